@@ -11,7 +11,8 @@
 //   4. leaf-ordered triangle array: 3 float4 per triangle (v0.w = id bits)
 //   5. binary tree: by default binned-SAH splits top-down down to ranges of
 //      at most J3DG_SAH_TOP triangles (section 5c), then PLOC clustering
-//      within each range (section 5b); with J3DG_BUILD_LBVH the LBVH,
+//      within each range (section 5b), both by one block in shared memory
+//      below kSmallTask triangles (section 5d); with J3DG_BUILD_LBVH the LBVH,
 //      bottom-up in one pass
 //      (Apetrei 2014, "Fast and Simple Agglomerative LBVH Construction"),
 //      with a strict total order on the split keys (xor of neighbouring
@@ -585,30 +586,21 @@ __global__ void k_collapse(const uint2* __restrict__ child, const BinNode* __res
 // -------------------------------------------------------- 5b. PLOC ----
 //
 // Parallel locally-ordered clustering (Meister and Bittner 2018, "Parallel
-// Locally-Ordered Clustering for Bounding Volume Hierarchy Construction"):
-// the Morton-sorted leaves start as clusters; every cluster picks the
-// cluster within kPlocRadius list positions whose union box has the smallest
-// surface area (equal areas: the smaller position; with the pair order this
-// is a total order, so the globally best pair is always mutual and every
-// round merges); mutual pairs become a new binary node at the lower
-// position; the list is compacted (two exclusive scans) and the rounds
-// repeat until one cluster is left. Subtrees are no longer Morton ranges, so
-// the collapse below carries each subtree's first position in the new leaf
-// order and writes the triangles there.
+// Locally-Ordered Clustering for Bounding Volume Hierarchy Construction") of
+// a segment of at most J3DG_SAH_TOP triangles (section 5d runs it): the
+// Morton-ordered leaves start as clusters; every cluster picks the cluster
+// within kPlocRadius list positions whose union box has the smallest surface
+// area (equal areas: the smaller position; with the pair order this is a
+// total order, so the best pair is always mutual and every round merges);
+// mutual pairs become a new binary node at the lower position; the list is
+// compacted and the rounds repeat until one cluster is left. Subtrees are no
+// longer Morton ranges, so the collapse below carries each subtree's first
+// position in the new leaf order and writes the triangles there.
 
 #ifndef J3DG_PLOC_RADIUS
 #define J3DG_PLOC_RADIUS 8  // 2..64 measured on the torus frames: 8 visits the fewest nodes
 #endif
 static const int kPlocRadius = J3DG_PLOC_RADIUS;
-static const int kPlocBlock = 256;
-
-__global__ void k_ploc_init(const float4* __restrict__ tris, uint32_t n, uint32_t* __restrict__ C,
-                            float4* __restrict__ lo, float4* __restrict__ hi) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  C[i] = 0x80000000u | i;
-  leaf_box(tris, i, lo[i], hi[i]);
-}
 
 __device__ __forceinline__ float merged_area(float4 alo, float4 ahi, float4 blo, float4 bhi) {
   const float dx = fmaxf(ahi.x, bhi.x) - fminf(alo.x, blo.x);
@@ -616,168 +608,6 @@ __device__ __forceinline__ float merged_area(float4 alo, float4 ahi, float4 blo,
   const float dz = fmaxf(ahi.z, bhi.z) - fminf(alo.z, blo.z);
   const float a = dx * dy + dy * dz + dz * dx;
   return a == a ? a : FLT_MAX;  // boxes with NaN planes still get an order
-}
-
-// Clusters are searched within their own segment (seg: the segment of each
-// list position, all 0 for one segment); a cluster alone in its segment gets
-// no neighbour (0xffffffff) and so never merges.
-__global__ void __launch_bounds__(kPlocBlock) k_ploc_nn(const float4* __restrict__ lo, const float4* __restrict__ hi,
-                                                       const uint32_t* __restrict__ seg,
-                                                       const uint32_t* __restrict__ m_p,
-                                                       const uint32_t* __restrict__ n_seg_p, uint32_t* __restrict__ nn) {
-  __shared__ float4 slo[kPlocBlock + 2 * kPlocRadius], shi[kPlocBlock + 2 * kPlocRadius];
-  __shared__ uint32_t sseg[kPlocBlock + 2 * kPlocRadius];
-  const uint32_t m = *m_p;
-  if (m <= *n_seg_p) return;  // every segment is one cluster: no round
-  for (uint32_t tile = blockIdx.x; tile * kPlocBlock < m; tile += gridDim.x) {  // uniform over the block
-    const int base = (int)(tile * kPlocBlock) - kPlocRadius;
-    for (int k = threadIdx.x; k < kPlocBlock + 2 * kPlocRadius; k += blockDim.x) {
-      const int j = base + k;
-      if (j >= 0 && j < (int)m) {
-        slo[k] = lo[j];
-        shi[k] = hi[j];
-        sseg[k] = seg[j];
-      }
-    }
-    __syncthreads();
-    const int i = (int)(tile * kPlocBlock + threadIdx.x);
-    if (i < (int)m) {
-      const int si = threadIdx.x + kPlocRadius;
-      const float4 alo = slo[si], ahi = shi[si];
-      const uint32_t my = sseg[si];
-      float best = INFINITY;
-      uint32_t bj = 0xffffffffu;
-      for (int o = -kPlocRadius; o <= kPlocRadius; ++o) {
-        const int j = i + o;
-        if (o == 0 || j < 0 || j >= (int)m || sseg[si + o] != my) continue;
-        const float a = merged_area(alo, ahi, slo[si + o], shi[si + o]);
-        if (a < best) {  // increasing j: the first of equal areas is the smaller position
-          best = a;
-          bj = (uint32_t)j;
-        }
-      }
-      nn[i] = bj;
-    }
-    __syncthreads();  // the tile's shared copies are read before the next tile overwrites them
-  }
-}
-
-// a PLOC round's two compactions in one pass: position i creates a node if it
-// and its nearest neighbour j are mutual with i < j, and survives (keeps a
-// list slot) unless it is the j > i side of a mutual pair. Each chunk of 1024
-// positions (256 threads x 4) writes the exclusive scans of both flags
-// within the chunk (cps, sps) and its two totals (csum, ssum; scanned by
-// k_scan_sums, whose grand totals are the round's creates and survivors).
-__global__ void __launch_bounds__(256) k_ploc_flag_scan(const uint32_t* __restrict__ nn, const uint32_t* __restrict__ m_p,
-                                                        const uint32_t* __restrict__ n_seg_p,
-                                                        uint32_t* __restrict__ cps, uint32_t* __restrict__ sps,
-                                                        uint32_t* __restrict__ csum, uint32_t* __restrict__ ssum) {
-  __shared__ uint32_t wsum[2][8];
-  const uint32_t m = *m_p;
-  if (m <= *n_seg_p || blockIdx.x * 1024u >= m) return;  // no round, or past the list
-  const uint32_t base = blockIdx.x * 1024u + threadIdx.x * 4u;
-  uint32_t c[4] = {0u, 0u, 0u, 0u}, v[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const uint32_t i = base + k;
-    if (i < m) {
-      const uint32_t j = nn[i];
-      const bool mutual = j < m && nn[j] == i;
-      c[k] = (mutual && i < j) ? 1u : 0u;
-      v[k] = (!mutual || i < j) ? 1u : 0u;
-    }
-  }
-  const uint32_t ct = c[0] + c[1] + c[2] + c[3], vt = v[0] + v[1] + v[2] + v[3];
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  uint32_t ci = ct, vi = vt;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t yc = __shfl_up_sync(0xffffffffu, ci, o);
-    const uint32_t yv = __shfl_up_sync(0xffffffffu, vi, o);
-    if (lane >= (uint32_t)o) {
-      ci += yc;
-      vi += yv;
-    }
-  }
-  if (lane == 31) {
-    wsum[0][warp] = ci;
-    wsum[1][warp] = vi;
-  }
-  __syncthreads();
-  uint32_t co = 0, vo = 0, call = 0, vall = 0;
-#pragma unroll
-  for (uint32_t w = 0; w < 8; ++w) {
-    const uint32_t xc = wsum[0][w], xv = wsum[1][w];
-    co += w < warp ? xc : 0u;
-    vo += w < warp ? xv : 0u;
-    call += xc;
-    vall += xv;
-  }
-  const uint32_t ec = co + ci - ct, ev = vo + vi - vt;
-  const uint4 oc = make_uint4(ec, ec + c[0], ec + c[0] + c[1], ec + c[0] + c[1] + c[2]);
-  const uint4 ov = make_uint4(ev, ev + v[0], ev + v[0] + v[1], ev + v[0] + v[1] + v[2]);
-  if (base + 3 < m) {
-    *reinterpret_cast<uint4*>(cps + base) = oc;
-    *reinterpret_cast<uint4*>(sps + base) = ov;
-  } else {
-    const uint32_t a4[4] = {oc.x, oc.y, oc.z, oc.w}, b4[4] = {ov.x, ov.y, ov.z, ov.w};
-    for (uint32_t k = 0; k < 4 && base + k < m; ++k) {
-      cps[base + k] = a4[k];
-      sps[base + k] = b4[k];
-    }
-  }
-  if (threadIdx.x == 0) {
-    csum[blockIdx.x] = call;
-    ssum[blockIdx.x] = vall;
-  }
-}
-
-__device__ __forceinline__ void ploc_merge_one(const uint32_t* __restrict__ C, const float4* __restrict__ lo,
-                                               const float4* __restrict__ hi, const uint32_t* __restrict__ seg,
-                                               const uint32_t* __restrict__ nn, const uint32_t* __restrict__ cps,
-                                               const uint32_t* __restrict__ sps, const uint32_t* __restrict__ csum,
-                                               const uint32_t* __restrict__ ssum, uint32_t i, uint32_t m,
-                                               uint32_t node_base, uint32_t* __restrict__ C2,
-                                               float4* __restrict__ lo2, float4* __restrict__ hi2,
-                                               uint32_t* __restrict__ seg2, uint2* __restrict__ child,
-                                               BinNode* __restrict__ box, uint32_t* __restrict__ count) {
-  const uint32_t j = nn[i];
-  const bool mutual = j < m && nn[j] == i;
-  if (mutual && i > j) return;  // merged into the node made at j
-  const uint32_t pos = sps[i] + ssum[i >> 10];  // survivors before i
-  seg2[pos] = seg[i];
-  if (!mutual) {
-    C2[pos] = C[i];
-    lo2[pos] = lo[i];
-    hi2[pos] = hi[i];
-    return;
-  }
-  const uint32_t p = node_base + cps[i] + csum[i >> 10];  // nodes made before i's
-  const uint32_t a = C[i], b = C[j];
-  const float4 l = make_float4(fminf(lo[i].x, lo[j].x), fminf(lo[i].y, lo[j].y), fminf(lo[i].z, lo[j].z), 0.f);
-  const float4 h = make_float4(fmaxf(hi[i].x, hi[j].x), fmaxf(hi[i].y, hi[j].y), fmaxf(hi[i].z, hi[j].z), 0.f);
-  child[p] = make_uint2(a, b);
-  box[p].lo = l;
-  box[p].hi = h;
-  count[p] = ((a & 0x80000000u) ? 1u : count[a]) + ((b & 0x80000000u) ? 1u : count[b]);
-  C2[pos] = p;
-  lo2[pos] = l;
-  hi2[pos] = h;
-}
-
-__global__ void k_ploc_merge(const uint32_t* __restrict__ C, const float4* __restrict__ lo,
-                             const float4* __restrict__ hi, const uint32_t* __restrict__ seg,
-                             const uint32_t* __restrict__ nn, const uint32_t* __restrict__ cps,
-                             const uint32_t* __restrict__ sps, const uint32_t* __restrict__ csum,
-                             const uint32_t* __restrict__ ssum, const uint32_t* __restrict__ m_p,
-                             const uint32_t* __restrict__ n_seg_p, const uint32_t* __restrict__ node_base_p,
-                             uint32_t* __restrict__ C2, float4* __restrict__ lo2, float4* __restrict__ hi2,
-                             uint32_t* __restrict__ seg2, uint2* __restrict__ child, BinNode* __restrict__ box,
-                             uint32_t* __restrict__ count) {
-  const uint32_t m = *m_p, node_base = *node_base_p;
-  if (m <= *n_seg_p) return;  // no round
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
-    ploc_merge_one(C, lo, hi, seg, nn, cps, sps, csum, ssum, i, m, node_base, C2, lo2, hi2, seg2, child, box, count);
 }
 
 // ------------------------------------------- 6b. cost-optimal collapse ----
@@ -790,8 +620,9 @@ __global__ void k_ploc_merge(const uint32_t* __restrict__ C, const float4* __res
 //   C(n, 1)   = min(leaf: A(n) N(n) c_t if N(n) <= leaf_size,
 //                   node: A(n) c_n + min_k C(left, k) + C(right, 4 - k))
 //   C(n, i)   = min(C(n, i - 1), min_k C(left, k) + C(right, i - k))
-// Children are made in earlier PLOC rounds, so one launch per round, in
-// round order, sees its children's costs. The decisions steer the collapse:
+// Children come before their parents: within a small task (section 5d) the
+// costs are made as its nodes are; the top nodes follow level by level,
+// deepest first. The decisions steer the collapse:
 // dec.x = the k of the node case (bit 7 set: the leaf case is cheaper);
 // dec.y, .z, .w for i = 2, 3, 4: 0 = as i - 1, else the k of the best split.
 
@@ -820,19 +651,13 @@ __device__ __forceinline__ void sub_costs(const float* __restrict__ cost, const 
   }
 }
 
-// cost: W floats per binary node (C(n, 1..W)); dec: W bytes per node
-// (dec[0] = the k of the node case | 0x80 when the leaf case is cheaper;
-// dec[i - 1], i = 2..W: 0 = as i - 1, else the k of the best split)
+// the programme's step at a node of half area A over N triangles from its
+// children's costs: C(n, 1..W) and the W decision bytes (d[0] = the k of the
+// node case | 0x80 when the leaf case is cheaper; d[i - 1], i = 2..W: 0 = as
+// i - 1, else the k of the best split)
 template <int W>
-__device__ __forceinline__ void collapse_cost_one(const uint2* __restrict__ child, const BinNode* __restrict__ box,
-                                                  const uint32_t* __restrict__ count, const float4* __restrict__ tris,
-                                                  uint32_t n, uint32_t leaf_size, float* __restrict__ cost,
-                                                  uint8_t* __restrict__ dec) {
-  const uint2 c = child[n];
-  float cl[W + 1], cr[W + 1], C[W + 1];
-  sub_costs<W>(cost, tris, c.x, cl);
-  sub_costs<W>(cost, tris, c.y, cr);
-  const float A = half_area4(box[n].lo, box[n].hi);
+__device__ __forceinline__ void collapse_step(const float (&cl)[W + 1], const float (&cr)[W + 1], float A, uint32_t N,
+                                              uint32_t leaf_size, float (&C)[W + 1], uint8_t (&d)[W]) {
   float best = FLT_MAX;
   uint32_t bk = 1;
 #pragma unroll
@@ -842,15 +667,14 @@ __device__ __forceinline__ void collapse_cost_one(const uint2* __restrict__ chil
       bk = k;
     }
   const float node = A + best;  // c_n = 1
-  const uint32_t N = count[n];
   const float leaf = N <= leaf_size ? A * (float)N * J3DG_SAH_CTRI : FLT_MAX;
   C[1] = fminf(leaf, node);
-  uint8_t d[W];
   d[0] = (uint8_t)(bk | (leaf <= node ? 0x80u : 0u));
 #pragma unroll
   for (uint32_t i = 2; i <= (uint32_t)W; ++i) {
     float v = C[i - 1];
     uint32_t dk = 0;
+#pragma unroll
     for (uint32_t k = 1; k < i; ++k)
       if (cl[k] + cr[i - k] < v) {
         v = cl[k] + cr[i - k];
@@ -859,22 +683,48 @@ __device__ __forceinline__ void collapse_cost_one(const uint2* __restrict__ chil
     C[i] = v;
     d[i - 1] = (uint8_t)dk;
   }
+}
+
+// the W decision bytes of node n in one store
+template <int W>
+__device__ __forceinline__ void store_dec(uint8_t* __restrict__ dec, uint32_t n, const uint8_t (&d)[W]) {
+  if constexpr (W == 2) {
+    reinterpret_cast<uint16_t*>(dec)[n] = (uint16_t)(d[0] | (d[1] << 8));
+  } else {
 #pragma unroll
-  for (int i = 1; i <= W; ++i) {
-    cost[(size_t)n * W + i - 1] = C[i];
-    dec[(size_t)n * W + i - 1] = d[i - 1];
+    for (int q = 0; q < W / 4; ++q)
+      reinterpret_cast<uint32_t*>(dec)[(size_t)n * (W / 4) + q] =
+          (uint32_t)d[4 * q] | ((uint32_t)d[4 * q + 1] << 8) | ((uint32_t)d[4 * q + 2] << 16) |
+          ((uint32_t)d[4 * q + 3] << 24);
   }
+}
+
+// cost: W floats per binary node (C(n, 1..W)); dec: W bytes per node
+template <int W>
+__device__ __forceinline__ void collapse_cost_one(const uint2* __restrict__ child, const BinNode* __restrict__ box,
+                                                  const uint32_t* __restrict__ count, const float4* __restrict__ tris,
+                                                  uint32_t n, uint32_t leaf_size, float* __restrict__ cost,
+                                                  uint8_t* __restrict__ dec) {
+  const uint2 c = child[n];
+  float cl[W + 1], cr[W + 1], C[W + 1];
+  uint8_t d[W];
+  sub_costs<W>(cost, tris, c.x, cl);
+  sub_costs<W>(cost, tris, c.y, cr);
+  collapse_step<W>(cl, cr, half_area4(box[n].lo, box[n].hi), count[n], leaf_size, C, d);
+#pragma unroll
+  for (int i = 1; i <= W; ++i) cost[(size_t)n * W + i - 1] = C[i];
+  store_dec<W>(dec, n, d);
 }
 
 template <int W>
 __global__ void k_collapse_cost(const uint2* __restrict__ child, const BinNode* __restrict__ box,
                                 const uint32_t* __restrict__ count, const float4* __restrict__ tris,
-                                const uint32_t* __restrict__ lohi, uint32_t leaf_size, float* __restrict__ cost,
-                                uint8_t* __restrict__ dec) {
-  // the pass's binary nodes [lohi[0], lohi[1]) (device memory)
+                                const uint32_t* __restrict__ list, const uint32_t* __restrict__ lohi,
+                                uint32_t leaf_size, float* __restrict__ cost, uint8_t* __restrict__ dec) {
+  // the pass's binary nodes: entries [lohi[0], lohi[1]) of the list (device memory)
   const uint32_t lo = lohi[0], hi = lohi[1];
-  for (uint32_t n = lo + blockIdx.x * blockDim.x + threadIdx.x; n < hi; n += gridDim.x * blockDim.x)
-    collapse_cost_one<W>(child, box, count, tris, n, leaf_size, cost, dec);
+  for (uint32_t k = lo + blockIdx.x * blockDim.x + threadIdx.x; k < hi; k += gridDim.x * blockDim.x)
+    collapse_cost_one<W>(child, box, count, tris, list[k], leaf_size, cost, dec);
 }
 
 struct PlaceItem {
@@ -1163,14 +1013,14 @@ static uint32_t wave_blocks128() {
 }
 
 static void launch_collapse_cost(uint32_t W, const uint2* child, const BinNode* box, const uint32_t* count,
-                                 const float4* tris, const uint32_t* lohi, uint32_t leaf_size, float* cost,
-                                 uint8_t* dec, cudaStream_t st) {
+                                 const float4* tris, const uint32_t* list, const uint32_t* lohi, uint32_t leaf_size,
+                                 float* cost, uint8_t* dec, cudaStream_t st) {
   if (W == 2)
-    k_collapse_cost<2><<<kStrideBlocks, 256, 0, st>>>(child, box, count, tris, lohi, leaf_size, cost, dec);
+    k_collapse_cost<2><<<kStrideBlocks, 256, 0, st>>>(child, box, count, tris, list, lohi, leaf_size, cost, dec);
   else if (W == 8)
-    k_collapse_cost<8><<<kStrideBlocks, 256, 0, st>>>(child, box, count, tris, lohi, leaf_size, cost, dec);
+    k_collapse_cost<8><<<kStrideBlocks, 256, 0, st>>>(child, box, count, tris, list, lohi, leaf_size, cost, dec);
   else
-    k_collapse_cost<4><<<kStrideBlocks, 256, 0, st>>>(child, box, count, tris, lohi, leaf_size, cost, dec);
+    k_collapse_cost<4><<<kStrideBlocks, 256, 0, st>>>(child, box, count, tris, list, lohi, leaf_size, cost, dec);
 }
 
 static void launch_collapse_place(uint32_t W, const uint2* child, const BinNode* box, const uint32_t* count,
@@ -1193,18 +1043,23 @@ static void launch_collapse_place(uint32_t W, const uint2* child, const BinNode*
 //
 // Above J3DG_SAH_TOP triangles a node is split top-down by binned SAH (Wald
 // 2007, "On fast Construction of SAH-based Bounding Volume Hierarchies"):
-// per level, every task (a range of the triangle order `ord`) bins its
-// triangles' centroids into kTopBins bins per axis (per-block bins in shared
-// memory, then merged into the task's bins; tasks of at most kTopWarpTask
-// triangles are binned by one warp each), one warp per task finds the split
-// of least A_L N_L + A_R N_R from prefix and suffix unions of the bins
-// (shuffles, lanes = bins), and a stable partition
-// (flags from the bin codes that binning stored per position, one exclusive
-// scan) reorders the range. A stable partition of the
-// Morton-sorted order keeps every range in Morton order, so each range of at
-// most J3DG_SAH_TOP triangles (a segment) is then clustered by PLOC on its
-// own (neighbours searched within the segment only), and the segment roots
-// are linked under the top nodes.
+// every task (a range of the triangle order `ord`) bins its triangles'
+// centroids into kTopBins bins per axis, one warp finds the split of least
+// A_L N_L + A_R N_R from prefix and suffix unions of the bins (shuffles,
+// lanes = bins), and a stable partition reorders the range. A stable
+// partition of the Morton-sorted order keeps every range in Morton order, so
+// each range of at most J3DG_SAH_TOP triangles (a segment) is then clustered
+// by PLOC on its own (neighbours searched within the segment only).
+// Tasks above kSmallTask triangles are split level by level over the whole
+// mesh (per-block bins in shared memory, merged into the task's bins; flags
+// from the bin codes that binning stored per position, one exclusive scan);
+// a task of at most kSmallTask is taken through the rest of its subtree by
+// one block (section 5d).
+//
+// Binary nodes are numbered by position: the node that splits its range at
+// position mid is node mid, and the nodes that PLOC makes in a segment take
+// the segment's positions but the first: every position but position 0
+// numbers one node, without a counter.
 
 // segment size below which PLOC takes over (0: PLOC over the whole mesh).
 // Measured on the 28M-triangle torus frames (node visits per ray, ms per
@@ -1222,10 +1077,14 @@ static_assert(kTopBins <= 16, "bin codes keep 4 bits per axis");
 // task the two ranges differ by about one triangle
 static const int kTopVals = 7;
 static const uint32_t kNoTask = 0xffffffffu;
-static const uint32_t kPendingRef = 0xfffffffeu;  // child slot filled by a segment root later
+static const uint32_t kMaxTopLevels = 1024;  // SAH levels of a tree, top and small together
+
+static const uint32_t kNoParent = 0xffffffffu;  // the parent of the root
 
 struct TopTask {
-  uint32_t begin, end, node, pad;
+  uint32_t begin, end;
+  uint32_t parent;   // the node whose child it becomes (kNoParent: the root)
+  uint32_t side;     // which child (bit 0) | the task's level << 1
   float4 clo, chi;  // centroid bounds
 };
 
@@ -1247,8 +1106,19 @@ __global__ void k_top_boxes(const float4* __restrict__ tris, uint32_t n, float4*
 }
 
 struct TopRange {  // a finished range: a segment for PLOC
-  uint32_t begin, end, parent, side;
+  uint32_t begin, end, parent, side;  // parent and side as in TopTask
 };
+
+// puts a finished subtree under its parent (or makes it the root)
+__device__ __forceinline__ void link_child(uint2* __restrict__ child, uint32_t* __restrict__ root, uint32_t parent,
+                                           uint32_t side, uint32_t ref) {
+  if (parent == kNoParent)
+    *root = ref;
+  else if (side & 1u)
+    child[parent].y = ref;
+  else
+    child[parent].x = ref;
+}
 
 // float <-> uint32 with the same order (for atomic min / max)
 __device__ __forceinline__ uint32_t f2o(float f) {
@@ -1264,23 +1134,28 @@ __device__ __forceinline__ int top_bin(float c, float lo, float hi) {
   return b < 0 ? 0 : (b >= kTopBins ? kTopBins - 1 : b);
 }
 
-static const int kTopChunk = 2048;
-// Tasks up to this size are binned by one warp each (k_top_bin_warp): at
-// that depth 32 neighbouring triangles span many bins, so grouping lanes by
-// bin (match + reductions per group) serialises; plain shared atomics do not.
-static const uint32_t kTopWarpTask = 2048;
+// top_bin by a product with scale = kTopBins / (hi - lo) instead of a division:
+// the two differ by under 4e-6, so away from a bin's edge the bin is the
+// same; within 1e-4 of an edge (and for NaN and infinite values) the division
+// decides
+__device__ __forceinline__ int top_bin_scaled(float c, float lo, float hi, float scale) {
+  const float q = (c - lo) * scale;
+  if (!(fabsf(q - rintf(q)) > 1e-4f)) return top_bin(c, lo, hi);
+  const int b = (int)q;
+  return b < 0 ? 0 : (b >= kTopBins ? kTopBins - 1 : b);
+}
 
-// global bins of the tasks larger than kTopWarpTask (k_top_bin's); the
-// smaller tasks keep their bins in shared memory
-// (the level's task count and largest task are read from device memory;
-// levels with no task above kTopWarpTask have nothing to do here)
-__global__ void k_top_bins_init(uint32_t* __restrict__ bins, const uint32_t* __restrict__ n_tasks_p,
-                                const uint32_t* __restrict__ max_task_p, const TopTask* __restrict__ tasks) {
-  if (*max_task_p <= kTopWarpTask) return;
+static const int kTopChunk = 2048;
+// Tasks up to this size leave the level loop for section 5d.
+#ifndef J3DG_SMALL_TASK
+#define J3DG_SMALL_TASK 1024
+#endif
+static const uint32_t kSmallTask = J3DG_SMALL_TASK;
+
+// the level's task count is read from device memory
+__global__ void k_top_bins_init(uint32_t* __restrict__ bins, const uint32_t* __restrict__ n_tasks_p) {
   const uint32_t n_words = *n_tasks_p * 3 * kTopBins * kTopVals;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_words; i += gridDim.x * blockDim.x) {
-    const TopTask& T = tasks[i / (3 * kTopBins * kTopVals)];
-    if (T.end - T.begin <= kTopWarpTask) continue;
     const uint32_t v = i % kTopVals;
     bins[i] = v == 0 ? 0u : (((v - 1) % 6) < 3 ? 0xffffffffu : 0u);  // lo fields: max code, hi fields: 0
   }
@@ -1291,18 +1166,17 @@ __global__ void k_top_bins_init(uint32_t* __restrict__ bins, const uint32_t* __r
 __global__ void __launch_bounds__(256) k_top_bin(const uint32_t* __restrict__ ord, const float4* __restrict__ blo,
                                                  const float4* __restrict__ bhi, const uint32_t* __restrict__ task_of,
                                                  const TopTask* __restrict__ tasks,
-                                                 const uint32_t* __restrict__ n_tasks_p,
-                                                 const uint32_t* __restrict__ max_task_p, uint32_t n,
+                                                 const uint32_t* __restrict__ n_tasks_p, uint32_t n,
                                                  uint32_t* __restrict__ bins, uint16_t* __restrict__ code) {
   __shared__ uint32_t sb[3 * kTopBins * kTopVals];
   __shared__ uint32_t s_task;
   const uint32_t n_tasks = *n_tasks_p;
-  if (n_tasks == 0 || *max_task_p <= kTopWarpTask) return;  // k_top_bin_warp's level, or no level
+  if (n_tasks == 0) return;  // no level
   const uint32_t c0 = blockIdx.x * kTopChunk, c1 = min(n, c0 + kTopChunk);
   if (c0 >= n) return;
   if (threadIdx.x == 0) {
     const uint32_t a = task_of[c0], b = task_of[c1 - 1];
-    s_task = (a == b && a < n_tasks && tasks[a].end - tasks[a].begin > kTopWarpTask) ? a : kNoTask;
+    s_task = (a == b && a < n_tasks) ? a : kNoTask;
   }
   for (uint32_t k = threadIdx.x; k < 3 * kTopBins * kTopVals; k += blockDim.x) {
     const uint32_t v = k % kTopVals;
@@ -1313,8 +1187,7 @@ __global__ void __launch_bounds__(256) k_top_bin(const uint32_t* __restrict__ or
   const uint32_t lane = threadIdx.x & 31u;
   for (uint32_t base = c0; base < c1; base += blockDim.x) {  // uniform trip count: whole warps
     const uint32_t p = base + threadIdx.x;
-    uint32_t t = p < c1 ? (st != kNoTask ? st : task_of[p]) : kNoTask;
-    if (st == kNoTask && t < n_tasks && tasks[t].end - tasks[t].begin <= kTopWarpTask) t = kNoTask;  // k_top_bin_warp's
+    const uint32_t t = p < c1 ? (st != kNoTask ? st : task_of[p]) : kNoTask;
     const bool valid = t < n_tasks;
     float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo, c = lo;
     int bx = 0, by = 0, bz = 0;
@@ -1381,14 +1254,15 @@ __device__ __forceinline__ float box_half_area(float lx, float ly, float lz, flo
 
 // One warp: the split of least SAH cost A_L N_L + A_R N_R over the task's
 // bins B ([axis][bin][kTopVals], shared or global memory); writes the split,
-// the node's box and its triangle count. Lanes b and b + 16 hold bin b of
+// the node's box and its triangle count, and returns its left count
+// (warp-uniform). Lanes b and b + 16 hold bin b of
 // the axis in hand; prefix and suffix unions of the bins come from shuffles
 // within the 16 lanes. Among equal costs the lowest (axis, bin) wins, the
 // split a sweep over the axes and bins in order with a strict comparison
 // takes. Bins with no triangle carry no box (their encoded fields would
 // decode to NaN).
-__device__ void warp_top_split(const uint32_t* B, const TopTask& T, TopSplit* __restrict__ split,
-                               BinNode* __restrict__ box, uint32_t* __restrict__ count) {
+__device__ uint32_t warp_top_split(const uint32_t* B, const TopTask& T, TopSplit* split, BinNode* __restrict__ box,
+                                   uint32_t* __restrict__ count) {
   const uint32_t lane = threadIdx.x & 31u, b = lane & 15u;
   const uint32_t n = T.end - T.begin;
   float best = FLT_MAX;
@@ -1480,6 +1354,10 @@ __device__ void warp_top_split(const uint32_t* B, const TopTask& T, TopSplit* __
       wi = oi;
     }
   }
+  // the left count: the winner's, or half for a split by position
+  const uint32_t win = __ballot_sync(0xffffffffu, best_idx == wi);
+  const uint32_t left = __shfl_sync(0xffffffffu, best_lc, __ffs(win) - 1);
+  const uint32_t nleft = wi == 0xffffffffu ? n / 2 : left;
   if (wi == 0xffffffffu) {  // no usable SAH split: split by position
     if (lane == 0) {
       TopSplit S;
@@ -1508,80 +1386,22 @@ __device__ void warp_top_split(const uint32_t* B, const TopTask& T, TopSplit* __
     *split = S;
   }
   if (lane == 0) {
-    box[T.node].lo = make_float4(nlo[0], nlo[1], nlo[2], 0.f);
-    box[T.node].hi = make_float4(nhi[0], nhi[1], nhi[2], 0.f);
-    count[T.node] = n;
+    const uint32_t node = T.begin + nleft;
+    box[node].lo = make_float4(nlo[0], nlo[1], nlo[2], 0.f);
+    box[node].hi = make_float4(nhi[0], nhi[1], nhi[2], 0.f);
+    count[node] = n;
   }
+  return nleft;
 }
 
-// one warp bins task T (index t) into its shared bins `my` and splits it
-__device__ __forceinline__ void top_bin_warp_task(const uint32_t* __restrict__ ord, const float4* __restrict__ blo,
-                                                       const float4* __restrict__ bhi, const TopTask& T, uint32_t t,
-                                                       uint32_t* my, uint32_t lane, TopSplit* __restrict__ splits,
-                                                       BinNode* __restrict__ box, uint32_t* __restrict__ count,
-                                                       uint16_t* __restrict__ code) {
-  for (uint32_t k = lane; k < 3 * kTopBins * kTopVals; k += 32) {
-    const uint32_t v = k % kTopVals;
-    my[k] = v == 0 ? 0u : (((v - 1) % 6) < 3 ? 0xffffffffu : 0u);
-  }
-  __syncwarp();
-  for (uint32_t p = T.begin + lane; p < T.end; p += 32) {
-    const uint32_t tri = ord[p];
-    const float4 lo = blo[tri], hi = bhi[tri];
-    const float4 c = make_float4(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z), 0.f);
-    const int bins3[3] = {top_bin(c.x, T.clo.x, T.chi.x), top_bin(c.y, T.clo.y, T.chi.y),
-                          top_bin(c.z, T.clo.z, T.chi.z)};
-    code[p] = (uint16_t)(bins3[0] | (bins3[1] << 4) | (bins3[2] << 8));
-    const uint32_t v[6] = {f2o(lo.x), f2o(lo.y), f2o(lo.z), f2o(hi.x), f2o(hi.y), f2o(hi.z)};
-#pragma unroll
-    for (int ax = 0; ax < 3; ++ax) {
-      uint32_t* b = my + (ax * kTopBins + bins3[ax]) * kTopVals;
-      atomicAdd(b, 1u);
-#pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        if (k < 3)
-          atomicMin(b + 1 + k, v[k]);
-        else
-          atomicMax(b + 1 + k, v[k]);
-      }
-    }
-  }
-  __syncwarp();
-  warp_top_split(my, T, splits + t, box, count);
-  __syncwarp();  // the split has read the bins before the warp's next task resets them
-}
-
-// tasks of at most kTopWarpTask triangles: one warp bins a whole task into
-// its own shared-memory bins with per-lane shared atomics, then splits it
-// from those bins (its bins never go to global memory)
-__global__ void __launch_bounds__(256) k_top_bin_warp(const uint32_t* __restrict__ ord, const float4* __restrict__ blo,
-                                                      const float4* __restrict__ bhi, const TopTask* __restrict__ tasks,
-                                                      const uint32_t* __restrict__ n_tasks_p,
-                                                      TopSplit* __restrict__ splits, BinNode* __restrict__ box,
-                                                      uint32_t* __restrict__ count, uint16_t* __restrict__ code) {
-  __shared__ uint32_t sb[8][3 * kTopBins * kTopVals];
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-  const uint32_t n_tasks = *n_tasks_p;
-  // whole warps take tasks together (a warp-stride loop over the level's tasks)
-  for (uint32_t t = blockIdx.x * 8u + warp; t < n_tasks; t += gridDim.x * 8u) {
-    const TopTask T = tasks[t];
-    if (T.end - T.begin > kTopWarpTask) continue;
-    top_bin_warp_task(ord, blo, bhi, T, t, sb[warp], lane, splits, box, count, code);
-  }
-}
-
-// one warp per task larger than kTopWarpTask (the smaller ones were split
-// by k_top_bin_warp from their shared-memory bins)
+// one warp per task
 __global__ void __launch_bounds__(128) k_top_split(const TopTask* __restrict__ tasks,
                                                    const uint32_t* __restrict__ n_tasks_p,
-                                                   const uint32_t* __restrict__ max_task_p,
                                                    const uint32_t* __restrict__ bins, TopSplit* __restrict__ splits,
                                                    BinNode* __restrict__ box, uint32_t* __restrict__ count) {
-  if (*max_task_p <= kTopWarpTask) return;
   const uint32_t n_tasks = *n_tasks_p;
   for (uint32_t t = blockIdx.x * 4u + (threadIdx.x >> 5); t < n_tasks; t += gridDim.x * 4u) {  // whole warps
     const TopTask T = tasks[t];
-    if (T.end - T.begin <= kTopWarpTask) continue;
     warp_top_split(bins + (size_t)t * 3 * kTopBins * kTopVals, T, splits + t, box, count);
   }
 }
@@ -1713,69 +1533,70 @@ __global__ void __launch_bounds__(256) k_top_scatter(const uint32_t* __restrict_
   }
 }
 
-// children of every task: a new task above J3DG_SAH_TOP triangles, else a
-// finished range (segment) whose root PLOC supplies later
+// children of every task: a task of the next level above kSmallTask
+// triangles, a small task above J3DG_SAH_TOP, else a finished range; the
+// task's own node goes under its parent and into the list of top nodes
+// counters: [0] top nodes, [1] next tasks, [2] ranges, [3] small tasks
 __device__ __forceinline__ void top_children_of(const TopTask* __restrict__ tasks, TopSplit* __restrict__ splits,
-                                                uint32_t t, uint32_t seg_max, uint32_t* __restrict__ counters,
-                                                TopTask* __restrict__ next, TopRange* __restrict__ ranges,
-                                                uint2* __restrict__ child, uint32_t cap_tasks, uint32_t cap_ranges,
-                                                uint32_t max_nodes, uint32_t* status) {
+                                                uint32_t t, uint32_t* __restrict__ counters,
+                                                TopTask* __restrict__ next, TopTask* __restrict__ small,
+                                                TopRange* __restrict__ ranges, uint32_t* __restrict__ list,
+                                                uint2* __restrict__ child, uint32_t* __restrict__ root,
+                                                uint32_t cap_tasks, uint32_t cap_small, uint32_t nt, uint32_t* status) {
   const TopTask T = tasks[t];
   TopSplit S = splits[t];
-  const uint32_t n = T.end - T.begin;
-  uint32_t nl = S.nleft;
-  if (nl == 0 || nl >= n) {  // cannot happen (both sides of a split are non-empty); kept safe
-    atomicOr(status, J3DG_DEV_BAD_INDEX);
-    nl = n / 2;
-    S.axis = 3;
-    S.nleft = nl;
-  }
-  const uint32_t mid = T.begin + nl;
-  uint32_t ref[2];
+  const uint32_t n = T.end - T.begin, nl = S.nleft;
   S.task[0] = S.task[1] = kNoTask;
-  for (int side = 0; side < 2; ++side) {
-    const uint32_t b = side ? mid : T.begin, e = side ? T.end : mid;
-    if (e - b > seg_max) {
-      const uint32_t q = atomicAdd(counters + 1, 1u);
-      const uint32_t node = atomicAdd(counters + 0, 1u);
-      if (q >= cap_tasks || node >= max_nodes) {
-        atomicOr(status, J3DG_DEV_BAD_INDEX);
-        ref[side] = kPendingRef;
-        continue;
-      }
-      atomicMax(counters + 3, e - b);  // the next level's largest task
+  if (nl == 0 || nl >= n) {  // cannot happen: both sides of a split are non-empty
+    atomicOr(status, J3DG_DEV_BAD_INDEX);
+    splits[t] = S;
+    return;
+  }
+  const uint32_t node = T.begin + nl;
+  const uint32_t k = atomicAdd(counters + 0, 1u);
+  if (k < nt)
+    list[k] = node;
+  else
+    atomicOr(status, J3DG_DEV_BAD_INDEX);
+  link_child(child, root, T.parent, T.side, node);
+  for (uint32_t side = 0; side < 2; ++side) {
+    const uint32_t b = side ? node : T.begin, e = side ? T.end : node;
+    const uint32_t tag = side | (((T.side >> 1) + 1u) << 1);
+    if (e - b > J3DG_SAH_TOP) {
       TopTask C;
       C.begin = b;
       C.end = e;
-      C.node = node;
-      C.pad = 0;
+      C.parent = node;
+      C.side = tag;
       C.clo = side ? S.rclo : S.lclo;
       C.chi = side ? S.rchi : S.lchi;
-      next[q] = C;
-      ref[side] = node;
-      S.task[side] = q;
+      const bool again = e - b > kSmallTask;
+      const uint32_t q = atomicAdd(counters + (again ? 1 : 3), 1u);
+      if (q >= (again ? cap_tasks : cap_small)) {
+        atomicOr(status, J3DG_DEV_BAD_INDEX);
+        continue;
+      }
+      (again ? next : small)[q] = C;
+      if (again) S.task[side] = q;
     } else {
       const uint32_t q = atomicAdd(counters + 2, 1u);
-      if (q < cap_ranges)
-        ranges[q] = TopRange{b, e, T.node, (uint32_t)side};
+      if (q < nt)
+        ranges[q] = TopRange{b, e, node, tag};
       else
         atomicOr(status, J3DG_DEV_BAD_INDEX);
-      ref[side] = kPendingRef;
     }
   }
-  child[T.node] = make_uint2(ref[0], ref[1]);
   splits[t] = S;
 }
 
 __global__ void k_top_children(const TopTask* __restrict__ tasks, TopSplit* __restrict__ splits,
-                               const uint32_t* __restrict__ n_tasks_p, uint32_t seg_max,
-                               uint32_t* __restrict__ counters, TopTask* __restrict__ next,
-                               TopRange* __restrict__ ranges, uint2* __restrict__ child, uint32_t cap_tasks,
-                               uint32_t cap_ranges, uint32_t max_nodes, uint32_t* status) {
-  // counters: [0] nodes allocated, [1] next tasks, [2] ranges, [3] largest next task
+                               const uint32_t* __restrict__ n_tasks_p, uint32_t* __restrict__ counters,
+                               TopTask* __restrict__ next, TopTask* __restrict__ small, TopRange* __restrict__ ranges,
+                               uint32_t* __restrict__ list, uint2* __restrict__ child, uint32_t* __restrict__ root,
+                               uint32_t cap_tasks, uint32_t cap_small, uint32_t nt, uint32_t* status) {
   const uint32_t n_tasks = *n_tasks_p;
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n_tasks; t += gridDim.x * blockDim.x)
-    top_children_of(tasks, splits, t, seg_max, counters, next, ranges, child, cap_tasks, cap_ranges, max_nodes,
+    top_children_of(tasks, splits, t, counters, next, small, ranges, list, child, root, cap_tasks, cap_small, nt,
                     status);
 }
 
@@ -1784,50 +1605,612 @@ __global__ void k_iota(uint32_t* __restrict__ a, uint32_t n) {
   if (i < n) a[i] = i;
 }
 
-// segment starts: flags[begin] = 1 for every finished range
-__global__ void k_top_seg_starts(const TopRange* __restrict__ ranges, const uint32_t* __restrict__ n_ranges_p,
-                                 uint32_t n, uint32_t* __restrict__ flags) {
-  const uint32_t n_ranges = *n_ranges_p;
-  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n_ranges; r += gridDim.x * blockDim.x)
-    if (ranges[r].begin < n) flags[ranges[r].begin] = 1u;
+// -------------------------------------------------- 5d. small tasks ----
+//
+// One block takes a task of at most kSmallTask triangles through the rest of
+// its subtree in shared memory: the SAH levels down to segments (the same
+// bins, splits and stable partitions as the level loop's), PLOC in every
+// segment, and the cost programme of every node it makes. Done level by
+// level over the whole mesh, these levels were bound by launches on small
+// meshes (82k triangles: 17 PLOC rounds, 6 SAH levels and 23 cost passes of
+// 2-5 us kernels) and by passes over memory on large ones (28M triangles:
+// about 12 of the build's 30 ms).
+//
+// The boxes stay in shared memory; the levels permute 16-bit indices to
+// them. In a level every thread bins a run of consecutive positions with
+// shared atomics: the lanes of a warp are then some positions apart, so that
+// fewer of them meet in one bin than with neighbouring positions, which in
+// Morton order mostly share their bins.
+//
+// Then the boxes are put in the final order and all segments are clustered
+// together, as one list: the clusters of 20 segments and more fill the lanes
+// that a segment on its own (44 triangles on average, a few after three
+// rounds) would leave idle. Each cluster carries a node number that no node
+// below it uses, at first its position: a merge makes the node of the higher
+// cluster's number and keeps the lower one's, so a segment's nodes take its
+// positions but the first, and what is left at the end tells the segment.
+// The cost of a cluster sits beside it, so the programme reads no memory.
+//
+// Measured (GB300): this kernel 5.9 ms for 28.09M triangles where the levels,
+// rounds and cost passes it replaces took 11.5; builds of 82k / 2M / 28M
+// triangles with their first frame 1.88 -> 1.45, 5.10 -> 4.20 and 33.0 -> 28.4
+// ms. It is bound by instruction issue and latency (40 % of issue slots), so
+// a block of 192 threads with four blocks an SM (24 warps, 85 registers) is
+// the best of 64-512 threads and tasks of 512-2048 triangles: 0.424 ms for 2M
+// triangles in 700-triangle tasks, against 0.444 at 256 threads (64
+// registers, spills), 0.472 at 128, and 0.68 for 2048-triangle tasks.
+
+#ifndef J3DG_SMALL_THREADS
+#define J3DG_SMALL_THREADS 192
+#endif
+#ifndef J3DG_SMALL_BLOCKS
+#define J3DG_SMALL_BLOCKS 4
+#endif
+#ifndef J3DG_SMALL_BINS
+#define J3DG_SMALL_BINS 8
+#endif
+static const int kSmallThreads = J3DG_SMALL_THREADS;
+static const int kSmallWarps = kSmallThreads / 32;
+static const int kSmallPer = (J3DG_SMALL_TASK + kSmallThreads - 1) / kSmallThreads;  // positions per thread
+static const uint32_t kSmallBins = J3DG_SMALL_BINS;  // local tasks binned at once
+static const uint32_t kSmallTasks = kSmallTask / (J3DG_SAH_TOP + 1u) + 1u;  // tasks of one local level
+static const uint32_t kBinWords = 3 * kTopBins * kTopVals;
+static_assert(kSmallPer <= 32 && kSmallPer * kSmallWarps <= 64, "flag bits and list counts per thread");
+static_assert(kSmallTask <= 4096u && kSmallTasks < 255u && kSmallTasks <= kSmallThreads,
+              "12-bit positions, 8-bit local tasks, one thread per task");
+static_assert(J3DG_SAH_TOP <= 128u && kPlocRadius <= 8, "cluster sizes in a byte, neighbours within a warp's pass");
+
+struct SmallTaskMem {   // while the levels run
+  uint16_t ord[2][kSmallTask];
+  uint16_t code[kSmallTask];
+  uint8_t tk[2][kSmallTask];
+  uint32_t bins[kSmallBins * kBinWords];
+};
+template <int W>
+struct SmallClusterMem {  // while the segments are clustered
+  float cost[W][kSmallTask];
+  uint16_t spare[kSmallTask];  // the cluster's unused node number
+  uint8_t cnt[kSmallTask];     // its triangles
+  uint8_t nn[kSmallTask];      // its nearest neighbour's offset + kPlocRadius, or 255
+};
+template <int W>
+struct SmallMem {
+  float2 box[3][kSmallTask];     // lo, hi per axis
+  uint32_t ref[kSmallTask];      // triangle, then cluster reference
+  uint16_t seg[kSmallTask];      // each position's segment: its first position
+  uint16_t par[kSmallTask];      // at a segment's first position: its parent node << 1 | side, later its cluster
+  union {
+    SmallTaskMem t;
+    SmallClusterMem<W> c;
+  };
+  union {
+    struct {  // while the levels run
+      TopTask task[2][kSmallTasks];
+      TopSplit split[kSmallTasks];
+      uint32_t pre[kSmallTasks];  // left flags before each task's first position
+    };
+    float edge[kSmallWarps][kPlocRadius][kPlocRadius];  // clustering: areas that reach into the next warp's clusters
+  };
+  uint32_t wsum[64];
+  uint32_t n_task[2], n_seg, n_rec, job, bad;
+};
+
+template <int W>
+static size_t small_smem() {
+  return sizeof(SmallMem<W>);
 }
 
-// PLOC's initial clusters in the order `ord`, with the segment of each position
-// (seg = inclusive scan of the starts - 1)
-__global__ void k_ploc_init_seg(const float4* __restrict__ tris, const uint32_t* __restrict__ ord_a,
-                                const uint32_t* __restrict__ ord_b, const uint32_t* __restrict__ parity, uint32_t n,
-                                const uint32_t* __restrict__ starts, const uint32_t* __restrict__ scan,
-                                uint32_t* __restrict__ C, float4* __restrict__ lo, float4* __restrict__ hi,
-                                uint32_t* __restrict__ seg) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t t = (*parity ? ord_b : ord_a)[i];  // the final order is where the last level put it
-  C[i] = 0x80000000u | t;
-  leaf_box(tris, t, lo[i], hi[i]);
-  seg[i] = scan[i] + starts[i] - 1u;
+// the SAH levels of the task in s.task[0][0] (n triangles from global
+// position b0); leaves the order in s.t.ord[return value], the segments in
+// s.seg and s.par and a record (begin | mid << 16, end | level << 16) per
+// node in rec
+template <int W>
+__device__ int small_levels(SmallMem<W>& s, uint32_t b0, uint32_t n, uint2* __restrict__ rec,
+                            uint2* __restrict__ child, uint32_t* __restrict__ root, BinNode* __restrict__ box,
+                            uint32_t* __restrict__ count, uint32_t* __restrict__ error, uint32_t* status) {
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t K = (n + kSmallThreads - 1) / kSmallThreads, p0 = min(n, tid * K), p1 = min(n, p0 + K);
+  int cur = 0;
+  for (uint32_t level = 0;; ++level) {
+    const uint32_t nlt = s.n_task[cur];
+    if (nlt == 0) return cur;
+    if ((s.task[cur][0].side >> 1) >= kMaxTopLevels) {  // every task of a local level has its level
+      if (tid == 0) atomicOr(error, 1u);
+      __syncthreads();
+      if (tid == 0) s.bad = 1u;
+      __syncthreads();
+      return cur;
+    }
+    if (tid == 0) s.n_task[cur ^ 1] = 0;
+    for (uint32_t base = 0; base < nlt; base += kSmallBins) {
+      const uint32_t m = min(kSmallBins, nlt - base);
+      for (uint32_t k = tid; k < m * kBinWords; k += kSmallThreads) {
+        const uint32_t v = k % kTopVals;
+        s.t.bins[k] = v == 0 ? 0u : (v < 4 ? 0xffffffffu : 0u);
+      }
+      __syncthreads();
+      {
+        uint32_t last = kNoTask;
+        float4 clo = make_float4(0.f, 0.f, 0.f, 0.f), chi = clo;
+        float sx = 0.f, sy = 0.f, sz = 0.f;
+        const uint32_t q0 = min(n, (lane * kSmallWarps + warp) * K), q1 = min(n, q0 + K);  // lanes far apart
+        for (uint32_t p = q0; p < q1; ++p) {
+          const uint32_t t = (uint32_t)s.t.tk[cur][p] - base;  // 255: no task
+          if (t >= m) continue;
+          if (t != last) {
+            clo = s.task[cur][base + t].clo;
+            chi = s.task[cur][base + t].chi;
+            sx = (float)kTopBins / (chi.x - clo.x);
+            sy = (float)kTopBins / (chi.y - clo.y);
+            sz = (float)kTopBins / (chi.z - clo.z);
+            last = t;
+          }
+          const uint32_t i = s.t.ord[cur][p];
+          const float2 fx = s.box[0][i], fy = s.box[1][i], fz = s.box[2][i];
+          const uint32_t v[6] = {f2o(fx.x), f2o(fy.x), f2o(fz.x), f2o(fx.y), f2o(fy.y), f2o(fz.y)};
+          const int bx = top_bin_scaled(0.5f * (fx.x + fx.y), clo.x, chi.x, sx),
+                    by = top_bin_scaled(0.5f * (fy.x + fy.y), clo.y, chi.y, sy),
+                    bz = top_bin_scaled(0.5f * (fz.x + fz.y), clo.z, chi.z, sz);
+          s.t.code[p] = (uint16_t)(bx | (by << 4) | (bz << 8));
+          const int bin[3] = {bx, kTopBins + by, 2 * kTopBins + bz};
+#pragma unroll
+          for (int ax = 0; ax < 3; ++ax) {
+            uint32_t* b = s.t.bins + t * kBinWords + bin[ax] * kTopVals;
+            atomicAdd(b, 1u);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) atomicMin(b + 1 + k, v[k]);
+#pragma unroll
+            for (int k = 3; k < 6; ++k) atomicMax(b + 1 + k, v[k]);
+          }
+        }
+      }
+      __syncthreads();
+      for (uint32_t t = warp; t < m; t += kSmallWarps)
+        warp_top_split(s.t.bins + t * kBinWords, s.task[cur][base + t], &s.split[base + t], box, count);
+      __syncthreads();
+    }
+    // the children's tasks
+    if (tid < nlt) {
+      const TopTask T = s.task[cur][tid];
+      TopSplit& S = s.split[tid];
+      const uint32_t mid = T.begin + S.nleft;  // the node's number too
+      link_child(child, root, T.parent, T.side, mid);
+      // at most kSmallTask - 1 nodes: their records fit the task's own range
+      const uint32_t r = atomicAdd(&s.n_rec, 1u);
+      rec[b0 + r] = make_uint2((T.begin - b0) | ((mid - b0) << 16), (T.end - b0) | (level << 16));
+#pragma unroll
+      for (uint32_t side = 0; side < 2; ++side) {
+        const uint32_t b = side ? mid : T.begin, e = side ? T.end : mid;
+        S.task[side] = 255u;
+        if (e - b > J3DG_SAH_TOP) {
+          const uint32_t q = atomicAdd(&s.n_task[cur ^ 1], 1u);
+          TopTask& C = s.task[cur ^ 1][q];
+          C.begin = b;
+          C.end = e;
+          C.parent = mid;
+          C.side = side | (((T.side >> 1) + 1u) << 1);
+          C.clo = side ? S.rclo : S.lclo;
+          C.chi = side ? S.rchi : S.lchi;
+          S.task[side] = q;
+        } else {
+          s.par[b - b0] = (uint16_t)(((mid - b0) << 1) | side);
+          atomicAdd(&s.n_seg, 1u);
+        }
+      }
+    }
+    // stable partition: lefts before each position by one scan
+    uint32_t f = 0, cnt = 0;
+    for (uint32_t p = p0; p < p1; ++p) {
+      const uint32_t t = s.t.tk[cur][p];
+      if (t >= nlt) continue;
+      if (top_goes_left(b0 + p, s.t.code[p], s.task[cur][t], s.split[t])) {
+        f |= 1u << (p - p0);
+        ++cnt;
+      }
+    }
+    uint32_t inc = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= (uint32_t)o) inc += y;
+    }
+    if (lane == 31) s.wsum[warp] = inc;
+    __syncthreads();
+    uint32_t run = inc - cnt;
+    for (uint32_t w = 0; w < warp; ++w) run += s.wsum[w];
+    {
+      uint32_t at = run;
+      for (uint32_t p = p0; p < p1; ++p) {
+        const uint32_t t = s.t.tk[cur][p];
+        if (t < nlt && s.task[cur][t].begin - b0 == p) s.pre[t] = at;
+        at += (f >> (p - p0)) & 1u;
+      }
+    }
+    __syncthreads();
+    for (uint32_t p = p0; p < p1; ++p) {
+      const uint32_t t = s.t.tk[cur][p], left = (f >> (p - p0)) & 1u;
+      uint32_t d = p, next = 255u;
+      if (t < nlt) {
+        const uint32_t begin = s.task[cur][t].begin - b0, l = run - s.pre[t], mid = begin + s.split[t].nleft;
+        d = left ? begin + l : mid + (p - begin - l);
+        next = s.split[t].task[left ? 0 : 1];
+        run += left;
+        if (d >= n) {
+          atomicOr(status, J3DG_DEV_BAD_INDEX);
+          continue;
+        }
+        if (next == 255u) s.seg[d] = (uint16_t)(left ? begin : mid);
+      }
+      s.t.ord[cur ^ 1][d] = s.t.ord[cur][p];
+      s.t.tk[cur ^ 1][d] = (uint8_t)next;
+    }
+    __syncthreads();  // the level's tasks and splits are read before the next level writes them
+    cur ^= 1;
+  }
 }
 
-// the root of segment s (its one cluster left, at list position s) fills the
-// child slot of the top node that made the segment
-// (the clusters are in C0 or C1, by the parity of the PLOC rounds run)
-__global__ void k_top_link(const TopRange* __restrict__ ranges, const uint32_t* __restrict__ n_ranges_p,
-                           const uint32_t* __restrict__ starts, const uint32_t* __restrict__ scan,
-                           const uint32_t* __restrict__ C0, const uint32_t* __restrict__ C1,
-                           const uint32_t* __restrict__ parity, const uint32_t* __restrict__ n_seg_p,
-                           uint2* __restrict__ child, uint32_t* status) {
-  const uint32_t n_ranges = *n_ranges_p, n_seg = *n_seg_p;
-  const uint32_t* C = *parity ? C1 : C0;
-  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n_ranges; r += gridDim.x * blockDim.x) {
-    const TopRange R = ranges[r];
-    const uint32_t s = scan[R.begin] + starts[R.begin] - 1u;
-    if (s >= n_seg) {
-      atomicOr(status, J3DG_DEV_BAD_INDEX);
+__device__ __forceinline__ float merged_area2(const float2 (&a)[3], const float2 (&b)[3]) {
+  return merged_area(make_float4(a[0].x, a[1].x, a[2].x, 0.f), make_float4(a[0].y, a[1].y, a[2].y, 0.f),
+                     make_float4(b[0].x, b[1].x, b[2].x, 0.f), make_float4(b[0].y, b[1].y, b[2].y, 0.f));
+}
+__device__ __forceinline__ float half_area2(const float2 (&a)[3]) {
+  return half_area4(make_float4(a[0].x, a[1].x, a[2].x, 0.f), make_float4(a[0].y, a[1].y, a[2].y, 0.f));
+}
+
+// PLOC over the block's m clusters (one list, neighbours within a segment
+// only) until n_seg are left, one a segment, in segment order
+template <int W>
+__device__ uint32_t small_cluster(SmallMem<W>& s, uint32_t b0, uint32_t m, uint32_t n_seg, uint32_t leaf_size,
+                                  uint2* __restrict__ child, BinNode* __restrict__ box, uint32_t* __restrict__ count,
+                                  uint8_t* __restrict__ dec, uint32_t* __restrict__ error) {
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, below = (1u << lane) - 1u;
+  while (m > n_seg) {
+    const uint32_t passes = (m + kSmallThreads - 1) / kSmallThreads;
+    // nearest neighbours: each warp's clusters are consecutive, 32 at a time.
+    // A pair's area is made once, by its lower cluster (right[o]: with the
+    // cluster o positions on), and handed to the higher one, which lies in
+    // the same pass or, where the lane index wraps, in the next; the areas
+    // that reach into the next warp's clusters go through shared memory.
+    // Candidates are compared in increasing position: the first of equal
+    // areas wins.
+    const uint32_t lo = warp * passes * 32u;
+    uint32_t first_bo = 255u;
+    float first_best = INFINITY;
+    {
+      float before[kPlocRadius + 1];
+#pragma unroll
+      for (int o = 1; o <= kPlocRadius; ++o) before[o] = INFINITY;
+      for (uint32_t i0 = lo; i0 < min(m, lo + passes * 32u); i0 += 32u) {
+        const uint32_t i = i0 + lane;
+        const bool act = i < m;
+        // how many of the following clusters are of the cluster's segment
+        // (up to the radius): by the segments' first clusters
+        const uint32_t sg = act ? s.seg[i] : 0xffffu;
+        const uint32_t sg2 = i + 32u < m ? s.seg[i + 32u] : 0xffffu;
+        const uint32_t sn = __shfl_sync(0xffffffffu, lane == 0 ? sg2 : sg, (lane + 1u) & 31u);
+        const uint32_t sn2 = __shfl_down_sync(0xffffffffu, sg2, 1);
+        // bit l: the cluster after i0 + l starts another segment
+        const uint64_t ends = (uint64_t)__ballot_sync(0xffffffffu, sn != sg) |
+                              ((uint64_t)__ballot_sync(0xffffffffu, sn2 != sg2) << 32);
+        const uint32_t run = act ? min((uint32_t)kPlocRadius, (uint32_t)__ffsll(ends >> lane | 1ull << 31) - 1u) : 0u;
+        float2 a[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) a[k] = act ? s.box[k][i] : make_float2(0.f, 0.f);
+        float right[kPlocRadius + 1], best = INFINITY;
+        uint32_t bo = 255u;
+#pragma unroll
+        for (int o = kPlocRadius; o >= 1; --o) {
+          right[o] = INFINITY;
+          if ((uint32_t)o <= run) {
+            float2 b[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) b[k] = s.box[k][i + o];
+            right[o] = merged_area2(a, b);
+          }
+          const float left = __shfl_sync(0xffffffffu, lane + o < 32u ? right[o] : before[o], (lane - o) & 31u);
+          if (left < best) {
+            best = left;
+            bo = kPlocRadius - o;
+          }
+          before[o] = right[o];
+        }
+#pragma unroll
+        for (int o = 1; o <= kPlocRadius; ++o)
+          if (right[o] < best) {
+            best = right[o];
+            bo = kPlocRadius + o;
+          }
+        if (i0 == lo) {
+          first_best = best;
+          first_bo = bo;
+        } else if (act) {
+          s.c.nn[i] = (uint8_t)bo;
+        }
+      }
+      if (lane >= 32u - kPlocRadius)
+#pragma unroll
+        for (int o = 1; o <= kPlocRadius; ++o) s.edge[warp][lane - (32u - kPlocRadius)][o - 1] = before[o];
+    }
+    __syncthreads();
+    if (lo + lane < m) {
+      if (lane < (uint32_t)kPlocRadius && lo) {
+        // the clusters of the warp before, which come first: they win ties
+        float best = INFINITY;
+        uint32_t bo = 255u;
+#pragma unroll
+        for (int o = kPlocRadius; o >= 1; --o)
+          if ((uint32_t)o > lane) {
+            const float left = s.edge[warp - 1][kPlocRadius + lane - o][o - 1];
+            if (left < best) {
+              best = left;
+              bo = kPlocRadius - o;
+            }
+          }
+        if (best <= first_best && bo != 255u) first_bo = bo;
+      }
+      s.c.nn[lo + lane] = (uint8_t)first_bo;
+    }
+    __syncthreads();
+    // survivors before each pass's warp
+    uint32_t flags = 0;  // 2 bits per pass: keep, create
+    for (uint32_t pass = 0; pass < passes; ++pass) {
+      if (pass * kSmallThreads + warp * 32u >= m) {  // past the list: the warp has nothing
+        if (lane == 0) s.wsum[pass * kSmallWarps + warp] = 0;
+        continue;
+      }
+      const uint32_t i = pass * kSmallThreads + tid;
+      bool keep = false, create = false;
+      if (i < m) {
+        const uint32_t o = s.c.nn[i];
+        const bool mutual = o != 255u && s.c.nn[i + o - kPlocRadius] == 2u * kPlocRadius - o;
+        create = mutual && o > (uint32_t)kPlocRadius;
+        keep = !mutual || create;
+      }
+      flags |= ((keep ? 1u : 0u) | (create ? 2u : 0u)) << (2u * pass);
+      const uint32_t k = __popc(__ballot_sync(0xffffffffu, keep));
+      if (lane == 0) s.wsum[pass * kSmallWarps + warp] = k;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const uint32_t c = passes * kSmallWarps;
+      const uint32_t x = lane < c ? s.wsum[lane] : 0u, y = lane + 32u < c ? s.wsum[lane + 32u] : 0u;
+      uint32_t xi = x, yi = y;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, xi, o), v = __shfl_up_sync(0xffffffffu, yi, o);
+        if (lane >= (uint32_t)o) {
+          xi += u;
+          yi += v;
+        }
+      }
+      const uint32_t half = __shfl_sync(0xffffffffu, xi, 31);
+      if (lane < c) s.wsum[lane] = xi - x;
+      if (lane + 32u < c) s.wsum[lane + 32u] = half + yi - y;
+      if (lane == 31) s.job = half + yi;  // the survivors
+    }
+    __syncthreads();
+    const uint32_t m2 = s.job;
+    // merges and compaction, a block's width of clusters at a time: a
+    // survivor moves to a position at or below its own, so what later passes
+    // read is in place
+    for (uint32_t pass = 0; pass < passes; ++pass) {
+      const uint32_t i = pass * kSmallThreads + tid;
+      if (pass * kSmallThreads + warp * 32u >= m) {
+        __syncthreads();
+        __syncthreads();
+        continue;
+      }
+      const bool keep = (flags >> (2u * pass)) & 1u, create = (flags >> (2u * pass)) & 2u;
+      const uint32_t bk = __ballot_sync(0xffffffffu, keep);
+      const uint32_t pos = s.wsum[pass * kSmallWarps + warp] + __popc(bk & below);
+      float2 a[3];
+      uint32_t ref = 0, num = 0, sg = 0, spare = 0;
+      float C[W + 1];
+      if (keep) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) a[k] = s.box[k][i];
+        ref = s.ref[i];
+        num = s.c.cnt[i];
+        sg = s.seg[i];
+        spare = s.c.spare[i];
+#pragma unroll
+        for (int k = 1; k <= W; ++k) C[k] = s.c.cost[k - 1][i];
+      }
+      if (create) {
+        const uint32_t j = i + s.c.nn[i] - kPlocRadius, node = b0 + s.c.spare[j];
+        float cr[W + 1], cn[W + 1];
+        uint8_t d[W];
+#pragma unroll
+        for (int k = 1; k <= W; ++k) cr[k] = s.c.cost[k - 1][j];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const float2 b = s.box[k][j];
+          a[k] = make_float2(fminf(a[k].x, b.x), fmaxf(a[k].y, b.y));
+        }
+        num += s.c.cnt[j];
+        collapse_step<W>(C, cr, half_area2(a), num, leaf_size, cn, d);
+        child[node] = make_uint2(ref, s.ref[j]);
+        box[node].lo = make_float4(a[0].x, a[1].x, a[2].x, 0.f);
+        box[node].hi = make_float4(a[0].y, a[1].y, a[2].y, 0.f);
+        count[node] = num;
+        store_dec<W>(dec, node, d);
+        ref = node;
+#pragma unroll
+        for (int k = 1; k <= W; ++k) C[k] = cn[k];
+      }
+      __syncthreads();
+      if (keep && (create || pos != i)) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) s.box[k][pos] = a[k];
+        s.ref[pos] = ref;
+        s.c.cnt[pos] = (uint8_t)num;
+        s.seg[pos] = (uint16_t)sg;
+        s.c.spare[pos] = (uint16_t)spare;
+#pragma unroll
+        for (int k = 1; k <= W; ++k) s.c.cost[k - 1][pos] = C[k];
+      }
+      __syncthreads();
+    }
+    if (m2 >= m) {  // no pair merges (areas past the largest float)
+      if (tid == 0) atomicOr(error, 2u);
+      break;
+    }
+    m = m2;
+  }
+  return m;
+}
+
+template <int W>
+__global__ void __launch_bounds__(kSmallThreads, W == 8 ? J3DG_SMALL_BLOCKS - 1 : J3DG_SMALL_BLOCKS)
+    k_small_tasks(const uint32_t* __restrict__ ord_a, const uint32_t* __restrict__ ord_b,
+                  const uint32_t* __restrict__ parity, const float4* __restrict__ blo, const float4* __restrict__ bhi,
+                  const TopTask* __restrict__ tasks, const TopRange* __restrict__ ranges,
+                  const uint32_t* __restrict__ counters, uint32_t* __restrict__ next_job, uint32_t* __restrict__ error,
+                  uint32_t leaf_size, uint32_t nt, uint32_t cap_small, uint2* __restrict__ rec,
+                  uint2* __restrict__ child, uint32_t* __restrict__ root, BinNode* __restrict__ box,
+                  uint32_t* __restrict__ count, float* __restrict__ cost, uint8_t* __restrict__ dec, uint32_t* status) {
+  extern __shared__ __align__(16) uint8_t small_raw[];
+  SmallMem<W>& s = *reinterpret_cast<SmallMem<W>*>(small_raw);
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t n_tasks = min(counters[3], cap_small), n_jobs = n_tasks + min(counters[2], nt);
+  const uint32_t* ord = *parity ? ord_b : ord_a;  // the final order is where the last level put it
+  for (;;) {
+    if (tid == 0) s.job = atomicAdd(next_job, 1u);
+    __syncthreads();
+    const uint32_t job = s.job;
+    if (job >= n_jobs) return;
+    TopTask T;
+    if (job < n_tasks) {
+      T = tasks[job];
+    } else {
+      const TopRange R = ranges[job - n_tasks];
+      T.begin = R.begin;
+      T.end = R.end;
+      T.parent = R.parent;
+      T.side = R.side;
+      T.clo = T.chi = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const uint32_t b0 = T.begin, n = T.end - T.begin;
+    if (T.end > nt || T.begin >= T.end || n > (job < n_tasks ? kSmallTask : J3DG_SAH_TOP)) {  // block-uniform
+      if (tid == 0) atomicOr(status, J3DG_DEV_BAD_INDEX);
+      __syncthreads();
       continue;
     }
-    if (R.side)
-      child[R.parent].y = C[s];
-    else
-      child[R.parent].x = C[s];
+    if (tid == 0) {
+      s.task[0][0] = T;
+      s.n_task[0] = 1;
+      s.n_seg = s.n_rec = s.bad = 0;
+    }
+    for (uint32_t p = tid; p < n; p += kSmallThreads) {
+      const uint32_t t = ord[b0 + p];
+      const float4 lo = blo[t], hi = bhi[t];
+      s.ref[p] = t;
+      s.box[0][p] = make_float2(lo.x, hi.x);
+      s.box[1][p] = make_float2(lo.y, hi.y);
+      s.box[2][p] = make_float2(lo.z, hi.z);
+      s.t.ord[0][p] = (uint16_t)p;
+      s.t.tk[0][p] = 0;
+      s.seg[p] = 0;
+    }
+    __syncthreads();
+    if (n > J3DG_SAH_TOP) {
+      const int cur = small_levels<W>(s, b0, n, rec, child, root, box, count, error, status);
+      if (s.bad) {
+        __syncthreads();
+        continue;
+      }
+      // boxes and triangles into the final order, one array at a time
+      uint32_t idx[kSmallPer];
+#pragma unroll
+      for (int k = 0; k < kSmallPer; ++k) {
+        const uint32_t p = tid + k * kSmallThreads;
+        idx[k] = p < n ? s.t.ord[cur][p] : 0u;
+      }
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        float2 v[kSmallPer];
+#pragma unroll
+        for (int k = 0; k < kSmallPer; ++k) v[k] = s.box[a][idx[k]];
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kSmallPer; ++k)
+          if (tid + k * kSmallThreads < n) s.box[a][tid + k * kSmallThreads] = v[k];
+      }
+      uint32_t r[kSmallPer];
+#pragma unroll
+      for (int k = 0; k < kSmallPer; ++k) r[k] = s.ref[idx[k]];
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < kSmallPer; ++k)
+        if (tid + k * kSmallThreads < n) s.ref[tid + k * kSmallThreads] = r[k];
+    } else if (tid == 0) {
+      s.par[0] = 0xffffu;  // one segment: its root is the task's
+      s.n_seg = 1;
+    }
+    __syncthreads();
+    for (uint32_t p = tid; p < n; p += kSmallThreads) {
+      s.ref[p] |= 0x80000000u;
+      s.c.cnt[p] = 1;
+      s.c.spare[p] = (uint16_t)p;
+      const float2 a[3] = {s.box[0][p], s.box[1][p], s.box[2][p]};
+      const float v = half_area2(a) * J3DG_SAH_CTRI;
+#pragma unroll
+      for (int k = 0; k < W; ++k) s.c.cost[k][p] = v;
+    }
+    __syncthreads();
+    const uint32_t m = small_cluster<W>(s, b0, n, s.n_seg, leaf_size, child, box, count, dec, error);
+    if (m != s.n_seg) {  // an error was raised: nothing is linked
+      __syncthreads();
+      continue;
+    }
+    // every cluster is a segment's root, its number left over the segment's
+    // first position: the root goes under its parent, its costs are found there
+    for (uint32_t c = tid; c < m; c += kSmallThreads) {
+      const uint32_t first = s.c.spare[c], par = s.par[first];
+      if (par == 0xffffu)
+        link_child(child, root, T.parent, T.side, s.ref[c]);
+      else
+        link_child(child, root, b0 + (par >> 1), par & 1u, s.ref[c]);
+      s.par[first] = (uint16_t)c;
+    }
+    __syncthreads();
+    // the levels' nodes, deepest first: a subtree's costs are kept at its
+    // first position's cluster
+    if (warp == 0) {
+      uint32_t at = s.n_rec;
+      while (at > 0) {
+        const bool have = lane < at;
+        const uint2 x = have ? rec[b0 + at - 1u - lane] : make_uint2(0u, 0u);
+        const uint32_t lv = __shfl_sync(0xffffffffu, x.y >> 16, 0);
+        const uint32_t same = __ballot_sync(0xffffffffu, have && (x.y >> 16) == lv);
+        const uint32_t take = same == 0xffffffffu ? 32u : (uint32_t)__ffs(~same) - 1u;  // one level's records
+        if (lane < take) {
+          const uint32_t mid = x.x >> 16, node = b0 + mid;
+          const uint32_t cb = s.par[x.x & 0xffffu], cm = s.par[mid];
+          float cl[W + 1], cr[W + 1], C[W + 1];
+          uint8_t d[W];
+#pragma unroll
+          for (int k = 1; k <= W; ++k) {
+            cl[k] = s.c.cost[k - 1][cb];
+            cr[k] = s.c.cost[k - 1][cm];
+          }
+          collapse_step<W>(cl, cr, half_area4(box[node].lo, box[node].hi), (x.y & 0xffffu) - (x.x & 0xffffu), leaf_size,
+                           C, d);
+#pragma unroll
+          for (int k = 1; k <= W; ++k) s.c.cost[k - 1][cb] = C[k];
+          store_dec<W>(dec, node, d);
+        }
+        at -= take;
+        __syncwarp();
+      }
+    }
+    __syncthreads();
+    // the task's root under a top node: its costs, for the top nodes' passes
+    if (tid < (uint32_t)W && n > 1u && T.parent != kNoParent) {
+      const uint32_t r = T.side & 1u ? child[T.parent].y : child[T.parent].x;
+      cost[(size_t)r * W + tid] = s.c.cost[tid][s.par[0]];
+    }
+    __syncthreads();  // the block's memory is free for the next job
   }
 }
 
@@ -1844,10 +2227,11 @@ __global__ void k_top_link(const TopRange* __restrict__ ranges, const uint32_t* 
   } while (0)
 
 // slot_of[id] = leaf position of triangle id (ids are a permutation of 0..nt)
-__global__ void k_slot_of(const float4* __restrict__ tris, uint32_t nt, uint32_t* __restrict__ slot_of,
-                          uint32_t* status) {
+// (n_wide, if given: the number of wide nodes; 0 when the build failed and placed nothing)
+__global__ void k_slot_of(const float4* __restrict__ tris, uint32_t nt, const uint32_t* __restrict__ n_wide,
+                          uint32_t* __restrict__ slot_of, uint32_t* status) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nt) return;
+  if (i >= nt || (n_wide && *n_wide == 0u)) return;
   const uint32_t id = __float_as_uint(tris[3 * (size_t)i].w);
   if (id >= nt) {
     atomicOr(status, J3DG_DEV_BAD_INDEX);
@@ -1879,97 +2263,74 @@ __global__ void k_slot_of(const float4* __restrict__ tris, uint32_t nt, uint32_t
 // capture): j3dg_mesh_build captures and launches it for one mesh, and a
 // batch captures it for all its meshes ahead of its frames.
 
-static const uint32_t kMaxTopLevels = 1024, kMaxRounds = 1024, kMaxPlaceLevels = 128;
+static const uint32_t kMaxPlaceLevels = 128;
 
 struct BuildCtl {
-  uint32_t top_ctr[4];  // k_top_children: [0] top nodes, [1] next level's tasks, [2] ranges, [3] largest next task
+  uint32_t top_ctr[4];  // k_top_children: [0] top nodes, [1] next level's tasks, [2] ranges, [3] small tasks
                         // (LBVH: [0] the root that k_lbvh found)
-  uint32_t n_tasks, max_task, ord_parity, top_levels;
-  uint32_t mcount, n_seg, node_base, c_parity, rounds, tot[2];
+  uint32_t n_tasks, ord_parity, top_levels;
+  uint32_t root;      // the binary tree's root
+  uint32_t next_job;  // the next small task or range to be taken (k_small_tasks)
   uint32_t lohi[2];  // the running pass's node range (collapse costs, depth-first levels)
   uint32_t pass, n_pass;
   uint32_t n_in, n_out, n_wide, place_levels, max_depth;
   int32_t dfs_level;
-  uint32_t error;  // a loop overran its bound: 1 SAH levels, 2 PLOC, 4 placement / collapse
-  uint32_t top_end[kMaxTopLevels];     // top nodes of level L end at top_end[L]
-  uint32_t round_end[kMaxRounds];      // binary nodes of PLOC round r end at round_end[r]
+  uint32_t error;  // 1 SAH levels overran their bound, 2 PLOC, 4 placement / collapse
+  uint32_t top_end[kMaxTopLevels];     // top nodes of level L end at top_end[L] (in their list)
   uint32_t level_end[kMaxPlaceLevels]; // wide nodes of level L end at level_end[L]
 };
 
-__global__ void k_ctl_init(BuildCtl* __restrict__ c, TopTask* __restrict__ tasks, const float* __restrict__ bb,
-                           uint32_t nt, uint32_t top) {
+// the root task, by its size: split level by level, by one block, or a segment
+__global__ void k_ctl_init(BuildCtl* __restrict__ c, TopTask* __restrict__ tasks, TopTask* __restrict__ small,
+                           TopRange* __restrict__ ranges, const float* __restrict__ bb, uint32_t nt, uint32_t top) {
   if (top) {
     TopTask r0;
     r0.begin = 0;
     r0.end = nt;
-    r0.node = 0;
-    r0.pad = 0;
+    r0.parent = kNoParent;
+    r0.side = 0;
     r0.clo = make_float4(bb[0], bb[1], bb[2], 0.f);  // the vertex bbox holds every centroid
     r0.chi = make_float4(bb[3], bb[4], bb[5], 0.f);
-    tasks[0] = r0;
-    c->top_ctr[0] = 1;  // the root node
-    c->n_tasks = 1;
-    c->max_task = nt;
-    c->top_levels = 1;
-    c->top_end[0] = 1;
+    if (nt > kSmallTask) {
+      tasks[0] = r0;
+      c->n_tasks = 1;
+    } else if (nt > J3DG_SAH_TOP) {
+      small[0] = r0;
+      c->top_ctr[3] = 1;
+    } else {
+      ranges[0] = TopRange{0, nt, kNoParent, 0};
+      c->top_ctr[2] = 1;
+    }
   }
-  c->mcount = nt;
-  c->n_seg = 1;
   c->n_in = 1;  // the placement's root item
   c->n_wide = 1;
   c->place_levels = 1;
   c->level_end[0] = 1;
 }
 
-__global__ void k_top_step(BuildCtl* __restrict__ c, uint32_t cap_tasks, uint32_t nt, cudaGraphConditionalHandle h,
-                           uint32_t set) {
+__global__ void k_top_step(BuildCtl* __restrict__ c, uint32_t cap_tasks, uint32_t cap_small, uint32_t nt,
+                           cudaGraphConditionalHandle h, uint32_t set) {
   if (c->n_tasks) {  // the level ran
     uint32_t next = c->top_ctr[1];
-    if (next > cap_tasks || c->top_ctr[2] > nt || c->top_ctr[0] > nt - 1 || c->top_levels >= kMaxTopLevels) {
+    if (next > cap_tasks || c->top_ctr[3] > cap_small || c->top_ctr[2] > nt || c->top_ctr[0] > nt - 1 ||
+        c->top_levels >= kMaxTopLevels) {
       c->error |= 1u;
       next = 0;
-    } else if (c->top_ctr[0] > c->top_end[c->top_levels - 1]) {
+    } else {
       c->top_end[c->top_levels++] = c->top_ctr[0];
     }
     c->n_tasks = next;
-    c->max_task = c->top_ctr[3];
     c->top_ctr[1] = 0;
-    c->top_ctr[3] = 0;
     c->ord_parity ^= 1u;
   }
   if (set) cudaGraphSetConditional(h, c->n_tasks > 0 ? 1u : 0u);
 }
 
-__global__ void k_ploc_setup(BuildCtl* __restrict__ c) {  // after the SAH levels: one segment per range
-  c->n_seg = c->top_ctr[2];
-  c->node_base = c->top_ctr[0];
-}
-
-__global__ void k_ploc_step(BuildCtl* __restrict__ c, uint32_t nt, cudaGraphConditionalHandle h, uint32_t set) {
-  if (c->mcount > c->n_seg) {  // the round ran
-    const uint32_t creates = c->tot[0], surv = c->tot[1];
-    if (creates == 0 || surv >= c->mcount || c->node_base + creates > nt - 1 || c->rounds >= kMaxRounds) {
-      c->error |= 2u;  // no progress or past the node bound
-      c->mcount = c->n_seg;
-    } else {
-      c->node_base += creates;
-      c->round_end[c->rounds++] = c->node_base;
-      c->mcount = surv;
-      c->c_parity ^= 1u;
-    }
-  }
-  if (set) cudaGraphSetConditional(h, c->mcount > c->n_seg ? 1u : 0u);
-}
-
-// pass p of the cost programme: the PLOC rounds in order, then the top levels
-// deepest first (children before parents)
-__device__ __forceinline__ void cost_range(BuildCtl* c, uint32_t p, uint32_t top) {
+// pass p of the cost programme: the top levels, deepest first (children before parents)
+__device__ __forceinline__ void cost_range(BuildCtl* c, uint32_t p) {
   uint32_t lo = 0, hi = 0;
-  if (p < c->rounds) {
-    lo = p ? c->round_end[p - 1] : (top ? c->top_ctr[0] : 0u);
-    hi = c->round_end[p];
-  } else if (p < c->n_pass) {
-    const uint32_t k = c->top_levels - 1 - (p - c->rounds);
+  if (p < c->n_pass) {
+    const uint32_t k = c->top_levels - 1 - p;
     lo = k ? c->top_end[k - 1] : 0u;
     hi = c->top_end[k];
   }
@@ -1977,19 +2338,23 @@ __device__ __forceinline__ void cost_range(BuildCtl* c, uint32_t p, uint32_t top
   c->lohi[1] = hi;
 }
 
-__global__ void k_ploc_done(BuildCtl* __restrict__ c, uint32_t nt, uint32_t top, const uint32_t* __restrict__ C0,
-                            const uint32_t* __restrict__ C1, PlaceItem* __restrict__ qa) {
-  const uint32_t root = top ? 0u : (c->c_parity ? C1 : C0)[0];
-  if (c->node_base != nt - 1 || (root & 0x80000000u)) c->error |= 2u;  // a malformed tree
+// the binary tree is complete: the placement starts at its root
+__global__ void k_tree_done(BuildCtl* __restrict__ c, uint32_t nt, PlaceItem* __restrict__ qa) {
+  uint32_t root = c->root;
+  if (root == 0u || root >= nt) {  // a malformed tree (a mesh of one leaf is not built here)
+    c->error |= 2u;
+    root = 0;
+  }
+  if (c->error) c->n_in = c->n_wide = c->place_levels = 0;  // nothing is placed or numbered
   qa[0] = PlaceItem{root, 0u, 1u, 0u};
-  c->n_pass = c->rounds + (top ? c->top_levels : 0u);
+  c->n_pass = c->error ? 0u : c->top_levels;
   c->pass = 0;
-  cost_range(c, 0, top);
+  cost_range(c, 0);
 }
 
-__global__ void k_cost_step(BuildCtl* __restrict__ c, uint32_t top, cudaGraphConditionalHandle h, uint32_t set) {
+__global__ void k_cost_step(BuildCtl* __restrict__ c, cudaGraphConditionalHandle h, uint32_t set) {
   ++c->pass;
-  cost_range(c, c->pass, top);  // past the last pass: an empty range
+  cost_range(c, c->pass);  // past the last pass: an empty range
   if (set) cudaGraphSetConditional(h, c->pass < c->n_pass ? 1u : 0u);
 }
 
@@ -2089,7 +2454,7 @@ static cudaError_t capture_while(cudaStream_t st, cudaStream_t side, Body&& body
 // where the tree decides: the wide nodes, the queues).
 struct BuildPlan {
   uint32_t nv = 0, nt = 0, W = 4, leaf = 2;
-  bool top = false;   // binned-SAH top levels (the default builder, large meshes)
+  bool top = false;   // the default builder (binned-SAH top levels, PLOC below them)
   bool lbvh = false;  // this build is an LBVH (J3DG_BUILD_LBVH)
   // the builders the scratch serves: PLOC (the default) and / or LBVH (a
   // batch's rebuild lane may serve both)
@@ -2099,18 +2464,16 @@ struct BuildPlan {
   float* bb = nullptr;
   uint64_t *k0 = nullptr, *k1 = nullptr;
   uint32_t *v0 = nullptr, *v1 = nullptr, *hist = nullptr, *sums = nullptr;
-  uint32_t *ord_a = nullptr, *ord_b = nullptr, *task_of = nullptr, *task_of2 = nullptr, *seg_starts = nullptr,
-           *seg_scan = nullptr, *top_bins = nullptr;
+  uint32_t *ord_a = nullptr, *ord_b = nullptr, *task_of = nullptr, *task_of2 = nullptr, *top_list = nullptr,
+           *top_bins = nullptr, *cscan = nullptr, *pl_sums = nullptr;
   float4 *tbox_lo = nullptr, *tbox_hi = nullptr;
   uint16_t* codes = nullptr;
-  TopTask *tasks_a = nullptr, *tasks_b = nullptr;
+  TopTask *tasks_a = nullptr, *tasks_b = nullptr, *small = nullptr;
   TopSplit* splits = nullptr;
   TopRange* ranges = nullptr;
   uint2* child = nullptr;
   BinNode* box = nullptr;
-  uint32_t *count = nullptr, *C0 = nullptr, *C1 = nullptr, *nn = nullptr, *cscan = nullptr, *sscan = nullptr,
-           *pl_sums = nullptr, *pl_sums2 = nullptr, *seg0 = nullptr, *seg1 = nullptr;
-  float4 *lo0 = nullptr, *hi0 = nullptr, *lo1 = nullptr, *hi1 = nullptr;
+  uint32_t* count = nullptr;
   float* dp_cost = nullptr;
   uint8_t* dp_dec = nullptr;
   float4* wide = nullptr;
@@ -2122,7 +2485,9 @@ struct BuildPlan {
   // outputs (the mesh keeps them)
   float4 *normals = nullptr, *soup = nullptr, *tris_out = nullptr, *nodes = nullptr;
   uint32_t* slot_of = nullptr;
-  uint32_t cap_tasks() const { return nt / J3DG_SAH_TOP + 1; }  // tasks of one level are disjoint, each > J3DG_SAH_TOP
+  // tasks of one level are disjoint, each above kSmallTask; so are the small tasks, each above J3DG_SAH_TOP
+  uint32_t cap_tasks() const { return nt / kSmallTask + 1; }
+  uint32_t cap_small() const { return nt / J3DG_SAH_TOP + 1; }
   uint32_t n_tiles() const { return (nt + kSortTile - 1) / kSortTile; }
   uint32_t hist_n() const { return 256 * n_tiles(); }
   uint32_t scan_blocks() const { return (hist_n() + 1023) / 1024; }
@@ -2148,7 +2513,7 @@ static cudaError_t plan_alloc(BuildPlan& P, cudaStream_t st, bool outputs = true
   A(P.v1, sizeof(uint32_t) * nt);
   A(P.hist, sizeof(uint32_t) * P.hist_n());
   A(P.sums, sizeof(uint32_t) * (P.scan_blocks() + 1));
-  if (P.top) {
+  if (P.need_ploc) {
     A(P.ord_a, sizeof(uint32_t) * nt);
     A(P.ord_b, sizeof(uint32_t) * nt);
     A(P.task_of, sizeof(uint32_t) * nt);
@@ -2156,33 +2521,22 @@ static cudaError_t plan_alloc(BuildPlan& P, cudaStream_t st, bool outputs = true
     A(P.tbox_lo, sizeof(float4) * nt);
     A(P.tbox_hi, sizeof(float4) * nt);
     A(P.codes, sizeof(uint16_t) * nt);
-    A(P.seg_starts, sizeof(uint32_t) * nt);
-    A(P.seg_scan, sizeof(uint32_t) * nt);
+    A(P.cscan, sizeof(uint32_t) * nt);
+    A(P.pl_sums, sizeof(uint32_t) * (P.sblocks() + 1));
+    A(P.top_list, sizeof(uint32_t) * nt);
     A(P.top_bins, sizeof(uint32_t) * (size_t)P.cap_tasks() * 3 * kTopBins * kTopVals);
     A(P.tasks_a, sizeof(TopTask) * P.cap_tasks());
     A(P.tasks_b, sizeof(TopTask) * P.cap_tasks());
+    A(P.small, sizeof(TopTask) * P.cap_small());
     A(P.splits, sizeof(TopSplit) * P.cap_tasks());
     A(P.ranges, sizeof(TopRange) * nt);  // at most one range per triangle
   }
-  A(P.child, sizeof(uint2) * (nt - 1));
-  A(P.box, sizeof(BinNode) * (nt - 1));
-  A(P.count, sizeof(uint32_t) * (nt - 1));  // LBVH: the sibling handshake of k_lbvh
+  A(P.child, sizeof(uint2) * nt);
+  A(P.box, sizeof(BinNode) * nt);
+  A(P.count, sizeof(uint32_t) * nt);  // LBVH: the sibling handshake of k_lbvh
   if (P.need_ploc) {
-    A(P.C0, sizeof(uint32_t) * nt);
-    A(P.C1, sizeof(uint32_t) * nt);
-    A(P.nn, sizeof(uint32_t) * nt);
-    A(P.cscan, sizeof(uint32_t) * nt);
-    A(P.sscan, sizeof(uint32_t) * nt);
-    A(P.pl_sums, sizeof(uint32_t) * (P.sblocks() + 1));
-    A(P.pl_sums2, sizeof(uint32_t) * (P.sblocks() + 1));
-    A(P.seg0, sizeof(uint32_t) * nt);
-    A(P.seg1, sizeof(uint32_t) * nt);
-    A(P.lo0, sizeof(float4) * nt);
-    A(P.hi0, sizeof(float4) * nt);
-    A(P.lo1, sizeof(float4) * nt);
-    A(P.hi1, sizeof(float4) * nt);
-    A(P.dp_cost, sizeof(float) * P.W * (nt - 1));
-    A(P.dp_dec, sizeof(uint8_t) * P.W * (nt - 1));
+    A(P.dp_cost, sizeof(float) * P.W * nt);
+    A(P.dp_dec, sizeof(uint8_t) * P.W * nt);
     A(P.pa, sizeof(PlaceItem) * nt);
     A(P.pb, sizeof(PlaceItem) * nt);
     A(P.soup, sizeof(float4) * 3 * nt);  // the LBVH gathers straight into the leaf order
@@ -2208,10 +2562,9 @@ static cudaError_t plan_alloc(BuildPlan& P, cudaStream_t st, bool outputs = true
 // frees the scratch (outputs the caller took over are null)
 static void plan_free(BuildPlan& P, cudaStream_t st) {
   void* ps[] = {P.part, P.bb, P.k0, P.k1, P.v0, P.v1, P.hist, P.sums, P.ord_a, P.ord_b, P.task_of, P.task_of2,
-                P.seg_starts, P.seg_scan, P.top_bins, P.tbox_lo, P.tbox_hi, P.codes, P.tasks_a, P.tasks_b, P.splits,
-                P.ranges, P.child, P.box, P.count, P.C0, P.C1, P.nn, P.cscan, P.sscan, P.pl_sums, P.pl_sums2, P.seg0,
-                P.seg1, P.lo0, P.hi0, P.lo1, P.hi1, P.dp_cost, P.dp_dec, P.wide, P.pa, P.pb, P.range, P.qa, P.qb,
-                P.dfs_size, P.dfs_pos, P.ctl, P.normals, P.soup, P.tris_out, P.nodes, P.slot_of};
+                P.cscan, P.pl_sums, P.top_list, P.top_bins, P.tbox_lo, P.tbox_hi, P.codes, P.tasks_a, P.tasks_b,
+                P.small, P.splits, P.ranges, P.child, P.box, P.count, P.dp_cost, P.dp_dec, P.wide, P.pa, P.pb, P.range,
+                P.qa, P.qb, P.dfs_size, P.dfs_pos, P.ctl, P.normals, P.soup, P.tris_out, P.nodes, P.slot_of};
   for (void* p : ps)
     if (p) cudaFreeAsync(p, st);
   P = BuildPlan{};
@@ -2223,29 +2576,56 @@ static void plan_free(BuildPlan& P, cudaStream_t st) {
     if (e == cudaSuccess) e = cudaGetLastError(); \
   } while (0)
 
+// section 5d over every small task and range: persistent blocks, as many as
+// the device holds at the kernel's shared memory
+template <int W>
+static cudaError_t launch_small_tasks_w(BuildPlan& P, cudaStream_t st, uint32_t* d_status) {
+  BuildCtl* c = P.ctl;
+  const size_t smem = small_smem<W>();
+  cudaError_t e = cudaFuncSetAttribute(k_small_tasks<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int dev = 0, sms = 0, per = 0;
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_small_tasks<W>, kSmallThreads, smem);
+  if (e != cudaSuccess) return e;
+  const uint32_t grid = std::min((uint32_t)std::max(1, sms * per), P.cap_small());
+  k_small_tasks<W><<<grid, kSmallThreads, smem, st>>>(
+      P.ord_a, P.ord_b, &c->ord_parity, P.tbox_lo, P.tbox_hi, P.small, P.ranges, c->top_ctr, &c->next_job, &c->error,
+      P.leaf, P.nt, P.cap_small(), reinterpret_cast<uint2*>(P.pb), P.child, &c->root, P.box, P.count, P.dp_cost, P.dp_dec,
+      d_status);
+  return cudaGetLastError();
+}
+
+static cudaError_t launch_small_tasks(uint32_t W, BuildPlan& P, cudaStream_t st, uint32_t* d_status) {
+  if (W == 2) return launch_small_tasks_w<2>(P, st, d_status);
+  if (W == 8) return launch_small_tasks_w<8>(P, st, d_status);
+  return launch_small_tasks_w<4>(P, st, d_status);
+}
+
 // the default builder's binary tree and wide nodes (P.wide, level ranges in
-// c->level_end): binned-SAH top levels over PLOC ranges (or PLOC alone), the
-// cost programme, the placement; the leaf-ordered triangles go to P.tris_out
+// c->level_end): binned-SAH levels down to small tasks, each small task's
+// subtree by one block, the cost programme of the top nodes, the placement;
+// the leaf-ordered triangles go to P.tris_out
 static cudaError_t enqueue_tree_ploc(BuildPlan& P, cudaStream_t st, cudaStream_t side, uint32_t* d_status) {
   const uint32_t nt = P.nt, W = P.W;
   BuildCtl* c = P.ctl;
   cudaError_t e = cudaSuccess;
   const float4* soup = P.soup;
-  if (P.top) {
-    k_top_boxes<<<(nt + 255) / 256, 256, 0, st>>>(soup, nt, P.tbox_lo, P.tbox_hi);
-    k_iota<<<(nt + 255) / 256, 256, 0, st>>>(P.ord_a, nt);
+  k_top_boxes<<<(nt + 255) / 256, 256, 0, st>>>(soup, nt, P.tbox_lo, P.tbox_hi);
+  k_iota<<<(nt + 255) / 256, 256, 0, st>>>(P.ord_a, nt);
+  J3DG_EQ(cudaSuccess);
+  if (nt > kSmallTask) {
     J3DG_EQ(cudaMemsetAsync(P.task_of, 0, sizeof(uint32_t) * nt, st));
     // one SAH level: tasks ti, order oi, task of each position si -> the next level's
     auto level = [&](cudaStream_t s, TopTask* ti, TopTask* to, uint32_t* oi, uint32_t* oo, uint32_t* si,
                      uint32_t* so) {
-      k_top_bins_init<<<kStrideBlocks, 256, 0, s>>>(P.top_bins, &c->n_tasks, &c->max_task, ti);
-      k_top_bin<<<(nt + kTopChunk - 1) / kTopChunk, 256, 0, s>>>(oi, P.tbox_lo, P.tbox_hi, si, ti, &c->n_tasks,
-                                                                 &c->max_task, nt, P.top_bins, P.codes);
-      k_top_bin_warp<<<kStrideBlocks, 256, 0, s>>>(oi, P.tbox_lo, P.tbox_hi, ti, &c->n_tasks, P.splits, P.box,
-                                                   P.count, P.codes);
-      k_top_split<<<kStrideBlocks, 128, 0, s>>>(ti, &c->n_tasks, &c->max_task, P.top_bins, P.splits, P.box, P.count);
-      k_top_children<<<kStrideBlocks, 128, 0, s>>>(ti, P.splits, &c->n_tasks, J3DG_SAH_TOP, c->top_ctr, to, P.ranges,
-                                                   P.child, P.cap_tasks(), nt, nt - 1, d_status);
+      k_top_bins_init<<<kStrideBlocks, 256, 0, s>>>(P.top_bins, &c->n_tasks);
+      k_top_bin<<<(nt + kTopChunk - 1) / kTopChunk, 256, 0, s>>>(oi, P.tbox_lo, P.tbox_hi, si, ti, &c->n_tasks, nt,
+                                                                 P.top_bins, P.codes);
+      k_top_split<<<kStrideBlocks, 128, 0, s>>>(ti, &c->n_tasks, P.top_bins, P.splits, P.box, P.count);
+      k_top_children<<<kStrideBlocks, 128, 0, s>>>(ti, P.splits, &c->n_tasks, c->top_ctr, to, P.small, P.ranges,
+                                                   P.top_list, P.child, &c->root, P.cap_tasks(), P.cap_small(), nt,
+                                                   d_status);
       k_top_flag_scan<<<P.sblocks(), 256, 0, s>>>(si, P.codes, ti, P.splits, &c->n_tasks, nt, P.cscan, P.pl_sums);
       k_scan_sums<<<1, 1024, 0, s>>>(P.pl_sums, nullptr, P.sblocks(), nullptr);
       k_top_scatter<<<(nt + 1023) / 1024, 256, 0, s>>>(oi, oo, si, so, P.codes, ti, P.splits, &c->n_tasks, P.cscan,
@@ -2253,53 +2633,22 @@ static cudaError_t enqueue_tree_ploc(BuildPlan& P, cudaStream_t st, cudaStream_t
     };
     J3DG_EQ(capture_while(st, side, [&](cudaStream_t s, cudaGraphConditionalHandle h) {
       level(s, P.tasks_a, P.tasks_b, P.ord_a, P.ord_b, P.task_of, P.task_of2);
-      k_top_step<<<1, 1, 0, s>>>(c, P.cap_tasks(), nt, h, 0u);
+      k_top_step<<<1, 1, 0, s>>>(c, P.cap_tasks(), P.cap_small(), nt, h, 0u);
       level(s, P.tasks_b, P.tasks_a, P.ord_b, P.ord_a, P.task_of2, P.task_of);
-      k_top_step<<<1, 1, 0, s>>>(c, P.cap_tasks(), nt, h, 1u);
+      k_top_step<<<1, 1, 0, s>>>(c, P.cap_tasks(), P.cap_small(), nt, h, 1u);
     }));
-    k_ploc_setup<<<1, 1, 0, st>>>(c);
-    // segments numbered in position order: a flag at each range's start, one scan
-    J3DG_EQ(cudaMemsetAsync(P.seg_starts, 0, sizeof(uint32_t) * nt, st));
-    k_top_seg_starts<<<kStrideBlocks, 256, 0, st>>>(P.ranges, &c->top_ctr[2], nt, P.seg_starts);
-    k_scan_chunks<<<P.sblocks(), 256, 0, st>>>(P.seg_starts, P.seg_scan, nt, P.pl_sums);
-    k_scan_sums<<<1, 1024, 0, st>>>(P.pl_sums, nullptr, P.sblocks(), nullptr);
-    k_scan_add<<<P.sblocks(), 256, 0, st>>>(P.seg_scan, nt, P.pl_sums);
-    k_ploc_init_seg<<<(nt + 255) / 256, 256, 0, st>>>(soup, P.ord_a, P.ord_b, &c->ord_parity, nt, P.seg_starts,
-                                                      P.seg_scan, P.C0, P.lo0, P.hi0, P.seg0);
-  } else {
-    k_ploc_init<<<(nt + 255) / 256, 256, 0, st>>>(soup, nt, P.C0, P.lo0, P.hi0);
-    J3DG_EQ(cudaMemsetAsync(P.seg0, 0, sizeof(uint32_t) * nt, st));
   }
+  J3DG_EQ(launch_small_tasks(W, P, st, d_status));
+  k_tree_done<<<1, 1, 0, st>>>(c, nt, P.pa);
   J3DG_EQ(cudaSuccess);
-  // PLOC rounds: clusters (C, lo, hi, seg) in -> out
-  auto round = [&](cudaStream_t s, const uint32_t* Ci, const float4* li, const float4* hi_, const uint32_t* si,
-                   uint32_t* Co, float4* lo_, float4* ho, uint32_t* so) {
-    k_ploc_nn<<<kStrideBlocks, kPlocBlock, 0, s>>>(li, hi_, si, &c->mcount, &c->n_seg, P.nn);
-    k_ploc_flag_scan<<<P.sblocks(), 256, 0, s>>>(P.nn, &c->mcount, &c->n_seg, P.cscan, P.sscan, P.pl_sums,
-                                                 P.pl_sums2);
-    k_scan_sums<<<1, 1024, 0, s>>>(P.pl_sums, P.pl_sums2, 0u, c->tot, &c->mcount);
-    k_ploc_merge<<<kStrideBlocks, 256, 0, s>>>(Ci, li, hi_, si, P.nn, P.cscan, P.sscan, P.pl_sums, P.pl_sums2,
-                                               &c->mcount, &c->n_seg, &c->node_base, Co, lo_, ho, so, P.child, P.box,
-                                               P.count);
-  };
-  J3DG_EQ(capture_while(st, side, [&](cudaStream_t s, cudaGraphConditionalHandle h) {
-    round(s, P.C0, P.lo0, P.hi0, P.seg0, P.C1, P.lo1, P.hi1, P.seg1);
-    k_ploc_step<<<1, 1, 0, s>>>(c, nt, h, 0u);
-    round(s, P.C1, P.lo1, P.hi1, P.seg1, P.C0, P.lo0, P.hi0, P.seg0);
-    k_ploc_step<<<1, 1, 0, s>>>(c, nt, h, 1u);
-  }));
-  if (P.top)
-    k_top_link<<<kStrideBlocks, 256, 0, st>>>(P.ranges, &c->top_ctr[2], P.seg_starts, P.seg_scan, P.C0, P.C1,
-                                              &c->c_parity, &c->n_seg, P.child, d_status);
-  k_ploc_done<<<1, 1, 0, st>>>(c, nt, P.top ? 1u : 0u, P.C0, P.C1, P.pa);
-  J3DG_EQ(cudaSuccess);
-  // cost programme, children before parents
-  J3DG_EQ(capture_while(st, side, [&](cudaStream_t s, cudaGraphConditionalHandle h) {
-    launch_collapse_cost(W, P.child, P.box, P.count, soup, c->lohi, P.leaf, P.dp_cost, P.dp_dec, s);
-    k_cost_step<<<1, 1, 0, s>>>(c, P.top ? 1u : 0u, h, 0u);
-    launch_collapse_cost(W, P.child, P.box, P.count, soup, c->lohi, P.leaf, P.dp_cost, P.dp_dec, s);
-    k_cost_step<<<1, 1, 0, s>>>(c, P.top ? 1u : 0u, h, 1u);
-  }));
+  // the top nodes' cost programme, children before parents
+  if (nt > kSmallTask)
+    J3DG_EQ(capture_while(st, side, [&](cudaStream_t s, cudaGraphConditionalHandle h) {
+      launch_collapse_cost(W, P.child, P.box, P.count, soup, P.top_list, c->lohi, P.leaf, P.dp_cost, P.dp_dec, s);
+      k_cost_step<<<1, 1, 0, s>>>(c, h, 0u);
+      launch_collapse_cost(W, P.child, P.box, P.count, soup, P.top_list, c->lohi, P.leaf, P.dp_cost, P.dp_dec, s);
+      k_cost_step<<<1, 1, 0, s>>>(c, h, 1u);
+    }));
   // placement, level by level
   J3DG_EQ(capture_while(st, side, [&](cudaStream_t s, cudaGraphConditionalHandle h) {
     launch_collapse_place(W, P.child, P.box, P.count, soup, P.pa, &c->n_in, P.pb, &c->n_out, &c->n_wide, P.wide,
@@ -2349,7 +2698,7 @@ static cudaError_t enqueue_prefix(BuildPlan& P, const float* dV, const uint32_t*
   J3DG_EQ(cudaMemsetAsync(c, 0, sizeof(BuildCtl), st));
   k_bbox_partial<<<kBBoxBlocks, 256, 0, st>>>(dV, nv, P.part);
   k_bbox_final<<<1, 32, 0, st>>>(P.part, kBBoxBlocks, P.bb);
-  k_ctl_init<<<1, 1, 0, st>>>(c, P.tasks_a, P.bb, nt, P.top ? 1u : 0u);
+  k_ctl_init<<<1, 1, 0, st>>>(c, P.tasks_a, P.small, P.ranges, P.bb, nt, P.top ? 1u : 0u);
   k_tri_prep<<<(nt + 255) / 256, 256, 0, st>>>(dV, nv, dT, nt, P.bb, P.normals, P.k0, P.v0, d_status);
   J3DG_EQ(cudaSuccess);
   {
@@ -2407,7 +2756,7 @@ static cudaError_t enqueue_tree(BuildPlan& P, cudaStream_t st, cudaStream_t side
     dfs(std::integral_constant<int, 8>());
   else
     dfs(std::integral_constant<int, 4>());
-  k_slot_of<<<(nt + 255) / 256, 256, 0, st>>>(P.tris_out, nt, P.slot_of, d_status);
+  k_slot_of<<<(nt + 255) / 256, 256, 0, st>>>(P.tris_out, nt, &c->n_wide, P.slot_of, d_status);
   J3DG_EQ(cudaSuccess);
   return e;
 }
@@ -2436,7 +2785,7 @@ static int build_bvh_graph(j3dg_mesh* m, const float* dV, const uint32_t* dT, cu
   P.lbvh = (m->build_flags & J3DG_BUILD_LBVH) != 0;
   P.need_ploc = !P.lbvh;
   P.need_lbvh = P.lbvh;
-  P.top = !P.lbvh && J3DG_SAH_TOP > 0 && m->nt > J3DG_SAH_TOP;
+  P.top = !P.lbvh;
   cudaStream_t side = nullptr;
   cudaGraph_t g = nullptr;
   cudaGraphExec_t ex = nullptr;
@@ -2554,7 +2903,7 @@ int rebuild_lane_alloc(uint32_t nt_max, uint32_t nv_max, uint32_t W, bool ploc, 
   L->P.W = W;
   L->P.need_ploc = ploc;
   L->P.need_lbvh = lbvh;
-  L->P.top = ploc && J3DG_SAH_TOP > 0 && nt_max > J3DG_SAH_TOP;
+  L->P.top = ploc;
   const cudaError_t e = plan_alloc(L->P, st, false);
   if (e != cudaSuccess) {
     plan_free(L->P, st);
@@ -2580,7 +2929,7 @@ cudaError_t rebuild_enqueue(RebuildLane* L, const j3dg_mesh* m, cudaStream_t st,
   Pm.nv = m->nv;
   Pm.leaf = m->leaf_size;
   Pm.lbvh = (m->build_flags & J3DG_BUILD_LBVH) != 0;
-  Pm.top = !Pm.lbvh && J3DG_SAH_TOP > 0 && m->nt > J3DG_SAH_TOP;
+  Pm.top = !Pm.lbvh;
   if (Pm.lbvh ? !Pm.need_lbvh : !Pm.need_ploc) return cudaErrorInvalidValue;  // the lane has no scratch for it
   Pm.normals = (float4*)m->d_normals;
   Pm.tris_out = (float4*)m->d_tris;
@@ -2637,7 +2986,7 @@ int build_bvh(j3dg_mesh* m, const float* dV, const uint32_t* dT, cudaStream_t st
   J3DG_CK(cudaMallocAsync(&m->d_nodes, sizeof(float4) * F4, st));
   J3DG_CK(cudaMemsetAsync(m->d_nodes, 0, sizeof(float4) * F4, st));
   J3DG_CK(cudaMallocAsync(&m->d_slot_of, sizeof(uint32_t) * (size_t)nt, st));
-  k_slot_of<<<1, 256, 0, st>>>((const float4*)m->d_tris, nt, (uint32_t*)m->d_slot_of, d_status);
+  k_slot_of<<<1, 256, 0, st>>>((const float4*)m->d_tris, nt, nullptr, (uint32_t*)m->d_slot_of, d_status);
   J3DG_CK(cudaGetLastError());
   if (done) J3DG_CK(cudaEventRecord(done, st));
 
