@@ -159,11 +159,11 @@ __global__ void k_radix_hist(const uint64_t* __restrict__ keys, uint32_t n, int 
   hist[(size_t)threadIdx.x * num_tiles + blockIdx.x] = h[threadIdx.x];
 }
 
-// exclusive scan helpers (three phases over chunks of 1024 elements):
+// exclusive scan helpers (over chunks of 1024 elements):
 // k_scan_chunks scans each chunk (256 threads x 4 elements: a sequential
 // scan of the thread's uint4, a shuffle scan of the warp's totals, the
 // eight warp totals through shared memory) and writes the chunk total,
-// k_scan_sums scans the chunk totals, k_scan_add adds them back. in and out
+// k_scan_sums scans the chunk totals, which the readers add. in and out
 // are 16-byte aligned (device allocations); elements past n read as 0 and
 // are not written.
 __global__ void __launch_bounds__(256) k_scan_chunks(const uint32_t* in, uint32_t* out, uint32_t n,
@@ -207,68 +207,41 @@ __global__ void __launch_bounds__(256) k_scan_chunks(const uint32_t* in, uint32_
   if (threadIdx.x == 0) sums[blockIdx.x] = all;
 }
 
-__global__ void __launch_bounds__(1024) k_scan_sums(uint32_t* __restrict__ sums_a, uint32_t* __restrict__ sums_b,
-                                                    uint32_t n, uint32_t* __restrict__ totals,
-                                                    const uint32_t* __restrict__ len_p = nullptr) {
-  // len_p (if given): the scanned list's length in device memory; the chunk
-  // totals to scan are then ceil(len / 1024)
-  if (len_p) n = (*len_p + 1023u) / 1024u;
-  // single block of 1024 threads, over one array of chunk totals (sums_b
-  // null) or two: each thread sums a strip of consecutive chunk totals, the
-  // strip sums are scanned by warp shuffles (within each warp, then the 32
-  // warp totals by warp 0), and each thread rewrites its strip as exclusive
-  // prefixes; totals (if not null) receives each array's grand total
+__global__ void __launch_bounds__(1024) k_scan_sums(uint32_t* __restrict__ sums, uint32_t n) {
+  // single block of 1024 threads: each thread sums a strip of consecutive
+  // chunk totals, the strip sums are scanned by warp shuffles (within each
+  // warp, then the 32 warp totals by warp 0), and each thread rewrites its
+  // strip as exclusive prefixes
   __shared__ uint32_t wtot[32];
   const uint32_t per = (n + 1023) / 1024;
   const uint32_t b = threadIdx.x * per, e = min(n, b + per);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  for (int q = 0; q < 2; ++q) {
-    uint32_t* sums = q ? sums_b : sums_a;
-    if (!sums) break;  // uniform over the block
-    uint32_t acc = 0;
-    for (uint32_t i = b; i < e; ++i) acc += sums[i];
-    uint32_t inc = acc;
+  uint32_t acc = 0;
+  for (uint32_t i = b; i < e; ++i) acc += sums[i];
+  uint32_t inc = acc;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= (uint32_t)o) inc += y;
+  }
+  if (lane == 31) wtot[warp] = inc;
+  __syncthreads();
+  if (warp == 0) {
+    const uint32_t x = wtot[lane];
+    uint32_t xi = x;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= (uint32_t)o) inc += y;
+      const uint32_t y = __shfl_up_sync(0xffffffffu, xi, o);
+      if (lane >= (uint32_t)o) xi += y;
     }
-    if (lane == 31) wtot[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-      const uint32_t x = wtot[lane];
-      uint32_t xi = x;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, xi, o);
-        if (lane >= (uint32_t)o) xi += y;
-      }
-      wtot[lane] = xi - x;
-      if (lane == 31 && totals) totals[q] = xi;
-    }
-    __syncthreads();
-    uint32_t run = wtot[warp] + inc - acc;
-    for (uint32_t i = b; i < e; ++i) {
-      const uint32_t x = sums[i];
-      sums[i] = run;
-      run += x;
-    }
-    __syncthreads();  // wtot is reused by the second array
+    wtot[lane] = xi - x;
   }
-}
-
-__global__ void __launch_bounds__(256) k_scan_add(uint32_t* __restrict__ out, uint32_t n,
-                                                  const uint32_t* __restrict__ sums) {
-  const uint32_t base = blockIdx.x * 1024u + threadIdx.x * 4u, add = sums[blockIdx.x];
-  if (base + 3 < n) {
-    uint4 v = *reinterpret_cast<const uint4*>(out + base);
-    v.x += add;
-    v.y += add;
-    v.z += add;
-    v.w += add;
-    *reinterpret_cast<uint4*>(out + base) = v;
-  } else {
-    for (uint32_t k = base; k < n && k < base + 4u; ++k) out[k] += add;
+  __syncthreads();
+  uint32_t run = wtot[warp] + inc - acc;
+  for (uint32_t i = b; i < e; ++i) {
+    const uint32_t x = sums[i];
+    sums[i] = run;
+    run += x;
   }
 }
 
@@ -1050,11 +1023,10 @@ static void launch_collapse_place(uint32_t W, const uint2* child, const BinNode*
 // partition of the Morton-sorted order keeps every range in Morton order, so
 // each range of at most J3DG_SAH_TOP triangles (a segment) is then clustered
 // by PLOC on its own (neighbours searched within the segment only).
-// Tasks above kSmallTask triangles are split level by level over the whole
-// mesh (per-block bins in shared memory, merged into the task's bins; flags
-// from the bin codes that binning stored per position, one exclusive scan);
-// a task of at most kSmallTask is taken through the rest of its subtree by
-// one block (section 5d).
+// Tasks above kSmallTask triangles are split level by level, each cut into
+// items of at most `chunk` positions that a block bins and partitions; a task
+// of at most kSmallTask is taken through the rest of its subtree by one block
+// (section 5d).
 //
 // Binary nodes are numbered by position: the node that splits its range at
 // position mid is node mid, and the nodes that PLOC makes in a segment take
@@ -1098,11 +1070,16 @@ struct TopSplit {
   float4 lclo, lchi, rclo, rchi;  // children's centroid bounds
 };
 
-// triangle boxes by triangle, computed once for the top levels
-__global__ void k_top_boxes(const float4* __restrict__ tris, uint32_t n, float4* __restrict__ blo,
-                            float4* __restrict__ bhi) {
+// triangle boxes by triangle, computed once for the SAH levels, and the order they start from
+__global__ void k_top_boxes(const float4* __restrict__ tris, uint32_t n, BinNode* __restrict__ tbox,
+                            uint32_t* __restrict__ ord) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) leaf_box(tris, i, blo[i], bhi[i]);
+  if (i >= n) return;
+  float4 lo, hi;
+  leaf_box(tris, i, lo, hi);
+  tbox[i].lo = lo;
+  tbox[i].hi = hi;
+  ord[i] = i;
 }
 
 struct TopRange {  // a finished range: a segment for PLOC
@@ -1134,118 +1111,43 @@ __device__ __forceinline__ int top_bin(float c, float lo, float hi) {
   return b < 0 ? 0 : (b >= kTopBins ? kTopBins - 1 : b);
 }
 
-// top_bin by a product with scale = kTopBins / (hi - lo) instead of a division:
-// the two differ by under 4e-6, so away from a bin's edge the bin is the
-// same; within 1e-4 of an edge (and for NaN and infinite values) the division
-// decides
-__device__ __forceinline__ int top_bin_scaled(float c, float lo, float hi, float scale) {
-  const float q = (c - lo) * scale;
-  if (!(fabsf(q - rintf(q)) > 1e-4f)) return top_bin(c, lo, hi);
-  const int b = (int)q;
-  return b < 0 ? 0 : (b >= kTopBins ? kTopBins - 1 : b);
-}
+// top_bin on three axes (packed 4 bits each, x lowest) by products with
+// kTopBins / (hi - lo) instead of divisions: the two differ by under 4e-6, so
+// away from a bin's edge the bin is the same; where an axis is within 1e-4 of
+// an edge or out of the range (or NaN or infinite), the divisions decide
+struct TopBinner {
+  float lx, ly, lz, sx, sy, sz;
+  __device__ __forceinline__ void set(const TopTask& T) {
+    lx = T.clo.x, ly = T.clo.y, lz = T.clo.z;
+    sx = (float)kTopBins / (T.chi.x - lx);
+    sy = (float)kTopBins / (T.chi.y - ly);
+    sz = (float)kTopBins / (T.chi.z - lz);
+  }
+  // q - 0.5 rounded to an integer is the floor of a q away from its edges;
+  // the bits of 1.5 2^23 + that are the integer itself
+  __device__ __forceinline__ static float floor_off(float q, uint32_t& b) {
+    const float t = q - 0.5f, m = t + 12582912.f;
+    b = __float_as_uint(m) - 0x4b400000u;
+    return fabsf(t - (m - 12582912.f));
+  }
+  __device__ __forceinline__ uint32_t code(float cx, float cy, float cz, const TopTask& T) const {
+    uint32_t bx, by, bz;
+    const float ox = floor_off((cx - lx) * sx, bx), oy = floor_off((cy - ly) * sy, by),
+                oz = floor_off((cz - lz) * sz, bz);
+    if (!(ox < 0.4999f && oy < 0.4999f && oz < 0.4999f) || (bx | by | bz) >= (uint32_t)kTopBins) {
+      bx = top_bin(cx, T.clo.x, T.chi.x);
+      by = top_bin(cy, T.clo.y, T.chi.y);
+      bz = top_bin(cz, T.clo.z, T.chi.z);
+    }
+    return bx | (by << 4) | (bz << 8);
+  }
+};
 
-static const int kTopChunk = 2048;
 // Tasks up to this size leave the level loop for section 5d.
 #ifndef J3DG_SMALL_TASK
 #define J3DG_SMALL_TASK 1024
 #endif
 static const uint32_t kSmallTask = J3DG_SMALL_TASK;
-
-// the level's task count is read from device memory
-__global__ void k_top_bins_init(uint32_t* __restrict__ bins, const uint32_t* __restrict__ n_tasks_p) {
-  const uint32_t n_words = *n_tasks_p * 3 * kTopBins * kTopVals;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_words; i += gridDim.x * blockDim.x) {
-    const uint32_t v = i % kTopVals;
-    bins[i] = v == 0 ? 0u : (((v - 1) % 6) < 3 ? 0xffffffffu : 0u);  // lo fields: max code, hi fields: 0
-  }
-}
-
-
-// bins of every active task: [task][axis][bin][kTopVals]
-__global__ void __launch_bounds__(256) k_top_bin(const uint32_t* __restrict__ ord, const float4* __restrict__ blo,
-                                                 const float4* __restrict__ bhi, const uint32_t* __restrict__ task_of,
-                                                 const TopTask* __restrict__ tasks,
-                                                 const uint32_t* __restrict__ n_tasks_p, uint32_t n,
-                                                 uint32_t* __restrict__ bins, uint16_t* __restrict__ code) {
-  __shared__ uint32_t sb[3 * kTopBins * kTopVals];
-  __shared__ uint32_t s_task;
-  const uint32_t n_tasks = *n_tasks_p;
-  if (n_tasks == 0) return;  // no level
-  const uint32_t c0 = blockIdx.x * kTopChunk, c1 = min(n, c0 + kTopChunk);
-  if (c0 >= n) return;
-  if (threadIdx.x == 0) {
-    const uint32_t a = task_of[c0], b = task_of[c1 - 1];
-    s_task = (a == b && a < n_tasks) ? a : kNoTask;
-  }
-  for (uint32_t k = threadIdx.x; k < 3 * kTopBins * kTopVals; k += blockDim.x) {
-    const uint32_t v = k % kTopVals;
-    sb[k] = v == 0 ? 0u : (((v - 1) % 6) < 3 ? 0xffffffffu : 0u);
-  }
-  __syncthreads();
-  const uint32_t st = s_task;
-  const uint32_t lane = threadIdx.x & 31u;
-  for (uint32_t base = c0; base < c1; base += blockDim.x) {  // uniform trip count: whole warps
-    const uint32_t p = base + threadIdx.x;
-    const uint32_t t = p < c1 ? (st != kNoTask ? st : task_of[p]) : kNoTask;
-    const bool valid = t < n_tasks;
-    float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo, c = lo;
-    int bx = 0, by = 0, bz = 0;
-    if (valid) {
-      const uint32_t tri = ord[p];
-      lo = blo[tri];
-      hi = bhi[tri];
-      c = make_float4(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z), 0.f);
-      const TopTask T = tasks[t];
-      bx = top_bin(c.x, T.clo.x, T.chi.x);
-      by = top_bin(c.y, T.clo.y, T.chi.y);
-      bz = top_bin(c.z, T.clo.z, T.chi.z);
-      code[p] = (uint16_t)(bx | (by << 4) | (bz << 8));
-    }
-    // neighbouring triangles (Morton order) mostly share a task and bins:
-    // lanes of one (task, bin) reduce in registers and one lane updates the
-    // bin -- in shared memory when the whole chunk is one task, else in the
-    // task's global bins
-    const uint32_t vm = __ballot_sync(0xffffffffu, valid);
-    if (valid) {
-      const uint32_t v[6] = {f2o(lo.x), f2o(lo.y), f2o(lo.z), f2o(hi.x), f2o(hi.y), f2o(hi.z)};
-      const int bins3[3] = {bx, by, bz};
-      uint32_t* dst = st != kNoTask ? sb : bins + (size_t)t * 3 * kTopBins * kTopVals;
-#pragma unroll
-      for (int ax = 0; ax < 3; ++ax) {
-        const uint32_t g = __match_any_sync(vm, t * (uint32_t)kTopBins + (uint32_t)bins3[ax]);
-        const uint32_t n_g = (uint32_t)__popc(g);
-        uint32_t r[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) r[k] = k < 3 ? __reduce_min_sync(g, v[k]) : __reduce_max_sync(g, v[k]);
-        if (lane == (uint32_t)(__ffs(g) - 1)) {
-          uint32_t* b = dst + (ax * kTopBins + bins3[ax]) * kTopVals;
-          atomicAdd(b, n_g);
-#pragma unroll
-          for (int k = 0; k < 6; ++k) {
-            if (k < 3)
-              atomicMin(b + 1 + k, r[k]);
-            else
-              atomicMax(b + 1 + k, r[k]);
-          }
-        }
-      }
-    }
-  }
-  if (st == kNoTask) return;
-  __syncthreads();
-  uint32_t* g = bins + (size_t)st * 3 * kTopBins * kTopVals;
-  for (uint32_t k = threadIdx.x; k < 3 * kTopBins * kTopVals; k += blockDim.x) {
-    const uint32_t v = k % kTopVals;
-    if (v == 0) {
-      if (sb[k]) atomicAdd(g + k, sb[k]);
-    } else if (((v - 1) % 6) < 3) {
-      atomicMin(g + k, sb[k]);
-    } else {
-      atomicMax(g + k, sb[k]);
-    }
-  }
-}
 
 __device__ __forceinline__ float box_half_area(float lx, float ly, float lz, float hx, float hy, float hz) {
   const float dx = hx - lx, dy = hy - ly, dz = hz - lz;
@@ -1394,215 +1296,420 @@ __device__ uint32_t warp_top_split(const uint32_t* B, const TopTask& T, TopSplit
   return nleft;
 }
 
-// one warp per task
-__global__ void __launch_bounds__(128) k_top_split(const TopTask* __restrict__ tasks,
-                                                   const uint32_t* __restrict__ n_tasks_p,
-                                                   const uint32_t* __restrict__ bins, TopSplit* __restrict__ splits,
-                                                   BinNode* __restrict__ box, uint32_t* __restrict__ count) {
-  const uint32_t n_tasks = *n_tasks_p;
-  for (uint32_t t = blockIdx.x * 4u + (threadIdx.x >> 5); t < n_tasks; t += gridDim.x * 4u) {  // whole warps
-    const TopTask T = tasks[t];
-    warp_top_split(bins + (size_t)t * 3 * kTopBins * kTopVals, T, splits + t, box, count);
+// Work of a level: items of at most `chunk` positions of one task. A task's
+// items are consecutive; a task of one item is split and partitioned by the
+// block that bins it.
+struct TopItem {
+  uint32_t task, first;  // the task's first item
+  uint32_t begin, n;     // positions
+};
+static const int kLevelThreads = 256;
+static const uint32_t kTopBinWords = 3 * kTopBins * kTopVals;
+
+__device__ __forceinline__ uint32_t top_bin_empty(uint32_t k) {  // word k of a task's empty bins
+  const uint32_t v = k % kTopVals;
+  return v == 0 ? 0u : (v < 4 ? 0xffffffffu : 0u);  // lo fields: max code, hi fields: 0
+}
+
+// the first level: the root task's items and empty bins
+__global__ void k_top_items(TopItem* __restrict__ items, uint32_t* __restrict__ bins, uint32_t nt, uint32_t chunk) {
+  const uint32_t n_items = (nt + chunk - 1) / chunk;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_items; i += gridDim.x * blockDim.x)
+    items[i] = TopItem{0u, 0u, i * chunk, min(chunk, nt - i * chunk)};
+  if (blockIdx.x == 0)
+    for (uint32_t k = threadIdx.x; k < kTopBinWords; k += blockDim.x) bins[k] = top_bin_empty(k);
+}
+
+// adds a box of ordered-float codes (n of them) to a bin
+__device__ __forceinline__ void bin_update(uint32_t* b, uint32_t n, const uint32_t (&v)[6]) {
+  atomicAdd(b, n);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) atomicMin(b + 1 + k, v[k]);
+#pragma unroll
+  for (int k = 3; k < 6; ++k) atomicMax(b + 1 + k, v[k]);
+}
+
+// the same to the three bins of a code
+__device__ __forceinline__ void bin_update3(uint32_t* __restrict__ bins, uint32_t code, uint32_t n, const uint32_t (&v)[6]) {
+#pragma unroll
+  for (uint32_t ax = 0; ax < 3; ++ax)
+    bin_update(bins + (ax * kTopBins + ((code >> (4 * ax)) & 15u)) * kTopVals, n, v);
+}
+
+// a run of the binning: the code that a thread's last positions share and what
+// they gathered (boxes without NaN, whose minima and maxima order as their
+// codes do)
+struct BinRun {
+  uint32_t at;  // the code, or kNoTask
+  uint32_t n;
+  float v[6];
+  __device__ __forceinline__ void flush(uint32_t* __restrict__ bins) const {
+    if (at == kNoTask) return;
+    const uint32_t c[6] = {f2o(v[0]), f2o(v[1]), f2o(v[2]), f2o(v[3]), f2o(v[4]), f2o(v[5])};
+    bin_update3(bins, at, n, c);
   }
-}
-
-// 1 if position p (of task t) goes left: its bin on the split axis (the
-// bin codes that binning wrote: 4 bits per axis) is at most the split bin,
-// or, for a split by position, it lies in the first nleft positions
-__device__ __forceinline__ uint32_t top_goes_left(uint32_t p, uint32_t code, const TopTask& T, const TopSplit& S) {
-  if (S.axis < 3) return ((code >> (4 * S.axis)) & 15u) <= S.bin ? 1u : 0u;
-  return (p - T.begin) < S.nleft ? 1u : 0u;
-}
-
-// the flags of the stable partition and the first phase of their exclusive
-// scan in one pass: each chunk of 1024 positions (256 threads x 4) scans its
-// flags into pscan and writes its total to sums (scanned by k_scan_sums;
-// k_top_scatter adds a chunk's offset itself)
-__global__ void __launch_bounds__(256) k_top_flag_scan(const uint32_t* __restrict__ task_of,
-                                                       const uint16_t* __restrict__ code,
-                                                       const TopTask* __restrict__ tasks,
-                                                       const TopSplit* __restrict__ splits,
-                                                       const uint32_t* __restrict__ n_tasks_p, uint32_t n,
-                                                       uint32_t* __restrict__ pscan, uint32_t* __restrict__ sums) {
-  __shared__ uint32_t wsum[8];
-  const uint32_t n_tasks = *n_tasks_p;
-  if (n_tasks == 0) return;  // no level
-  const uint32_t base = blockIdx.x * 1024u + threadIdx.x * 4u;
-  uint32_t f[4] = {0u, 0u, 0u, 0u}, tk[4] = {kNoTask, kNoTask, kNoTask, kNoTask}, cd[4] = {0u, 0u, 0u, 0u};
-  if (base + 3 < n) {  // task_of, code: 16- and 8-byte aligned groups of 4
-    const uint4 t4 = *reinterpret_cast<const uint4*>(task_of + base);
-    const uint2 c4 = *reinterpret_cast<const uint2*>(code + base);
-    tk[0] = t4.x, tk[1] = t4.y, tk[2] = t4.z, tk[3] = t4.w;
-    cd[0] = c4.x & 0xffffu, cd[1] = c4.x >> 16, cd[2] = c4.y & 0xffffu, cd[3] = c4.y >> 16;
-  } else {
-    for (uint32_t k = 0; k < 4 && base + k < n; ++k) {
-      tk[k] = task_of[base + k];
-      cd[k] = code[base + k];
+  __device__ __forceinline__ void add(uint32_t* __restrict__ bins, uint32_t code, const float (&x)[6]) {
+    if (code != at) {
+      flush(bins);
+      at = code;
+      n = 1;
+#pragma unroll
+      for (int k = 0; k < 6; ++k) v[k] = x[k];
+    } else {
+      ++n;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) v[k] = fminf(v[k], x[k]);
+#pragma unroll
+      for (int k = 3; k < 6; ++k) v[k] = fmaxf(v[k], x[k]);
     }
   }
+  // the runs of a whole warp at its end: one update per distinct code where
+  // they are few (each costs a round of reductions), else one per lane
+  __device__ __forceinline__ void flush_warp(uint32_t* __restrict__ bins) const {
+    const uint32_t g = __match_any_sync(0xffffffffu, at), lane = threadIdx.x & 31u;
+    const bool leader = lane == (uint32_t)__ffs(g) - 1u;
+    if (__popc(__ballot_sync(0xffffffffu, leader)) > 8) {
+      flush(bins);
+      return;
+    }
+    const uint32_t c[6] = {f2o(v[0]), f2o(v[1]), f2o(v[2]), f2o(v[3]), f2o(v[4]), f2o(v[5])};
+    uint32_t r[6];
 #pragma unroll
-  for (int k = 0; k < 4; ++k)
-    if (tk[k] < n_tasks) f[k] = top_goes_left(base + k, cd[k], tasks[tk[k]], splits[tk[k]]);
-  const uint32_t tot = f[0] + f[1] + f[2] + f[3];
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  uint32_t inc = tot;
+    for (int k = 0; k < 3; ++k) r[k] = __reduce_min_sync(g, c[k]);
+#pragma unroll
+    for (int k = 3; k < 6; ++k) r[k] = __reduce_max_sync(g, c[k]);
+    const uint32_t m = __reduce_add_sync(g, n);
+    if (at != kNoTask && leader) bin_update3(bins, at, m, r);
+  }
+};
+
+// the exclusive scan of per-pass, per-warp counts in s_cnt[K][8] (in place), by the first warp
+template <int K>
+__device__ __forceinline__ void scan_counts(uint32_t* s_cnt) {
+  constexpr uint32_t n = K * (kLevelThreads / 32);
+  static_assert(n <= 64, "two counts a lane");
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t x = lane < n ? s_cnt[lane] : 0u, y = lane + 32u < n ? s_cnt[lane + 32u] : 0u;
+  uint32_t xi = x, yi = y;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= (uint32_t)o) inc += y;
+    const uint32_t u = __shfl_up_sync(0xffffffffu, xi, o), v = __shfl_up_sync(0xffffffffu, yi, o);
+    if (lane >= (uint32_t)o) {
+      xi += u;
+      yi += v;
+    }
   }
-  if (lane == 31) wsum[warp] = inc;
+  const uint32_t half = __shfl_sync(0xffffffffu, xi, 31);
+  if (lane < n) s_cnt[lane] = xi - x;
+  if (lane + 32u < n) s_cnt[lane + 32u] = half + yi - y;
+}
+
+// 1 if a position (the k-th of task T) goes left: its bin on the split axis
+// (the bin codes that binning wrote: 4 bits per axis) is at most the split
+// bin, or, for a split by position, it lies in the first nleft positions
+__device__ __forceinline__ bool top_goes_left(uint32_t k, uint32_t code, const TopSplit& S) {
+  return S.axis < 3 ? ((code >> (4 * S.axis)) & 15u) <= S.bin : k < S.nleft;
+}
+
+// Stable partition of an item's n positions (from position p0 of its task,
+// which begins at `begin`): left0 of the task's earlier positions go left.
+// Whole block; code_of(k), ord_of(k): the k-th position's.
+template <int K, class Code, class Ord>
+__device__ __forceinline__ void partition_item(const TopSplit& S, uint32_t begin, uint32_t p0, uint32_t n, uint32_t end,
+                                               uint32_t left0, uint32_t* s_cnt, Code code_of, Ord ord_of,
+                                               uint32_t* __restrict__ ord2, uint32_t* status) {
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  uint32_t f = 0, o[K];  // the order is fetched with the codes: one wait for both
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    const uint32_t k = (uint32_t)j * kLevelThreads + tid;
+    o[j] = k < n ? ord_of(k) : 0u;
+  }
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    const uint32_t k = (uint32_t)j * kLevelThreads + tid;
+    const bool left = k < n && top_goes_left(p0 + k, code_of(k), S);
+    f |= (left ? 1u : 0u) << j;
+    const uint32_t c = __popc(__ballot_sync(0xffffffffu, left));
+    if (lane == 0) s_cnt[j * (kLevelThreads / 32) + warp] = c;
+  }
   __syncthreads();
-  uint32_t woff = 0, all = 0;
+  if (warp == 0) scan_counts<K>(s_cnt);
+  __syncthreads();
 #pragma unroll
-  for (uint32_t w = 0; w < 8; ++w) {
-    const uint32_t x = wsum[w];
-    woff += w < warp ? x : 0u;
-    all += x;
-  }
-  const uint32_t e = woff + inc - tot;
-  const uint4 o4 = make_uint4(e, e + f[0], e + f[0] + f[1], e + f[0] + f[1] + f[2]);
-  if (base + 3 < n) {
-    *reinterpret_cast<uint4*>(pscan + base) = o4;
-  } else {
-    if (base < n) pscan[base] = o4.x;
-    if (base + 1 < n) pscan[base + 1] = o4.y;
-    if (base + 2 < n) pscan[base + 2] = o4.z;
-  }
-  if (threadIdx.x == 0) sums[blockIdx.x] = all;
-}
-
-// stable partition of every active task's range: the lefts before p within
-// its task are the exclusive scan (chunk scan + chunk offset) at p minus that
-// at the task's first position; task_of2 gets each position's task of the
-// next level
-__global__ void __launch_bounds__(256) k_top_scatter(const uint32_t* __restrict__ ord, uint32_t* __restrict__ ord2,
-                                                     const uint32_t* __restrict__ task_of,
-                                                     uint32_t* __restrict__ task_of2, const uint16_t* __restrict__ code,
-                                                     const TopTask* __restrict__ tasks,
-                                                     const TopSplit* __restrict__ splits,
-                                                     const uint32_t* __restrict__ n_tasks_p,
-                                                     const uint32_t* __restrict__ pscan,
-                                                     const uint32_t* __restrict__ sums, uint32_t n, uint32_t* status) {
-  const uint32_t n_tasks = *n_tasks_p;
-  if (n_tasks == 0) return;  // no level: the order stays where it is
-  // 4 consecutive positions per thread (one chunk of the scan: base is a multiple of 4)
-  const uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) * 4u;
-  if (base >= n) return;
-  uint32_t tk[4] = {kNoTask, kNoTask, kNoTask, kNoTask}, cd[4] = {0u, 0u, 0u, 0u}, ps[4] = {0u, 0u, 0u, 0u},
-           od[4] = {0u, 0u, 0u, 0u};
-  const uint32_t m = min(4u, n - base);
-  if (m == 4) {
-    const uint4 t4 = *reinterpret_cast<const uint4*>(task_of + base);
-    const uint2 c4 = *reinterpret_cast<const uint2*>(code + base);
-    const uint4 p4 = *reinterpret_cast<const uint4*>(pscan + base);
-    const uint4 o4 = *reinterpret_cast<const uint4*>(ord + base);
-    tk[0] = t4.x, tk[1] = t4.y, tk[2] = t4.z, tk[3] = t4.w;
-    cd[0] = c4.x & 0xffffu, cd[1] = c4.x >> 16, cd[2] = c4.y & 0xffffu, cd[3] = c4.y >> 16;
-    ps[0] = p4.x, ps[1] = p4.y, ps[2] = p4.z, ps[3] = p4.w;
-    od[0] = o4.x, od[1] = o4.y, od[2] = o4.z, od[3] = o4.w;
-  } else {
-    for (uint32_t k = 0; k < m; ++k) {
-      tk[k] = task_of[base + k];
-      cd[k] = code[base + k];
-      ps[k] = pscan[base + k];
-      od[k] = ord[base + k];
-    }
-  }
-  const uint32_t chunk_off = sums[base >> 10];
-#pragma unroll
-  for (uint32_t k = 0; k < 4; ++k) {
-    if (k >= m) break;
-    const uint32_t p = base + k, t = tk[k];
-    uint32_t d = p, next = kNoTask;
-    if (t < n_tasks) {
-      const TopTask T = tasks[t];
-      const TopSplit S = splits[t];
-      const uint32_t f = top_goes_left(p, cd[k], T, S);
-      // lefts before p within its task: the exclusive scan at p minus that at the task's first position
-      const uint32_t l = (ps[k] + chunk_off) - (pscan[T.begin] + sums[T.begin >> 10]);
-      d = f ? T.begin + l : T.begin + S.nleft + (p - T.begin - l);
-      next = S.task[f ? 0 : 1];
-      if (d < T.begin || d >= T.end) {
-        atomicOr(status, J3DG_DEV_BAD_INDEX);
-        continue;
-      }
-    }
-    ord2[d] = od[k];
-    task_of2[d] = next;
+  for (int j = 0; j < K; ++j) {
+    const uint32_t k = (uint32_t)j * kLevelThreads + tid;
+    const bool left = (f >> j) & 1u;
+    const uint32_t bal = __ballot_sync(0xffffffffu, left);
+    if (k >= n) continue;
+    const uint32_t l = left0 + s_cnt[j * (kLevelThreads / 32) + warp] + __popc(bal & ((1u << lane) - 1u));
+    const uint32_t d = begin + (left ? l : S.nleft + (p0 + k - l));
+    if (d < end)
+      ord2[d] = o[j];
+    else
+      atomicOr(status, J3DG_DEV_BAD_INDEX);
   }
 }
 
-// children of every task: a task of the next level above kSmallTask
-// triangles, a small task above J3DG_SAH_TOP, else a finished range; the
-// task's own node goes under its parent and into the list of top nodes
-// counters: [0] top nodes, [1] next tasks, [2] ranges, [3] small tasks
-__device__ __forceinline__ void top_children_of(const TopTask* __restrict__ tasks, TopSplit* __restrict__ splits,
-                                                uint32_t t, uint32_t* __restrict__ counters,
-                                                TopTask* __restrict__ next, TopTask* __restrict__ small,
-                                                TopRange* __restrict__ ranges, uint32_t* __restrict__ list,
-                                                uint2* __restrict__ child, uint32_t* __restrict__ root,
-                                                uint32_t cap_tasks, uint32_t cap_small, uint32_t nt, uint32_t* status) {
-  const TopTask T = tasks[t];
-  TopSplit S = splits[t];
-  const uint32_t n = T.end - T.begin, nl = S.nleft;
-  S.task[0] = S.task[1] = kNoTask;
-  if (nl == 0 || nl >= n) {  // cannot happen: both sides of a split are non-empty
-    atomicOr(status, J3DG_DEV_BAD_INDEX);
-    splits[t] = S;
-    return;
-  }
-  const uint32_t node = T.begin + nl;
-  const uint32_t k = atomicAdd(counters + 0, 1u);
-  if (k < nt)
-    list[k] = node;
-  else
-    atomicOr(status, J3DG_DEV_BAD_INDEX);
-  link_child(child, root, T.parent, T.side, node);
-  for (uint32_t side = 0; side < 2; ++side) {
-    const uint32_t b = side ? node : T.begin, e = side ? T.end : node;
-    const uint32_t tag = side | (((T.side >> 1) + 1u) << 1);
-    if (e - b > J3DG_SAH_TOP) {
-      TopTask C;
-      C.begin = b;
-      C.end = e;
-      C.parent = node;
-      C.side = tag;
-      C.clo = side ? S.rclo : S.lclo;
-      C.chi = side ? S.rchi : S.lchi;
-      const bool again = e - b > kSmallTask;
-      const uint32_t q = atomicAdd(counters + (again ? 1 : 3), 1u);
-      if (q >= (again ? cap_tasks : cap_small)) {
-        atomicOr(status, J3DG_DEV_BAD_INDEX);
-        continue;
+// Bins the items of a level. The item's boxes are staged in shared memory
+// (neighbouring threads fetch neighbouring positions), then every thread bins
+// a run of consecutive positions: in Morton order they mostly share their
+// bins, so a run is gathered in registers and its bin updated when it ends.
+// The bins of a task of several items are merged in global memory, and each
+// item leaves its counts of bins 0..b per axis (icum, one row per axis and
+// bin), from which its lefts follow for any split; a task of one item is
+// split and partitioned here.
+//
+// Bound: 32 B of box and 4 of order in, 2 or 4 out per triangle; staging them
+// alone takes 8.9 ps a triangle (2.1M triangles in one task, 4.7 TB/s), the
+// whole kernel 13.4, at 3000-triangle tasks 21. One update of the bins per
+// run, and of all three axes together, is what counts: a run per axis took
+// 17.6, the same with a bin's values encoded for every triangle and runs read
+// across the banks 19.6. The pass that binned whole chunks of positions, with
+// one warp reduction per 32 triangles and global atomics where a chunk held
+// two tasks, took 0.43 ms a level at 28.09M triangles and, with the passes for
+// flags, scan and scatter, 0.66; this kernel, the split and the scatter take
+// 0.52. Builds of 82k / 2M / 28.09M triangles with their first frame: 1449 ->
+// 1230, 4201 -> 3729, 28412 -> 26443 us.
+// the place of an item's k-th box in shared memory: threads read runs of 2, 4
+// or 8 positions, and the low bits are mixed so that the threads of a half
+// warp meet in no bank (a run of 8 boxes of 8 bytes spans half the banks)
+__device__ __forceinline__ uint32_t top_slot(uint32_t k) { return (k & ~15u) | ((k ^ (k >> 4)) & 15u); }
+
+template <int K>
+struct TopBinMem {
+  float2 box[3][K * kLevelThreads];
+  __align__(16) uint16_t code[K * kLevelThreads];
+  uint32_t bins[kTopBinWords];
+  uint32_t cnt[64];
+  TopSplit split;
+};
+#ifndef J3DG_LEVEL_BLOCKS
+#define J3DG_LEVEL_BLOCKS 4
+#endif
+// K positions a thread: items of K * kLevelThreads
+template <int K>
+__global__ void __launch_bounds__(kLevelThreads, J3DG_LEVEL_BLOCKS) k_top_bin(
+    const uint32_t* __restrict__ ord, uint32_t* __restrict__ ord2, const BinNode* __restrict__ tbox,
+    const TopItem* __restrict__ items, const uint32_t* __restrict__ n_items_p, const TopTask* __restrict__ tasks,
+    uint32_t cap_items, uint32_t* __restrict__ bins, uint16_t* __restrict__ code, uint32_t* __restrict__ icum,
+    TopSplit* __restrict__ splits, BinNode* __restrict__ box, uint32_t* __restrict__ count, uint32_t* status) {
+  constexpr uint32_t chunk = K * kLevelThreads;
+  extern __shared__ __align__(16) uint8_t top_raw[];
+  TopBinMem<K>& s = *reinterpret_cast<TopBinMem<K>*>(top_raw);
+  uint32_t* const sb = s.bins;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t n_items = min(*n_items_p, cap_items);
+  for (uint32_t it = blockIdx.x; it < n_items; it += gridDim.x) {  // uniform over the block
+    const TopItem I = items[it];
+    const TopTask T = tasks[I.task];
+    if (tid < 3 * kTopBins)
+#pragma unroll
+      for (int v = 0; v < kTopVals; ++v) sb[tid * kTopVals + v] = top_bin_empty(v);
+    constexpr int kFlight = K < 4 ? K : 4;
+#pragma unroll
+    for (int j0 = 0; j0 < K; j0 += kFlight) {  // four boxes in flight per thread
+      uint32_t t[kFlight];
+#pragma unroll
+      for (int j = 0; j < kFlight; ++j) {
+        const uint32_t k = (uint32_t)(j0 + j) * kLevelThreads + tid;
+        t[j] = k < I.n ? ord[I.begin + k] : 0u;
       }
-      (again ? next : small)[q] = C;
-      if (again) S.task[side] = q;
+      float4 lo[kFlight], hi[kFlight];
+#pragma unroll
+      for (int j = 0; j < kFlight; ++j) {  // (a position past the item reads triangle 0's box and drops it)
+        lo[j] = tbox[t[j]].lo;
+        hi[j] = tbox[t[j]].hi;
+      }
+#pragma unroll
+      for (int j = 0; j < kFlight; ++j) {
+        const uint32_t q = top_slot((uint32_t)(j0 + j) * kLevelThreads + tid);
+        s.box[0][q] = make_float2(lo[j].x, hi[j].x);
+        s.box[1][q] = make_float2(lo[j].y, hi[j].y);
+        s.box[2][q] = make_float2(lo[j].z, hi[j].z);
+      }
+    }
+    __syncthreads();
+    {
+      TopBinner B;
+      B.set(T);
+      BinRun r;
+      r.at = kNoTask;
+      r.n = 0;
+#pragma unroll
+      for (int k = 0; k < 6; ++k) r.v[k] = 0.f;
+      const uint32_t k1 = min(I.n, tid * K + K);
+      for (uint32_t k = tid * K; k < k1; ++k) {
+        const uint32_t q = top_slot(k);
+        const float2 x = s.box[0][q], y = s.box[1][q], z = s.box[2][q];
+        const float v[6] = {x.x, y.x, z.x, x.y, y.y, z.y};
+        const float cx = 0.5f * (x.x + x.y), cy = 0.5f * (y.x + y.y), cz = 0.5f * (z.x + z.y);
+        const uint32_t cd = B.code(cx, cy, cz, T);
+        s.code[k] = (uint16_t)cd;
+        const float sum = cx + cy + cz;
+        if (!(sum == sum)) {  // a NaN (or infinities of both signs): by the codes' order, which ranks NaN too
+          const uint32_t c[6] = {f2o(v[0]), f2o(v[1]), f2o(v[2]), f2o(v[3]), f2o(v[4]), f2o(v[5])};
+          bin_update3(sb, cd, 1u, c);
+          continue;
+        }
+        r.add(sb, cd, v);
+      }
+      __syncwarp();
+      r.flush_warp(sb);
+    }
+    __syncthreads();
+    if (T.end - T.begin <= chunk) {
+      // the whole task is here
+      if (warp == 0) {
+        warp_top_split(sb, T, &s.split, box, count);
+        __syncwarp();
+        if (lane == 0) splits[I.task] = s.split;
+      }
+      __syncthreads();
+      partition_item<K>(s.split, T.begin, 0u, I.n, T.end, 0u, s.cnt, [&](uint32_t k) { return (uint32_t)s.code[k]; },
+                        [&](uint32_t k) { return ord[I.begin + k]; }, ord2, status);
     } else {
-      const uint32_t q = atomicAdd(counters + 2, 1u);
-      if (q < nt)
-        ranges[q] = TopRange{b, e, node, tag};
+      // the codes in one store a thread (2 K bytes, by item), the bins to the task's
+      constexpr int kWords = K / 2;
+      const uint32_t* cs = reinterpret_cast<const uint32_t*>(s.code) + tid * kWords;
+      uint32_t* cg = reinterpret_cast<uint32_t*>(code) + ((size_t)it * kLevelThreads + tid) * kWords;
+      if constexpr (K == 8)
+        *reinterpret_cast<uint4*>(cg) = *reinterpret_cast<const uint4*>(cs);
+      else if constexpr (K == 4)
+        *reinterpret_cast<uint2*>(cg) = *reinterpret_cast<const uint2*>(cs);
+      else
+        *cg = *cs;
+      if (tid < 3 * kTopBins) {
+        const uint32_t* b = sb + tid * kTopVals;
+        uint32_t* g = bins + (size_t)I.task * kTopBinWords + tid * kTopVals;
+        if (b[0]) {
+          const uint32_t v[6] = {b[1], b[2], b[3], b[4], b[5], b[6]};
+          bin_update(g, b[0], v);
+        }
+        uint32_t c = 0;
+        for (uint32_t k = tid & ~15u; k <= tid; ++k) c += sb[k * kTopVals];
+        icum[(size_t)tid * cap_items + it] = c;
+      }
+    }
+    __syncthreads();  // the block's memory is free for the next item
+  }
+}
+
+// one warp per task: the split of a task of several items; then the children:
+// a task of the next level above kSmallTask triangles (with its items and, if
+// they are several, empty bins), a small task above J3DG_SAH_TOP, else a
+// finished range; the task's own node goes under its parent and into the list
+// of top nodes
+// counters: [0] top nodes, [1] next tasks, [2] ranges, [3] small tasks, [4] next items
+__global__ void __launch_bounds__(128) k_top_split(
+    const TopTask* __restrict__ tasks, const uint32_t* __restrict__ n_tasks_p, uint32_t chunk,
+    const uint32_t* __restrict__ bins, uint32_t* __restrict__ bins2, TopSplit* __restrict__ splits,
+    uint32_t* __restrict__ counters, TopTask* __restrict__ next, TopItem* __restrict__ items2,
+    TopTask* __restrict__ small, TopRange* __restrict__ ranges, uint32_t* __restrict__ list, uint2* __restrict__ child,
+    uint32_t* __restrict__ root, BinNode* __restrict__ box, uint32_t* __restrict__ count, uint32_t cap_tasks,
+    uint32_t cap_small, uint32_t cap_items, uint32_t nt, uint32_t* status) {
+  const uint32_t n_tasks = min(*n_tasks_p, cap_tasks), lane = threadIdx.x & 31u;
+  for (uint32_t t = blockIdx.x * 4u + (threadIdx.x >> 5); t < n_tasks; t += gridDim.x * 4u) {  // whole warps
+    const TopTask T = tasks[t];
+    const uint32_t n = T.end - T.begin;
+    if (n > chunk) {
+      warp_top_split(bins + (size_t)t * kTopBinWords, T, splits + t, box, count);
+      __syncwarp();
+    }
+    const TopSplit S = splits[t];
+    const uint32_t nl = S.nleft;
+    if (nl == 0 || nl >= n) {  // cannot happen: both sides of a split are non-empty
+      if (lane == 0) atomicOr(status, J3DG_DEV_BAD_INDEX);
+      continue;
+    }
+    const uint32_t node = T.begin + nl;
+    if (lane == 0) {
+      const uint32_t k = atomicAdd(counters + 0, 1u);
+      if (k < nt)
+        list[k] = node;
       else
         atomicOr(status, J3DG_DEV_BAD_INDEX);
+      link_child(child, root, T.parent, T.side, node);
+    }
+    for (uint32_t side = 0; side < 2; ++side) {
+      const uint32_t b = side ? node : T.begin, e = side ? T.end : node, len = e - b;
+      const uint32_t tag = side | (((T.side >> 1) + 1u) << 1);
+      const bool again = len > kSmallTask;
+      uint32_t q = 0, i0 = 0;
+      const uint32_t m = (len + chunk - 1) / chunk;
+      if (lane == 0) {
+        if (len > J3DG_SAH_TOP) {
+          q = atomicAdd(counters + (again ? 1 : 3), 1u);
+          if (again) i0 = atomicAdd(counters + 4, m);
+          if (q >= (again ? cap_tasks : cap_small) || (again && i0 + m > cap_items)) {
+            atomicOr(status, J3DG_DEV_BAD_INDEX);
+            q = kNoTask;
+          } else {
+            TopTask C;
+            C.begin = b;
+            C.end = e;
+            C.parent = node;
+            C.side = tag;
+            C.clo = side ? S.rclo : S.lclo;
+            C.chi = side ? S.rchi : S.lchi;
+            (again ? next : small)[q] = C;
+          }
+        } else {
+          q = atomicAdd(counters + 2, 1u);
+          if (q < nt)
+            ranges[q] = TopRange{b, e, node, tag};
+          else
+            atomicOr(status, J3DG_DEV_BAD_INDEX);
+        }
+      }
+      if (!again) continue;
+      q = __shfl_sync(0xffffffffu, q, 0);
+      i0 = __shfl_sync(0xffffffffu, i0, 0);
+      if (q == kNoTask) continue;
+      for (uint32_t k = lane; k < m; k += 32u) items2[i0 + k] = TopItem{q, i0, b + k * chunk, min(chunk, len - k * chunk)};
+      if (m > 1u)
+        for (uint32_t k = lane; k < kTopBinWords; k += 32u) bins2[(size_t)q * kTopBinWords + k] = top_bin_empty(k);
     }
   }
-  splits[t] = S;
 }
 
-__global__ void k_top_children(const TopTask* __restrict__ tasks, TopSplit* __restrict__ splits,
-                               const uint32_t* __restrict__ n_tasks_p, uint32_t* __restrict__ counters,
-                               TopTask* __restrict__ next, TopTask* __restrict__ small, TopRange* __restrict__ ranges,
-                               uint32_t* __restrict__ list, uint2* __restrict__ child, uint32_t* __restrict__ root,
-                               uint32_t cap_tasks, uint32_t cap_small, uint32_t nt, uint32_t* status) {
-  const uint32_t n_tasks = *n_tasks_p;
-  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n_tasks; t += gridDim.x * blockDim.x)
-    top_children_of(tasks, splits, t, counters, next, small, ranges, list, child, root, cap_tasks, cap_small, nt,
-                    status);
-}
-
-__global__ void k_iota(uint32_t* __restrict__ a, uint32_t n) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) a[i] = i;
+// the stable partition of the tasks of several items: an item's lefts go
+// after those of the task's earlier items (a row of icum)
+template <int K>
+__global__ void __launch_bounds__(kLevelThreads) k_top_scatter(
+    const uint32_t* __restrict__ ord, uint32_t* __restrict__ ord2, const TopItem* __restrict__ items,
+    const uint32_t* __restrict__ n_items_p, const TopTask* __restrict__ tasks, uint32_t cap_items, const uint16_t* __restrict__ code, const uint32_t* __restrict__ icum, const TopSplit* __restrict__ splits,
+    uint32_t* status) {
+  constexpr uint32_t chunk = K * kLevelThreads;
+  __shared__ uint32_t s_cnt[64], s_sum[kLevelThreads / 32];
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t n_items = min(*n_items_p, cap_items);
+  for (uint32_t it = blockIdx.x; it < n_items; it += gridDim.x) {  // uniform over the block
+    const TopItem I = items[it];
+    const TopTask T = tasks[I.task];
+    if (T.end - T.begin <= chunk) continue;  // partitioned where it was binned
+    const TopSplit S = splits[I.task];
+    uint32_t before = 0;  // lefts of the task's earlier items
+    if (S.axis < 3) {
+      const uint32_t* row = icum + (size_t)(S.axis * kTopBins + S.bin) * cap_items;
+      for (uint32_t k = I.first + tid; k < it; k += kLevelThreads) before += row[k];
+      before = __reduce_add_sync(0xffffffffu, before);
+      if (lane == 0) s_sum[warp] = before;
+    }
+    __syncthreads();
+    uint32_t left0;
+    if (S.axis < 3) {
+      left0 = 0;
+#pragma unroll
+      for (int w = 0; w < kLevelThreads / 32; ++w) left0 += s_sum[w];
+    } else {
+      left0 = min(S.nleft, I.begin - T.begin);
+    }
+    partition_item<K>(S, T.begin, I.begin - T.begin, I.n, T.end, left0, s_cnt,
+                   [&](uint32_t k) { return (uint32_t)code[(size_t)it * chunk + k]; },
+                   [&](uint32_t k) { return ord[I.begin + k]; }, ord2, status);
+    __syncthreads();  // the counts are read before the next item resets them
+  }
 }
 
 // -------------------------------------------------- 5d. small tasks ----
@@ -1731,37 +1838,23 @@ __device__ int small_levels(SmallMem<W>& s, uint32_t b0, uint32_t n, uint2* __re
       __syncthreads();
       {
         uint32_t last = kNoTask;
-        float4 clo = make_float4(0.f, 0.f, 0.f, 0.f), chi = clo;
-        float sx = 0.f, sy = 0.f, sz = 0.f;
+        TopBinner B;
+        B.lx = B.ly = B.lz = B.sx = B.sy = B.sz = 0.f;
         const uint32_t q0 = min(n, (lane * kSmallWarps + warp) * K), q1 = min(n, q0 + K);  // lanes far apart
         for (uint32_t p = q0; p < q1; ++p) {
           const uint32_t t = (uint32_t)s.t.tk[cur][p] - base;  // 255: no task
           if (t >= m) continue;
           if (t != last) {
-            clo = s.task[cur][base + t].clo;
-            chi = s.task[cur][base + t].chi;
-            sx = (float)kTopBins / (chi.x - clo.x);
-            sy = (float)kTopBins / (chi.y - clo.y);
-            sz = (float)kTopBins / (chi.z - clo.z);
+            B.set(s.task[cur][base + t]);
             last = t;
           }
           const uint32_t i = s.t.ord[cur][p];
           const float2 fx = s.box[0][i], fy = s.box[1][i], fz = s.box[2][i];
           const uint32_t v[6] = {f2o(fx.x), f2o(fy.x), f2o(fz.x), f2o(fx.y), f2o(fy.y), f2o(fz.y)};
-          const int bx = top_bin_scaled(0.5f * (fx.x + fx.y), clo.x, chi.x, sx),
-                    by = top_bin_scaled(0.5f * (fy.x + fy.y), clo.y, chi.y, sy),
-                    bz = top_bin_scaled(0.5f * (fz.x + fz.y), clo.z, chi.z, sz);
-          s.t.code[p] = (uint16_t)(bx | (by << 4) | (bz << 8));
-          const int bin[3] = {bx, kTopBins + by, 2 * kTopBins + bz};
-#pragma unroll
-          for (int ax = 0; ax < 3; ++ax) {
-            uint32_t* b = s.t.bins + t * kBinWords + bin[ax] * kTopVals;
-            atomicAdd(b, 1u);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) atomicMin(b + 1 + k, v[k]);
-#pragma unroll
-            for (int k = 3; k < 6; ++k) atomicMax(b + 1 + k, v[k]);
-          }
+          const uint32_t cd = B.code(0.5f * (fx.x + fx.y), 0.5f * (fy.x + fy.y), 0.5f * (fz.x + fz.y),
+                                     s.task[cur][base + t]);
+          s.t.code[p] = (uint16_t)cd;
+          bin_update3(s.t.bins + t * kBinWords, cd, 1u, v);
         }
       }
       __syncthreads();
@@ -1803,7 +1896,7 @@ __device__ int small_levels(SmallMem<W>& s, uint32_t b0, uint32_t n, uint2* __re
     for (uint32_t p = p0; p < p1; ++p) {
       const uint32_t t = s.t.tk[cur][p];
       if (t >= nlt) continue;
-      if (top_goes_left(b0 + p, s.t.code[p], s.task[cur][t], s.split[t])) {
+      if (top_goes_left(b0 + p - s.task[cur][t].begin, s.t.code[p], s.split[t])) {
         f |= 1u << (p - p0);
         ++cnt;
       }
@@ -2063,8 +2156,7 @@ __device__ uint32_t small_cluster(SmallMem<W>& s, uint32_t b0, uint32_t m, uint3
 template <int W>
 __global__ void __launch_bounds__(kSmallThreads, W == 8 ? J3DG_SMALL_BLOCKS - 1 : J3DG_SMALL_BLOCKS)
     k_small_tasks(const uint32_t* __restrict__ ord_a, const uint32_t* __restrict__ ord_b,
-                  const uint32_t* __restrict__ parity, const float4* __restrict__ blo, const float4* __restrict__ bhi,
-                  const TopTask* __restrict__ tasks, const TopRange* __restrict__ ranges,
+                  const BinNode* __restrict__ tbox, const TopTask* __restrict__ tasks, const TopRange* __restrict__ ranges,
                   const uint32_t* __restrict__ counters, uint32_t* __restrict__ next_job, uint32_t* __restrict__ error,
                   uint32_t leaf_size, uint32_t nt, uint32_t cap_small, uint2* __restrict__ rec,
                   uint2* __restrict__ child, uint32_t* __restrict__ root, BinNode* __restrict__ box,
@@ -2073,7 +2165,6 @@ __global__ void __launch_bounds__(kSmallThreads, W == 8 ? J3DG_SMALL_BLOCKS - 1 
   SmallMem<W>& s = *reinterpret_cast<SmallMem<W>*>(small_raw);
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const uint32_t n_tasks = min(counters[3], cap_small), n_jobs = n_tasks + min(counters[2], nt);
-  const uint32_t* ord = *parity ? ord_b : ord_a;  // the final order is where the last level put it
   for (;;) {
     if (tid == 0) s.job = atomicAdd(next_job, 1u);
     __syncthreads();
@@ -2096,6 +2187,7 @@ __global__ void __launch_bounds__(kSmallThreads, W == 8 ? J3DG_SMALL_BLOCKS - 1 
       __syncthreads();
       continue;
     }
+    const uint32_t* ord = (T.side >> 1) & 1u ? ord_b : ord_a;  // the levels alternate: where the last one put the task
     if (tid == 0) {
       s.task[0][0] = T;
       s.n_task[0] = 1;
@@ -2103,7 +2195,7 @@ __global__ void __launch_bounds__(kSmallThreads, W == 8 ? J3DG_SMALL_BLOCKS - 1 
     }
     for (uint32_t p = tid; p < n; p += kSmallThreads) {
       const uint32_t t = ord[b0 + p];
-      const float4 lo = blo[t], hi = bhi[t];
+      const float4 lo = tbox[t].lo, hi = tbox[t].hi;
       s.ref[p] = t;
       s.box[0][p] = make_float2(lo.x, hi.x);
       s.box[1][p] = make_float2(lo.y, hi.y);
@@ -2266,9 +2358,9 @@ __global__ void k_slot_of(const float4* __restrict__ tris, uint32_t nt, const ui
 static const uint32_t kMaxPlaceLevels = 128;
 
 struct BuildCtl {
-  uint32_t top_ctr[4];  // k_top_children: [0] top nodes, [1] next level's tasks, [2] ranges, [3] small tasks
-                        // (LBVH: [0] the root that k_lbvh found)
-  uint32_t n_tasks, ord_parity, top_levels;
+  uint32_t top_ctr[5];  // k_top_split: [0] top nodes, [1] next level's tasks, [2] ranges, [3] small tasks,
+                        // [4] next level's items (LBVH: [0] the root that k_lbvh found)
+  uint32_t n_tasks, n_items, top_levels;
   uint32_t root;      // the binary tree's root
   uint32_t next_job;  // the next small task or range to be taken (k_small_tasks)
   uint32_t lohi[2];  // the running pass's node range (collapse costs, depth-first levels)
@@ -2282,7 +2374,8 @@ struct BuildCtl {
 
 // the root task, by its size: split level by level, by one block, or a segment
 __global__ void k_ctl_init(BuildCtl* __restrict__ c, TopTask* __restrict__ tasks, TopTask* __restrict__ small,
-                           TopRange* __restrict__ ranges, const float* __restrict__ bb, uint32_t nt, uint32_t top) {
+                           TopRange* __restrict__ ranges, const float* __restrict__ bb, uint32_t nt, uint32_t top,
+                           uint32_t chunk) {
   if (top) {
     TopTask r0;
     r0.begin = 0;
@@ -2294,6 +2387,7 @@ __global__ void k_ctl_init(BuildCtl* __restrict__ c, TopTask* __restrict__ tasks
     if (nt > kSmallTask) {
       tasks[0] = r0;
       c->n_tasks = 1;
+      c->n_items = (nt + chunk - 1) / chunk;
     } else if (nt > J3DG_SAH_TOP) {
       small[0] = r0;
       c->top_ctr[3] = 1;
@@ -2308,20 +2402,20 @@ __global__ void k_ctl_init(BuildCtl* __restrict__ c, TopTask* __restrict__ tasks
   c->level_end[0] = 1;
 }
 
-__global__ void k_top_step(BuildCtl* __restrict__ c, uint32_t cap_tasks, uint32_t cap_small, uint32_t nt,
-                           cudaGraphConditionalHandle h, uint32_t set) {
+__global__ void k_top_step(BuildCtl* __restrict__ c, uint32_t cap_tasks, uint32_t cap_small, uint32_t cap_items,
+                           uint32_t nt, cudaGraphConditionalHandle h, uint32_t set) {
   if (c->n_tasks) {  // the level ran
     uint32_t next = c->top_ctr[1];
     if (next > cap_tasks || c->top_ctr[3] > cap_small || c->top_ctr[2] > nt || c->top_ctr[0] > nt - 1 ||
-        c->top_levels >= kMaxTopLevels) {
+        c->top_ctr[4] > cap_items || c->top_levels >= kMaxTopLevels) {
       c->error |= 1u;
       next = 0;
     } else {
       c->top_end[c->top_levels++] = c->top_ctr[0];
     }
     c->n_tasks = next;
-    c->top_ctr[1] = 0;
-    c->ord_parity ^= 1u;
+    c->n_items = next ? c->top_ctr[4] : 0u;
+    c->top_ctr[1] = c->top_ctr[4] = 0;
   }
   if (set) cudaGraphSetConditional(h, c->n_tasks > 0 ? 1u : 0u);
 }
@@ -2464,10 +2558,11 @@ struct BuildPlan {
   float* bb = nullptr;
   uint64_t *k0 = nullptr, *k1 = nullptr;
   uint32_t *v0 = nullptr, *v1 = nullptr, *hist = nullptr, *sums = nullptr;
-  uint32_t *ord_a = nullptr, *ord_b = nullptr, *task_of = nullptr, *task_of2 = nullptr, *top_list = nullptr,
-           *top_bins = nullptr, *cscan = nullptr, *pl_sums = nullptr;
-  float4 *tbox_lo = nullptr, *tbox_hi = nullptr;
+  uint32_t *ord_a = nullptr, *ord_b = nullptr, *top_list = nullptr, *bins_a = nullptr, *bins_b = nullptr,
+           *icum = nullptr;
+  BinNode* tbox = nullptr;
   uint16_t* codes = nullptr;
+  TopItem *items_a = nullptr, *items_b = nullptr;
   TopTask *tasks_a = nullptr, *tasks_b = nullptr, *small = nullptr;
   TopSplit* splits = nullptr;
   TopRange* ranges = nullptr;
@@ -2491,7 +2586,12 @@ struct BuildPlan {
   uint32_t n_tiles() const { return (nt + kSortTile - 1) / kSortTile; }
   uint32_t hist_n() const { return 256 * n_tiles(); }
   uint32_t scan_blocks() const { return (hist_n() + 1023) / 1024; }
-  uint32_t sblocks() const { return (nt + 1023) / 1024; }
+  // positions per item of the SAH levels: large ones keep the runs of the
+  // binning long and the bins to merge few; below two items an SM (304 on 152
+  // SMs) smaller items fill the device instead (82k triangles: 160 items of
+  // 512; with 2048 its levels took 23 us a bin pass instead of 7)
+  uint32_t chunk() const { return nt >= 600000u ? 2048u : (nt >= 300000u ? 1024u : 512u); }
+  uint32_t cap_items() const { return nt / chunk() + cap_tasks() + 1; }
 };
 
 static const int kBBoxBlocks = 1024;
@@ -2516,15 +2616,16 @@ static cudaError_t plan_alloc(BuildPlan& P, cudaStream_t st, bool outputs = true
   if (P.need_ploc) {
     A(P.ord_a, sizeof(uint32_t) * nt);
     A(P.ord_b, sizeof(uint32_t) * nt);
-    A(P.task_of, sizeof(uint32_t) * nt);
-    A(P.task_of2, sizeof(uint32_t) * nt);
-    A(P.tbox_lo, sizeof(float4) * nt);
-    A(P.tbox_hi, sizeof(float4) * nt);
-    A(P.codes, sizeof(uint16_t) * nt);
-    A(P.cscan, sizeof(uint32_t) * nt);
-    A(P.pl_sums, sizeof(uint32_t) * (P.sblocks() + 1));
+    A(P.tbox, sizeof(BinNode) * nt);
+    // (a lane's smaller meshes may have more items, of smaller chunks)
+    const uint32_t items = std::max(P.cap_items(), std::min(P.nt, 600000u) / 512u + P.cap_tasks() + 1);
+    A(P.codes, sizeof(uint16_t) * std::max((size_t)P.cap_items() * P.chunk(), (size_t)items * 512));
     A(P.top_list, sizeof(uint32_t) * nt);
-    A(P.top_bins, sizeof(uint32_t) * (size_t)P.cap_tasks() * 3 * kTopBins * kTopVals);
+    A(P.bins_a, sizeof(uint32_t) * (size_t)P.cap_tasks() * kTopBinWords);
+    A(P.bins_b, sizeof(uint32_t) * (size_t)P.cap_tasks() * kTopBinWords);
+    A(P.icum, sizeof(uint32_t) * (size_t)items * 3 * kTopBins);
+    A(P.items_a, sizeof(TopItem) * items);
+    A(P.items_b, sizeof(TopItem) * items);
     A(P.tasks_a, sizeof(TopTask) * P.cap_tasks());
     A(P.tasks_b, sizeof(TopTask) * P.cap_tasks());
     A(P.small, sizeof(TopTask) * P.cap_small());
@@ -2561,8 +2662,8 @@ static cudaError_t plan_alloc(BuildPlan& P, cudaStream_t st, bool outputs = true
 
 // frees the scratch (outputs the caller took over are null)
 static void plan_free(BuildPlan& P, cudaStream_t st) {
-  void* ps[] = {P.part, P.bb, P.k0, P.k1, P.v0, P.v1, P.hist, P.sums, P.ord_a, P.ord_b, P.task_of, P.task_of2,
-                P.cscan, P.pl_sums, P.top_list, P.top_bins, P.tbox_lo, P.tbox_hi, P.codes, P.tasks_a, P.tasks_b,
+  void* ps[] = {P.part, P.bb, P.k0, P.k1, P.v0, P.v1, P.hist, P.sums, P.ord_a, P.ord_b, P.top_list, P.bins_a,
+                P.bins_b, P.icum, P.items_a, P.items_b, P.tbox, P.codes, P.tasks_a, P.tasks_b,
                 P.small, P.splits, P.ranges, P.child, P.box, P.count, P.dp_cost, P.dp_dec, P.wide, P.pa, P.pb, P.range,
                 P.qa, P.qb, P.dfs_size, P.dfs_pos, P.ctl, P.normals, P.soup, P.tris_out, P.nodes, P.slot_of};
   for (void* p : ps)
@@ -2575,6 +2676,43 @@ static void plan_free(BuildPlan& P, cudaStream_t st) {
     if (e == cudaSuccess) e = (x);                \
     if (e == cudaSuccess) e = cudaGetLastError(); \
   } while (0)
+
+// a level's items, a block at a time: as many blocks as are resident or the
+// level can have items
+template <int K>
+static void launch_top_bin_k(BuildPlan& P, cudaStream_t s, const uint32_t* oi, uint32_t* oo, const TopItem* items,
+                             const TopTask* tasks, uint32_t* bins, uint32_t* d_status) {
+  BuildCtl* c = P.ctl;
+  const uint32_t blocks = std::min(wave_blocks128() / 16u * J3DG_LEVEL_BLOCKS, P.cap_items());
+  cudaFuncSetAttribute(k_top_bin<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TopBinMem<K>));
+  k_top_bin<K><<<blocks, kLevelThreads, sizeof(TopBinMem<K>), s>>>(oi, oo, P.tbox, items, &c->n_items, tasks,
+                                                                   P.cap_items(), bins, P.codes, P.icum, P.splits, P.box,
+                                                                   P.count, d_status);
+}
+static void launch_top_bin(BuildPlan& P, cudaStream_t s, const uint32_t* oi, uint32_t* oo, const TopItem* items,
+                           const TopTask* tasks, uint32_t* bins, uint32_t* d_status) {
+  switch (P.chunk() / kLevelThreads) {
+    case 8: return launch_top_bin_k<8>(P, s, oi, oo, items, tasks, bins, d_status);
+    case 4: return launch_top_bin_k<4>(P, s, oi, oo, items, tasks, bins, d_status);
+    default: return launch_top_bin_k<2>(P, s, oi, oo, items, tasks, bins, d_status);
+  }
+}
+
+static void launch_top_scatter(BuildPlan& P, cudaStream_t s, const uint32_t* oi, uint32_t* oo, const TopItem* items,
+                               const TopTask* tasks, uint32_t* d_status) {
+  BuildCtl* c = P.ctl;
+  const uint32_t blocks = std::min(wave_blocks128() / 2u, P.cap_items()), cap = P.cap_items();
+  switch (P.chunk() / kLevelThreads) {
+    case 8:
+      k_top_scatter<8><<<blocks, kLevelThreads, 0, s>>>(oi, oo, items, &c->n_items, tasks, cap, P.codes, P.icum, P.splits, d_status);
+      break;
+    case 4:
+      k_top_scatter<4><<<blocks, kLevelThreads, 0, s>>>(oi, oo, items, &c->n_items, tasks, cap, P.codes, P.icum, P.splits, d_status);
+      break;
+    default:
+      k_top_scatter<2><<<blocks, kLevelThreads, 0, s>>>(oi, oo, items, &c->n_items, tasks, cap, P.codes, P.icum, P.splits, d_status);
+  }
+}
 
 // section 5d over every small task and range: persistent blocks, as many as
 // the device holds at the kernel's shared memory
@@ -2590,7 +2728,7 @@ static cudaError_t launch_small_tasks_w(BuildPlan& P, cudaStream_t st, uint32_t*
   if (e != cudaSuccess) return e;
   const uint32_t grid = std::min((uint32_t)std::max(1, sms * per), P.cap_small());
   k_small_tasks<W><<<grid, kSmallThreads, smem, st>>>(
-      P.ord_a, P.ord_b, &c->ord_parity, P.tbox_lo, P.tbox_hi, P.small, P.ranges, c->top_ctr, &c->next_job, &c->error,
+      P.ord_a, P.ord_b, P.tbox, P.small, P.ranges, c->top_ctr, &c->next_job, &c->error,
       P.leaf, P.nt, P.cap_small(), reinterpret_cast<uint2*>(P.pb), P.child, &c->root, P.box, P.count, P.dp_cost, P.dp_dec,
       d_status);
   return cudaGetLastError();
@@ -2611,31 +2749,26 @@ static cudaError_t enqueue_tree_ploc(BuildPlan& P, cudaStream_t st, cudaStream_t
   BuildCtl* c = P.ctl;
   cudaError_t e = cudaSuccess;
   const float4* soup = P.soup;
-  k_top_boxes<<<(nt + 255) / 256, 256, 0, st>>>(soup, nt, P.tbox_lo, P.tbox_hi);
-  k_iota<<<(nt + 255) / 256, 256, 0, st>>>(P.ord_a, nt);
+  k_top_boxes<<<(nt + 255) / 256, 256, 0, st>>>(soup, nt, P.tbox, P.ord_a);
   J3DG_EQ(cudaSuccess);
   if (nt > kSmallTask) {
-    J3DG_EQ(cudaMemsetAsync(P.task_of, 0, sizeof(uint32_t) * nt, st));
-    // one SAH level: tasks ti, order oi, task of each position si -> the next level's
-    auto level = [&](cudaStream_t s, TopTask* ti, TopTask* to, uint32_t* oi, uint32_t* oo, uint32_t* si,
-                     uint32_t* so) {
-      k_top_bins_init<<<kStrideBlocks, 256, 0, s>>>(P.top_bins, &c->n_tasks);
-      k_top_bin<<<(nt + kTopChunk - 1) / kTopChunk, 256, 0, s>>>(oi, P.tbox_lo, P.tbox_hi, si, ti, &c->n_tasks, nt,
-                                                                 P.top_bins, P.codes);
-      k_top_split<<<kStrideBlocks, 128, 0, s>>>(ti, &c->n_tasks, P.top_bins, P.splits, P.box, P.count);
-      k_top_children<<<kStrideBlocks, 128, 0, s>>>(ti, P.splits, &c->n_tasks, c->top_ctr, to, P.small, P.ranges,
-                                                   P.top_list, P.child, &c->root, P.cap_tasks(), P.cap_small(), nt,
-                                                   d_status);
-      k_top_flag_scan<<<P.sblocks(), 256, 0, s>>>(si, P.codes, ti, P.splits, &c->n_tasks, nt, P.cscan, P.pl_sums);
-      k_scan_sums<<<1, 1024, 0, s>>>(P.pl_sums, nullptr, P.sblocks(), nullptr);
-      k_top_scatter<<<(nt + 1023) / 1024, 256, 0, s>>>(oi, oo, si, so, P.codes, ti, P.splits, &c->n_tasks, P.cscan,
-                                                       P.pl_sums, nt, d_status);
+    const uint32_t chunk = P.chunk();
+    k_top_items<<<std::min(kStrideBlocks, P.cap_items() / 256 + 1), 256, 0, st>>>(P.items_a, P.bins_a, nt, chunk);
+    const uint32_t split_blocks = std::min(kStrideBlocks, P.cap_tasks() / 4u + 1u);
+    // one SAH level: tasks ti, items ii, bins bi, order oi -> the next level's
+    auto level = [&](cudaStream_t s, TopTask* ti, TopTask* to, TopItem* ii, TopItem* io, uint32_t* bi, uint32_t* bo,
+                     uint32_t* oi, uint32_t* oo) {
+      launch_top_bin(P, s, oi, oo, ii, ti, bi, d_status);
+      k_top_split<<<split_blocks, 128, 0, s>>>(ti, &c->n_tasks, chunk, bi, bo, P.splits, c->top_ctr, to, io, P.small,
+                                               P.ranges, P.top_list, P.child, &c->root, P.box, P.count, P.cap_tasks(),
+                                               P.cap_small(), P.cap_items(), nt, d_status);
+      launch_top_scatter(P, s, oi, oo, ii, ti, d_status);
     };
     J3DG_EQ(capture_while(st, side, [&](cudaStream_t s, cudaGraphConditionalHandle h) {
-      level(s, P.tasks_a, P.tasks_b, P.ord_a, P.ord_b, P.task_of, P.task_of2);
-      k_top_step<<<1, 1, 0, s>>>(c, P.cap_tasks(), P.cap_small(), nt, h, 0u);
-      level(s, P.tasks_b, P.tasks_a, P.ord_b, P.ord_a, P.task_of2, P.task_of);
-      k_top_step<<<1, 1, 0, s>>>(c, P.cap_tasks(), P.cap_small(), nt, h, 1u);
+      level(s, P.tasks_a, P.tasks_b, P.items_a, P.items_b, P.bins_a, P.bins_b, P.ord_a, P.ord_b);
+      k_top_step<<<1, 1, 0, s>>>(c, P.cap_tasks(), P.cap_small(), P.cap_items(), nt, h, 0u);
+      level(s, P.tasks_b, P.tasks_a, P.items_b, P.items_a, P.bins_b, P.bins_a, P.ord_b, P.ord_a);
+      k_top_step<<<1, 1, 0, s>>>(c, P.cap_tasks(), P.cap_small(), P.cap_items(), nt, h, 1u);
     }));
   }
   J3DG_EQ(launch_small_tasks(W, P, st, d_status));
@@ -2698,7 +2831,7 @@ static cudaError_t enqueue_prefix(BuildPlan& P, const float* dV, const uint32_t*
   J3DG_EQ(cudaMemsetAsync(c, 0, sizeof(BuildCtl), st));
   k_bbox_partial<<<kBBoxBlocks, 256, 0, st>>>(dV, nv, P.part);
   k_bbox_final<<<1, 32, 0, st>>>(P.part, kBBoxBlocks, P.bb);
-  k_ctl_init<<<1, 1, 0, st>>>(c, P.tasks_a, P.small, P.ranges, P.bb, nt, P.top ? 1u : 0u);
+  k_ctl_init<<<1, 1, 0, st>>>(c, P.tasks_a, P.small, P.ranges, P.bb, nt, P.top ? 1u : 0u, P.chunk());
   k_tri_prep<<<(nt + 255) / 256, 256, 0, st>>>(dV, nv, dT, nt, P.bb, P.normals, P.k0, P.v0, d_status);
   J3DG_EQ(cudaSuccess);
   {
@@ -2708,7 +2841,7 @@ static cudaError_t enqueue_prefix(BuildPlan& P, const float* dV, const uint32_t*
       const int shift = 8 * pass;
       k_radix_hist<<<P.n_tiles(), kSortThreads, 0, st>>>(ka, nt, shift, P.n_tiles(), P.hist);
       k_scan_chunks<<<P.scan_blocks(), 256, 0, st>>>(P.hist, P.hist, P.hist_n(), P.sums);
-      k_scan_sums<<<1, 1024, 0, st>>>(P.sums, nullptr, P.scan_blocks(), nullptr);
+      k_scan_sums<<<1, 1024, 0, st>>>(P.sums, P.scan_blocks());
       k_radix_scatter<<<P.n_tiles(), kSortThreads, 0, st>>>(ka, va, kb, vb, nt, shift, P.n_tiles(), P.hist, P.sums,
                                                            d_status);
       std::swap(ka, kb);
