@@ -250,6 +250,15 @@ int upload_instances(j3dg_ctx* c, const j3dg_instance* objs, uint32_t n, const D
   return J3DG_OK;
 }
 
+// A scene of one object needs no table: its record goes with the kernel's
+// parameters. Checks the object as upload_instances does.
+int one_instance(j3dg_ctx* c, const j3dg_instance* obj, DevInst* out) {
+  if (!obj->mesh) return fail(c, J3DG_ERR_INVALID_ARGUMENT, "instance without a mesh");
+  if (obj->mesh->ctx != c) return fail(c, J3DG_ERR_INVALID_ARGUMENT, "mesh belongs to another context");
+  *out = to_dev(*obj);
+  return J3DG_OK;
+}
+
 int check_status(j3dg_ctx* c) {
   uint32_t st = 0;
   CK(c, cudaMemcpyAsync(&st, c->d_status, sizeof(st), cudaMemcpyDeviceToHost, S(c)), "status");
@@ -387,10 +396,29 @@ bool raster_layout(FrameParams& P, j3dg_canvas* cv, uint32_t n, uint32_t id_bits
   return true;
 }
 
+// A traced frame's objects: the only one by value, or the table of several.
+// (Frames that may be rasterised use the table, which their kernels read.)
+struct SceneRef {
+  const DevInst* table = nullptr;
+  bool top = false, embedded = false;
+  DevInst one;
+  void put(FrameParams& P) const {
+    P.top = top ? 1u : 0u;
+    P.embedded = embedded ? 1u : 0u;
+    if (embedded) P.one = one;
+  }
+};
+
+int scene_ref(j3dg_ctx* c, const j3dg_scene* s, SceneRef& R) {
+  const int mode = all(c)->ex.primary_mode;
+  R.embedded = s->n_objects == 1 && (mode == J3DG_PRIMARY_TRACE || (mode == J3DG_PRIMARY_AUTO && !kAutoRaster));
+  return R.embedded ? one_instance(c, s->objects, &R.one) : upload_instances(c, s->objects, s->n_objects, &R.table, &R.top);
+}
+
 void setup_raster(FrameParams& P, j3dg_canvas* cv, const j3dg_scene* s) {
   const int mode = all(cv->ctx)->ex.primary_mode;
   cv->last_primary = J3DG_PRIMARY_TRACE;
-  if (mode == J3DG_PRIMARY_TRACE || !s || s->n_objects == 0 || P.x1 < P.x0 || P.y1 < P.y0) return;
+  if (P.embedded || mode == J3DG_PRIMARY_TRACE || !s || s->n_objects == 0 || P.x1 < P.x0 || P.y1 < P.y0) return;
   const uint32_t n = s->n_objects;
   uint64_t total = 0;
   uint32_t max_nt = 0;
@@ -491,22 +519,28 @@ void canvas_writable(j3dg_canvas* cv) {
 // node-visit / triangle-test counters while counting is on, else null
 unsigned long long* ctx_counters(j3dg_ctx* c) { return all(c)->ex.counting ? all(c)->ex.d_counters : nullptr; }
 
-// The device instance table of one mesh with the identity transform.
-int mesh_devinst(j3dg_ctx* c, const j3dg_mesh* mesh, const DevInst** out) {
-  if (mesh->ctx != c) return fail(c, J3DG_ERR_INVALID_ARGUMENT, "mesh of another context");
+static j3dg_instance identity_instance(const j3dg_mesh* mesh) {
   j3dg_instance one;
   one.mesh = mesh;
   for (int i = 0; i < 16; ++i) one.cs[i] = (i % 5 == 0) ? 1.f : 0.f;
   one.db_id = 0;
   one.reserved = 0;
+  return one;
+}
+
+// The device instance table of one mesh with the identity transform.
+int mesh_devinst(j3dg_ctx* c, const j3dg_mesh* mesh, const DevInst** out) {
+  if (mesh->ctx != c) return fail(c, J3DG_ERR_INVALID_ARGUMENT, "mesh of another context");
+  const j3dg_instance one = identity_instance(mesh);
   return upload_instances(c, &one, 1, out);
 }
 
 // Plain closest hit of device rays against one mesh into device hits (async).
 int ray_query_device(j3dg_ctx* c, const j3dg_mesh* mesh, const j3dg_ray* d_rays, uint32_t n, j3dg_hit* d_hits) {
-  const DevInst* dinst = nullptr;
-  if (int rc = mesh_devinst(c, mesh, &dinst)) return rc;
-  CK(c, launch_rays(dinst, 1, false, (int)mesh->width, d_rays, n, d_hits, false, all(c)->ex.d_ray_counter, c->d_status,
+  j3dg_instance obj = identity_instance(mesh);
+  DevInst one;
+  if (int rc = one_instance(c, &obj, &one)) return rc;
+  CK(c, launch_rays(nullptr, &one, 1, false, (int)mesh->width, d_rays, n, d_hits, false, all(c)->ex.d_ray_counter, c->d_status,
                     nullptr, S(c)),
      "ray query");
   return J3DG_OK;
@@ -980,8 +1014,9 @@ static int ray_query(j3dg_ctx* c, const j3dg_instance* objs, uint32_t n_obj, con
   if (!c || (n && (!rays || !hits)) || (n_obj && !objs)) return J3DG_ERR_INVALID_ARGUMENT;
   cudaSetDevice(c->device);
   const DevInst* dinst = nullptr;
+  DevInst one;
   bool top = false;
-  int rc = upload_instances(c, objs, n_obj, &dinst, &top);
+  int rc = n_obj == 1 ? one_instance(c, objs, &one) : upload_instances(c, objs, n_obj, &dinst, &top);
   if (rc) return rc;
   if (n == 0) return J3DG_OK;
   const bool rays_dev = is_device_ptr(rays), hits_dev = is_device_ptr(hits);
@@ -992,7 +1027,7 @@ static int ray_query(j3dg_ctx* c, const j3dg_instance* objs, uint32_t n_obj, con
     CK(c, cudaMemcpyAsync(dr, rays, sizeof(j3dg_ray) * (size_t)n, cudaMemcpyHostToDevice, S(c)), "rays");
   }
   if (!hits_dev) CK(c, cudaMallocAsync((void**)&dh, sizeof(j3dg_hit) * (size_t)n, S(c)), "hits");
-  CK(c, j3dg::launch_rays(dinst, n_obj, top, n_obj ? (int)objs[0].mesh->width : 4, dr, n, dh, any,
+  CK(c, j3dg::launch_rays(dinst, n_obj == 1 ? &one : nullptr, n_obj, top, n_obj ? (int)objs[0].mesh->width : 4, dr, n, dh, any,
                           all(c)->ex.d_ray_counter, c->d_status, j3dg::ctx_counters(c),
                           S(c)),
      "find");
@@ -1267,9 +1302,8 @@ int j3dg_canvas_update_canvas(j3dg_canvas* cv, int x0, int y0, int x1, int y1, c
   if (cv->w == 0 || cv->h == 0) return J3DG_OK;
   cudaSetDevice(c->device);
   j3dg::canvas_writable(cv);
-  const DevInst* dinst = nullptr;
-  bool top = false;
-  if (int rc = upload_instances(c, s->objects, s->n_objects, &dinst, &top)) return rc;
+  SceneRef R;
+  if (int rc = scene_ref(c, s, R)) return rc;
   // canvas.cpp:681-698: clamp the rectangle
   const int w = (int)cv->w, h = (int)cv->h;
   auto clampv = [](int v, int hi) { return v < 0 ? 0 : (v >= hi ? hi - 1 : v); };
@@ -1278,8 +1312,8 @@ int j3dg_canvas_update_canvas(j3dg_canvas* cv, int x0, int y0, int x1, int y1, c
   x1 = clampv(x1, w);
   y1 = clampv(y1, h);
   FrameParams P;
-  fill_frame(P, cv, s, dinst, nullptr);
-  P.top = top ? 1u : 0u;
+  fill_frame(P, cv, s, R.table, nullptr);
+  R.put(P);
   next_frame_seq(P, cv);  // its counters; a rectangle writes no stamps and does not overlap
   P.x0 = x0;
   P.y0 = y0;
@@ -1349,10 +1383,9 @@ int j3dg_canvas_render_frame(j3dg_canvas* cv, const j3dg_scene* s, const j3dg_ma
   const bool after_frame = c->stream_ops == X.frame_ops || cv->expect_stamps;
   cv->expect_stamps = false;
   j3dg::canvas_writable(cv);
-  const DevInst* dinst = nullptr;
-  bool top = false;
+  SceneRef R;
   if (s)
-    if (int rc = upload_instances(c, s->objects, s->n_objects, &dinst, &top)) return rc;
+    if (int rc = scene_ref(c, s, R)) return rc;
   const int mode = shade_mode_of(cv->settings);
   if (!s) {
     const size_t n = (size_t)cv->w * cv->h;
@@ -1361,8 +1394,8 @@ int j3dg_canvas_render_frame(j3dg_canvas* cv, const j3dg_scene* s, const j3dg_ma
     return J3DG_OK;
   }
   FrameParams P;
-  fill_frame(P, cv, s, dinst, m);
-  P.top = top ? 1u : 0u;
+  fill_frame(P, cv, s, R.table, m);
+  R.put(P);
   setup_raster(P, cv, s);
   next_frame_seq(P, cv);
   // a traced frame in one kernel (plain shading) stamps its pixels and may

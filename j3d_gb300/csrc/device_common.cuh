@@ -350,8 +350,13 @@ __device__ __forceinline__ void sort_children(float (&tc)[W], uint32_t (&rc)[W])
 #undef J3DG_CX
 }
 
-template <int N, bool TOP = false, int W = 4>
+// ONE: the scene is one object, whose record comes by value with the kernel's
+// parameters (insts points there): its arrays are then read from the constant
+// bank in every step instead of being kept in registers, and the frame needs
+// no instance table in device memory.
+template <int N, bool TOP = false, int W = 4, bool ONE = false>
 struct TracerT {
+  static_assert(!(TOP && ONE), "one object has no top level");
 #if J3DG_COLD_SMEM & 1
   // world ray: read only when an object's walk starts, kept in shared memory
   __device__ __forceinline__ float& wr(int k) { return ColdSlots<N>::ray()[k * ColdSlots<N>::S + threadIdx.x]; }
@@ -371,10 +376,12 @@ struct TracerT {
   uint32_t budget;
 
   __device__ __forceinline__ void start_object(const DevInst* __restrict__ insts) {
-    const DevInst& I = insts[inst];
+    const DevInst& I = insts[ONE ? 0u : inst];
     if (I.width != (uint32_t)W) {  // a tree of another width: walk nothing (the host never launches that)
-      nodes = nullptr;
-      n_nodes = 0;
+      if (!ONE) {
+        nodes = nullptr;
+        n_nodes = 0;
+      }
       cur = J3DG_EMPTY_REF;
       budget = 0;
       return;
@@ -382,12 +389,14 @@ struct TracerT {
     float4 o = mat_vec(I.inv, wr(0), wr(1), wr(2), 1.f);
     float4 d = mat_vec(I.inv, wr(3), wr(4), wr(5), 0.f);
     r = make_ray(o.x, o.y, o.z, d.x, d.y, d.z, r.t_near, I.scale);
-    nodes = I.nodes;
-    tris = I.tris;
-    n_nodes = I.n_nodes;
-    nt = I.nt;
+    if (!ONE) {
+      nodes = I.nodes;
+      tris = I.tris;
+      n_nodes = I.n_nodes;
+      nt = I.nt;
+    }
     cur = I.root_ref;
-    budget = n_nodes + 1;
+    budget = I.n_nodes + 1;
   }
 
   // the top level with the world ray; its slab test is padded by
@@ -430,7 +439,7 @@ struct TracerT {
       start_top(insts, H.n_nodes + 1);
       cur = H.root;
     } else {
-      inst = 0;
+      if (!ONE) inst = 0;
       start_object(insts);
     }
     return false;
@@ -453,6 +462,7 @@ struct TracerT {
   __device__ __forceinline__ bool step(const DevInst* __restrict__ insts, uint32_t n_inst, uint32_t* status,
                                        uint32_t& visits, uint32_t& tests, uint2* __restrict__ stack) {
     {
+      const uint32_t c_nt = ONE ? insts[0].nt : nt, c_nodes = ONE ? insts[0].n_nodes : n_nodes;
       if (cur == J3DG_EMPTY_REF) {
         bool got = false;
         while (sp > 0) {
@@ -469,7 +479,7 @@ struct TracerT {
           }
         }
         if (!got) {
-          if (TOP) return true;
+          if (TOP || ONE) return true;
           if (++inst >= n_inst) return true;
           start_object(insts);
           return false;
@@ -477,7 +487,7 @@ struct TracerT {
       }
       if (cur & J3DG_LEAF_BIT) {
         const uint32_t first = (cur & 0x7fffffffu) >> 3, cnt = (cur & 7u) + 1u;
-        if (first + cnt > nt) {
+        if (first + cnt > (TOP ? nt : c_nt)) {
           atomicOr(status, J3DG_DEV_BAD_INDEX);
           return true;
         }
@@ -496,7 +506,7 @@ struct TracerT {
 #pragma unroll 1
         for (uint32_t k = 0; k < cnt; ++k) {
           ++tests;
-          if (tri_test(r, tris, first + k, inst, b, any) && any) return true;
+          if (tri_test(r, ONE ? insts[0].tris : tris, first + k, ONE ? 0u : inst, b, any) && any) return true;
         }
         cur = J3DG_EMPTY_REF;
         return false;
@@ -505,12 +515,12 @@ struct TracerT {
         atomicOr(status, J3DG_DEV_VISIT_CAP);
         return true;
       }
-      if (cur >= n_nodes) {
+      if (cur >= (TOP ? n_nodes : c_nodes)) {
         atomicOr(status, J3DG_DEV_BAD_INDEX);
         return true;
       }
       ++visits;
-      const float4* nd = nodes + J3DG_NODE_F4(W) * (size_t)cur;
+      const float4* nd = (ONE ? insts[0].nodes : nodes) + J3DG_NODE_F4(W) * (size_t)cur;
       // near / far planes by the ray's octant: the same values slab() selects,
       // picked by the load offsets instead of per-child selects
       NodeLoad<W> L;
@@ -548,8 +558,9 @@ struct TracerT {
       if (cur != J3DG_EMPTY_REF && !(TOP && inst == kTopInst)) {
         const bool leaf = (cur & J3DG_LEAF_BIT) != 0;
         const uint32_t first = (cur & 0x7fffffffu) >> 3;
-        if (leaf ? first + (cur & 7u) + 1u <= nt : cur < n_nodes) {  // the checks the next step makes
-          const float4* line = leaf ? tris + 3 * (size_t)first : nodes + J3DG_NODE_F4(W) * (size_t)cur;
+        if (leaf ? first + (cur & 7u) + 1u <= (TOP ? nt : c_nt) : cur < (TOP ? n_nodes : c_nodes)) {  // the checks the next step makes
+          const float4* line = leaf ? (ONE ? insts[0].tris : tris) + 3 * (size_t)first
+                                    : (ONE ? insts[0].nodes : nodes) + J3DG_NODE_F4(W) * (size_t)cur;
           asm volatile("prefetch.global.L1 [%0];" ::"l"(line));
         }
       }
@@ -565,11 +576,11 @@ struct TracerT {
 // (returns false when the item needs no tracing and was handled) and
 // finish(); ITERS node/leaf steps run between refills.
 // N: the kernel's block size.
-template <int ITERS, int N, bool TOP, int W, class Src>
+template <int ITERS, int N, bool TOP, int W, bool ONE = false, class Src>
 __device__ __forceinline__ void persistent_trace(Src& src, const DevInst* __restrict__ insts, uint32_t n_inst,
                                                  uint32_t* counter, uint32_t* status,
                                                  unsigned long long* counters) {
-  TracerT<N, TOP, W> T;
+  TracerT<N, TOP, W, ONE> T;
   uint2 stack[J3DG_STACK];
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t n = src.count();

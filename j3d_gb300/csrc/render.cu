@@ -310,11 +310,17 @@ __device__ __forceinline__ void primary_ray(const FrameParams& P, int x, int y, 
 
 __device__ __forceinline__ float primary_t_near(const FrameParams& P) { return __fdiv_rn(P.diagonal, 100.f); }
 
-template <class Tracer>
+// the frame's objects: its instance table, or the one object in its parameters
+template <bool ONE>
+__device__ __forceinline__ const DevInst* frame_insts(const FrameParams& P) {
+  return ONE ? &P.one : P.inst;
+}
+
+template <bool ONE = false, class Tracer>
 __device__ __forceinline__ void primary_begin(const FrameParams& P, Tracer& T, int x, int y) {
   float4 o, d;
   primary_ray(P, x, y, o, d);
-  T.begin(P.inst, P.n_inst, o.x, o.y, o.z, d.x, d.y, d.z, primary_t_near(P), FLT_MAX, false);
+  T.begin(frame_insts<ONE>(P), P.n_inst, o.x, o.y, o.z, d.x, d.y, d.z, primary_t_near(P), FLT_MAX, false);
 }
 
 
@@ -326,7 +332,7 @@ __device__ __forceinline__ float4 light_position(const FrameParams& P) {
 
 // Writes the hit record; returns true and sets up the shadow ray in T when
 // one is needed. w0 / su / sv keep what the final colour needs.
-template <class Tracer>
+template <bool ONE = false, class Tracer>
 __device__ __forceinline__ bool primary_finish(const FrameParams& P, Tracer& T, size_t pix, uint32_t& w0, float& su,
                                                float& sv) {
   await_pixel(P, pix);
@@ -336,7 +342,7 @@ __device__ __forceinline__ bool primary_finish(const FrameParams& P, Tracer& T, 
     return false;
   }
   j3dg_pixel* rec = P.gbuf + pix;
-  const DevInst& I = P.inst[b.inst()];
+  const DevInst& I = frame_insts<ONE>(P)[ONE ? 0u : b.inst()];
   // canvas.cpp:788-801
   const float4 N = __ldg(I.normals + b.tri());
   float4 n = mat_vec(P.cs_inv, N.x, N.y, N.z, 0.f);
@@ -402,7 +408,7 @@ __device__ __forceinline__ bool primary_finish(const FrameParams& P, Tracer& T, 
   const float px = fa(fa(fm(V0.x, wgt), fm(b.u(), V1.x)), fm(b.v(), V2.x));
   const float py = fa(fa(fm(V0.y, wgt), fm(b.u(), V1.y)), fm(b.v(), V2.y));
   const float pz = fa(fa(fm(V0.z, wgt), fm(b.u(), V1.z)), fm(b.v(), V2.z));
-  T.begin(P.inst, P.n_inst, px, py, pz, fs(light.x, px), fs(light.y, py), fs(light.z, pz), 1e-3f, FLT_MAX, true);
+  T.begin(frame_insts<ONE>(P), P.n_inst, px, py, pz, fs(light.x, px), fs(light.y, py), fs(light.z, pz), 1e-3f, FLT_MAX, true);
   return true;
 }
 
@@ -868,10 +874,10 @@ __global__ void __launch_bounds__(kTraceThreads, J3DG_TRACE_MINBLOCKS) k_shadow(
   persistent_trace<kIters, kTraceThreads, TOP, kWidth>(src, P.inst, P.n_inst, P.work + 2, P.status, P.counters);
 }
 
-template <bool kThroughput, bool TOP>
+template <bool kThroughput, bool TOP, bool ONE>
 __global__ void __launch_bounds__(kFrameThreads, kThroughput ? kFrameBlocksT : kFrameBlocksL)
-    k_frame(const FrameParams P) {
-  TracerT<kFrameThreads, TOP, kWidth> T;
+    k_frame(const __grid_constant__ FrameParams P) {
+  TracerT<kFrameThreads, TOP, kWidth, ONE> T;
   uint2 stack[J3DG_STACK];
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t n = primary_count(P);
@@ -891,7 +897,7 @@ __global__ void __launch_bounds__(kFrameThreads, kThroughput ? kFrameBlocksT : k
   auto finish = [&](int ph) {
     bool last;
     if (ph == 1 || ph == 3) {
-      phase = primary_finish(P, T, pix, w0, su, sv) ? 2 : 0;
+      phase = primary_finish<ONE>(P, T, pix, w0, su, sv) ? 2 : 0;
       last = phase == 0;
     } else {
       shadow_finish(P, T, pix, w0, su, sv);
@@ -923,7 +929,7 @@ __global__ void __launch_bounds__(kFrameThreads, kThroughput ? kFrameBlocksT : k
             write_miss(P, pix);
             stamp_pixel(P, pix);
           } else {
-            primary_begin(P, T, x, y);
+            primary_begin<ONE>(P, T, x, y);
             phase = 1;
           }
         }
@@ -937,7 +943,7 @@ __global__ void __launch_bounds__(kFrameThreads, kThroughput ? kFrameBlocksT : k
     // all lanes step together; leave to refill once enough lanes are idle
 #pragma unroll 1
     for (;;) {
-      if ((phase == 1 || phase == 2) && T.step(P.inst, P.n_inst, P.status, visits, tests, stack)) {
+      if ((phase == 1 || phase == 2) && T.step(frame_insts<ONE>(P), P.n_inst, P.status, visits, tests, stack)) {
 #if J3DG_DEFER_FINISH
         phase += 2;
 #else
@@ -986,13 +992,13 @@ struct BatchSrc {
   }
 };
 
-template <bool ANY, bool TOP>
-__global__ void __launch_bounds__(kTraceThreads) k_rays(const DevInst* __restrict__ inst, uint32_t n_inst,
-                                                        const j3dg_ray* __restrict__ rays, uint32_t n,
-                                                        j3dg_hit* __restrict__ hits, uint32_t* counter,
-                                                        uint32_t* status, unsigned long long* counters) {
+template <bool ANY, bool TOP, bool ONE>
+__global__ void __launch_bounds__(kTraceThreads)
+    k_rays(const DevInst* __restrict__ inst, const __grid_constant__ DevInst one, uint32_t n_inst,
+           const j3dg_ray* __restrict__ rays, uint32_t n, j3dg_hit* __restrict__ hits, uint32_t* counter,
+           uint32_t* status, unsigned long long* counters) {
   BatchSrc<ANY> src{rays, hits, n};
-  persistent_trace<kIters, kTraceThreads, TOP, kWidth>(src, inst, n_inst, counter, status, counters);
+  persistent_trace<kIters, kTraceThreads, TOP, kWidth, ONE>(src, ONE ? &one : inst, n_inst, counter, status, counters);
 }
 
 // Many frames (canvases, scenes, cameras, resolutions of uneven size) in one
@@ -1285,8 +1291,9 @@ __global__ void k_init_pixels(j3dg_pixel* __restrict__ G, size_t n) {
 
 // k_frame, as a programmatic dependent of the previous kernel on the stream
 // when the frame overlaps its canvas's previous frame
-template <bool kT, bool TOP>
-static cudaError_t launch_frame(int blocks, const FrameParams& P, bool overlap, cudaStream_t st) {
+template <bool kT, bool TOP, bool ONE>
+static cudaError_t launch_frame(const FrameParams& P, bool overlap, cudaStream_t st) {
+  static const int blocks = persistent_blocks(k_frame<kT, TOP, ONE>, kFrameThreads);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)blocks);
   cfg.blockDim = dim3((unsigned)kFrameThreads);
@@ -1297,19 +1304,12 @@ static cudaError_t launch_frame(int blocks, const FrameParams& P, bool overlap, 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = overlap ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, k_frame<kT, TOP>, P);
+  return cudaLaunchKernelEx(&cfg, k_frame<kT, TOP, ONE>, P);
 }
 
 cudaError_t launch_render(const FrameParams& P, cudaStream_t st) {
   const int rw = P.x1 - P.x0 + 1, rh = P.y1 - P.y0 + 1;
   if (rw <= 0 || rh <= 0) return cudaSuccess;
-  static int blocks_t = 0, blocks_l = 0, blocks_tt = 0, blocks_lt = 0;
-  if (!blocks_t) {
-    blocks_t = persistent_blocks(k_frame<true, false>, kFrameThreads);
-    blocks_l = persistent_blocks(k_frame<false, false>, kFrameThreads);
-    blocks_tt = persistent_blocks(k_frame<true, true>, kFrameThreads);
-    blocks_lt = persistent_blocks(k_frame<false, true>, kFrameThreads);
-  }
   // an overlapped frame finds its counter slot zeroed by the slot's
   // previous user (completed before this frame could start); any other
   // frame zeroes the canvas's slots here
@@ -1343,17 +1343,12 @@ cudaError_t launch_render(const FrameParams& P, cudaStream_t st) {
     // k_frame below returns at once unless the large-triangle list overflowed
   }
   const bool thr = primary_items(P) >= J3DG_THROUGHPUT_ITEMS;
-  if (P.top) {
-    if (thr)
-      e = launch_frame<true, true>(blocks_tt, P, overlap, st);
-    else
-      e = launch_frame<false, true>(blocks_lt, P, overlap, st);
-  } else {
-    if (thr)
-      e = launch_frame<true, false>(blocks_t, P, overlap, st);
-    else
-      e = launch_frame<false, false>(blocks_l, P, overlap, st);
-  }
+  if (P.embedded)
+    e = thr ? launch_frame<true, false, true>(P, overlap, st) : launch_frame<false, false, true>(P, overlap, st);
+  else if (P.top)
+    e = thr ? launch_frame<true, true, false>(P, overlap, st) : launch_frame<false, true, false>(P, overlap, st);
+  else
+    e = thr ? launch_frame<true, false, false>(P, overlap, st) : launch_frame<false, false, false>(P, overlap, st);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
@@ -1439,29 +1434,27 @@ cudaError_t launch_frame_from_hits(const FrameParams& P, const j3dg_hit* hits, c
   return cudaGetLastError();
 }
 
-cudaError_t launch_rays(const DevInst* inst, uint32_t n_inst, bool top, int, const j3dg_ray* rays, uint32_t n,
-                        j3dg_hit* hits, bool any, uint32_t* counter, uint32_t* status, unsigned long long* counters,
-                        cudaStream_t st) {
+template <bool ANY, bool TOP, bool ONE>
+static cudaError_t launch_rays_k(const DevInst* inst, const DevInst* one, uint32_t n_inst, const j3dg_ray* rays,
+                                 uint32_t n, j3dg_hit* hits, uint32_t* counter, uint32_t* status,
+                                 unsigned long long* counters, cudaStream_t st) {
+  static const int blocks = persistent_blocks(k_rays<ANY, TOP, ONE>);
+  const DevInst none = {};
+  k_rays<ANY, TOP, ONE><<<blocks, kTraceThreads, 0, st>>>(inst, one ? *one : none, n_inst, rays, n, hits, counter,
+                                                          status, counters);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_rays(const DevInst* inst, const DevInst* one, uint32_t n_inst, bool top, int, const j3dg_ray* rays,
+                        uint32_t n, j3dg_hit* hits, bool any, uint32_t* counter, uint32_t* status,
+                        unsigned long long* counters, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  static int blocks_c = 0, blocks_a = 0;
-  if (!blocks_c) {
-    blocks_c = persistent_blocks(k_rays<false, false>);
-    blocks_a = persistent_blocks(k_rays<true, false>);
-  }
   cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(uint32_t), st);
   if (e != cudaSuccess) return e;
-  if (top) {
-    if (any)
-      k_rays<true, true><<<blocks_a, kTraceThreads, 0, st>>>(inst, n_inst, rays, n, hits, counter, status, counters);
-    else
-      k_rays<false, true><<<blocks_c, kTraceThreads, 0, st>>>(inst, n_inst, rays, n, hits, counter, status, counters);
-  } else {
-    if (any)
-      k_rays<true, false><<<blocks_a, kTraceThreads, 0, st>>>(inst, n_inst, rays, n, hits, counter, status, counters);
-    else
-      k_rays<false, false><<<blocks_c, kTraceThreads, 0, st>>>(inst, n_inst, rays, n, hits, counter, status, counters);
-  }
-  return cudaGetLastError();
+  auto go = [&](auto k) { return k(inst, one, n_inst, rays, n, hits, counter, status, counters, st); };
+  if (one) return any ? go(launch_rays_k<true, false, true>) : go(launch_rays_k<false, false, true>);
+  if (top) return any ? go(launch_rays_k<true, true, false>) : go(launch_rays_k<false, true, false>);
+  return any ? go(launch_rays_k<true, false, false>) : go(launch_rays_k<false, false, false>);
 }
 
 }  // namespace J3DG_WNS

@@ -4,10 +4,9 @@
 #include <stdint.h>
 
 #include "../../include/j3dg.h"
+#include "device_common.cuh"
 
 namespace j3dg {
-
-struct DevInst;
 
 // Primary hits by conservative rasterisation (FrameParams::raster): per
 // instance, the object -> clip matrix of the frame's camera and the slab
@@ -80,6 +79,9 @@ struct FrameParams {
   // had completed)
   uint32_t* ring;
   uint32_t launch;
+  // a scene of one object: its record by value (embedded = 1, inst unused)
+  uint32_t embedded;
+  DevInst one;
 };
 static const uint32_t kFrameDepth = 4;                     // frame kernels in flight at most
 static const uint32_t kCanvasWorkWords = 4 + 2 * kFrameDepth;  // FrameParams::work
@@ -103,8 +105,9 @@ cudaError_t launch_frame_from_hits(const FrameParams& P, const j3dg_hit* hits, c
 cudaError_t launch_copy_u32(uint32_t* dst, const uint32_t* src, size_t n, cudaStream_t st);
 cudaError_t launch_clear_ids(j3dg_pixel* G, size_t n, cudaStream_t st);
 cudaError_t launch_init_pixels(j3dg_pixel* G, size_t n, cudaStream_t st);
-cudaError_t launch_rays(const DevInst* inst, uint32_t n_inst, bool top, int width, const j3dg_ray* rays, uint32_t n,
-                        j3dg_hit* hits, bool any, uint32_t* counter, uint32_t* status, unsigned long long* counters,
-                        cudaStream_t st);
+// one: the only object's record (host memory; inst is then unused), or null
+cudaError_t launch_rays(const DevInst* inst, const DevInst* one, uint32_t n_inst, bool top, int width,
+                        const j3dg_ray* rays, uint32_t n, j3dg_hit* hits, bool any, uint32_t* counter, uint32_t* status,
+                        unsigned long long* counters, cudaStream_t st);
 
 }  // namespace j3dg

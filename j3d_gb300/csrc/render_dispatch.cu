@@ -19,9 +19,9 @@ namespace j3dg {
   cudaError_t launch_copy_u32(uint32_t* dst, const uint32_t* src, size_t n, cudaStream_t st);                     \
   cudaError_t launch_clear_ids(j3dg_pixel* G, size_t n, cudaStream_t st);                                         \
   cudaError_t launch_init_pixels(j3dg_pixel* G, size_t n, cudaStream_t st);                                       \
-  cudaError_t launch_rays(const DevInst* inst, uint32_t n_inst, bool top, int width, const j3dg_ray* rays,        \
-                          uint32_t n, j3dg_hit* hits, bool any, uint32_t* counter, uint32_t* status,              \
-                          unsigned long long* counters, cudaStream_t st);
+  cudaError_t launch_rays(const DevInst* inst, const DevInst* one, uint32_t n_inst, bool top, int width,          \
+                          const j3dg_ray* rays, uint32_t n, j3dg_hit* hits, bool any, uint32_t* counter,          \
+                          uint32_t* status, unsigned long long* counters, cudaStream_t st);
 
 namespace w2 {
 J3DG_RENDER_DECLS
@@ -56,13 +56,13 @@ cudaError_t launch_frame_from_hits(const FrameParams& P, const j3dg_hit* hits, c
   return w4::launch_frame_from_hits(P, hits, st);
 }
 
-cudaError_t launch_rays(const DevInst* inst, uint32_t n_inst, bool top, int width, const j3dg_ray* rays, uint32_t n,
-                        j3dg_hit* hits, bool any, uint32_t* counter, uint32_t* status, unsigned long long* counters,
-                        cudaStream_t st) {
-  if (width == 2) return w2::launch_rays(inst, n_inst, top, 2, rays, n, hits, any, counter, status, counters, st);
-  if (width == 8) return w8::launch_rays(inst, n_inst, top, 8, rays, n, hits, any, counter, status, counters, st);
+cudaError_t launch_rays(const DevInst* inst, const DevInst* one, uint32_t n_inst, bool top, int width,
+                        const j3dg_ray* rays, uint32_t n, j3dg_hit* hits, bool any, uint32_t* counter, uint32_t* status,
+                        unsigned long long* counters, cudaStream_t st) {
+  if (width == 2) return w2::launch_rays(inst, one, n_inst, top, 2, rays, n, hits, any, counter, status, counters, st);
+  if (width == 8) return w8::launch_rays(inst, one, n_inst, top, 8, rays, n, hits, any, counter, status, counters, st);
   if (width != 4) return cudaErrorInvalidValue;
-  return w4::launch_rays(inst, n_inst, top, 4, rays, n, hits, any, counter, status, counters, st);
+  return w4::launch_rays(inst, one, n_inst, top, 4, rays, n, hits, any, counter, status, counters, st);
 }
 
 uint32_t primary_items(const FrameParams& P) { return w4::primary_items(P); }
