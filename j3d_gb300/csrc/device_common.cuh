@@ -281,10 +281,9 @@ __device__ __forceinline__ bool tri_test(const Ray& r, const float4* __restrict_
 // world boxes) with the world ray; a top-level leaf pushes a kPopTop entry
 // (which carries the top level's remaining visit budget) and enters its
 // object; popping that entry takes the world ray back to the top level.
-// Without TOP the objects are walked one after the other. run() advances by
-// at most `iters` node or leaf steps, so persistent warps can refill lanes
-// whose rays have finished. Corrupt trees raise status bits instead of
-// trapping.
+// Without TOP the objects are walked one after the other. step() advances by
+// one node or leaf, so persistent warps can refill lanes whose rays have
+// finished. Corrupt trees raise status bits instead of trapping.
 // Child c's near / far planes of a width-W node for the ray's octant, and
 // its ref (the layout of J3DG_NODE_F4; the same values slab() selects).
 template <int W>
@@ -447,16 +446,7 @@ struct TracerT {
 
   // stack: the caller's per-thread traversal stack of (ref, entry t bits)
   // pairs, one 8-byte access per push or pop (kept out of the struct so
-  // that its scalar state can stay in registers)
-  __device__ __forceinline__ bool run(const DevInst* __restrict__ insts, uint32_t n_inst, int iters,
-                                      uint32_t* status, uint32_t& visits, uint32_t& tests,
-                                      uint2* __restrict__ stack) {
-#pragma unroll 1
-    for (int it = 0; it < iters; ++it)
-      if (step(insts, n_inst, status, visits, tests, stack)) return true;
-    return false;
-  }
-
+  // that its scalar state can stay in registers).
   // One traversal step: a pop, a leaf (its triangles, or with TOP an
   // object entered) or a node. Returns true when the ray is finished.
   __device__ __forceinline__ bool step(const DevInst* __restrict__ insts, uint32_t n_inst, uint32_t* status,
@@ -574,9 +564,10 @@ struct TracerT {
 // fetch"): every lane whose ray finished takes the next work item; the warp
 // fetches for all such lanes with one atomic. Src supplies count(), begin()
 // (returns false when the item needs no tracing and was handled) and
-// finish(); ITERS node/leaf steps run between refills.
+// finish(). All lanes step together; a lane whose ray finished waits until
+// REFILL lanes are idle, and those finish and refill together.
 // N: the kernel's block size.
-template <int ITERS, int N, bool TOP, int W, bool ONE = false, class Src>
+template <int REFILL, int N, bool TOP, int W, bool ONE = false, class Src>
 __device__ __forceinline__ void persistent_trace(Src& src, const DevInst* __restrict__ insts, uint32_t n_inst,
                                                  uint32_t* counter, uint32_t* status,
                                                  unsigned long long* counters) {
@@ -584,32 +575,35 @@ __device__ __forceinline__ void persistent_trace(Src& src, const DevInst* __rest
   uint2 stack[J3DG_STACK];
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t n = src.count();
-  int64_t idx = -1;
-  bool exhausted = false;
+  uint32_t idx = 0;
+  int phase = 0;  // 0 idle, 1 tracing, 2 finished, 3 no items left
   uint32_t visits = 0, tests = 0;
 #pragma unroll 1
   for (;;) {
-    const bool need = idx < 0 && !exhausted;
-    const uint32_t m = __ballot_sync(0xffffffffu, need);
+    if (phase == 2) {
+      src.finish(T, idx);
+      phase = 0;
+    }
+    const uint32_t m = __ballot_sync(0xffffffffu, phase == 0);
     if (m) {
       const int leader = __ffs(m) - 1;
       uint32_t base = 0;
       if ((int)lane == leader) base = atomicAdd(counter, (uint32_t)__popc(m));
       base = __shfl_sync(0xffffffffu, base, leader);
-      if (need) {
-        const uint32_t my = base + __popc(m & ((1u << lane) - 1u));
-        if (my < n) {
-          idx = my;
-          if (!src.begin(T, insts, n_inst, my)) idx = -1;  // handled without tracing
-        } else {
-          exhausted = true;
-        }
+      if (phase == 0) {
+        idx = base + __popc(m & ((1u << lane) - 1u));
+        if (idx >= n)
+          phase = 3;
+        else if (src.begin(T, insts, n_inst, idx))
+          phase = 1;  // else: handled without tracing
       }
     }
-    if (__all_sync(0xffffffffu, idx < 0 && exhausted)) break;
-    if (idx >= 0 && T.run(insts, n_inst, ITERS, status, visits, tests, stack)) {
-      src.finish(T, (uint32_t)idx);
-      idx = -1;
+    if (__all_sync(0xffffffffu, phase == 3)) break;
+#pragma unroll 1
+    for (;;) {
+      if (phase == 1 && T.step(insts, n_inst, status, visits, tests, stack)) phase = 2;
+      if (__all_sync(0xffffffffu, phase != 1)) break;
+      if (__popc(__ballot_sync(0xffffffffu, phase == 0 || phase == 2)) >= REFILL) break;
     }
   }
   if (counters) {

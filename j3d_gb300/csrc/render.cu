@@ -235,9 +235,9 @@ __device__ __forceinline__ void frame_exit(const FrameParams& P, bool handed_ove
 #ifndef J3DG_TRACE_MINBLOCKS
 #define J3DG_TRACE_MINBLOCKS 6
 #endif
-// A frame (or batch) of fewer primary items than J3DG_THROUGHPUT_ITEMS runs
-// the latency build instead: 5 blocks per SM with the pixel state in
-// registers. Measured on single frames: below about one 1920x1080 frame the
+// A batch of fewer primary items than J3DG_THROUGHPUT_ITEMS runs the latency
+// build instead: 5 blocks per SM with the pixel state in registers (single
+// frames: kTierItems below). Measured on single frames: below about one 1920x1080 frame the
 // extra warps of the throughput build lengthen the frame (a 512x512 frame
 // of the 28M-triangle torus 0.80 -> 0.89 ms); from there on they shorten it.
 #ifndef J3DG_LATENCY_MINBLOCKS
@@ -246,8 +246,15 @@ __device__ __forceinline__ void frame_exit(const FrameParams& P, bool handed_ove
 #ifndef J3DG_THROUGHPUT_ITEMS
 #define J3DG_THROUGHPUT_ITEMS 2000000u
 #endif
-#ifndef J3DG_TRACE_ITERS
-#define J3DG_TRACE_ITERS 16
+// the same for ray batches and shadow jobs (a million incoherent rays on 2M
+// triangles: 4 lanes 525 us, 8 506, 12 504, 16 508; any hit: 469, 442, 447,
+// 446; 24 objects: 809, 807, 825, 848; letting each lane run 16 steps on its
+// own between refills 516), with 28 warps an SM (32: 508, any hit 458)
+#ifndef J3DG_RAY_REFILL
+#define J3DG_RAY_REFILL 8
+#endif
+#ifndef J3DG_RAY_BLOCKS
+#define J3DG_RAY_BLOCKS 7
 #endif
 // idle lanes that make a warp stop tracing and fetch new pixels (16: with
 // overlapped frames and in batches; 12 was best for frames run one by one,
@@ -263,7 +270,6 @@ __device__ __forceinline__ void frame_exit(const FrameParams& P, bool handed_ove
 #define J3DG_DEFER_FINISH 1
 #endif
 static const int kTraceThreads = J3DG_TRACE_THREADS;
-static const int kIters = J3DG_TRACE_ITERS;
 // k_frame runs two warps per block, with the warps per SM of the builds
 // above: when a frame's last rays keep a few warps busy, every block that is
 // done frees its slot for the canvas's next frame (overlapped frames, below;
@@ -272,8 +278,24 @@ static const int kIters = J3DG_TRACE_ITERS;
 #define J3DG_FRAME_THREADS 64
 #endif
 static const int kFrameThreads = J3DG_FRAME_THREADS;
-static const int kFrameBlocksT = J3DG_TRACE_MINBLOCKS * 128 / kFrameThreads;
-static const int kFrameBlocksL = J3DG_LATENCY_MINBLOCKS * 128 / kFrameThreads;
+// The builds of k_frame, by the frame's primary items: more warps an SM hide
+// more of the fetches' latency once a frame has the pixels to feed them, fewer
+// let a small frame's last rays run faster.
+//   0 (below 400k items): 20 warps an SM, pixel state in registers
+//   1 (below 2M): 24 warps (a 1280x720 frame of a 1M-triangle torus with
+//     shadows 229 -> 210 us, 800x600 of 24 objects 538 -> 508; a 512x512 frame
+//     of the 28.09M-triangle torus would take 228 instead of 218)
+//   2: pixel state in shared memory, 28 warps at width 4, whose 72 registers
+//     hold the step without spills now that a single object's arrays come from
+//     the constant bank (1920x1080 of the 28.09M-triangle torus with shadows
+//     525 -> 489 us; 32 warps spill: 497)
+static const int kTiers = 3;
+static const uint32_t kTierItems[kTiers - 1] = {400000u, J3DG_THROUGHPUT_ITEMS};
+__host__ __device__ constexpr int tier_blocks(int tier) {  // blocks of kFrameThreads an SM
+  return (tier == 0 ? J3DG_LATENCY_MINBLOCKS
+                    : (tier == 1 || J3DG_W != 4 ? J3DG_TRACE_MINBLOCKS : J3DG_TRACE_MINBLOCKS + 1)) *
+         128 / kFrameThreads;
+}
 
 // Pixel and colour state of a lane: read only at a pixel's start and
 // finish. The throughput build keeps it in a per-block shared array
@@ -871,11 +893,11 @@ template <bool TOP>
 __global__ void __launch_bounds__(kTraceThreads, J3DG_TRACE_MINBLOCKS) k_shadow(const FrameParams P) {
   if (P.rlist[1]) return;
   ShadowSrc src{&P, shadow_jobs(P), P.work[1], light_position(P)};
-  persistent_trace<kIters, kTraceThreads, TOP, kWidth>(src, P.inst, P.n_inst, P.work + 2, P.status, P.counters);
+  persistent_trace<J3DG_RAY_REFILL, kTraceThreads, TOP, kWidth>(src, P.inst, P.n_inst, P.work + 2, P.status, P.counters);
 }
 
-template <bool kThroughput, bool TOP, bool ONE>
-__global__ void __launch_bounds__(kFrameThreads, kThroughput ? kFrameBlocksT : kFrameBlocksL)
+template <int kTier, bool TOP, bool ONE>
+__global__ void __launch_bounds__(kFrameThreads, tier_blocks(kTier))
     k_frame(const __grid_constant__ FrameParams P) {
   TracerT<kFrameThreads, TOP, kWidth, ONE> T;
   uint2 stack[J3DG_STACK];
@@ -886,7 +908,7 @@ __global__ void __launch_bounds__(kFrameThreads, kThroughput ? kFrameBlocksT : k
   // the raster kernels made this frame: nothing to take (the exit still runs)
   bool exhausted = P.raster && P.rlist[1] == 0u, handed_over = false;
   PixState local;
-  PixState& ps = pix_state<kThroughput && (J3DG_COLD_SMEM & 4) != 0, kFrameThreads>(local);
+  PixState& ps = pix_state<kTier == 2 && (J3DG_COLD_SMEM & 4) != 0, kFrameThreads>(local);
   ps = PixState{0, 0u, 0u, 0.f, 0.f};
   size_t& pix = ps.pix;
   uint32_t& w0 = ps.w0;
@@ -993,12 +1015,12 @@ struct BatchSrc {
 };
 
 template <bool ANY, bool TOP, bool ONE>
-__global__ void __launch_bounds__(kTraceThreads)
+__global__ void __launch_bounds__(kTraceThreads, J3DG_RAY_BLOCKS)
     k_rays(const DevInst* __restrict__ inst, const __grid_constant__ DevInst one, uint32_t n_inst,
            const j3dg_ray* __restrict__ rays, uint32_t n, j3dg_hit* __restrict__ hits, uint32_t* counter,
            uint32_t* status, unsigned long long* counters) {
   BatchSrc<ANY> src{rays, hits, n};
-  persistent_trace<kIters, kTraceThreads, TOP, kWidth, ONE>(src, ONE ? &one : inst, n_inst, counter, status, counters);
+  persistent_trace<J3DG_RAY_REFILL, kTraceThreads, TOP, kWidth, ONE>(src, ONE ? &one : inst, n_inst, counter, status, counters);
 }
 
 // Many frames (canvases, scenes, cameras, resolutions of uneven size) in one
@@ -1291,9 +1313,9 @@ __global__ void k_init_pixels(j3dg_pixel* __restrict__ G, size_t n) {
 
 // k_frame, as a programmatic dependent of the previous kernel on the stream
 // when the frame overlaps its canvas's previous frame
-template <bool kT, bool TOP, bool ONE>
-static cudaError_t launch_frame(const FrameParams& P, bool overlap, cudaStream_t st) {
-  static const int blocks = persistent_blocks(k_frame<kT, TOP, ONE>, kFrameThreads);
+template <int kTier, bool TOP, bool ONE>
+static cudaError_t launch_frame_tier(const FrameParams& P, bool overlap, cudaStream_t st) {
+  static const int blocks = persistent_blocks(k_frame<kTier, TOP, ONE>, kFrameThreads);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)blocks);
   cfg.blockDim = dim3((unsigned)kFrameThreads);
@@ -1304,7 +1326,15 @@ static cudaError_t launch_frame(const FrameParams& P, bool overlap, cudaStream_t
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = overlap ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, k_frame<kT, TOP, ONE>, P);
+  return cudaLaunchKernelEx(&cfg, k_frame<kTier, TOP, ONE>, P);
+}
+
+template <bool TOP, bool ONE>
+static cudaError_t launch_frame(const FrameParams& P, bool overlap, cudaStream_t st) {
+  const uint32_t items = primary_items(P);
+  if (items < kTierItems[0]) return launch_frame_tier<0, TOP, ONE>(P, overlap, st);
+  if (items < kTierItems[1]) return launch_frame_tier<1, TOP, ONE>(P, overlap, st);
+  return launch_frame_tier<2, TOP, ONE>(P, overlap, st);
 }
 
 cudaError_t launch_render(const FrameParams& P, cudaStream_t st) {
@@ -1342,13 +1372,10 @@ cudaError_t launch_render(const FrameParams& P, cudaStream_t st) {
       k_shadow<false><<<blocks_s, kTraceThreads, 0, st>>>(P);
     // k_frame below returns at once unless the large-triangle list overflowed
   }
-  const bool thr = primary_items(P) >= J3DG_THROUGHPUT_ITEMS;
   if (P.embedded)
-    e = thr ? launch_frame<true, false, true>(P, overlap, st) : launch_frame<false, false, true>(P, overlap, st);
-  else if (P.top)
-    e = thr ? launch_frame<true, true, false>(P, overlap, st) : launch_frame<false, true, false>(P, overlap, st);
+    e = launch_frame<false, true>(P, overlap, st);
   else
-    e = thr ? launch_frame<true, false, false>(P, overlap, st) : launch_frame<false, false, false>(P, overlap, st);
+    e = P.top ? launch_frame<true, false>(P, overlap, st) : launch_frame<false, false>(P, overlap, st);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
