@@ -535,11 +535,16 @@ int mesh_devinst(j3dg_ctx* c, const j3dg_mesh* mesh, const DevInst** out) {
   return upload_instances(c, &one, 1, out);
 }
 
+// The same as a record by value.
+int mesh_record(j3dg_ctx* c, const j3dg_mesh* mesh, DevInst* out) {
+  const j3dg_instance one = identity_instance(mesh);
+  return one_instance(c, &one, out);
+}
+
 // Plain closest hit of device rays against one mesh into device hits (async).
 int ray_query_device(j3dg_ctx* c, const j3dg_mesh* mesh, const j3dg_ray* d_rays, uint32_t n, j3dg_hit* d_hits) {
-  j3dg_instance obj = identity_instance(mesh);
   DevInst one;
-  if (int rc = one_instance(c, &obj, &one)) return rc;
+  if (int rc = mesh_record(c, mesh, &one)) return rc;
   CK(c, launch_rays(nullptr, &one, 1, false, (int)mesh->width, d_rays, n, d_hits, false, all(c)->ex.d_ray_counter, c->d_status,
                     nullptr, S(c)),
      "ray query");
