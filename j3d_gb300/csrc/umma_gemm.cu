@@ -2,11 +2,19 @@
 // accumulator in tensor memory, and the fused epilogues the network's
 // training and layer-by-layer inference need:
 //   C[M x N] = epilogue(A[M x K] . Bt[N x K]^T)   (A and Bt row-major, K-major)
-// One CTA of 4 warps per 128 x BN tile. K advances in chunks of 64 through a
-// two-stage shared-memory ring: all threads copy the next chunk into the
-// canonical no-swizzle layout while the tensor core works on the previous
-// one; thread 0 issues the four K = 16 MMAs of a chunk and commits them to
-// the stage's mbarrier, which frees the stage for the chunk after next.
+// One CTA of 4 warps per 128 x BN tile, two CTAs an SM (each takes BN TMEM
+// columns), so that one's epilogue overlaps the other's MMAs. K advances in
+// chunks of 64 through a shared-memory ring of 3 (BN = 128) or 2 stages that
+// asynchronous copies (16 bytes each, straight into the canonical no-swizzle
+// layout) fill ahead; thread 0 issues the four K = 16 MMAs of a chunk and
+// commits them to the stage's mbarrier, which frees the stage for the chunk
+// that follows the ring's last.
+// What bounds it: operands and results in memory (K = 128: 268 MB of logits
+// for 16384 rows). With copies through registers and one CTA an SM every
+// chunk waited a memory latency. For 16384 rows, before and after: logits 197
+// -> 142 us, the gradient through the last layer (K = 4096) and the three
+// small ones 235 -> 135, the last layer's weight gradient 147 -> 83, the
+// others' 67 -> 43.
 // The epilogue moves each warp's 32 accumulator rows out of TMEM with
 // tcgen05.ld. Every wait is bounded (clock budget); on timeout the kernel
 // raises J3DG_DEV_VISIT_CAP in the status word, skips the epilogue and still
@@ -29,28 +37,35 @@ namespace {
 
 const int kChunkK = 64;                     // K per stage
 const long long kWaitBudget = 500000000ll;  // ~0.25 s at 2 GHz
-const uint32_t kTmemCols = 512;             // whole TMEM: one CTA per SM
 
 template <int BN>
 struct GemmSmem {
   static constexpr uint32_t a_bytes = 128 * kChunkK * 2;  // 16 KB
   static constexpr uint32_t b_bytes = BN * kChunkK * 2;
   static constexpr uint32_t stage_bytes = a_bytes + b_bytes;
-  // + alignment slack; at least 120 KB so that one CTA runs per SM (each
-  // takes all 512 TMEM columns)
-  static constexpr uint32_t total = 2 * stage_bytes + 1024 > 122880u ? 2 * stage_bytes + 1024 : 122880u;
+  static constexpr int stages = BN == 128 ? 3 : 2;
+  static constexpr uint32_t total = stages * stage_bytes + 1024;  // + alignment slack: 97 KB, two CTAs an SM
 };
 
-// Copies rows [r0, r0 + rows) x K-chunk [k0, k0 + 64) of a row-major bf16
-// matrix into the canonical layout (8 core matrices along K).
-__device__ __forceinline__ void copy_chunk(const __nv_bfloat16* __restrict__ src, int ld, int r0, int rows, int k0,
-                                           uint8_t* dst) {
-  const int pieces = rows * (kChunkK / 8);
-  for (int p = threadIdx.x; p < pieces; p += blockDim.x) {
-    const int row = p >> 3, kg = p & 7;
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(src + (size_t)(r0 + row) * ld + k0 + kg * 8));
-    *reinterpret_cast<uint4*>(dst + umma::tile_offset(row, kg * 8, kChunkK / 8)) = v;
+// Starts copying rows [r0, r0 + ROWS) x K-chunk [k0, k0 + 64) of a row-major
+// bf16 matrix into the canonical layout (8 core matrices along K). A warp's
+// 32 copies take 8 rows x 4 pieces: 64 bytes of a row from memory, and all
+// of shared memory's banks.
+template <int ROWS>
+__device__ __forceinline__ void copy_chunk(const __nv_bfloat16* __restrict__ src, int ld, int r0, int k0, uint8_t* dst) {
+#pragma unroll
+  for (int p = threadIdx.x; p < ROWS * (kChunkK / 8); p += 128) {
+    const int row = (p >> 6) * 8 + (p & 7), kg = (p >> 3) & 7;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                     umma::smem_u32(dst + umma::tile_offset(row, kg * 8, kChunkK / 8))),
+                 "l"(src + (size_t)(r0 + row) * ld + k0 + kg * 8)
+                 : "memory");
   }
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copies_wait() {  // all but the last N groups have landed
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
 // The epilogue of thread `lane` of warp w: accumulator row m0 + 32 w + lane,
@@ -117,9 +132,9 @@ __device__ __forceinline__ void epilogue(const UmmaArgs& g, uint32_t taddr, int 
 }
 
 template <int BN, int EPI>
-__global__ void __launch_bounds__(128, 1) k_umma_gemm(const UmmaArgs g, uint32_t* status, int withhold) {
+__global__ void __launch_bounds__(128, 2) k_umma_gemm(const UmmaArgs g, uint32_t* status, int withhold) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t mbar[2];
+  __shared__ __align__(8) uint64_t mbar[GemmSmem<BN>::stages];
   __shared__ uint32_t taddr_s;
   uint8_t* sm = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -129,12 +144,11 @@ __global__ void __launch_bounds__(128, 1) k_umma_gemm(const UmmaArgs g, uint32_t
   // a CTA that timed out raised the status word: the rest of the grid stops
   if (*reinterpret_cast<volatile uint32_t*>(status) & J3DG_DEV_VISIT_CAP) return;
   if (warp == 0) {
-    umma::tmem_alloc(umma::smem_u32(&taddr_s), kTmemCols);
+    umma::tmem_alloc(umma::smem_u32(&taddr_s), BN);
     umma::tmem_relinquish();
   }
   if (threadIdx.x == 0) {
-    umma::mbar_init(umma::smem_u32(&mbar[0]), 1);
-    umma::mbar_init(umma::smem_u32(&mbar[1]), 1);
+    for (int i = 0; i < L::stages; ++i) umma::mbar_init(umma::smem_u32(&mbar[i]), 1);
   }
   umma::fence_before_sync();
   __syncthreads();
@@ -147,31 +161,41 @@ __global__ void __launch_bounds__(128, 1) k_umma_gemm(const UmmaArgs g, uint32_t
   const int kc0 = (int)((long long)nk_all * blockIdx.z / gridDim.z);
   const int kc1 = (int)((long long)nk_all * (blockIdx.z + 1) / gridDim.z);
   const int nk = kc1 - kc0;
+  constexpr int S = L::stages;
+  auto load = [&](int it) {  // chunk it into its stage; one group a chunk, empty past the last
+    if (it < nk) {
+      uint8_t* sA = sm + (it % S) * L::stage_bytes;
+      copy_chunk<128>(g.A, g.lda, m0, (kc0 + it) * kChunkK, sA);
+      copy_chunk<BN>(g.Bt, g.ldb, n0, (kc0 + it) * kChunkK, sA + L::a_bytes);
+    }
+    copies_commit();
+  };
   bool ok = true;
+  for (int it = 0; it < S - 1; ++it) load(it);
   for (int it = 0; it < nk; ++it) {
-    const int s = it & 1;
-    uint8_t* sA = sm + s * L::stage_bytes;
-    uint8_t* sB = sA + L::a_bytes;
-    if (it >= 2) ok = umma::mbar_wait(umma::smem_u32(&mbar[s]), ((it - 2) >> 1) & 1, kWaitBudget);
+    const int s = it % S;
+    copies_wait<S - 2>();      // this thread's copies of chunk it
+    umma::fence_async_smem();  // ... before the tensor core reads them
     if (!__syncthreads_and(ok)) {
       ok = false;
       break;
     }
-    copy_chunk(g.A, g.lda, m0, 128, (kc0 + it) * kChunkK, sA);
-    copy_chunk(g.Bt, g.ldb, n0, BN, (kc0 + it) * kChunkK, sB);
-    umma::fence_async_smem();
-    __syncthreads();
     if (threadIdx.x == 0 && !withhold) {  // withhold: nothing completes the barrier (failure-path test)
       umma::fence_after_sync();
-      const uint32_t a0 = umma::smem_u32(sA), b0 = umma::smem_u32(sB);
+      const uint32_t a0 = umma::smem_u32(sm + s * L::stage_bytes), b0 = a0 + L::a_bytes;
 #pragma unroll
       for (int k = 0; k < kChunkK / 16; ++k)
         umma::mma_bf16(taddr, umma::desc(a0 + k * 256, 128, (kChunkK / 8) * 128),
                        umma::desc(b0 + k * 256, 128, (kChunkK / 8) * 128), idesc, (it | k) != 0);
       umma::commit(umma::smem_u32(&mbar[s]));
     }
+    // chunk it + S - 1 takes the stage of chunk it - 1, once its MMAs are done
+    if (it > 0 && it + S - 1 < nk)
+      ok = umma::mbar_wait(umma::smem_u32(&mbar[(it - 1) % S]), ((it - 1) / S) & 1, kWaitBudget);
+    if (ok) load(it + S - 1);
   }
-  if (ok && nk > 0) ok = umma::mbar_wait(umma::smem_u32(&mbar[(nk - 1) & 1]), ((nk - 1) >> 1) & 1, kWaitBudget);
+  copies_wait<0>();  // (a timed-out CTA's copies too)
+  if (ok && nk > 0) ok = umma::mbar_wait(umma::smem_u32(&mbar[(nk - 1) % S]), ((nk - 1) / S) & 1, kWaitBudget);
   ok = __syncthreads_and(ok);
   umma::fence_after_sync();
   if (ok && nk > 0) {
@@ -183,7 +207,7 @@ __global__ void __launch_bounds__(128, 1) k_umma_gemm(const UmmaArgs g, uint32_t
   __syncthreads();
   if (warp == 0) {
     umma::fence_after_sync();
-    umma::tmem_dealloc(taddr, kTmemCols);
+    umma::tmem_dealloc(taddr, BN);
   }
 }
 
