@@ -18,9 +18,10 @@
 //      with a strict total order on the split keys (xor of neighbouring
 //      codes, then i ^ (i+1), then i)
 //   6. collapse to 4-wide nodes level by level: slots and leaves chosen by
-//      the SAH cost programme of section 6b (LBVH: open the largest-area
+//      the SAH cost programme of section 6b, which also tells every wide
+//      node's place in depth-first order (LBVH: open the largest-area
 //      child until four children, subtrees of <= leaf_size triangles become
-//      leaves); then the wide nodes are numbered depth-first (section 7).
+//      leaves; then the wide nodes are renumbered depth-first, section 7).
 // Child boxes are exact unions of triangle boxes, which the traversal's
 // topology-independence argument requires.
 #include <cuda_runtime.h>
@@ -75,11 +76,29 @@ __global__ void k_bbox_partial(const float* __restrict__ V, uint32_t nv, float* 
   }
 }
 
-__global__ void k_bbox_final(const float* __restrict__ part, int n, float* __restrict__ out) {
-  if (threadIdx.x < 6) {
-    float v = part[threadIdx.x];
-    for (int b = 1; b < n; ++b) v = threadIdx.x < 3 ? fminf(v, part[6 * b + threadIdx.x]) : fmaxf(v, part[6 * b + threadIdx.x]);
-    out[threadIdx.x] = v;
+// one block over at most 1024 partial boxes, one a thread (one warp walking
+// them took 41 us)
+__global__ void __launch_bounds__(1024) k_bbox_final(const float* __restrict__ part, int n, float* __restrict__ out) {
+  __shared__ float s[6][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int b = min((int)threadIdx.x, n - 1);  // (a box read twice changes nothing)
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    float v = part[6 * b + k];
+    for (int o = 16; o > 0; o >>= 1) {
+      const float y = __shfl_xor_sync(0xffffffffu, v, o);
+      v = k < 3 ? fminf(v, y) : fmaxf(v, y);
+    }
+    if (lane == 0) s[k][warp] = v;
+  }
+  __syncthreads();
+  if (warp < 6) {
+    float v = s[warp][lane];
+    for (int o = 16; o > 0; o >>= 1) {
+      const float y = __shfl_xor_sync(0xffffffffu, v, o);
+      v = warp < 3 ? fminf(v, y) : fmaxf(v, y);
+    }
+    if (lane == 0) out[warp] = v;
   }
 }
 
@@ -367,9 +386,22 @@ __global__ void k_soup(const float* __restrict__ V, const uint32_t* __restrict__
 
 // ------------------------------------------------------------- 5. LBVH ----
 
-struct BinNode {   // binary node n (split between sorted leaves n and n+1)
-  float4 lo, hi;   // box (w unused)
+// A binary node. LBVH: node n splits between sorted leaves n and n + 1, the
+// w fields are unused. The default builder keeps the two children's refs
+// there (bit 31: a triangle, in Morton order), so that one 32-byte sector
+// holds what the collapse follows.
+struct BinNode {
+  float4 lo, hi;
 };
+// ... and what the collapse's decisions need of it (default builder)
+struct __align__(16) NodeMeta {
+  uint32_t count;   // triangles
+  uint32_t wide;    // wide nodes its subtree becomes unless it is a leaf
+  uint32_t dec[2];  // the decisions of section 6b, a byte each
+};
+// a BinNode's children
+__device__ __forceinline__ uint32_t left_ref(const float4& lo) { return __float_as_uint(lo.w); }
+__device__ __forceinline__ uint32_t right_ref(const float4& hi) { return __float_as_uint(hi.w); }
 
 __device__ __forceinline__ void leaf_box(const float4* __restrict__ tris, uint32_t i, float4& lo, float4& hi) {
   float4 a = tris[3 * (size_t)i], b = tris[3 * (size_t)i + 1], c = tris[3 * (size_t)i + 2];
@@ -606,98 +638,66 @@ __device__ __forceinline__ float merged_area(float4 alo, float4 ahi, float4 blo,
 #define J3DG_SAH_CTRI 0.5f  // cost of a triangle test relative to a node visit
 #endif
 
-__device__ __forceinline__ float half_area4(float4 lo, float4 hi);
-
-// costs C(r, 1..W) of subtree r (a triangle: its area times c_t for any i)
+// what the programme keeps of a subtree: C(n, 1..W), and how many wide nodes
+// it becomes with 1..W slots (a triangle: none), from which every wide node's
+// place in depth-first order follows before any is made
 template <int W>
-__device__ __forceinline__ void sub_costs(const float* __restrict__ cost, const float4* __restrict__ tris, uint32_t r,
-                                          float (&c)[W + 1]) {
-  if (r & 0x80000000u) {
-    float4 lo, hi;
-    leaf_box(tris, r & 0x7fffffffu, lo, hi);
-    const float v = half_area4(lo, hi) * J3DG_SAH_CTRI;
+struct Covering {
+  float cost[W + 1];
+  uint32_t wide[W + 1];
+  __device__ __forceinline__ void triangle(float half_area) {
 #pragma unroll
-    for (int i = 1; i <= W; ++i) c[i] = v;
-  } else {
-#pragma unroll
-    for (int i = 1; i <= W; ++i) c[i] = cost[(size_t)r * W + i - 1];
+    for (int i = 1; i <= W; ++i) {
+      cost[i] = half_area * J3DG_SAH_CTRI;
+      wide[i] = 0u;
+    }
   }
-}
+};
 
 // the programme's step at a node of half area A over N triangles from its
-// children's costs: C(n, 1..W) and the W decision bytes (d[0] = the k of the
-// node case | 0x80 when the leaf case is cheaper; d[i - 1], i = 2..W: 0 = as
+// children's coverings; M.dec: the W decision bytes (byte 0 = the k of the node
+// case | 0x80 when the leaf case is cheaper; byte i - 1, i = 2..W: 0 = as
 // i - 1, else the k of the best split)
 template <int W>
-__device__ __forceinline__ void collapse_step(const float (&cl)[W + 1], const float (&cr)[W + 1], float A, uint32_t N,
-                                              uint32_t leaf_size, float (&C)[W + 1], uint8_t (&d)[W]) {
+__device__ __forceinline__ void collapse_step(const Covering<W>& l, const Covering<W>& r, float A, uint32_t N,
+                                              uint32_t leaf_size, Covering<W>& c, NodeMeta& M) {
   float best = FLT_MAX;
-  uint32_t bk = 1;
+  uint32_t bk = 1, bw = l.wide[1] + r.wide[W - 1];
 #pragma unroll
   for (uint32_t k = 1; k < (uint32_t)W; ++k)
-    if (cl[k] + cr[W - k] < best) {
-      best = cl[k] + cr[W - k];
+    if (l.cost[k] + r.cost[W - k] < best) {
+      best = l.cost[k] + r.cost[W - k];
       bk = k;
+      bw = l.wide[k] + r.wide[W - k];
     }
   const float node = A + best;  // c_n = 1
   const float leaf = N <= leaf_size ? A * (float)N * J3DG_SAH_CTRI : FLT_MAX;
-  C[1] = fminf(leaf, node);
-  d[0] = (uint8_t)(bk | (leaf <= node ? 0x80u : 0u));
+  c.cost[1] = fminf(leaf, node);
+  const bool is_leaf = leaf <= node && N <= J3DG_MAX_LEAF;  // (areas past the largest float: at equal costs)
+  c.wide[1] = is_leaf ? 0u : 1u + bw;
+  M.count = N;
+  M.wide = 1u + bw;
+  M.dec[0] = bk | (is_leaf ? 0x80u : 0u);
+  M.dec[1] = 0u;
 #pragma unroll
   for (uint32_t i = 2; i <= (uint32_t)W; ++i) {
-    float v = C[i - 1];
-    uint32_t dk = 0;
+    float v = c.cost[i - 1];
+    uint32_t dk = 0, w = c.wide[i - 1];
 #pragma unroll
     for (uint32_t k = 1; k < i; ++k)
-      if (cl[k] + cr[i - k] < v) {
-        v = cl[k] + cr[i - k];
+      if (l.cost[k] + r.cost[i - k] < v) {
+        v = l.cost[k] + r.cost[i - k];
         dk = k;
+        w = l.wide[k] + r.wide[i - k];
       }
-    C[i] = v;
-    d[i - 1] = (uint8_t)dk;
+    c.cost[i] = v;
+    c.wide[i] = w;
+    M.dec[(i - 1) >> 2] |= dk << (8 * ((i - 1) & 3u));
   }
 }
 
-// the W decision bytes of node n in one store
-template <int W>
-__device__ __forceinline__ void store_dec(uint8_t* __restrict__ dec, uint32_t n, const uint8_t (&d)[W]) {
-  if constexpr (W == 2) {
-    reinterpret_cast<uint16_t*>(dec)[n] = (uint16_t)(d[0] | (d[1] << 8));
-  } else {
-#pragma unroll
-    for (int q = 0; q < W / 4; ++q)
-      reinterpret_cast<uint32_t*>(dec)[(size_t)n * (W / 4) + q] =
-          (uint32_t)d[4 * q] | ((uint32_t)d[4 * q + 1] << 8) | ((uint32_t)d[4 * q + 2] << 16) |
-          ((uint32_t)d[4 * q + 3] << 24);
-  }
-}
-
-// cost: W floats per binary node (C(n, 1..W)); dec: W bytes per node
-template <int W>
-__device__ __forceinline__ void collapse_cost_one(const uint2* __restrict__ child, const BinNode* __restrict__ box,
-                                                  const uint32_t* __restrict__ count, const float4* __restrict__ tris,
-                                                  uint32_t n, uint32_t leaf_size, float* __restrict__ cost,
-                                                  uint8_t* __restrict__ dec) {
-  const uint2 c = child[n];
-  float cl[W + 1], cr[W + 1], C[W + 1];
-  uint8_t d[W];
-  sub_costs<W>(cost, tris, c.x, cl);
-  sub_costs<W>(cost, tris, c.y, cr);
-  collapse_step<W>(cl, cr, half_area4(box[n].lo, box[n].hi), count[n], leaf_size, C, d);
-#pragma unroll
-  for (int i = 1; i <= W; ++i) cost[(size_t)n * W + i - 1] = C[i];
-  store_dec<W>(dec, n, d);
-}
-
-template <int W>
-__global__ void k_collapse_cost(const uint2* __restrict__ child, const BinNode* __restrict__ box,
-                                const uint32_t* __restrict__ count, const float4* __restrict__ tris,
-                                const uint32_t* __restrict__ list, const uint32_t* __restrict__ lohi,
-                                uint32_t leaf_size, float* __restrict__ cost, uint8_t* __restrict__ dec) {
-  // the pass's binary nodes: entries [lohi[0], lohi[1]) of the list (device memory)
-  const uint32_t lo = lohi[0], hi = lohi[1];
-  for (uint32_t k = lo + blockIdx.x * blockDim.x + threadIdx.x; k < hi; k += gridDim.x * blockDim.x)
-    collapse_cost_one<W>(child, box, count, tris, list[k], leaf_size, cost, dec);
+__device__ __forceinline__ uint32_t dec_byte(const NodeMeta& m, uint32_t i) {
+  return (m.dec[i >> 2] >> (8 * (i & 3u))) & 0xffu;
 }
 
 struct PlaceItem {
@@ -709,98 +709,66 @@ struct PlaceItem {
 
 // The collapse of k_collapse over a tree whose subtrees are not ranges of the
 // sorted leaves: each slot carries its subtree's first position; leaves are
-// written to tris_out at those positions in depth-first order.
+// written to tris_out at those positions in depth-first order (and the
+// triangles' positions to slot_of). A wide node's place in depth-first order
+// is its parent's, plus one, plus the wide nodes of the slots before it: the
+// wide nodes are written where they stay.
 template <int W>
-__device__ __forceinline__ void collapse_place_one(const uint2* __restrict__ child, const BinNode* __restrict__ box,
-                                                   const uint32_t* __restrict__ count, const float4* __restrict__ tris,
+__device__ __forceinline__ void collapse_place_one(const BinNode* __restrict__ node, const NodeMeta* __restrict__ meta,
+                                                   const BinNode* __restrict__ tbox, const float4* __restrict__ tris,
                                                    const PlaceItem* __restrict__ qin, uint32_t t, uint32_t n_in,
                                                    PlaceItem* __restrict__ qout, uint32_t* __restrict__ n_out,
-                                                   uint32_t wide_base, float4* __restrict__ wide, uint32_t leaf_size,
+                                                   uint32_t n_wide, float4* __restrict__ wide,
                                                    uint32_t* __restrict__ max_depth, float4* __restrict__ tris_out,
-                                                   uint32_t nt, uint32_t* status, const uint8_t* __restrict__ dec) {
+                                                   uint32_t* __restrict__ slot_of, uint32_t nt, uint32_t* status) {
   // whole warps come here together (the next level's slots are allocated per
   // warp); lanes past n_in place nothing
   const uint32_t lane = threadIdx.x & 31u;
   const bool valid = t < n_in;
   const PlaceItem it = valid ? qin[t] : PlaceItem{0u, 0u, 0u, 0u};
-  uint32_t ref[W], cnt[W], start[W];
+  // the slots the cost decisions give: expand(left, k) then expand(right, W - k)
+  uint32_t ref[W], cnt[W], start[W], sub[W];  // sub: wide nodes in the slot (0: a leaf)
   float4 lo[W], hi[W];
-  auto load = [&](uint32_t r, int s, uint32_t first) {
-    ref[s] = r;
-    start[s] = first;
-    if (r & 0x80000000u) {
-      leaf_box(tris, r & 0x7fffffffu, lo[s], hi[s]);
-      cnt[s] = 1;
-    } else {
-      lo[s] = box[r].lo;
-      hi[s] = box[r].hi;
-      cnt[s] = count[r];
-    }
-  };
-  const uint2 c = valid ? child[it.bin] : make_uint2(0u, 0u);
   int m = 0;
-  if (!valid) {
-  } else if (dec) {
-    // the slots the cost decisions give: expand(left, k) then expand(right, W - k)
+  auto count_of = [&](uint32_t r) { return (r & 0x80000000u) ? 1u : meta[r].count; };
+  if (valid) {
     struct Slot {
       uint32_t r, i, start;
     };
     Slot stk[2 * W];
     int sp = 0;
-    const uint32_t k = dec[(size_t)it.bin * W] & 0x7fu;
-    const uint32_t nl = (c.x & 0x80000000u) ? 1u : count[c.x];
-    stk[sp++] = Slot{c.y, (uint32_t)W - k, it.start + nl};
-    stk[sp++] = Slot{c.x, k, it.start};
+    const uint32_t k = dec_byte(meta[it.bin], 0) & 0x7fu;
+    const uint32_t cl = left_ref(node[it.bin].lo), cr = right_ref(node[it.bin].hi);
+    stk[sp++] = Slot{cr, (uint32_t)W - k, it.start + count_of(cl)};
+    stk[sp++] = Slot{cl, k, it.start};
     while (sp > 0 && m < W) {
       const Slot e = stk[--sp];
-      if ((e.r & 0x80000000u) || e.i <= 1u) {
-        load(e.r, m++, e.start);
+      if (e.r & 0x80000000u) {
+        const BinNode b = tbox[e.r & 0x7fffffffu];
+        ref[m] = e.r, start[m] = e.start, cnt[m] = 1u, sub[m] = 0u, lo[m] = b.lo, hi[m] = b.hi;
+        ++m;
         continue;
       }
-      const uint32_t d = dec[(size_t)e.r * W + e.i - 1];
-      if (d == 0u || sp + 2 > 2 * W) {
-        stk[sp++] = Slot{e.r, e.i - 1u, e.start};
+      const BinNode b = node[e.r];
+      const NodeMeta M = meta[e.r];
+      uint32_t i = e.i, d = 0u;
+      while (i > 1u && (d = dec_byte(M, i - 1u)) == 0u) --i;  // 0: as with a slot less
+      if (i <= 1u || sp + 2 > 2 * W) {
+        ref[m] = e.r, start[m] = e.start, cnt[m] = M.count, lo[m] = b.lo, hi[m] = b.hi;
+        sub[m] = (M.dec[0] & 0x80u) ? 0u : M.wide;
+        ++m;
         continue;
       }
-      const uint2 cc = child[e.r];
-      const uint32_t ml = (cc.x & 0x80000000u) ? 1u : count[cc.x];
-      stk[sp++] = Slot{cc.y, e.i - d, e.start + ml};
-      stk[sp++] = Slot{cc.x, d, e.start};
+      const uint32_t l = left_ref(b.lo);
+      stk[sp++] = Slot{right_ref(b.hi), i - d, e.start + count_of(l)};
+      stk[sp++] = Slot{l, d, e.start};
     }
-  } else {
-    load(c.x, 0, it.start);
-    load(c.y, 1, it.start + cnt[0]);
-    m = 2;
   }
-  while (valid && !dec && m < W) {
-    int best = -1;
-    float ba = -1.f;
-    for (int s = 0; s < m; ++s)
-      if (cnt[s] > leaf_size) {
-        const float a = half_area(lo[s], hi[s]);
-        if (a > ba) {
-          ba = a;
-          best = s;
-        }
-      }
-    if (best < 0) break;
-    const uint2 cc = child[ref[best]];
-    const uint32_t s0 = start[best];
-    load(cc.x, best, s0);
-    load(cc.y, m, s0 + cnt[best]);
-    ++m;
-  }
-  // slots placed as leaves, and the next level's queue slots for the rest:
-  // one atomic per warp (a warp-wide scan of the lanes' internal slots)
-  uint32_t leaf_mask = 0u, n_int = 0u;
-  for (int s = 0; s < m; ++s) {
-    const bool as_leaf = (ref[s] & 0x80000000u) ||
-                         (dec ? (dec[(size_t)ref[s] * W] & 0x80u) != 0 : cnt[s] <= leaf_size);
-    if (as_leaf && cnt[s] <= J3DG_MAX_LEAF)
-      leaf_mask |= 1u << s;
-    else
-      ++n_int;
-  }
+  // the next level's queue slots: one atomic per warp (a warp-wide scan of the
+  // lanes' internal slots)
+  uint32_t n_int = 0u;
+#pragma unroll
+  for (int s = 0; s < W; ++s) n_int += s < m && sub[s] != 0u ? 1u : 0u;
   uint32_t incl = n_int;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -817,6 +785,8 @@ __device__ __forceinline__ void collapse_place_one(const uint2* __restrict__ chi
   float F[4 * J3DG_NODE_F4(W)];
 #pragma unroll
   for (int k = 0; k < 4 * J3DG_NODE_F4(W); ++k) F[k] = 0.f;
+  uint32_t next = it.wide + 1u;
+#pragma unroll
   for (int s = 0; s < W; ++s) {
     uint32_t out_ref = J3DG_EMPTY_REF;
     if (s < m) {
@@ -826,7 +796,7 @@ __device__ __forceinline__ void collapse_place_one(const uint2* __restrict__ chi
       F[3 * W + s] = hi[s].y;
       F[4 * W + s] = lo[s].z;
       F[5 * W + s] = hi[s].z;
-      if (leaf_mask & (1u << s)) {
+      if (sub[s] == 0u) {
         out_ref = J3DG_LEAF_BIT | (start[s] << 3) | (cnt[s] - 1u);
         uint32_t stk[J3DG_MAX_LEAF];
         int sp = 0;
@@ -837,31 +807,37 @@ __device__ __forceinline__ void collapse_place_one(const uint2* __restrict__ chi
           if (r & 0x80000000u) {
             const uint32_t src = r & 0x7fffffffu, dst = start[s] + k++;
             if (src < nt && dst < nt) {
-              tris_out[3 * (size_t)dst] = tris[3 * (size_t)src];
-              tris_out[3 * (size_t)dst + 1] = tris[3 * (size_t)src + 1];
-              tris_out[3 * (size_t)dst + 2] = tris[3 * (size_t)src + 2];
+              const float4 v0 = tris[3 * (size_t)src], v1 = tris[3 * (size_t)src + 1], v2 = tris[3 * (size_t)src + 2];
+              tris_out[3 * (size_t)dst] = v0;
+              tris_out[3 * (size_t)dst + 1] = v1;
+              tris_out[3 * (size_t)dst + 2] = v2;
+              const uint32_t id = __float_as_uint(v0.w);
+              if (id < nt)
+                slot_of[id] = dst;
+              else
+                atomicOr(status, J3DG_DEV_BAD_INDEX);
             } else {
               atomicOr(status, J3DG_DEV_BAD_INDEX);
             }
           } else if (sp + 2 <= (int)J3DG_MAX_LEAF) {
-            const uint2 cc = child[r];
-            stk[sp++] = cc.y;
-            stk[sp++] = cc.x;
+            const BinNode b = node[r];
+            stk[sp++] = right_ref(b.hi);
+            stk[sp++] = left_ref(b.lo);
           } else {
             atomicOr(status, J3DG_DEV_STACK_OVERFLOW);
             break;
           }
         }
       } else {
-        // the next level's wide nodes follow this level's, in queue order
-        // (the queue and the node array hold nt entries: a malformed tree
-        // is stopped here)
-        if (q < nt && wide_base + q < nt) {
-          qout[q] = PlaceItem{ref[s], wide_base + q, it.depth + 1, start[s]};
+        // (the queue holds nt entries, the tree n_wide nodes: a malformed
+        // tree is stopped here)
+        if (q < nt && next < n_wide) {
+          qout[q] = PlaceItem{ref[s], next, it.depth + 1, start[s]};
         } else {
           atomicOr(status, J3DG_DEV_BAD_INDEX);
         }
-        out_ref = wide_base + q;
+        out_ref = next;
+        next += sub[s];
         ++q;
       }
     } else {
@@ -870,7 +846,7 @@ __device__ __forceinline__ void collapse_place_one(const uint2* __restrict__ chi
     }
     F[6 * W + s] = __uint_as_float(out_ref);
   }
-  if (it.wide >= nt) {
+  if (it.wide >= n_wide) {
     atomicOr(status, J3DG_DEV_BAD_INDEX);
     return;
   }
@@ -879,33 +855,34 @@ __device__ __forceinline__ void collapse_place_one(const uint2* __restrict__ chi
   for (int k = 0; k < J3DG_NODE_F4(W); ++k) Wn[k] = make_float4(F[4 * k], F[4 * k + 1], F[4 * k + 2], F[4 * k + 3]);
 }
 
-// a level of the placement: the queue's n_in items (device memory) with
-// their wide nodes from wide_base on (device memory); warp-uniform strides
+// a level of the placement: the queue's n_in items (device memory);
+// warp-uniform strides
 template <int W>
-__global__ void k_collapse_place(const uint2* __restrict__ child, const BinNode* __restrict__ box,
-                                 const uint32_t* __restrict__ count, const float4* __restrict__ tris,
+__global__ void k_collapse_place(const BinNode* __restrict__ node, const NodeMeta* __restrict__ meta,
+                                 const BinNode* __restrict__ tbox, const float4* __restrict__ tris,
                                  const PlaceItem* __restrict__ qin, const uint32_t* __restrict__ n_in_p,
                                  PlaceItem* __restrict__ qout, uint32_t* __restrict__ n_out,
-                                 const uint32_t* __restrict__ wide_base_p, float4* __restrict__ wide,
-                                 uint32_t leaf_size, uint32_t* __restrict__ max_depth, float4* __restrict__ tris_out,
-                                 uint32_t nt, uint32_t* status, const uint8_t* __restrict__ dec) {
-  const uint32_t n_in = *n_in_p, wide_base = *wide_base_p;
+                                 const uint32_t* __restrict__ n_wide_p, float4* __restrict__ wide,
+                                 uint32_t* __restrict__ max_depth, float4* __restrict__ tris_out,
+                                 uint32_t* __restrict__ slot_of, uint32_t nt, uint32_t* status) {
+  const uint32_t n_in = *n_in_p, n_wide = *n_wide_p;
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t t0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); t0 < n_in; t0 += stride)
-    collapse_place_one<W>(child, box, count, tris, qin, t0 + (threadIdx.x & 31u), n_in, qout, n_out, wide_base, wide,
-                          leaf_size, max_depth, tris_out, nt, status, dec);
+    collapse_place_one<W>(node, meta, tbox, tris, qin, t0 + (threadIdx.x & 31u), n_in, qout, n_out, n_wide, wide,
+                          max_depth, tris_out, slot_of, nt, status);
 }
 
 // ------------------------------------------------ 7. depth-first order ----
 //
-// The collapse numbers wide nodes level by level, so the nodes on one ray's
-// path from the root to a leaf lie far apart in memory (one per level, each
-// level hundreds of MB wide at the bottom). Renumbering in depth-first order
-// puts every subtree in one contiguous range: the deep part of a path, and
-// the paths of neighbouring rays, then fall in the same few pages. Each
+// The LBVH's collapse numbers wide nodes level by level, so the nodes on one
+// ray's path from the root to a leaf lie far apart in memory (one per level,
+// each level hundreds of MB wide at the bottom). Renumbering in depth-first
+// order puts every subtree in one contiguous range: the deep part of a path,
+// and the paths of neighbouring rays, then fall in the same few pages. Each
 // level is a contiguous index range (a collapse launch allocates exactly the
 // next level), so subtree sizes go bottom-up and new positions top-down, one
-// launch per level.
+// launch per level. (The default builder knows every subtree's size before it
+// makes the wide nodes, and places them in this order at once.)
 
 template <int W>
 __device__ __forceinline__ void child_refs(const float4* __restrict__ wide, uint32_t i, uint32_t (&r)[W]) {
@@ -985,31 +962,20 @@ static uint32_t wave_blocks128() {
   return blocks;
 }
 
-static void launch_collapse_cost(uint32_t W, const uint2* child, const BinNode* box, const uint32_t* count,
-                                 const float4* tris, const uint32_t* list, const uint32_t* lohi, uint32_t leaf_size,
-                                 float* cost, uint8_t* dec, cudaStream_t st) {
-  if (W == 2)
-    k_collapse_cost<2><<<kStrideBlocks, 256, 0, st>>>(child, box, count, tris, list, lohi, leaf_size, cost, dec);
-  else if (W == 8)
-    k_collapse_cost<8><<<kStrideBlocks, 256, 0, st>>>(child, box, count, tris, list, lohi, leaf_size, cost, dec);
-  else
-    k_collapse_cost<4><<<kStrideBlocks, 256, 0, st>>>(child, box, count, tris, list, lohi, leaf_size, cost, dec);
-}
-
-static void launch_collapse_place(uint32_t W, const uint2* child, const BinNode* box, const uint32_t* count,
+static void launch_collapse_place(uint32_t W, const BinNode* node, const NodeMeta* meta, const BinNode* tbox,
                                   const float4* tris, const PlaceItem* qin, const uint32_t* n_in, PlaceItem* qout,
-                                  uint32_t* n_out, const uint32_t* wide_base, float4* wide, uint32_t leaf_size,
-                                  uint32_t* max_depth, float4* tris_out, uint32_t nt, uint32_t* status,
-                                  const uint8_t* dec, cudaStream_t st) {
+                                  uint32_t* n_out, const uint32_t* n_wide, float4* wide, uint32_t* max_depth,
+                                  float4* tris_out, uint32_t* slot_of, uint32_t nt, uint32_t* status, cudaStream_t st) {
+  auto go = [&](auto k) {
+    k<<<wave_blocks128(), 128, 0, st>>>(node, meta, tbox, tris, qin, n_in, qout, n_out, n_wide, wide, max_depth,
+                                        tris_out, slot_of, nt, status);
+  };
   if (W == 2)
-    k_collapse_place<2><<<wave_blocks128(), 128, 0, st>>>(child, box, count, tris, qin, n_in, qout, n_out, wide_base, wide,
-                                                      leaf_size, max_depth, tris_out, nt, status, dec);
+    go(k_collapse_place<2>);
   else if (W == 8)
-    k_collapse_place<8><<<wave_blocks128(), 128, 0, st>>>(child, box, count, tris, qin, n_in, qout, n_out, wide_base, wide,
-                                                      leaf_size, max_depth, tris_out, nt, status, dec);
+    go(k_collapse_place<8>);
   else
-    k_collapse_place<4><<<wave_blocks128(), 128, 0, st>>>(child, box, count, tris, qin, n_in, qout, n_out, wide_base, wide,
-                                                      leaf_size, max_depth, tris_out, nt, status, dec);
+    go(k_collapse_place<4>);
 }
 
 // -------------------------------------------------- 5c. SAH top levels ----
@@ -1086,15 +1052,26 @@ struct TopRange {  // a finished range: a segment for PLOC
   uint32_t begin, end, parent, side;  // parent and side as in TopTask
 };
 
+// the binary tree under construction
+struct Tree {
+  BinNode* node;
+  NodeMeta* meta;
+  uint32_t* up;      // a top node's parent (kNoParent: the root)
+  uint32_t* done;    // a top node's finished children
+  float* cost;       // coverings (W entries) of the top nodes and of the small tasks' roots
+  uint32_t* wide;
+  uint32_t* root;
+  uint32_t* error;
+};
+
 // puts a finished subtree under its parent (or makes it the root)
-__device__ __forceinline__ void link_child(uint2* __restrict__ child, uint32_t* __restrict__ root, uint32_t parent,
-                                           uint32_t side, uint32_t ref) {
+__device__ __forceinline__ void link_child(const Tree& tr, uint32_t parent, uint32_t side, uint32_t ref) {
   if (parent == kNoParent)
-    *root = ref;
+    *tr.root = ref;
   else if (side & 1u)
-    child[parent].y = ref;
+    tr.node[parent].hi.w = __uint_as_float(ref);
   else
-    child[parent].x = ref;
+    tr.node[parent].lo.w = __uint_as_float(ref);
 }
 
 // float <-> uint32 with the same order (for atomic min / max)
@@ -1145,7 +1122,7 @@ struct TopBinner {
 
 // Tasks up to this size leave the level loop for section 5d.
 #ifndef J3DG_SMALL_TASK
-#define J3DG_SMALL_TASK 1024
+#define J3DG_SMALL_TASK 960
 #endif
 static const uint32_t kSmallTask = J3DG_SMALL_TASK;
 
@@ -1163,8 +1140,7 @@ __device__ __forceinline__ float box_half_area(float lx, float ly, float lz, flo
 // split a sweep over the axes and bins in order with a strict comparison
 // takes. Bins with no triangle carry no box (their encoded fields would
 // decode to NaN).
-__device__ uint32_t warp_top_split(const uint32_t* B, const TopTask& T, TopSplit* split, BinNode* __restrict__ box,
-                                   uint32_t* __restrict__ count) {
+__device__ uint32_t warp_top_split(const uint32_t* B, const TopTask& T, TopSplit* split, const Tree& tr) {
   const uint32_t lane = threadIdx.x & 31u, b = lane & 15u;
   const uint32_t n = T.end - T.begin;
   float best = FLT_MAX;
@@ -1289,9 +1265,9 @@ __device__ uint32_t warp_top_split(const uint32_t* B, const TopTask& T, TopSplit
   }
   if (lane == 0) {
     const uint32_t node = T.begin + nleft;
-    box[node].lo = make_float4(nlo[0], nlo[1], nlo[2], 0.f);
-    box[node].hi = make_float4(nhi[0], nhi[1], nhi[2], 0.f);
-    count[node] = n;
+    tr.node[node].lo = make_float4(nlo[0], nlo[1], nlo[2], 0.f);
+    tr.node[node].hi = make_float4(nhi[0], nhi[1], nhi[2], 0.f);
+    tr.meta[node].count = n;
   }
   return nleft;
 }
@@ -1493,7 +1469,7 @@ __global__ void __launch_bounds__(kLevelThreads, J3DG_LEVEL_BLOCKS) k_top_bin(
     const uint32_t* __restrict__ ord, uint32_t* __restrict__ ord2, const BinNode* __restrict__ tbox,
     const TopItem* __restrict__ items, const uint32_t* __restrict__ n_items_p, const TopTask* __restrict__ tasks,
     uint32_t cap_items, uint32_t* __restrict__ bins, uint16_t* __restrict__ code, uint32_t* __restrict__ icum,
-    TopSplit* __restrict__ splits, BinNode* __restrict__ box, uint32_t* __restrict__ count, uint32_t* status) {
+    TopSplit* __restrict__ splits, const Tree tr, uint32_t* status) {
   constexpr uint32_t chunk = K * kLevelThreads;
   extern __shared__ __align__(16) uint8_t top_raw[];
   TopBinMem<K>& s = *reinterpret_cast<TopBinMem<K>*>(top_raw);
@@ -1561,7 +1537,7 @@ __global__ void __launch_bounds__(kLevelThreads, J3DG_LEVEL_BLOCKS) k_top_bin(
     if (T.end - T.begin <= chunk) {
       // the whole task is here
       if (warp == 0) {
-        warp_top_split(sb, T, &s.split, box, count);
+        warp_top_split(sb, T, &s.split, tr);
         __syncwarp();
         if (lane == 0) splits[I.task] = s.split;
       }
@@ -1598,38 +1574,36 @@ __global__ void __launch_bounds__(kLevelThreads, J3DG_LEVEL_BLOCKS) k_top_bin(
 // one warp per task: the split of a task of several items; then the children:
 // a task of the next level above kSmallTask triangles (with its items and, if
 // they are several, empty bins), a small task above J3DG_SAH_TOP, else a
-// finished range; the task's own node goes under its parent and into the list
-// of top nodes
-// counters: [0] top nodes, [1] next tasks, [2] ranges, [3] small tasks, [4] next items
+// finished range; the task's own node goes under its parent
+// counters: [1] next tasks, [2] ranges, [3] small tasks, [4] next items
 __global__ void __launch_bounds__(128) k_top_split(
     const TopTask* __restrict__ tasks, const uint32_t* __restrict__ n_tasks_p, uint32_t chunk,
     const uint32_t* __restrict__ bins, uint32_t* __restrict__ bins2, TopSplit* __restrict__ splits,
     uint32_t* __restrict__ counters, TopTask* __restrict__ next, TopItem* __restrict__ items2,
-    TopTask* __restrict__ small, TopRange* __restrict__ ranges, uint32_t* __restrict__ list, uint2* __restrict__ child,
-    uint32_t* __restrict__ root, BinNode* __restrict__ box, uint32_t* __restrict__ count, uint32_t cap_tasks,
-    uint32_t cap_small, uint32_t cap_items, uint32_t nt, uint32_t* status) {
+    TopTask* __restrict__ small, TopRange* __restrict__ ranges, const Tree tr, uint32_t cap_tasks, uint32_t cap_small,
+    uint32_t cap_items, uint32_t nt, uint32_t* status) {
   const uint32_t n_tasks = min(*n_tasks_p, cap_tasks), lane = threadIdx.x & 31u;
   for (uint32_t t = blockIdx.x * 4u + (threadIdx.x >> 5); t < n_tasks; t += gridDim.x * 4u) {  // whole warps
     const TopTask T = tasks[t];
     const uint32_t n = T.end - T.begin;
     if (n > chunk) {
-      warp_top_split(bins + (size_t)t * kTopBinWords, T, splits + t, box, count);
+      warp_top_split(bins + (size_t)t * kTopBinWords, T, splits + t, tr);
       __syncwarp();
     }
     const TopSplit S = splits[t];
     const uint32_t nl = S.nleft;
     if (nl == 0 || nl >= n) {  // cannot happen: both sides of a split are non-empty
-      if (lane == 0) atomicOr(status, J3DG_DEV_BAD_INDEX);
+      if (lane == 0) {
+        atomicOr(status, J3DG_DEV_BAD_INDEX);
+        atomicOr(tr.error, 1u);
+      }
       continue;
     }
     const uint32_t node = T.begin + nl;
     if (lane == 0) {
-      const uint32_t k = atomicAdd(counters + 0, 1u);
-      if (k < nt)
-        list[k] = node;
-      else
-        atomicOr(status, J3DG_DEV_BAD_INDEX);
-      link_child(child, root, T.parent, T.side, node);
+      tr.up[node] = T.parent;
+      tr.done[node] = 0u;
+      link_child(tr, T.parent, T.side, node);
     }
     for (uint32_t side = 0; side < 2; ++side) {
       const uint32_t b = side ? node : T.begin, e = side ? T.end : node, len = e - b;
@@ -1643,6 +1617,7 @@ __global__ void __launch_bounds__(128) k_top_split(
           if (again) i0 = atomicAdd(counters + 4, m);
           if (q >= (again ? cap_tasks : cap_small) || (again && i0 + m > cap_items)) {
             atomicOr(status, J3DG_DEV_BAD_INDEX);
+            atomicOr(tr.error, 1u);
             q = kNoTask;
           } else {
             TopTask C;
@@ -1659,7 +1634,7 @@ __global__ void __launch_bounds__(128) k_top_split(
           if (q < nt)
             ranges[q] = TopRange{b, e, node, tag};
           else
-            atomicOr(status, J3DG_DEV_BAD_INDEX);
+            atomicOr(tr.error, 1u);
         }
       }
       if (!again) continue;
@@ -1738,7 +1713,7 @@ __global__ void __launch_bounds__(kLevelThreads) k_top_scatter(
 // positions but the first, and what is left at the end tells the segment.
 // The cost of a cluster sits beside it, so the programme reads no memory.
 //
-// Measured (GB300): this kernel 5.9 ms for 28.09M triangles where the levels,
+// Measured (GB300): this kernel 6.2 ms for 28.09M triangles where the levels,
 // rounds and cost passes it replaces took 11.5; builds of 82k / 2M / 28M
 // triangles with their first frame 1.88 -> 1.45, 5.10 -> 4.20 and 33.0 -> 28.4
 // ms. It is bound by instruction issue and latency (40 % of issue slots), so
@@ -1775,14 +1750,18 @@ struct SmallTaskMem {   // while the levels run
 };
 template <int W>
 struct SmallClusterMem {  // while the segments are clustered
-  float cost[W][kSmallTask];
+  float cost[W][kSmallTask];   // a cluster's covering: costs, and wide nodes (at most 63)
+  uint8_t wide[W][kSmallTask];
   uint16_t spare[kSmallTask];  // the cluster's unused node number
   uint8_t cnt[kSmallTask];     // its triangles
   uint8_t nn[kSmallTask];      // its nearest neighbour's offset + kPlocRadius, or 255
 };
 template <int W>
 struct SmallMem {
-  float2 box[3][kSmallTask];     // lo, hi per axis
+  union {
+    float2 box[3][kSmallTask];     // lo, hi per axis
+    uint16_t wide16[W][kSmallTask];  // after the clustering: wide nodes of the segments' roots and the nodes above
+  };
   uint32_t ref[kSmallTask];      // triangle, then cluster reference
   uint16_t seg[kSmallTask];      // each position's segment: its first position
   uint16_t par[kSmallTask];      // at a segment's first position: its parent node << 1 | side, later its cluster
@@ -1813,8 +1792,7 @@ static size_t small_smem() {
 // node in rec
 template <int W>
 __device__ int small_levels(SmallMem<W>& s, uint32_t b0, uint32_t n, uint2* __restrict__ rec,
-                            uint2* __restrict__ child, uint32_t* __restrict__ root, BinNode* __restrict__ box,
-                            uint32_t* __restrict__ count, uint32_t* __restrict__ error, uint32_t* status) {
+                            const Tree& tr, uint32_t* status) {
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const uint32_t K = (n + kSmallThreads - 1) / kSmallThreads, p0 = min(n, tid * K), p1 = min(n, p0 + K);
   int cur = 0;
@@ -1822,7 +1800,7 @@ __device__ int small_levels(SmallMem<W>& s, uint32_t b0, uint32_t n, uint2* __re
     const uint32_t nlt = s.n_task[cur];
     if (nlt == 0) return cur;
     if ((s.task[cur][0].side >> 1) >= kMaxTopLevels) {  // every task of a local level has its level
-      if (tid == 0) atomicOr(error, 1u);
+      if (tid == 0) atomicOr(tr.error, 1u);
       __syncthreads();
       if (tid == 0) s.bad = 1u;
       __syncthreads();
@@ -1859,7 +1837,7 @@ __device__ int small_levels(SmallMem<W>& s, uint32_t b0, uint32_t n, uint2* __re
       }
       __syncthreads();
       for (uint32_t t = warp; t < m; t += kSmallWarps)
-        warp_top_split(s.t.bins + t * kBinWords, s.task[cur][base + t], &s.split[base + t], box, count);
+        warp_top_split(s.t.bins + t * kBinWords, s.task[cur][base + t], &s.split[base + t], tr);
       __syncthreads();
     }
     // the children's tasks
@@ -1867,7 +1845,7 @@ __device__ int small_levels(SmallMem<W>& s, uint32_t b0, uint32_t n, uint2* __re
       const TopTask T = s.task[cur][tid];
       TopSplit& S = s.split[tid];
       const uint32_t mid = T.begin + S.nleft;  // the node's number too
-      link_child(child, root, T.parent, T.side, mid);
+      link_child(tr, T.parent, T.side, mid);
       // at most kSmallTask - 1 nodes: their records fit the task's own range
       const uint32_t r = atomicAdd(&s.n_rec, 1u);
       rec[b0 + r] = make_uint2((T.begin - b0) | ((mid - b0) << 16), (T.end - b0) | (level << 16));
@@ -1954,8 +1932,7 @@ __device__ __forceinline__ float half_area2(const float2 (&a)[3]) {
 // only) until n_seg are left, one a segment, in segment order
 template <int W>
 __device__ uint32_t small_cluster(SmallMem<W>& s, uint32_t b0, uint32_t m, uint32_t n_seg, uint32_t leaf_size,
-                                  uint2* __restrict__ child, BinNode* __restrict__ box, uint32_t* __restrict__ count,
-                                  uint8_t* __restrict__ dec, uint32_t* __restrict__ error) {
+                                  const Tree& tr) {
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, below = (1u << lane) - 1u;
   while (m > n_seg) {
     const uint32_t passes = (m + kSmallThreads - 1) / kSmallThreads;
@@ -2098,7 +2075,14 @@ __device__ uint32_t small_cluster(SmallMem<W>& s, uint32_t b0, uint32_t m, uint3
       const uint32_t pos = s.wsum[pass * kSmallWarps + warp] + __popc(bk & below);
       float2 a[3];
       uint32_t ref = 0, num = 0, sg = 0, spare = 0;
-      float C[W + 1];
+      Covering<W> C;
+      auto covering = [&](uint32_t p, Covering<W>& c) {
+#pragma unroll
+        for (int k = 1; k <= W; ++k) {
+          c.cost[k] = s.c.cost[k - 1][p];
+          c.wide[k] = s.c.wide[k - 1][p];
+        }
+      };
       if (keep) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) a[k] = s.box[k][i];
@@ -2106,30 +2090,25 @@ __device__ uint32_t small_cluster(SmallMem<W>& s, uint32_t b0, uint32_t m, uint3
         num = s.c.cnt[i];
         sg = s.seg[i];
         spare = s.c.spare[i];
-#pragma unroll
-        for (int k = 1; k <= W; ++k) C[k] = s.c.cost[k - 1][i];
+        covering(i, C);
       }
       if (create) {
         const uint32_t j = i + s.c.nn[i] - kPlocRadius, node = b0 + s.c.spare[j];
-        float cr[W + 1], cn[W + 1];
-        uint8_t d[W];
-#pragma unroll
-        for (int k = 1; k <= W; ++k) cr[k] = s.c.cost[k - 1][j];
+        Covering<W> cr, cn;
+        NodeMeta M;
+        covering(j, cr);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
           const float2 b = s.box[k][j];
           a[k] = make_float2(fminf(a[k].x, b.x), fmaxf(a[k].y, b.y));
         }
         num += s.c.cnt[j];
-        collapse_step<W>(C, cr, half_area2(a), num, leaf_size, cn, d);
-        child[node] = make_uint2(ref, s.ref[j]);
-        box[node].lo = make_float4(a[0].x, a[1].x, a[2].x, 0.f);
-        box[node].hi = make_float4(a[0].y, a[1].y, a[2].y, 0.f);
-        count[node] = num;
-        store_dec<W>(dec, node, d);
+        collapse_step<W>(C, cr, half_area2(a), num, leaf_size, cn, M);
+        tr.node[node].lo = make_float4(a[0].x, a[1].x, a[2].x, __uint_as_float(ref));
+        tr.node[node].hi = make_float4(a[0].y, a[1].y, a[2].y, __uint_as_float(s.ref[j]));
+        tr.meta[node] = M;
         ref = node;
-#pragma unroll
-        for (int k = 1; k <= W; ++k) C[k] = cn[k];
+        C = cn;
       }
       __syncthreads();
       if (keep && (create || pos != i)) {
@@ -2140,12 +2119,15 @@ __device__ uint32_t small_cluster(SmallMem<W>& s, uint32_t b0, uint32_t m, uint3
         s.seg[pos] = (uint16_t)sg;
         s.c.spare[pos] = (uint16_t)spare;
 #pragma unroll
-        for (int k = 1; k <= W; ++k) s.c.cost[k - 1][pos] = C[k];
+        for (int k = 1; k <= W; ++k) {
+          s.c.cost[k - 1][pos] = C.cost[k];
+          s.c.wide[k - 1][pos] = (uint8_t)C.wide[k];
+        }
       }
       __syncthreads();
     }
     if (m2 >= m) {  // no pair merges (areas past the largest float)
-      if (tid == 0) atomicOr(error, 2u);
+      if (tid == 0) atomicOr(tr.error, 2u);
       break;
     }
     m = m2;
@@ -2153,14 +2135,57 @@ __device__ uint32_t small_cluster(SmallMem<W>& s, uint32_t b0, uint32_t m, uint3
   return m;
 }
 
+// (The covering carries the wide nodes too: k_collapse_place then writes every
+// wide node where it stays, without the two passes over the levels that
+// counted and numbered them and the permutation: with the top nodes' coverings
+// made below instead of in a pass per level, and the bounding box's last step
+// by a block, builds of 82k and 2M triangles with their first frame went from
+// 1230 to 992 and from 3729 to 3322 us.)
+
+// A small task's subtree is complete: the covering of every top node whose
+// two children are. The second of a node's two to arrive makes it and goes on
+// upwards (the nodes above were made by earlier launches, the coverings by
+// blocks of this one, on any SM).
+template <int W>
+__device__ void climb(const Tree& tr, const BinNode* __restrict__ tbox, uint32_t n, uint32_t leaf_size) {
+  auto covering = [&](uint32_t r, Covering<W>& c) {
+    if (r & 0x80000000u) {
+      const BinNode b = tbox[r & 0x7fffffffu];
+      c.triangle(half_area4(b.lo, b.hi));
+    } else {
+#pragma unroll
+      for (int i = 1; i <= W; ++i) {
+        c.cost[i] = __ldcg(tr.cost + (size_t)r * W + i - 1);
+        c.wide[i] = __ldcg(tr.wide + (size_t)r * W + i - 1);
+      }
+    }
+  };
+  while (n != kNoParent) {
+    __threadfence();
+    if (atomicAdd(tr.done + n, 1u) == 0u) return;
+    __threadfence();
+    const float4 lo = __ldcg(&tr.node[n].lo), hi = __ldcg(&tr.node[n].hi);
+    Covering<W> l, r, c;
+    NodeMeta M;
+    covering(left_ref(lo), l);
+    covering(right_ref(hi), r);
+    collapse_step<W>(l, r, half_area4(lo, hi), tr.meta[n].count, leaf_size, c, M);
+#pragma unroll
+    for (int i = 1; i <= W; ++i) {
+      tr.cost[(size_t)n * W + i - 1] = c.cost[i];
+      tr.wide[(size_t)n * W + i - 1] = c.wide[i];
+    }
+    tr.meta[n] = M;
+    n = tr.up[n];
+  }
+}
+
 template <int W>
 __global__ void __launch_bounds__(kSmallThreads, W == 8 ? J3DG_SMALL_BLOCKS - 1 : J3DG_SMALL_BLOCKS)
     k_small_tasks(const uint32_t* __restrict__ ord_a, const uint32_t* __restrict__ ord_b,
                   const BinNode* __restrict__ tbox, const TopTask* __restrict__ tasks, const TopRange* __restrict__ ranges,
-                  const uint32_t* __restrict__ counters, uint32_t* __restrict__ next_job, uint32_t* __restrict__ error,
-                  uint32_t leaf_size, uint32_t nt, uint32_t cap_small, uint2* __restrict__ rec,
-                  uint2* __restrict__ child, uint32_t* __restrict__ root, BinNode* __restrict__ box,
-                  uint32_t* __restrict__ count, float* __restrict__ cost, uint8_t* __restrict__ dec, uint32_t* status) {
+                  const uint32_t* __restrict__ counters, uint32_t* __restrict__ next_job, uint32_t leaf_size,
+                  uint32_t nt, uint32_t cap_small, uint2* __restrict__ rec, const Tree tr, uint32_t* status) {
   extern __shared__ __align__(16) uint8_t small_raw[];
   SmallMem<W>& s = *reinterpret_cast<SmallMem<W>*>(small_raw);
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -2183,7 +2208,10 @@ __global__ void __launch_bounds__(kSmallThreads, W == 8 ? J3DG_SMALL_BLOCKS - 1 
     }
     const uint32_t b0 = T.begin, n = T.end - T.begin;
     if (T.end > nt || T.begin >= T.end || n > (job < n_tasks ? kSmallTask : J3DG_SAH_TOP)) {  // block-uniform
-      if (tid == 0) atomicOr(status, J3DG_DEV_BAD_INDEX);
+      if (tid == 0) {
+        atomicOr(status, J3DG_DEV_BAD_INDEX);
+        atomicOr(tr.error, 1u);
+      }
       __syncthreads();
       continue;
     }
@@ -2206,7 +2234,7 @@ __global__ void __launch_bounds__(kSmallThreads, W == 8 ? J3DG_SMALL_BLOCKS - 1 
     }
     __syncthreads();
     if (n > J3DG_SAH_TOP) {
-      const int cur = small_levels<W>(s, b0, n, rec, child, root, box, count, error, status);
+      const int cur = small_levels<W>(s, b0, n, rec, tr, status);
       if (s.bad) {
         __syncthreads();
         continue;
@@ -2247,10 +2275,13 @@ __global__ void __launch_bounds__(kSmallThreads, W == 8 ? J3DG_SMALL_BLOCKS - 1 
       const float2 a[3] = {s.box[0][p], s.box[1][p], s.box[2][p]};
       const float v = half_area2(a) * J3DG_SAH_CTRI;
 #pragma unroll
-      for (int k = 0; k < W; ++k) s.c.cost[k][p] = v;
+      for (int k = 0; k < W; ++k) {
+        s.c.cost[k][p] = v;
+        s.c.wide[k][p] = 0;
+      }
     }
     __syncthreads();
-    const uint32_t m = small_cluster<W>(s, b0, n, s.n_seg, leaf_size, child, box, count, dec, error);
+    const uint32_t m = small_cluster<W>(s, b0, n, s.n_seg, leaf_size, tr);
     if (m != s.n_seg) {  // an error was raised: nothing is linked
       __syncthreads();
       continue;
@@ -2260,10 +2291,12 @@ __global__ void __launch_bounds__(kSmallThreads, W == 8 ? J3DG_SMALL_BLOCKS - 1 
     for (uint32_t c = tid; c < m; c += kSmallThreads) {
       const uint32_t first = s.c.spare[c], par = s.par[first];
       if (par == 0xffffu)
-        link_child(child, root, T.parent, T.side, s.ref[c]);
+        link_child(tr, T.parent, T.side, s.ref[c]);
       else
-        link_child(child, root, b0 + (par >> 1), par & 1u, s.ref[c]);
+        link_child(tr, b0 + (par >> 1), par & 1u, s.ref[c]);
       s.par[first] = (uint16_t)c;
+#pragma unroll
+      for (int k = 0; k < W; ++k) s.wide16[k][c] = s.c.wide[k][c];
     }
     __syncthreads();
     // the levels' nodes, deepest first: a subtree's costs are kept at its
@@ -2279,29 +2312,39 @@ __global__ void __launch_bounds__(kSmallThreads, W == 8 ? J3DG_SMALL_BLOCKS - 1 
         if (lane < take) {
           const uint32_t mid = x.x >> 16, node = b0 + mid;
           const uint32_t cb = s.par[x.x & 0xffffu], cm = s.par[mid];
-          float cl[W + 1], cr[W + 1], C[W + 1];
-          uint8_t d[W];
+          Covering<W> l, r, c;
+          NodeMeta M;
 #pragma unroll
           for (int k = 1; k <= W; ++k) {
-            cl[k] = s.c.cost[k - 1][cb];
-            cr[k] = s.c.cost[k - 1][cm];
+            l.cost[k] = s.c.cost[k - 1][cb];
+            r.cost[k] = s.c.cost[k - 1][cm];
+            l.wide[k] = s.wide16[k - 1][cb];
+            r.wide[k] = s.wide16[k - 1][cm];
           }
-          collapse_step<W>(cl, cr, half_area4(box[node].lo, box[node].hi), (x.y & 0xffffu) - (x.x & 0xffffu), leaf_size,
-                           C, d);
+          collapse_step<W>(l, r, half_area4(tr.node[node].lo, tr.node[node].hi), (x.y & 0xffffu) - (x.x & 0xffffu), leaf_size,
+                           c, M);
 #pragma unroll
-          for (int k = 1; k <= W; ++k) s.c.cost[k - 1][cb] = C[k];
-          store_dec<W>(dec, node, d);
+          for (int k = 1; k <= W; ++k) {
+            s.c.cost[k - 1][cb] = c.cost[k];
+            s.wide16[k - 1][cb] = (uint16_t)c.wide[k];
+          }
+          tr.meta[node] = M;
         }
         at -= take;
         __syncwarp();
       }
     }
     __syncthreads();
-    // the task's root under a top node: its costs, for the top nodes' passes
-    if (tid < (uint32_t)W && n > 1u && T.parent != kNoParent) {
-      const uint32_t r = T.side & 1u ? child[T.parent].y : child[T.parent].x;
-      cost[(size_t)r * W + tid] = s.c.cost[tid][s.par[0]];
+    // the task's root: its covering, for the top nodes above it
+    if (tid < (uint32_t)W && n > 1u) {
+      const uint32_t r = T.parent == kNoParent ? *tr.root
+                         : T.side & 1u         ? right_ref(tr.node[T.parent].hi)
+                                               : left_ref(tr.node[T.parent].lo);
+      tr.cost[(size_t)r * W + tid] = s.c.cost[tid][s.par[0]];
+      tr.wide[(size_t)r * W + tid] = s.wide16[tid][s.par[0]];
     }
+    __syncthreads();
+    if (tid == 0) climb<W>(tr, tbox, T.parent, leaf_size);
     __syncthreads();  // the block's memory is free for the next job
   }
 }
@@ -2319,11 +2362,10 @@ __global__ void __launch_bounds__(kSmallThreads, W == 8 ? J3DG_SMALL_BLOCKS - 1 
   } while (0)
 
 // slot_of[id] = leaf position of triangle id (ids are a permutation of 0..nt)
-// (n_wide, if given: the number of wide nodes; 0 when the build failed and placed nothing)
-__global__ void k_slot_of(const float4* __restrict__ tris, uint32_t nt, const uint32_t* __restrict__ n_wide,
-                          uint32_t* __restrict__ slot_of, uint32_t* status) {
+__global__ void k_slot_of(const float4* __restrict__ tris, uint32_t nt, uint32_t* __restrict__ slot_of,
+                          uint32_t* status) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nt || (n_wide && *n_wide == 0u)) return;
+  if (i >= nt) return;
   const uint32_t id = __float_as_uint(tris[3 * (size_t)i].w);
   if (id >= nt) {
     atomicOr(status, J3DG_DEV_BAD_INDEX);
@@ -2358,18 +2400,16 @@ __global__ void k_slot_of(const float4* __restrict__ tris, uint32_t nt, const ui
 static const uint32_t kMaxPlaceLevels = 128;
 
 struct BuildCtl {
-  uint32_t top_ctr[5];  // k_top_split: [0] top nodes, [1] next level's tasks, [2] ranges, [3] small tasks,
+  uint32_t top_ctr[5];  // k_top_split: [1] next level's tasks, [2] ranges, [3] small tasks,
                         // [4] next level's items (LBVH: [0] the root that k_lbvh found)
   uint32_t n_tasks, n_items, top_levels;
   uint32_t root;      // the binary tree's root
   uint32_t next_job;  // the next small task or range to be taken (k_small_tasks)
-  uint32_t lohi[2];  // the running pass's node range (collapse costs, depth-first levels)
-  uint32_t pass, n_pass;
+  uint32_t lohi[2];  // the running pass's node range (LBVH: depth-first levels)
   uint32_t n_in, n_out, n_wide, place_levels, max_depth;
   int32_t dfs_level;
   uint32_t error;  // 1 SAH levels overran their bound, 2 PLOC, 4 placement / collapse
-  uint32_t top_end[kMaxTopLevels];     // top nodes of level L end at top_end[L] (in their list)
-  uint32_t level_end[kMaxPlaceLevels]; // wide nodes of level L end at level_end[L]
+  uint32_t level_end[kMaxPlaceLevels]; // LBVH: wide nodes of level L end at level_end[L]
 };
 
 // the root task, by its size: split level by level, by one block, or a segment
@@ -2406,12 +2446,12 @@ __global__ void k_top_step(BuildCtl* __restrict__ c, uint32_t cap_tasks, uint32_
                            uint32_t nt, cudaGraphConditionalHandle h, uint32_t set) {
   if (c->n_tasks) {  // the level ran
     uint32_t next = c->top_ctr[1];
-    if (next > cap_tasks || c->top_ctr[3] > cap_small || c->top_ctr[2] > nt || c->top_ctr[0] > nt - 1 ||
-        c->top_ctr[4] > cap_items || c->top_levels >= kMaxTopLevels) {
+    if (next > cap_tasks || c->top_ctr[3] > cap_small || c->top_ctr[2] > nt || c->top_ctr[4] > cap_items ||
+        c->top_levels >= kMaxTopLevels) {
       c->error |= 1u;
       next = 0;
     } else {
-      c->top_end[c->top_levels++] = c->top_ctr[0];
+      ++c->top_levels;
     }
     c->n_tasks = next;
     c->n_items = next ? c->top_ctr[4] : 0u;
@@ -2420,47 +2460,27 @@ __global__ void k_top_step(BuildCtl* __restrict__ c, uint32_t cap_tasks, uint32_
   if (set) cudaGraphSetConditional(h, c->n_tasks > 0 ? 1u : 0u);
 }
 
-// pass p of the cost programme: the top levels, deepest first (children before parents)
-__device__ __forceinline__ void cost_range(BuildCtl* c, uint32_t p) {
-  uint32_t lo = 0, hi = 0;
-  if (p < c->n_pass) {
-    const uint32_t k = c->top_levels - 1 - p;
-    lo = k ? c->top_end[k - 1] : 0u;
-    hi = c->top_end[k];
-  }
-  c->lohi[0] = lo;
-  c->lohi[1] = hi;
-}
-
 // the binary tree is complete: the placement starts at its root
-__global__ void k_tree_done(BuildCtl* __restrict__ c, uint32_t nt, PlaceItem* __restrict__ qa) {
-  uint32_t root = c->root;
-  if (root == 0u || root >= nt) {  // a malformed tree (a mesh of one leaf is not built here)
-    c->error |= 2u;
-    root = 0;
+__global__ void k_tree_done(BuildCtl* __restrict__ c, const NodeMeta* __restrict__ meta, uint32_t nt,
+                            PlaceItem* __restrict__ qa) {
+  const uint32_t root = c->root;
+  if (!c->error && (root == 0u || root >= nt || meta[root].wide >= nt)) c->error |= 2u;  // a malformed tree
+  if (c->error) {  // nothing is placed
+    c->n_in = c->n_wide = 0;
+    return;
   }
-  if (c->error) c->n_in = c->n_wide = c->place_levels = 0;  // nothing is placed or numbered
+  c->n_wide = meta[root].wide;
   qa[0] = PlaceItem{root, 0u, 1u, 0u};
-  c->n_pass = c->error ? 0u : c->top_levels;
-  c->pass = 0;
-  cost_range(c, 0);
-}
-
-__global__ void k_cost_step(BuildCtl* __restrict__ c, cudaGraphConditionalHandle h, uint32_t set) {
-  ++c->pass;
-  cost_range(c, c->pass);  // past the last pass: an empty range
-  if (set) cudaGraphSetConditional(h, c->pass < c->n_pass ? 1u : 0u);
 }
 
 __global__ void k_place_step(BuildCtl* __restrict__ c, uint32_t nt, cudaGraphConditionalHandle h, uint32_t set) {
   if (c->n_in) {  // the level ran
     const uint32_t n_out = c->n_out;
-    c->n_wide += n_out;
-    if (c->n_wide > nt || c->place_levels >= kMaxPlaceLevels) {
+    if (n_out > nt || c->place_levels >= kMaxPlaceLevels) {
       c->error |= 4u;
       c->n_in = 0;
     } else {
-      if (n_out) c->level_end[c->place_levels++] = c->n_wide;
+      ++c->place_levels;
       c->n_in = n_out;
     }
     c->n_out = 0;
@@ -2558,7 +2578,7 @@ struct BuildPlan {
   float* bb = nullptr;
   uint64_t *k0 = nullptr, *k1 = nullptr;
   uint32_t *v0 = nullptr, *v1 = nullptr, *hist = nullptr, *sums = nullptr;
-  uint32_t *ord_a = nullptr, *ord_b = nullptr, *top_list = nullptr, *bins_a = nullptr, *bins_b = nullptr,
+  uint32_t *ord_a = nullptr, *ord_b = nullptr, *top_up = nullptr, *top_done = nullptr, *bins_a = nullptr, *bins_b = nullptr,
            *icum = nullptr;
   BinNode* tbox = nullptr;
   uint16_t* codes = nullptr;
@@ -2568,9 +2588,10 @@ struct BuildPlan {
   TopRange* ranges = nullptr;
   uint2* child = nullptr;
   BinNode* box = nullptr;
-  uint32_t* count = nullptr;
+  uint32_t* other = nullptr;  // LBVH: the sibling handshake of k_lbvh
+  NodeMeta* meta = nullptr;
   float* dp_cost = nullptr;
-  uint8_t* dp_dec = nullptr;
+  uint32_t* dp_wide = nullptr;
   float4* wide = nullptr;
   PlaceItem *pa = nullptr, *pb = nullptr;
   uint2* range = nullptr;  // LBVH: each binary node's leaf range
@@ -2587,11 +2608,11 @@ struct BuildPlan {
   uint32_t hist_n() const { return 256 * n_tiles(); }
   uint32_t scan_blocks() const { return (hist_n() + 1023) / 1024; }
   // positions per item of the SAH levels: large ones keep the runs of the
-  // binning long and the bins to merge few; below two items an SM (304 on 152
-  // SMs) smaller items fill the device instead (82k triangles: 160 items of
-  // 512; with 2048 its levels took 23 us a bin pass instead of 7)
+  // binning long and the bins to merge few; below about two items an SM (304
+  // on 152 SMs) smaller items fill the device instead
   uint32_t chunk() const { return nt >= 600000u ? 2048u : (nt >= 300000u ? 1024u : 512u); }
   uint32_t cap_items() const { return nt / chunk() + cap_tasks() + 1; }
+  Tree tree() const { return Tree{box, meta, top_up, top_done, dp_cost, dp_wide, &ctl->root, &ctl->error}; }
 };
 
 static const int kBBoxBlocks = 1024;
@@ -2620,7 +2641,8 @@ static cudaError_t plan_alloc(BuildPlan& P, cudaStream_t st, bool outputs = true
     // (a lane's smaller meshes may have more items, of smaller chunks)
     const uint32_t items = std::max(P.cap_items(), std::min(P.nt, 600000u) / 512u + P.cap_tasks() + 1);
     A(P.codes, sizeof(uint16_t) * std::max((size_t)P.cap_items() * P.chunk(), (size_t)items * 512));
-    A(P.top_list, sizeof(uint32_t) * nt);
+    A(P.top_up, sizeof(uint32_t) * nt);
+    A(P.top_done, sizeof(uint32_t) * nt);
     A(P.bins_a, sizeof(uint32_t) * (size_t)P.cap_tasks() * kTopBinWords);
     A(P.bins_b, sizeof(uint32_t) * (size_t)P.cap_tasks() * kTopBinWords);
     A(P.icum, sizeof(uint32_t) * (size_t)items * 3 * kTopBins);
@@ -2632,24 +2654,27 @@ static cudaError_t plan_alloc(BuildPlan& P, cudaStream_t st, bool outputs = true
     A(P.splits, sizeof(TopSplit) * P.cap_tasks());
     A(P.ranges, sizeof(TopRange) * nt);  // at most one range per triangle
   }
-  A(P.child, sizeof(uint2) * nt);
   A(P.box, sizeof(BinNode) * nt);
-  A(P.count, sizeof(uint32_t) * nt);  // LBVH: the sibling handshake of k_lbvh
   if (P.need_ploc) {
     A(P.dp_cost, sizeof(float) * P.W * nt);
-    A(P.dp_dec, sizeof(uint8_t) * P.W * nt);
+    A(P.dp_wide, sizeof(uint32_t) * P.W * nt);
+    A(P.meta, sizeof(NodeMeta) * nt);
     A(P.pa, sizeof(PlaceItem) * nt);
     A(P.pb, sizeof(PlaceItem) * nt);
     A(P.soup, sizeof(float4) * 3 * nt);  // the LBVH gathers straight into the leaf order
   }
   if (P.need_lbvh) {
+    A(P.child, sizeof(uint2) * nt);
+    A(P.other, sizeof(uint32_t) * nt);
+    A(P.dfs_size, sizeof(uint32_t) * nt);
+    A(P.dfs_pos, sizeof(uint32_t) * nt);
     A(P.range, sizeof(uint2) * (nt - 1));
     A(P.qa, sizeof(CollapseItem) * nt);
     A(P.qb, sizeof(CollapseItem) * nt);
   }
-  A(P.wide, sizeof(float4) * F4 * nt);
-  A(P.dfs_size, sizeof(uint32_t) * nt);
-  A(P.dfs_pos, sizeof(uint32_t) * nt);
+  // the wide nodes at their bound; the default builder writes them straight
+  // into a rebuildable mesh's array instead
+  if (P.need_lbvh || (outputs && !node_bound)) A(P.wide, sizeof(float4) * F4 * nt);
   A(P.ctl, sizeof(BuildCtl));
   if (outputs) {  // else the mesh's own arrays (a rebuild in place)
     A(P.normals, sizeof(float4) * nt);
@@ -2662,9 +2687,9 @@ static cudaError_t plan_alloc(BuildPlan& P, cudaStream_t st, bool outputs = true
 
 // frees the scratch (outputs the caller took over are null)
 static void plan_free(BuildPlan& P, cudaStream_t st) {
-  void* ps[] = {P.part, P.bb, P.k0, P.k1, P.v0, P.v1, P.hist, P.sums, P.ord_a, P.ord_b, P.top_list, P.bins_a,
+  void* ps[] = {P.part, P.bb, P.k0, P.k1, P.v0, P.v1, P.hist, P.sums, P.ord_a, P.ord_b, P.top_up, P.top_done, P.bins_a,
                 P.bins_b, P.icum, P.items_a, P.items_b, P.tbox, P.codes, P.tasks_a, P.tasks_b,
-                P.small, P.splits, P.ranges, P.child, P.box, P.count, P.dp_cost, P.dp_dec, P.wide, P.pa, P.pb, P.range,
+                P.small, P.splits, P.ranges, P.child, P.box, P.other, P.meta, P.dp_cost, P.dp_wide, P.wide, P.pa, P.pb, P.range,
                 P.qa, P.qb, P.dfs_size, P.dfs_pos, P.ctl, P.normals, P.soup, P.tris_out, P.nodes, P.slot_of};
   for (void* p : ps)
     if (p) cudaFreeAsync(p, st);
@@ -2686,8 +2711,8 @@ static void launch_top_bin_k(BuildPlan& P, cudaStream_t s, const uint32_t* oi, u
   const uint32_t blocks = std::min(wave_blocks128() / 16u * J3DG_LEVEL_BLOCKS, P.cap_items());
   cudaFuncSetAttribute(k_top_bin<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TopBinMem<K>));
   k_top_bin<K><<<blocks, kLevelThreads, sizeof(TopBinMem<K>), s>>>(oi, oo, P.tbox, items, &c->n_items, tasks,
-                                                                   P.cap_items(), bins, P.codes, P.icum, P.splits, P.box,
-                                                                   P.count, d_status);
+                                                                   P.cap_items(), bins, P.codes, P.icum, P.splits,
+                                                                   P.tree(), d_status);
 }
 static void launch_top_bin(BuildPlan& P, cudaStream_t s, const uint32_t* oi, uint32_t* oo, const TopItem* items,
                            const TopTask* tasks, uint32_t* bins, uint32_t* d_status) {
@@ -2728,9 +2753,8 @@ static cudaError_t launch_small_tasks_w(BuildPlan& P, cudaStream_t st, uint32_t*
   if (e != cudaSuccess) return e;
   const uint32_t grid = std::min((uint32_t)std::max(1, sms * per), P.cap_small());
   k_small_tasks<W><<<grid, kSmallThreads, smem, st>>>(
-      P.ord_a, P.ord_b, P.tbox, P.small, P.ranges, c->top_ctr, &c->next_job, &c->error,
-      P.leaf, P.nt, P.cap_small(), reinterpret_cast<uint2*>(P.pb), P.child, &c->root, P.box, P.count, P.dp_cost, P.dp_dec,
-      d_status);
+      P.ord_a, P.ord_b, P.tbox, P.small, P.ranges, c->top_ctr, &c->next_job, P.leaf, P.nt, P.cap_small(),
+      reinterpret_cast<uint2*>(P.pb), P.tree(), d_status);
   return cudaGetLastError();
 }
 
@@ -2740,11 +2764,12 @@ static cudaError_t launch_small_tasks(uint32_t W, BuildPlan& P, cudaStream_t st,
   return launch_small_tasks_w<4>(P, st, d_status);
 }
 
-// the default builder's binary tree and wide nodes (P.wide, level ranges in
-// c->level_end): binned-SAH levels down to small tasks, each small task's
-// subtree by one block, the cost programme of the top nodes, the placement;
-// the leaf-ordered triangles go to P.tris_out
-static cudaError_t enqueue_tree_ploc(BuildPlan& P, cudaStream_t st, cudaStream_t side, uint32_t* d_status) {
+// the default builder's binary tree and its wide nodes (`wide`, in depth-first
+// order): binned-SAH levels down to small tasks, each small task's subtree by
+// one block (and the cost programme up to the root), the placement; the
+// leaf-ordered triangles go to P.tris_out, their positions to P.slot_of
+static cudaError_t enqueue_tree_ploc(BuildPlan& P, float4* wide, cudaStream_t st, cudaStream_t side,
+                                     uint32_t* d_status) {
   const uint32_t nt = P.nt, W = P.W;
   BuildCtl* c = P.ctl;
   cudaError_t e = cudaSuccess;
@@ -2760,8 +2785,8 @@ static cudaError_t enqueue_tree_ploc(BuildPlan& P, cudaStream_t st, cudaStream_t
                      uint32_t* oi, uint32_t* oo) {
       launch_top_bin(P, s, oi, oo, ii, ti, bi, d_status);
       k_top_split<<<split_blocks, 128, 0, s>>>(ti, &c->n_tasks, chunk, bi, bo, P.splits, c->top_ctr, to, io, P.small,
-                                               P.ranges, P.top_list, P.child, &c->root, P.box, P.count, P.cap_tasks(),
-                                               P.cap_small(), P.cap_items(), nt, d_status);
+                                               P.ranges, P.tree(), P.cap_tasks(), P.cap_small(), P.cap_items(), nt,
+                                               d_status);
       launch_top_scatter(P, s, oi, oo, ii, ti, d_status);
     };
     J3DG_EQ(capture_while(st, side, [&](cudaStream_t s, cudaGraphConditionalHandle h) {
@@ -2772,23 +2797,17 @@ static cudaError_t enqueue_tree_ploc(BuildPlan& P, cudaStream_t st, cudaStream_t
     }));
   }
   J3DG_EQ(launch_small_tasks(W, P, st, d_status));
-  k_tree_done<<<1, 1, 0, st>>>(c, nt, P.pa);
+  k_tree_done<<<1, 1, 0, st>>>(c, P.meta, nt, P.pa);
   J3DG_EQ(cudaSuccess);
-  // the top nodes' cost programme, children before parents
-  if (nt > kSmallTask)
-    J3DG_EQ(capture_while(st, side, [&](cudaStream_t s, cudaGraphConditionalHandle h) {
-      launch_collapse_cost(W, P.child, P.box, P.count, soup, P.top_list, c->lohi, P.leaf, P.dp_cost, P.dp_dec, s);
-      k_cost_step<<<1, 1, 0, s>>>(c, h, 0u);
-      launch_collapse_cost(W, P.child, P.box, P.count, soup, P.top_list, c->lohi, P.leaf, P.dp_cost, P.dp_dec, s);
-      k_cost_step<<<1, 1, 0, s>>>(c, h, 1u);
-    }));
   // placement, level by level
+  auto place = [&](cudaStream_t s, const PlaceItem* qi, PlaceItem* qo) {
+    launch_collapse_place(W, P.box, P.meta, P.tbox, soup, qi, &c->n_in, qo, &c->n_out, &c->n_wide, wide, &c->max_depth,
+                          P.tris_out, P.slot_of, nt, d_status, s);
+  };
   J3DG_EQ(capture_while(st, side, [&](cudaStream_t s, cudaGraphConditionalHandle h) {
-    launch_collapse_place(W, P.child, P.box, P.count, soup, P.pa, &c->n_in, P.pb, &c->n_out, &c->n_wide, P.wide,
-                          P.leaf, &c->max_depth, P.tris_out, nt, d_status, P.dp_dec, s);
+    place(s, P.pa, P.pb);
     k_place_step<<<1, 1, 0, s>>>(c, nt, h, 0u);
-    launch_collapse_place(W, P.child, P.box, P.count, soup, P.pb, &c->n_in, P.pa, &c->n_out, &c->n_wide, P.wide,
-                          P.leaf, &c->max_depth, P.tris_out, nt, d_status, P.dp_dec, s);
+    place(s, P.pb, P.pa);
     k_place_step<<<1, 1, 0, s>>>(c, nt, h, 1u);
   }));
   return e;
@@ -2802,8 +2821,8 @@ static cudaError_t enqueue_tree_lbvh(BuildPlan& P, const uint64_t* keys, cudaStr
   const uint32_t nt = P.nt;
   BuildCtl* c = P.ctl;
   cudaError_t e = cudaSuccess;
-  J3DG_EQ(cudaMemsetAsync(P.count, 0xff, sizeof(uint32_t) * (nt - 1), st));
-  k_lbvh<<<(nt + 255) / 256, 256, 0, st>>>(keys, P.tris_out, nt, P.child, P.box, P.range, P.count, &c->top_ctr[0]);
+  J3DG_EQ(cudaMemsetAsync(P.other, 0xff, sizeof(uint32_t) * (nt - 1), st));
+  k_lbvh<<<(nt + 255) / 256, 256, 0, st>>>(keys, P.tris_out, nt, P.child, P.box, P.range, P.other, &c->top_ctr[0]);
   k_lbvh_root<<<1, 1, 0, st>>>(c, P.qa);
   J3DG_EQ(cudaSuccess);
   J3DG_EQ(capture_while(st, side, [&](cudaStream_t s, cudaGraphConditionalHandle h) {
@@ -2830,7 +2849,7 @@ static cudaError_t enqueue_prefix(BuildPlan& P, const float* dV, const uint32_t*
   cudaError_t e = cudaSuccess;
   J3DG_EQ(cudaMemsetAsync(c, 0, sizeof(BuildCtl), st));
   k_bbox_partial<<<kBBoxBlocks, 256, 0, st>>>(dV, nv, P.part);
-  k_bbox_final<<<1, 32, 0, st>>>(P.part, kBBoxBlocks, P.bb);
+  k_bbox_final<<<1, 1024, 0, st>>>(P.part, kBBoxBlocks, P.bb);
   k_ctl_init<<<1, 1, 0, st>>>(c, P.tasks_a, P.small, P.ranges, P.bb, nt, P.top ? 1u : 0u, P.chunk());
   k_tri_prep<<<(nt + 255) / 256, 256, 0, st>>>(dV, nv, dT, nt, P.bb, P.normals, P.k0, P.v0, d_status);
   J3DG_EQ(cudaSuccess);
@@ -2853,43 +2872,33 @@ static cudaError_t enqueue_prefix(BuildPlan& P, const float* dV, const uint32_t*
   return e;
 }
 
-// The rest: the tree, its wide nodes, the depth-first numbering (and, with
-// `permute`, the nodes written in that order into P.nodes) and the
-// triangles' slots; its level loops are conditional while nodes, so `st`
-// must be capturing.
-static cudaError_t enqueue_tree(BuildPlan& P, cudaStream_t st, cudaStream_t side, uint32_t* d_status,
-                                bool permute = true) {
-  const uint32_t nt = P.nt, W = P.W;
+// The rest: the tree, its wide nodes in depth-first order and the triangles'
+// slots; its level loops are conditional while nodes, so `st` must be
+// capturing. The nodes go to P.nodes where it is given, else to P.wide (LBVH:
+// the permutation into depth-first order is then left to the caller).
+static cudaError_t enqueue_tree(BuildPlan& P, cudaStream_t st, cudaStream_t side, uint32_t* d_status) {
+  const uint32_t nt = P.nt;
   BuildCtl* c = P.ctl;
   cudaError_t e = cudaSuccess;
-  J3DG_EQ(P.lbvh ? enqueue_tree_lbvh(P, sorted_keys(P), st, side, d_status)
-                 : enqueue_tree_ploc(P, st, side, d_status));
+  if (!P.lbvh) return enqueue_tree_ploc(P, P.nodes ? P.nodes : P.wide, st, side, d_status);
+  J3DG_EQ(enqueue_tree_lbvh(P, sorted_keys(P), st, side, d_status));
   // depth-first numbering: subtree sizes bottom-up, positions top-down, permute
-  auto dfs = [&](auto Wc) {
-    constexpr int WW = decltype(Wc)::value;
-    k_dfs_setup<<<1, 1, 0, st>>>(c, P.dfs_pos, 0u);
-    J3DG_EQ(capture_while(st, side, [&](cudaStream_t s, cudaGraphConditionalHandle h) {
-      k_dfs_size<WW><<<kStrideBlocks, 256, 0, s>>>(P.wide, c->lohi, P.dfs_size);
-      k_dfs_step<<<1, 1, 0, s>>>(c, 0u, h, 0u);
-      k_dfs_size<WW><<<kStrideBlocks, 256, 0, s>>>(P.wide, c->lohi, P.dfs_size);
-      k_dfs_step<<<1, 1, 0, s>>>(c, 0u, h, 1u);
-    }));
-    k_dfs_setup<<<1, 1, 0, st>>>(c, P.dfs_pos, 1u);
-    J3DG_EQ(capture_while(st, side, [&](cudaStream_t s, cudaGraphConditionalHandle h) {
-      k_dfs_place<WW><<<kStrideBlocks, 256, 0, s>>>(P.wide, c->lohi, P.dfs_size, P.dfs_pos);
-      k_dfs_step<<<1, 1, 0, s>>>(c, 1u, h, 0u);
-      k_dfs_place<WW><<<kStrideBlocks, 256, 0, s>>>(P.wide, c->lohi, P.dfs_size, P.dfs_pos);
-      k_dfs_step<<<1, 1, 0, s>>>(c, 1u, h, 1u);
-    }));
-    if (permute) k_dfs_permute<WW><<<(nt + 255) / 256, 256, 0, st>>>(P.wide, &c->n_wide, P.dfs_pos, P.nodes);
-  };
-  if (W == 2)
-    dfs(std::integral_constant<int, 2>());
-  else if (W == 8)
-    dfs(std::integral_constant<int, 8>());
-  else
-    dfs(std::integral_constant<int, 4>());
-  k_slot_of<<<(nt + 255) / 256, 256, 0, st>>>(P.tris_out, nt, &c->n_wide, P.slot_of, d_status);
+  k_dfs_setup<<<1, 1, 0, st>>>(c, P.dfs_pos, 0u);
+  J3DG_EQ(capture_while(st, side, [&](cudaStream_t s, cudaGraphConditionalHandle h) {
+    k_dfs_size<4><<<kStrideBlocks, 256, 0, s>>>(P.wide, c->lohi, P.dfs_size);
+    k_dfs_step<<<1, 1, 0, s>>>(c, 0u, h, 0u);
+    k_dfs_size<4><<<kStrideBlocks, 256, 0, s>>>(P.wide, c->lohi, P.dfs_size);
+    k_dfs_step<<<1, 1, 0, s>>>(c, 0u, h, 1u);
+  }));
+  k_dfs_setup<<<1, 1, 0, st>>>(c, P.dfs_pos, 1u);
+  J3DG_EQ(capture_while(st, side, [&](cudaStream_t s, cudaGraphConditionalHandle h) {
+    k_dfs_place<4><<<kStrideBlocks, 256, 0, s>>>(P.wide, c->lohi, P.dfs_size, P.dfs_pos);
+    k_dfs_step<<<1, 1, 0, s>>>(c, 1u, h, 0u);
+    k_dfs_place<4><<<kStrideBlocks, 256, 0, s>>>(P.wide, c->lohi, P.dfs_size, P.dfs_pos);
+    k_dfs_step<<<1, 1, 0, s>>>(c, 1u, h, 1u);
+  }));
+  if (P.nodes) k_dfs_permute<4><<<(nt + 255) / 256, 256, 0, st>>>(P.wide, &c->n_wide, P.dfs_pos, P.nodes);
+  k_slot_of<<<(nt + 255) / 256, 256, 0, st>>>(P.tris_out, nt, P.slot_of, d_status);
   J3DG_EQ(cudaSuccess);
   return e;
 }
@@ -2930,7 +2939,7 @@ static int build_bvh_graph(j3dg_mesh* m, const float* dV, const uint32_t* dT, cu
   if (e == cudaSuccess) e = enqueue_prefix(P, dV, dT, st, d_status);
   if (e == cudaSuccess) e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    const cudaError_t eq = enqueue_tree(P, st, side, d_status, false);
+    const cudaError_t eq = enqueue_tree(P, st, side, d_status);
     e = cudaStreamEndCapture(st, &g);
     if (eq != cudaSuccess) e = eq;
   }
@@ -2958,27 +2967,25 @@ static int build_bvh_graph(j3dg_mesh* m, const float* dV, const uint32_t* dT, cu
     m->n_nodes = h.n_wide;
     m->max_depth = h.max_depth;
     m->root_ref = 0;
-    // the nodes in depth-first order into an array of the tree's size (a
-    // rebuildable mesh keeps the array at the size bound: rebuilds write in
-    // place)
+    // the nodes into an array of the tree's size (a rebuildable mesh keeps the
+    // array at the size bound: its nodes are there already)
     const size_t bytes = sizeof(float4) * J3DG_NODE_F4(P.W) * (size_t)m->n_nodes;
     if (m->build_flags & J3DG_BUILD_REBUILDABLE) {
       m->d_nodes = P.nodes;
       P.nodes = nullptr;
     } else {
+      // the gathered triangles are not needed any more: their memory goes to
+      // the nodes (as an addition to the pool these took 0.85 ms at 778 MB)
+      if (P.soup) cudaFreeAsync(P.soup, st);
+      P.soup = nullptr;
       e = cudaMallocAsync(&m->d_nodes, bytes ? bytes : sizeof(float4) * J3DG_NODE_F4(P.W), st);
     }
-    if (e == cudaSuccess) {
-      float4* out = (float4*)m->d_nodes;
-      const uint32_t grid = (m->n_nodes + 255) / 256;
-      if (grid) {
-        if (P.W == 2)
-          k_dfs_permute<2><<<grid, 256, 0, st>>>(P.wide, &P.ctl->n_wide, P.dfs_pos, out);
-        else if (P.W == 8)
-          k_dfs_permute<8><<<grid, 256, 0, st>>>(P.wide, &P.ctl->n_wide, P.dfs_pos, out);
-        else
-          k_dfs_permute<4><<<grid, 256, 0, st>>>(P.wide, &P.ctl->n_wide, P.dfs_pos, out);
+    if (e == cudaSuccess && !(m->build_flags & J3DG_BUILD_REBUILDABLE) && m->n_nodes) {
+      if (P.lbvh) {
+        k_dfs_permute<4><<<(m->n_nodes + 255) / 256, 256, 0, st>>>(P.wide, &P.ctl->n_wide, P.dfs_pos, (float4*)m->d_nodes);
         e = cudaGetLastError();
+      } else {
+        e = cudaMemcpyAsync(m->d_nodes, P.wide, bytes, cudaMemcpyDeviceToDevice, st);
       }
     }
     if (e == cudaSuccess && done) e = cudaEventRecord(done, st);  // the BVH is ready; the rest is clean-up
@@ -3093,7 +3100,7 @@ int build_bvh(j3dg_mesh* m, const float* dV, const uint32_t* dT, cudaStream_t st
   J3DG_CK(cudaMallocAsync((void**)&d_part, sizeof(float) * 6 * bbox_blocks, st));
   J3DG_CK(cudaMallocAsync((void**)&d_bb, sizeof(float) * 6, st));
   k_bbox_partial<<<bbox_blocks, 256, 0, st>>>(dV, nv, d_part);
-  k_bbox_final<<<1, 32, 0, st>>>(d_part, bbox_blocks, d_bb);
+  k_bbox_final<<<1, 1024, 0, st>>>(d_part, bbox_blocks, d_bb);
   J3DG_CK(cudaGetLastError());
   J3DG_CK(cudaMemcpyAsync(hbb, d_bb, sizeof(hbb), cudaMemcpyDeviceToHost, st));
   J3DG_CK(cudaStreamSynchronize(st));
@@ -3119,7 +3126,7 @@ int build_bvh(j3dg_mesh* m, const float* dV, const uint32_t* dT, cudaStream_t st
   J3DG_CK(cudaMallocAsync(&m->d_nodes, sizeof(float4) * F4, st));
   J3DG_CK(cudaMemsetAsync(m->d_nodes, 0, sizeof(float4) * F4, st));
   J3DG_CK(cudaMallocAsync(&m->d_slot_of, sizeof(uint32_t) * (size_t)nt, st));
-  k_slot_of<<<1, 256, 0, st>>>((const float4*)m->d_tris, nt, nullptr, (uint32_t*)m->d_slot_of, d_status);
+  k_slot_of<<<1, 256, 0, st>>>((const float4*)m->d_tris, nt, (uint32_t*)m->d_slot_of, d_status);
   J3DG_CK(cudaGetLastError());
   if (done) J3DG_CK(cudaEventRecord(done, st));
 
