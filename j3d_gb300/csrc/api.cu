@@ -809,7 +809,7 @@ int mesh_build_on(j3dg_ctx* c, const float* V, uint32_t nv, const uint32_t* T, u
   float* dV = nullptr;
   bool ownV = false;
   int rc = J3DG_OK;
-  cudaError_t e = cudaMalloc(&m->d_index, sizeof(uint32_t) * 3 * (size_t)nt);
+  cudaError_t e = cudaMallocAsync(&m->d_index, sizeof(uint32_t) * 3 * (size_t)nt, st);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(m->d_index, T, sizeof(uint32_t) * 3 * (size_t)nt,
                         is_device_ptr(T) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st);

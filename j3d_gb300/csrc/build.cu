@@ -26,6 +26,7 @@
 // topology-independence argument requires.
 #include <cuda_runtime.h>
 #include <float.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #include <algorithm>
@@ -615,6 +616,37 @@ __device__ __forceinline__ float merged_area(float4 alo, float4 ahi, float4 blo,
   return a == a ? a : FLT_MAX;  // boxes with NaN planes still get an order
 }
 
+// ------------------------------------------------ a build's loop state ----
+
+static const uint32_t kMaxTopLevels = 1024;  // SAH levels of a tree, top and small together
+static const uint32_t kMaxPlaceLevels = 128;
+
+// In device memory. A level's kernels read their sizes from its entry and add
+// to the next one's: level `base + k` for the k that the launch gives (the
+// bases move only in the loops of a captured build). The first part is what
+// the host reads.
+struct BuildCtl {
+  float bb[6];
+  uint32_t n_wide, max_depth;
+  uint32_t error;     // 1 SAH levels overran their bound, 2 PLOC, 4 placement / collapse
+  uint32_t top_left;  // tasks that wait for more SAH levels than were launched
+  uint32_t place[kMaxPlaceLevels + 1];  // subtrees to be placed, by level
+  uint32_t root;                        // the binary tree's root
+  uint32_t top_base, place_base;
+  uint32_t n_small, n_ranges;           // small tasks and finished ranges
+  uint32_t next_job;                    // the next of them to be taken (k_small_tasks)
+  struct Level {
+    uint32_t tasks, items;
+  };
+  __align__(8) Level top[kMaxTopLevels + 1];
+  // the LBVH's loops
+  uint32_t lohi[2];  // the running pass's node range
+  uint32_t n_in, n_out, place_levels;
+  int32_t dfs_level;
+  uint32_t level_end[kMaxPlaceLevels];  // wide nodes of level L end at level_end[L]
+};
+static const size_t kCtlHead = offsetof(BuildCtl, root);
+
 // ------------------------------------------- 6b. cost-optimal collapse ----
 //
 // SAH cost of covering the subtree of binary node n with at most i = 1..4
@@ -855,23 +887,6 @@ __device__ __forceinline__ void collapse_place_one(const BinNode* __restrict__ n
   for (int k = 0; k < J3DG_NODE_F4(W); ++k) Wn[k] = make_float4(F[4 * k], F[4 * k + 1], F[4 * k + 2], F[4 * k + 3]);
 }
 
-// a level of the placement: the queue's n_in items (device memory);
-// warp-uniform strides
-template <int W>
-__global__ void k_collapse_place(const BinNode* __restrict__ node, const NodeMeta* __restrict__ meta,
-                                 const BinNode* __restrict__ tbox, const float4* __restrict__ tris,
-                                 const PlaceItem* __restrict__ qin, const uint32_t* __restrict__ n_in_p,
-                                 PlaceItem* __restrict__ qout, uint32_t* __restrict__ n_out,
-                                 const uint32_t* __restrict__ n_wide_p, float4* __restrict__ wide,
-                                 uint32_t* __restrict__ max_depth, float4* __restrict__ tris_out,
-                                 uint32_t* __restrict__ slot_of, uint32_t nt, uint32_t* status) {
-  const uint32_t n_in = *n_in_p, n_wide = *n_wide_p;
-  const uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t t0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); t0 < n_in; t0 += stride)
-    collapse_place_one<W>(node, meta, tbox, tris, qin, t0 + (threadIdx.x & 31u), n_in, qout, n_out, n_wide, wide,
-                          max_depth, tris_out, slot_of, nt, status);
-}
-
 // ------------------------------------------------ 7. depth-first order ----
 //
 // The LBVH's collapse numbers wide nodes level by level, so the nodes on one
@@ -962,13 +977,30 @@ static uint32_t wave_blocks128() {
   return blocks;
 }
 
+// level `base + k` of the placement; warp-uniform strides
+template <int W>
+__global__ void k_collapse_place(const BinNode* __restrict__ node, const NodeMeta* __restrict__ meta,
+                                 const BinNode* __restrict__ tbox, const float4* __restrict__ tris,
+                                 const PlaceItem* __restrict__ qin, PlaceItem* __restrict__ qout,
+                                 BuildCtl* __restrict__ c, uint32_t k, float4* __restrict__ wide,
+                                 float4* __restrict__ tris_out, uint32_t* __restrict__ slot_of, uint32_t nt,
+                                 uint32_t* status) {
+  const uint32_t L = c->place_base + k;
+  if (L >= kMaxPlaceLevels) return;
+  const uint32_t n_in = min(c->place[L], nt), n_wide = c->n_wide;
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint32_t t0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); t0 < n_in; t0 += stride)
+    collapse_place_one<W>(node, meta, tbox, tris, qin, t0 + (threadIdx.x & 31u), n_in, qout, &c->place[L + 1], n_wide,
+                          wide, &c->max_depth, tris_out, slot_of, nt, status);
+}
+
 static void launch_collapse_place(uint32_t W, const BinNode* node, const NodeMeta* meta, const BinNode* tbox,
-                                  const float4* tris, const PlaceItem* qin, const uint32_t* n_in, PlaceItem* qout,
-                                  uint32_t* n_out, const uint32_t* n_wide, float4* wide, uint32_t* max_depth,
-                                  float4* tris_out, uint32_t* slot_of, uint32_t nt, uint32_t* status, cudaStream_t st) {
-  auto go = [&](auto k) {
-    k<<<wave_blocks128(), 128, 0, st>>>(node, meta, tbox, tris, qin, n_in, qout, n_out, n_wide, wide, max_depth,
-                                        tris_out, slot_of, nt, status);
+                                  const float4* tris, const PlaceItem* qin, PlaceItem* qout, BuildCtl* c, uint32_t k,
+                                  float4* wide, float4* tris_out, uint32_t* slot_of, uint32_t nt, uint32_t* status,
+                                  cudaStream_t st) {
+  auto go = [&](auto kernel) {
+    kernel<<<wave_blocks128(), 128, 0, st>>>(node, meta, tbox, tris, qin, qout, c, k, wide, tris_out, slot_of, nt,
+                                             status);
   };
   if (W == 2)
     go(k_collapse_place<2>);
@@ -1015,8 +1047,6 @@ static_assert(kTopBins <= 16, "bin codes keep 4 bits per axis");
 // task the two ranges differ by about one triangle
 static const int kTopVals = 7;
 static const uint32_t kNoTask = 0xffffffffu;
-static const uint32_t kMaxTopLevels = 1024;  // SAH levels of a tree, top and small together
-
 static const uint32_t kNoParent = 0xffffffffu;  // the parent of the root
 
 struct TopTask {
@@ -1031,7 +1061,7 @@ struct TopSplit {
   uint32_t bin;    // bins 0..bin go left
   uint32_t nleft;
   uint32_t pad;
-  uint32_t task[2];  // the children's tasks of the next level (kNoTask: a finished range)
+  uint32_t task[2];  // section 5d: the children's tasks of the next level (255: a finished range)
   uint32_t pad2[2];
   float4 lclo, lchi, rclo, rchi;  // children's centroid bounds
 };
@@ -1132,7 +1162,7 @@ __device__ __forceinline__ float box_half_area(float lx, float ly, float lz, flo
 }
 
 // One warp: the split of least SAH cost A_L N_L + A_R N_R over the task's
-// bins B ([axis][bin][kTopVals], shared or global memory); writes the split,
+// bins B ([axis][bin][kTopVals], in shared memory); writes the split,
 // the node's box and its triangle count, and returns its left count
 // (warp-uniform). Lanes b and b + 16 hold bin b of
 // the axis in hand; prefix and suffix unions of the bins come from shuffles
@@ -1281,6 +1311,7 @@ struct TopItem {
 };
 static const int kLevelThreads = 256;
 static const uint32_t kTopBinWords = 3 * kTopBins * kTopVals;
+static const uint32_t kTopBinRow = kTopBinWords + 4;  // a task's bins in global memory, then its items done
 
 __device__ __forceinline__ uint32_t top_bin_empty(uint32_t k) {  // word k of a task's empty bins
   const uint32_t v = k % kTopVals;
@@ -1293,7 +1324,7 @@ __global__ void k_top_items(TopItem* __restrict__ items, uint32_t* __restrict__ 
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_items; i += gridDim.x * blockDim.x)
     items[i] = TopItem{0u, 0u, i * chunk, min(chunk, nt - i * chunk)};
   if (blockIdx.x == 0)
-    for (uint32_t k = threadIdx.x; k < kTopBinWords; k += blockDim.x) bins[k] = top_bin_empty(k);
+    for (uint32_t k = threadIdx.x; k < kTopBinRow; k += blockDim.x) bins[k] = k < kTopBinWords ? top_bin_empty(k) : 0u;
 }
 
 // adds a box of ordered-float codes (n of them) to a bin
@@ -1427,14 +1458,94 @@ __device__ __forceinline__ void partition_item(const TopSplit& S, uint32_t begin
   }
 }
 
+// where a level's tasks leave the next level's
+struct NextLevel {
+  TopTask* tasks;
+  TopItem* items;
+  uint32_t* bins;
+  TopTask* small;
+  TopRange* ranges;
+  uint32_t cap_tasks, cap_small, cap_items, nt;
+};
+
+// One warp, after the split S of task T: the children, lanes 0 and 1 one
+// each: a task of the next level above kSmallTask triangles (with its items
+// and, if they are several, empty bins), a small task above J3DG_SAH_TOP, else
+// a finished range; the task's own node goes under its parent.
+__device__ void warp_children(const TopTask& T, const TopSplit& S, uint32_t chunk, const NextLevel& N,
+                              BuildCtl* __restrict__ c, uint32_t level, const Tree& tr, uint32_t* status) {
+  const uint32_t lane = threadIdx.x & 31u, n = T.end - T.begin, nl = S.nleft;
+  if (nl == 0 || nl >= n) {  // (a split leaves both sides something: bins with a triangle on both)
+    if (lane == 0) {
+      atomicOr(status, J3DG_DEV_BAD_INDEX);
+      atomicOr(tr.error, 1u);
+    }
+    return;
+  }
+  const uint32_t node = T.begin + nl;
+  const uint32_t b = (lane & 1u) ? node : T.begin, e = (lane & 1u) ? T.end : node, len = e - b;
+  const uint32_t m = (len + chunk - 1) / chunk;
+  uint32_t q = kNoTask, i0 = 0;
+  if (lane < 2) {
+    const uint32_t tag = lane | (((T.side >> 1) + 1u) << 1);
+    if (len > J3DG_SAH_TOP) {
+      const bool again = len > kSmallTask;
+      if (again) {  // the task and its items in one atomic
+        const unsigned long long at = atomicAdd(reinterpret_cast<unsigned long long*>(&c->top[level + 1]),
+                                                1ull | ((unsigned long long)m << 32));
+        q = (uint32_t)at;
+        i0 = (uint32_t)(at >> 32);
+      } else {
+        q = atomicAdd(&c->n_small, 1u);
+      }
+      if (q >= (again ? N.cap_tasks : N.cap_small) ||
+          (again && (i0 + m > N.cap_items || level + 1u >= kMaxTopLevels))) {
+        atomicOr(tr.error, 1u);
+        q = kNoTask;
+      } else {
+        TopTask C;
+        C.begin = b;
+        C.end = e;
+        C.parent = node;
+        C.side = tag;
+        C.clo = lane ? S.rclo : S.lclo;
+        C.chi = lane ? S.rchi : S.lchi;
+        (again ? N.tasks : N.small)[q] = C;
+        if (!again) q = kNoTask;
+      }
+    } else {
+      const uint32_t r = atomicAdd(&c->n_ranges, 1u);
+      if (r < N.nt)
+        N.ranges[r] = TopRange{b, e, node, tag};
+      else
+        atomicOr(tr.error, 1u);
+    }
+  }
+  if (lane == 2) {
+    tr.up[node] = T.parent;
+    tr.done[node] = 0u;
+    link_child(tr, T.parent, T.side, node);
+  }
+  for (int side = 0; side < 2; ++side) {
+    const uint32_t qs = __shfl_sync(0xffffffffu, q, side), is = __shfl_sync(0xffffffffu, i0, side);
+    const uint32_t ms = __shfl_sync(0xffffffffu, m, side), bs = __shfl_sync(0xffffffffu, b, side);
+    const uint32_t ls = __shfl_sync(0xffffffffu, len, side);
+    if (qs == kNoTask) continue;
+    for (uint32_t k = lane; k < ms; k += 32u) N.items[is + k] = TopItem{qs, is, bs + k * chunk, min(chunk, ls - k * chunk)};
+    if (ms > 1u)
+      for (uint32_t k = lane; k < kTopBinRow; k += 32u)
+        N.bins[(size_t)qs * kTopBinRow + k] = k < kTopBinWords ? top_bin_empty(k) : 0u;
+  }
+}
+
 // Bins the items of a level. The item's boxes are staged in shared memory
 // (neighbouring threads fetch neighbouring positions), then every thread bins
 // a run of consecutive positions: in Morton order they mostly share their
 // bins, so a run is gathered in registers and its bin updated when it ends.
 // The bins of a task of several items are merged in global memory, and each
 // item leaves its counts of bins 0..b per axis (icum, one row per axis and
-// bin), from which its lefts follow for any split; a task of one item is
-// split and partitioned here.
+// bin), from which its lefts follow for any split; the last of a task's items
+// to be binned splits it. A task of one item is split and partitioned here.
 //
 // Bound: 32 B of box and 4 of order in, 2 or 4 out per triangle; staging them
 // alone takes 8.9 ps a triangle (2.1M triangles in one task, 4.7 TB/s), the
@@ -1458,24 +1569,37 @@ struct TopBinMem {
   __align__(16) uint16_t code[K * kLevelThreads];
   uint32_t bins[kTopBinWords];
   uint32_t cnt[64];
+  uint32_t last;
   TopSplit split;
 };
 #ifndef J3DG_LEVEL_BLOCKS
 #define J3DG_LEVEL_BLOCKS 4
 #endif
-// K positions a thread: items of K * kLevelThreads
+// Smaller builds split a task where its last item was binned: a level is two
+// launches (82k triangles: 12 + 4 us a level, against 7 + 6 + 3 and their
+// gaps). Where a block bins many items, waiting for each one's additions to
+// the task's bins before counting it costs more than a launch: 28.09M
+// triangles 8.2 ms in the binning, against 6.9 and 0.2 for the splits.
+template <int K>
+constexpr bool kSplitWhereBinned = K < 8;
+
+// K positions a thread: items of K * kLevelThreads; level `base + k`
 template <int K>
 __global__ void __launch_bounds__(kLevelThreads, J3DG_LEVEL_BLOCKS) k_top_bin(
     const uint32_t* __restrict__ ord, uint32_t* __restrict__ ord2, const BinNode* __restrict__ tbox,
-    const TopItem* __restrict__ items, const uint32_t* __restrict__ n_items_p, const TopTask* __restrict__ tasks,
-    uint32_t cap_items, uint32_t* __restrict__ bins, uint16_t* __restrict__ code, uint32_t* __restrict__ icum,
-    TopSplit* __restrict__ splits, const Tree tr, uint32_t* status) {
+    const TopItem* __restrict__ items, const TopTask* __restrict__ tasks, BuildCtl* __restrict__ c, uint32_t level_k,
+    uint32_t* __restrict__ bins, uint16_t* __restrict__ code, uint32_t* __restrict__ icum,
+    TopSplit* __restrict__ splits, const NextLevel next, const Tree tr, uint32_t* status) {
   constexpr uint32_t chunk = K * kLevelThreads;
   extern __shared__ __align__(16) uint8_t top_raw[];
   TopBinMem<K>& s = *reinterpret_cast<TopBinMem<K>*>(top_raw);
   uint32_t* const sb = s.bins;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  const uint32_t n_items = min(*n_items_p, cap_items);
+  const uint32_t level = c->top_base + level_k, cap_items = next.cap_items;
+  if (tid == 0) s.last = c->error;  // (other blocks may raise it meanwhile: one answer for the block)
+  __syncthreads();
+  if (level >= kMaxTopLevels || s.last) return;
+  const uint32_t n_items = min(c->top[level].items, cap_items);
   for (uint32_t it = blockIdx.x; it < n_items; it += gridDim.x) {  // uniform over the block
     const TopItem I = items[it];
     const TopTask T = tasks[I.task];
@@ -1538,12 +1662,16 @@ __global__ void __launch_bounds__(kLevelThreads, J3DG_LEVEL_BLOCKS) k_top_bin(
       // the whole task is here
       if (warp == 0) {
         warp_top_split(sb, T, &s.split, tr);
-        __syncwarp();
-        if (lane == 0) splits[I.task] = s.split;
       }
       __syncthreads();
       partition_item<K>(s.split, T.begin, 0u, I.n, T.end, 0u, s.cnt, [&](uint32_t k) { return (uint32_t)s.code[k]; },
                         [&](uint32_t k) { return ord[I.begin + k]; }, ord2, status);
+      if (warp == 0) {
+        if constexpr (kSplitWhereBinned<K>)
+          warp_children(T, s.split, chunk, next, c, level, tr, status);
+        else if (lane == 0)
+          splits[I.task] = s.split;
+      }
     } else {
       // the codes in one store a thread (2 K bytes, by item), the bins to the task's
       constexpr int kWords = K / 2;
@@ -1557,94 +1685,66 @@ __global__ void __launch_bounds__(kLevelThreads, J3DG_LEVEL_BLOCKS) k_top_bin(
         *cg = *cs;
       if (tid < 3 * kTopBins) {
         const uint32_t* b = sb + tid * kTopVals;
-        uint32_t* g = bins + (size_t)I.task * kTopBinWords + tid * kTopVals;
+        uint32_t* g = bins + (size_t)I.task * kTopBinRow + tid * kTopVals;
         if (b[0]) {
           const uint32_t v[6] = {b[1], b[2], b[3], b[4], b[5], b[6]};
           bin_update(g, b[0], v);
         }
-        uint32_t c = 0;
-        for (uint32_t k = tid & ~15u; k <= tid; ++k) c += sb[k * kTopVals];
-        icum[(size_t)tid * cap_items + it] = c;
+        uint32_t cum = 0;
+        for (uint32_t k = tid & ~15u; k <= tid; ++k) cum += sb[k * kTopVals];
+        icum[(size_t)tid * cap_items + it] = cum;
+      }
+      if constexpr (kSplitWhereBinned<K>) {  // the last of the task's items splits it
+        __syncthreads();
+        uint32_t* const row = bins + (size_t)I.task * kTopBinRow;
+        if (tid == 0) {
+          __threadfence();
+          const bool last = atomicAdd(row + kTopBinWords, 1u) == (T.end - T.begin + chunk - 1) / chunk - 1u;
+          __threadfence();
+          s.last = last ? 1u : 0u;
+        }
+        __syncthreads();
+        if (s.last) {
+          for (uint32_t k = tid; k < kTopBinWords; k += kLevelThreads) sb[k] = __ldcg(row + k);
+          __syncthreads();
+          if (warp == 0) {
+            warp_top_split(sb, T, &s.split, tr);
+            __syncwarp();
+            if (lane == 0) splits[I.task] = s.split;
+            warp_children(T, s.split, chunk, next, c, level, tr, status);
+          }
+        }
       }
     }
     __syncthreads();  // the block's memory is free for the next item
   }
 }
 
-// one warp per task: the split of a task of several items; then the children:
-// a task of the next level above kSmallTask triangles (with its items and, if
-// they are several, empty bins), a small task above J3DG_SAH_TOP, else a
-// finished range; the task's own node goes under its parent
-// counters: [1] next tasks, [2] ranges, [3] small tasks, [4] next items
-__global__ void __launch_bounds__(128) k_top_split(
-    const TopTask* __restrict__ tasks, const uint32_t* __restrict__ n_tasks_p, uint32_t chunk,
-    const uint32_t* __restrict__ bins, uint32_t* __restrict__ bins2, TopSplit* __restrict__ splits,
-    uint32_t* __restrict__ counters, TopTask* __restrict__ next, TopItem* __restrict__ items2,
-    TopTask* __restrict__ small, TopRange* __restrict__ ranges, const Tree tr, uint32_t cap_tasks, uint32_t cap_small,
-    uint32_t cap_items, uint32_t nt, uint32_t* status) {
-  const uint32_t n_tasks = min(*n_tasks_p, cap_tasks), lane = threadIdx.x & 31u;
-  for (uint32_t t = blockIdx.x * 4u + (threadIdx.x >> 5); t < n_tasks; t += gridDim.x * 4u) {  // whole warps
+// ... where not: a warp per task, the splits of the tasks of several items and
+// everyone's children
+__global__ void __launch_bounds__(128) k_top_split(const TopTask* __restrict__ tasks, uint32_t chunk,
+                                                   const uint32_t* __restrict__ bins, TopSplit* __restrict__ splits,
+                                                   BuildCtl* __restrict__ c, uint32_t level_k, const NextLevel next,
+                                                   const Tree tr, uint32_t* status) {
+  __shared__ uint32_t s_bins[4][kTopBinWords];
+  __shared__ TopSplit s_split[4];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, level = c->top_base + level_k;
+  if (level >= kMaxTopLevels) return;
+  const uint32_t n_tasks = min(c->top[level].tasks, next.cap_tasks);
+  for (uint32_t t = blockIdx.x * 4u + warp; t < n_tasks; t += gridDim.x * 4u) {  // whole warps
     const TopTask T = tasks[t];
-    const uint32_t n = T.end - T.begin;
-    if (n > chunk) {
-      warp_top_split(bins + (size_t)t * kTopBinWords, T, splits + t, tr);
+    if (T.end - T.begin > chunk) {
+      for (uint32_t k = lane; k < kTopBinWords; k += 32u) s_bins[warp][k] = bins[(size_t)t * kTopBinRow + k];
       __syncwarp();
+      warp_top_split(s_bins[warp], T, &s_split[warp], tr);
+      __syncwarp();
+      if (lane == 0) splits[t] = s_split[warp];
+    } else if (lane == 0) {
+      s_split[warp] = splits[t];
     }
-    const TopSplit S = splits[t];
-    const uint32_t nl = S.nleft;
-    if (nl == 0 || nl >= n) {  // cannot happen: both sides of a split are non-empty
-      if (lane == 0) {
-        atomicOr(status, J3DG_DEV_BAD_INDEX);
-        atomicOr(tr.error, 1u);
-      }
-      continue;
-    }
-    const uint32_t node = T.begin + nl;
-    if (lane == 0) {
-      tr.up[node] = T.parent;
-      tr.done[node] = 0u;
-      link_child(tr, T.parent, T.side, node);
-    }
-    for (uint32_t side = 0; side < 2; ++side) {
-      const uint32_t b = side ? node : T.begin, e = side ? T.end : node, len = e - b;
-      const uint32_t tag = side | (((T.side >> 1) + 1u) << 1);
-      const bool again = len > kSmallTask;
-      uint32_t q = 0, i0 = 0;
-      const uint32_t m = (len + chunk - 1) / chunk;
-      if (lane == 0) {
-        if (len > J3DG_SAH_TOP) {
-          q = atomicAdd(counters + (again ? 1 : 3), 1u);
-          if (again) i0 = atomicAdd(counters + 4, m);
-          if (q >= (again ? cap_tasks : cap_small) || (again && i0 + m > cap_items)) {
-            atomicOr(status, J3DG_DEV_BAD_INDEX);
-            atomicOr(tr.error, 1u);
-            q = kNoTask;
-          } else {
-            TopTask C;
-            C.begin = b;
-            C.end = e;
-            C.parent = node;
-            C.side = tag;
-            C.clo = side ? S.rclo : S.lclo;
-            C.chi = side ? S.rchi : S.lchi;
-            (again ? next : small)[q] = C;
-          }
-        } else {
-          q = atomicAdd(counters + 2, 1u);
-          if (q < nt)
-            ranges[q] = TopRange{b, e, node, tag};
-          else
-            atomicOr(tr.error, 1u);
-        }
-      }
-      if (!again) continue;
-      q = __shfl_sync(0xffffffffu, q, 0);
-      i0 = __shfl_sync(0xffffffffu, i0, 0);
-      if (q == kNoTask) continue;
-      for (uint32_t k = lane; k < m; k += 32u) items2[i0 + k] = TopItem{q, i0, b + k * chunk, min(chunk, len - k * chunk)};
-      if (m > 1u)
-        for (uint32_t k = lane; k < kTopBinWords; k += 32u) bins2[(size_t)q * kTopBinWords + k] = top_bin_empty(k);
-    }
+    __syncwarp();
+    warp_children(T, s_split[warp], chunk, next, c, level, tr, status);
+    __syncwarp();
   }
 }
 
@@ -1653,12 +1753,15 @@ __global__ void __launch_bounds__(128) k_top_split(
 template <int K>
 __global__ void __launch_bounds__(kLevelThreads) k_top_scatter(
     const uint32_t* __restrict__ ord, uint32_t* __restrict__ ord2, const TopItem* __restrict__ items,
-    const uint32_t* __restrict__ n_items_p, const TopTask* __restrict__ tasks, uint32_t cap_items, const uint16_t* __restrict__ code, const uint32_t* __restrict__ icum, const TopSplit* __restrict__ splits,
+    const TopTask* __restrict__ tasks, const BuildCtl* __restrict__ c, uint32_t level_k, uint32_t cap_items,
+    const uint16_t* __restrict__ code, const uint32_t* __restrict__ icum, const TopSplit* __restrict__ splits,
     uint32_t* status) {
   constexpr uint32_t chunk = K * kLevelThreads;
   __shared__ uint32_t s_cnt[64], s_sum[kLevelThreads / 32];
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  const uint32_t n_items = min(*n_items_p, cap_items);
+  const uint32_t level = c->top_base + level_k;
+  if (level >= kMaxTopLevels || c->error) return;
+  const uint32_t n_items = min(c->top[level].items, cap_items);
   for (uint32_t it = blockIdx.x; it < n_items; it += gridDim.x) {  // uniform over the block
     const TopItem I = items[it];
     const TopTask T = tasks[I.task];
@@ -2180,18 +2283,25 @@ __device__ void climb(const Tree& tr, const BinNode* __restrict__ tbox, uint32_t
   }
 }
 
+// tasks that still wait for SAH levels at level `base + k`
+__device__ __forceinline__ uint32_t top_tasks_left(const BuildCtl* c, uint32_t k) {
+  const uint32_t level = c->top_base + k;
+  return c->top[min(level, kMaxTopLevels)].tasks;
+}
+
 template <int W>
 __global__ void __launch_bounds__(kSmallThreads, W == 8 ? J3DG_SMALL_BLOCKS - 1 : J3DG_SMALL_BLOCKS)
     k_small_tasks(const uint32_t* __restrict__ ord_a, const uint32_t* __restrict__ ord_b,
                   const BinNode* __restrict__ tbox, const TopTask* __restrict__ tasks, const TopRange* __restrict__ ranges,
-                  const uint32_t* __restrict__ counters, uint32_t* __restrict__ next_job, uint32_t leaf_size,
-                  uint32_t nt, uint32_t cap_small, uint2* __restrict__ rec, const Tree tr, uint32_t* status) {
+                  BuildCtl* __restrict__ c, uint32_t level_k, uint32_t leaf_size, uint32_t nt,
+                  uint32_t cap_small, uint2* __restrict__ rec, const Tree tr, uint32_t* status) {
   extern __shared__ __align__(16) uint8_t small_raw[];
   SmallMem<W>& s = *reinterpret_cast<SmallMem<W>*>(small_raw);
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  const uint32_t n_tasks = min(counters[3], cap_small), n_jobs = n_tasks + min(counters[2], nt);
+  if (top_tasks_left(c, level_k)) return;  // more SAH levels come first
+  const uint32_t n_tasks = min(c->n_small, cap_small), n_jobs = n_tasks + min(c->n_ranges, nt);
   for (;;) {
-    if (tid == 0) s.job = atomicAdd(next_job, 1u);
+    if (tid == 0) s.job = atomicAdd(&c->next_job, 1u);
     __syncthreads();
     const uint32_t job = s.job;
     if (job >= n_jobs) return;
@@ -2384,39 +2494,26 @@ __global__ void k_slot_of(const float4* __restrict__ tris, uint32_t nt, uint32_t
 
 // ------------------------------------------------ device-driven build ----
 //
-// A build (the default: binned-SAH top levels, PLOC below them, the
-// cost-optimal collapse; or the LBVH: the one-pass tree and its collapse;
-// then the depth-first numbering) runs as one CUDA graph with no host round
-// trip: every level loop is a conditional while node whose
-// body ends in a one-thread step kernel, which advances the loop state kept
-// in device memory (BuildCtl) and sets the loop's condition. Kernels read
-// their sizes from BuildCtl and stride over them with fixed grids, so one
-// captured sequence serves every level. Loops whose levels alternate two
-// buffers run two levels per body (the second is a no-op when the first
-// ends the loop). enqueue_build only enqueues (it runs under a stream
-// capture): j3dg_mesh_build captures and launches it for one mesh, and a
-// batch captures it for all its meshes ahead of its frames.
-
-static const uint32_t kMaxPlaceLevels = 128;
-
-struct BuildCtl {
-  uint32_t top_ctr[5];  // k_top_split: [1] next level's tasks, [2] ranges, [3] small tasks,
-                        // [4] next level's items (LBVH: [0] the root that k_lbvh found)
-  uint32_t n_tasks, n_items, top_levels;
-  uint32_t root;      // the binary tree's root
-  uint32_t next_job;  // the next small task or range to be taken (k_small_tasks)
-  uint32_t lohi[2];  // the running pass's node range (LBVH: depth-first levels)
-  uint32_t n_in, n_out, n_wide, place_levels, max_depth;
-  int32_t dfs_level;
-  uint32_t error;  // 1 SAH levels overran their bound, 2 PLOC, 4 placement / collapse
-  uint32_t level_end[kMaxPlaceLevels]; // LBVH: wide nodes of level L end at level_end[L]
-};
+// A build runs with no host round trip but at its end: kernels read their
+// sizes from BuildCtl and stride over them with fixed grids, so the launches
+// do not depend on the tree. The default builder's levels (SAH, placement) are
+// launched a few more of than a balanced tree has; the tree that needs more
+// gets them after the host has looked (j3dg_mesh_build), or from a conditional
+// while node in a captured build (a batch rebuilds its meshes ahead of its
+// frames; a body ends in a one-thread kernel that sets the loop's condition).
+// A level past the last finds nothing and costs a launch (about 2 us), a round
+// of a loop 13-26 us between its levels, and making the graph of a single
+// build took longer than the radix sort that it ran beside. The LBVH's loops
+// (the collapse and both depth-first sweeps) are while nodes always. Builds of
+// 82k / 2M / 28.09M triangles with their first frame, as a graph of loops and
+// launched: 992 -> 906, 3322 -> 3224, 26262 -> 24598 us (the large one also by
+// its nodes' array, kStagedNodes, and the index array from the pool).
 
 // the root task, by its size: split level by level, by one block, or a segment
 __global__ void k_ctl_init(BuildCtl* __restrict__ c, TopTask* __restrict__ tasks, TopTask* __restrict__ small,
-                           TopRange* __restrict__ ranges, const float* __restrict__ bb, uint32_t nt, uint32_t top,
-                           uint32_t chunk) {
+                           TopRange* __restrict__ ranges, uint32_t nt, uint32_t top, uint32_t chunk) {
   if (top) {
+    const float* bb = c->bb;
     TopTask r0;
     r0.begin = 0;
     r0.end = nt;
@@ -2426,68 +2523,57 @@ __global__ void k_ctl_init(BuildCtl* __restrict__ c, TopTask* __restrict__ tasks
     r0.chi = make_float4(bb[3], bb[4], bb[5], 0.f);
     if (nt > kSmallTask) {
       tasks[0] = r0;
-      c->n_tasks = 1;
-      c->n_items = (nt + chunk - 1) / chunk;
+      c->top[0].tasks = 1;
+      c->top[0].items = (nt + chunk - 1) / chunk;
     } else if (nt > J3DG_SAH_TOP) {
       small[0] = r0;
-      c->top_ctr[3] = 1;
+      c->n_small = 1;
     } else {
       ranges[0] = TopRange{0, nt, kNoParent, 0};
-      c->top_ctr[2] = 1;
+      c->n_ranges = 1;
     }
   }
-  c->n_in = 1;  // the placement's root item
+  // LBVH: the collapse's root item
   c->n_wide = 1;
+  c->n_in = 1;
   c->place_levels = 1;
   c->level_end[0] = 1;
 }
 
-__global__ void k_top_step(BuildCtl* __restrict__ c, uint32_t cap_tasks, uint32_t cap_small, uint32_t cap_items,
-                           uint32_t nt, cudaGraphConditionalHandle h, uint32_t set) {
-  if (c->n_tasks) {  // the level ran
-    uint32_t next = c->top_ctr[1];
-    if (next > cap_tasks || c->top_ctr[3] > cap_small || c->top_ctr[2] > nt || c->top_ctr[4] > cap_items ||
-        c->top_levels >= kMaxTopLevels) {
-      c->error |= 1u;
-      next = 0;
-    } else {
-      ++c->top_levels;
-    }
-    c->n_tasks = next;
-    c->n_items = next ? c->top_ctr[4] : 0u;
-    c->top_ctr[1] = c->top_ctr[4] = 0;
-  }
-  if (set) cudaGraphSetConditional(h, c->n_tasks > 0 ? 1u : 0u);
-}
-
-// the binary tree is complete: the placement starts at its root
-__global__ void k_tree_done(BuildCtl* __restrict__ c, const NodeMeta* __restrict__ meta, uint32_t nt,
+// The SAH levels were launched up to `base + k`: if no task is left, the
+// binary tree is complete and the placement starts at its root; else nothing
+// happens here.
+__global__ void k_tree_done(BuildCtl* __restrict__ c, uint32_t k, const NodeMeta* __restrict__ meta, uint32_t nt,
                             PlaceItem* __restrict__ qa) {
+  c->n_wide = 0;
+  c->top_left = top_tasks_left(c, k);
+  if (c->error || c->top_left) return;
   const uint32_t root = c->root;
-  if (!c->error && (root == 0u || root >= nt || meta[root].wide >= nt)) c->error |= 2u;  // a malformed tree
-  if (c->error) {  // nothing is placed
-    c->n_in = c->n_wide = 0;
+  if (root == 0u || root >= nt || meta[root].wide >= nt) {  // a malformed tree: nothing is placed
+    c->error |= 2u;
     return;
   }
   c->n_wide = meta[root].wide;
+  c->place[0] = 1;
   qa[0] = PlaceItem{root, 0u, 1u, 0u};
 }
 
-__global__ void k_place_step(BuildCtl* __restrict__ c, uint32_t nt, cudaGraphConditionalHandle h, uint32_t set) {
-  if (c->n_in) {  // the level ran
-    const uint32_t n_out = c->n_out;
-    if (n_out > nt || c->place_levels >= kMaxPlaceLevels) {
-      c->error |= 4u;
-      c->n_in = 0;
-    } else {
-      ++c->place_levels;
-      c->n_in = n_out;
-    }
-    c->n_out = 0;
-  }
-  if (set) cudaGraphSetConditional(h, c->n_in > 0 ? 1u : 0u);
+// a captured build: the loop after the levels that were launched one by one
+// goes on from here while something is left
+__global__ void k_top_more(BuildCtl* __restrict__ c, uint32_t done, cudaGraphConditionalHandle h) {
+  c->top_base += done;
+  const bool left = c->top[min(c->top_base, kMaxTopLevels)].tasks > 0 && !c->error;
+  if (left && c->top_base >= kMaxTopLevels) c->error |= 1u;
+  cudaGraphSetConditional(h, left && c->top_base < kMaxTopLevels ? 1u : 0u);
+}
+__global__ void k_place_more(BuildCtl* __restrict__ c, uint32_t done, cudaGraphConditionalHandle h) {
+  c->place_base += done;
+  const bool left = c->place[min(c->place_base, kMaxPlaceLevels)] > 0 && !c->error;
+  if (left && c->place_base >= kMaxPlaceLevels) c->error |= 4u;
+  cudaGraphSetConditional(h, left && c->place_base < kMaxPlaceLevels ? 1u : 0u);
 }
 
+// node range [lohi[0], lohi[1]) of wide level l (empty outside the tree)
 __device__ __forceinline__ void level_range(BuildCtl* c, int32_t l) {
   const bool ok = l >= 0 && l < (int32_t)c->place_levels;
   c->lohi[0] = ok && l > 0 ? c->level_end[l - 1] : 0u;
@@ -2510,9 +2596,9 @@ __global__ void k_dfs_step(BuildCtl* __restrict__ c, uint32_t up, cudaGraphCondi
   if (set) cudaGraphSetConditional(h, (c->dfs_level >= 0 && c->dfs_level < (int32_t)c->place_levels) ? 1u : 0u);
 }
 
-// the LBVH's collapse starts at the root that k_lbvh left in top_ctr[0]
+// the LBVH's collapse starts at the root that k_lbvh left
 __global__ void k_lbvh_root(BuildCtl* __restrict__ c, CollapseItem* __restrict__ qa) {
-  qa[0] = CollapseItem{c->top_ctr[0], 0u, 1u};
+  qa[0] = CollapseItem{c->root, 0u, 1u};
 }
 
 // after an LBVH collapse level: k_collapse allocated its wide nodes itself
@@ -2530,11 +2616,12 @@ __global__ void k_lbvh_step(BuildCtl* __restrict__ c, uint32_t nt, cudaGraphCond
   if (set) cudaGraphSetConditional(h, c->n_in > 0 ? 1u : 0u);
 }
 
-// Appends a while node (condition initially 1) to the graph that `st` is
-// capturing; `body(side, handle)` enqueues the loop body on `side`, which
-// captures it into the node's body graph.
-template <class Body>
-static cudaError_t capture_while(cudaStream_t st, cudaStream_t side, Body&& body) {
+// Appends a while node to the graph that `st` is capturing: its condition is
+// initially 1, or what `before(handle)` enqueues on `st` sets;
+// `body(side, handle)` enqueues the loop body on `side`, which captures it
+// into the node's body graph.
+template <class Before, class Body>
+static cudaError_t capture_while(cudaStream_t st, cudaStream_t side, Before&& before, Body&& body) {
   cudaStreamCaptureStatus cs;
   unsigned long long id = 0;
   cudaGraph_t g = nullptr;
@@ -2545,6 +2632,9 @@ static cudaError_t capture_while(cudaStream_t st, cudaStream_t side, Body&& body
   if (cs != cudaStreamCaptureStatusActive) return cudaErrorStreamCaptureUnsupported;
   cudaGraphConditionalHandle h;
   if ((e = cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault)) != cudaSuccess) return e;
+  before(h);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if ((e = cudaStreamGetCaptureInfo(st, &cs, &id, &g, &deps, nullptr, &nd)) != cudaSuccess) return e;
   cudaGraphNodeParams p = {};
   p.type = cudaGraphNodeTypeConditional;
   p.conditional.handle = h;
@@ -2563,6 +2653,10 @@ static cudaError_t capture_while(cudaStream_t st, cudaStream_t side, Body&& body
   if (e != cudaSuccess) return e;
   return cudaStreamUpdateCaptureDependencies(st, &node, nullptr, 1, cudaStreamSetCaptureDependencies);
 }
+template <class Body>
+static cudaError_t capture_while(cudaStream_t st, cudaStream_t side, Body&& body) {
+  return capture_while(st, side, [](cudaGraphConditionalHandle) {}, body);
+}
 
 // Every buffer of one build, sized by the triangle count alone (upper bounds
 // where the tree decides: the wide nodes, the queues).
@@ -2573,9 +2667,10 @@ struct BuildPlan {
   // the builders the scratch serves: PLOC (the default) and / or LBVH (a
   // batch's rebuild lane may serve both)
   bool need_ploc = true, need_lbvh = false;
+  // what was allocated: the scratch's smaller arrays as one
+  std::vector<void*> owned;
   // scratch
   float* part = nullptr;
-  float* bb = nullptr;
   uint64_t *k0 = nullptr, *k1 = nullptr;
   uint32_t *v0 = nullptr, *v1 = nullptr, *hist = nullptr, *sums = nullptr;
   uint32_t *ord_a = nullptr, *ord_b = nullptr, *top_up = nullptr, *top_done = nullptr, *bins_a = nullptr, *bins_b = nullptr,
@@ -2598,7 +2693,7 @@ struct BuildPlan {
   CollapseItem *qa = nullptr, *qb = nullptr;
   uint32_t *dfs_size = nullptr, *dfs_pos = nullptr;
   BuildCtl* ctl = nullptr;
-  // outputs (the mesh keeps them)
+  // outputs (the mesh keeps them once `owned` does not)
   float4 *normals = nullptr, *soup = nullptr, *tris_out = nullptr, *nodes = nullptr;
   uint32_t* slot_of = nullptr;
   // tasks of one level are disjoint, each above kSmallTask; so are the small tasks, each above J3DG_SAH_TOP
@@ -2612,10 +2707,30 @@ struct BuildPlan {
   // on 152 SMs) smaller items fill the device instead
   uint32_t chunk() const { return nt >= 600000u ? 2048u : (nt >= 300000u ? 1024u : 512u); }
   uint32_t cap_items() const { return nt / chunk() + cap_tasks() + 1; }
+  // levels launched without looking: SAH splits halve at best, a placement
+  // level takes every subtree W ways at best; the trees of scans and of the
+  // procedural surfaces need 1-3 levels more (82k / 2M / 28.09M triangles: SAH
+  // 7, 12, 15 at best), even numbers for the loops behind them
+  uint32_t top_levels() const {
+    uint32_t l = 0;
+    while ((uint64_t)kSmallTask << l < nt) ++l;
+    return l ? (l + 4u) & ~1u : 0u;
+  }
+  uint32_t place_levels() const {
+    uint32_t l = 1;
+    for (uint64_t n = W * (uint64_t)leaf; n < nt; n *= W) ++l;
+    return std::min((l + 5u) & ~1u, kMaxPlaceLevels);
+  }
   Tree tree() const { return Tree{box, meta, top_up, top_done, dp_cost, dp_wide, &ctl->root, &ctl->error}; }
 };
 
 static const int kBBoxBlocks = 1024;
+
+// Up to this size the wide nodes are made in an array at their bound and then
+// copied into one of the tree's size: a copy of up to about 20 us, the time
+// that the host takes to look at the tree's size first. 28.09M triangles: 0.25
+// ms of copy and 3.6 GB less.
+static const size_t kStagedNodes = (size_t)256 << 20;
 
 // outputs: the mesh's arrays too (else the mesh's own: a rebuild in place);
 // node_bound: with them, a node array at the size bound (rebuildable meshes;
@@ -2623,11 +2738,25 @@ static const int kBBoxBlocks = 1024;
 static cudaError_t plan_alloc(BuildPlan& P, cudaStream_t st, bool outputs = true, bool node_bound = true) {
   const size_t nt = P.nt, F4 = J3DG_NODE_F4(P.W);
   cudaError_t e = cudaSuccess;
+  auto own = [&](void** p, size_t bytes) {
+    if (e == cudaSuccess) e = cudaMallocAsync(p, bytes, st);
+    if (e == cudaSuccess) P.owned.push_back(*p);
+  };
+  // arrays of at most 16 MB share one allocation (an allocation and its
+  // release take 1.6 us, and a small build has 35 arrays); a larger one has
+  // its own, which the pool can place where a freed one was
+  struct Part {
+    void** p;
+    size_t at;
+  };
+  std::vector<Part> parts;
+  size_t shared = 0;
   auto A = [&](auto*& p, size_t bytes) {
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&p, bytes, st);
+    if (bytes > ((size_t)16 << 20)) return own((void**)&p, bytes);
+    parts.push_back(Part{(void**)&p, shared});
+    shared += (bytes + 255) & ~(size_t)255;
   };
   A(P.part, sizeof(float) * 6 * kBBoxBlocks);
-  A(P.bb, sizeof(float) * 6);
   A(P.k0, sizeof(uint64_t) * nt);
   A(P.k1, sizeof(uint64_t) * nt);
   A(P.v0, sizeof(uint32_t) * nt);
@@ -2643,8 +2772,8 @@ static cudaError_t plan_alloc(BuildPlan& P, cudaStream_t st, bool outputs = true
     A(P.codes, sizeof(uint16_t) * std::max((size_t)P.cap_items() * P.chunk(), (size_t)items * 512));
     A(P.top_up, sizeof(uint32_t) * nt);
     A(P.top_done, sizeof(uint32_t) * nt);
-    A(P.bins_a, sizeof(uint32_t) * (size_t)P.cap_tasks() * kTopBinWords);
-    A(P.bins_b, sizeof(uint32_t) * (size_t)P.cap_tasks() * kTopBinWords);
+    A(P.bins_a, sizeof(uint32_t) * (size_t)P.cap_tasks() * kTopBinRow);
+    A(P.bins_b, sizeof(uint32_t) * (size_t)P.cap_tasks() * kTopBinRow);
     A(P.icum, sizeof(uint32_t) * (size_t)items * 3 * kTopBins);
     A(P.items_a, sizeof(TopItem) * items);
     A(P.items_b, sizeof(TopItem) * items);
@@ -2672,27 +2801,37 @@ static cudaError_t plan_alloc(BuildPlan& P, cudaStream_t st, bool outputs = true
     A(P.qa, sizeof(CollapseItem) * nt);
     A(P.qb, sizeof(CollapseItem) * nt);
   }
-  // the wide nodes at their bound; the default builder writes them straight
-  // into a rebuildable mesh's array instead
-  if (P.need_lbvh || (outputs && !node_bound)) A(P.wide, sizeof(float4) * F4 * nt);
+  // the wide nodes at their bound. The default builder writes them straight
+  // into the mesh's array where that is there before them (a rebuildable mesh)
+  // or worth waiting for (run_tree_ploc)
+  const size_t wide_bytes = sizeof(float4) * F4 * nt;
+  if (P.need_lbvh || (outputs && !node_bound && wide_bytes <= kStagedNodes)) A(P.wide, wide_bytes);
   A(P.ctl, sizeof(BuildCtl));
+  char* base = nullptr;
+  own((void**)&base, shared);
+  if (e == cudaSuccess)
+    for (const Part& q : parts) *q.p = base + q.at;
   if (outputs) {  // else the mesh's own arrays (a rebuild in place)
-    A(P.normals, sizeof(float4) * nt);
-    A(P.tris_out, sizeof(float4) * 3 * nt);
-    if (node_bound) A(P.nodes, sizeof(float4) * F4 * nt);  // the wide nodes are at most nt - 1
-    A(P.slot_of, sizeof(uint32_t) * nt);
+    own((void**)&P.normals, sizeof(float4) * nt);
+    own((void**)&P.tris_out, sizeof(float4) * 3 * nt);
+    if (node_bound) own((void**)&P.nodes, sizeof(float4) * F4 * nt);  // the wide nodes are at most nt - 1
+    own((void**)&P.slot_of, sizeof(uint32_t) * nt);
   }
   return e;
 }
 
-// frees the scratch (outputs the caller took over are null)
+// an output that the caller takes over
+template <class T>
+static void* plan_take(BuildPlan& P, T*& p) {
+  const auto it = std::find(P.owned.begin(), P.owned.end(), (void*)p);
+  if (it != P.owned.end()) P.owned.erase(it);
+  void* r = p;
+  p = nullptr;
+  return r;
+}
+// frees what is left
 static void plan_free(BuildPlan& P, cudaStream_t st) {
-  void* ps[] = {P.part, P.bb, P.k0, P.k1, P.v0, P.v1, P.hist, P.sums, P.ord_a, P.ord_b, P.top_up, P.top_done, P.bins_a,
-                P.bins_b, P.icum, P.items_a, P.items_b, P.tbox, P.codes, P.tasks_a, P.tasks_b,
-                P.small, P.splits, P.ranges, P.child, P.box, P.other, P.meta, P.dp_cost, P.dp_wide, P.wide, P.pa, P.pb, P.range,
-                P.qa, P.qb, P.dfs_size, P.dfs_pos, P.ctl, P.normals, P.soup, P.tris_out, P.nodes, P.slot_of};
-  for (void* p : ps)
-    if (p) cudaFreeAsync(p, st);
+  for (void* p : P.owned) cudaFreeAsync(p, st);
   P = BuildPlan{};
 }
 
@@ -2706,44 +2845,56 @@ static void plan_free(BuildPlan& P, cudaStream_t st) {
 // level can have items
 template <int K>
 static void launch_top_bin_k(BuildPlan& P, cudaStream_t s, const uint32_t* oi, uint32_t* oo, const TopItem* items,
-                             const TopTask* tasks, uint32_t* bins, uint32_t* d_status) {
-  BuildCtl* c = P.ctl;
+                             const TopTask* tasks, uint32_t* bins, const NextLevel& next, uint32_t k,
+                             uint32_t* d_status) {
   const uint32_t blocks = std::min(wave_blocks128() / 16u * J3DG_LEVEL_BLOCKS, P.cap_items());
   cudaFuncSetAttribute(k_top_bin<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TopBinMem<K>));
-  k_top_bin<K><<<blocks, kLevelThreads, sizeof(TopBinMem<K>), s>>>(oi, oo, P.tbox, items, &c->n_items, tasks,
-                                                                   P.cap_items(), bins, P.codes, P.icum, P.splits,
-                                                                   P.tree(), d_status);
+  k_top_bin<K><<<blocks, kLevelThreads, sizeof(TopBinMem<K>), s>>>(oi, oo, P.tbox, items, tasks, P.ctl, k, bins,
+                                                                   P.codes, P.icum, P.splits, next, P.tree(), d_status);
 }
 static void launch_top_bin(BuildPlan& P, cudaStream_t s, const uint32_t* oi, uint32_t* oo, const TopItem* items,
-                           const TopTask* tasks, uint32_t* bins, uint32_t* d_status) {
+                           const TopTask* tasks, uint32_t* bins, const NextLevel& next, uint32_t k, uint32_t* d_status) {
   switch (P.chunk() / kLevelThreads) {
-    case 8: return launch_top_bin_k<8>(P, s, oi, oo, items, tasks, bins, d_status);
-    case 4: return launch_top_bin_k<4>(P, s, oi, oo, items, tasks, bins, d_status);
-    default: return launch_top_bin_k<2>(P, s, oi, oo, items, tasks, bins, d_status);
+    case 8: return launch_top_bin_k<8>(P, s, oi, oo, items, tasks, bins, next, k, d_status);
+    case 4: return launch_top_bin_k<4>(P, s, oi, oo, items, tasks, bins, next, k, d_status);
+    default: return launch_top_bin_k<2>(P, s, oi, oo, items, tasks, bins, next, k, d_status);
   }
 }
 
 static void launch_top_scatter(BuildPlan& P, cudaStream_t s, const uint32_t* oi, uint32_t* oo, const TopItem* items,
-                               const TopTask* tasks, uint32_t* d_status) {
-  BuildCtl* c = P.ctl;
+                               const TopTask* tasks, uint32_t k, uint32_t* d_status) {
   const uint32_t blocks = std::min(wave_blocks128() / 2u, P.cap_items()), cap = P.cap_items();
+  auto go = [&](auto kernel) {
+    kernel<<<blocks, kLevelThreads, 0, s>>>(oi, oo, items, tasks, P.ctl, k, cap, P.codes, P.icum, P.splits, d_status);
+  };
   switch (P.chunk() / kLevelThreads) {
-    case 8:
-      k_top_scatter<8><<<blocks, kLevelThreads, 0, s>>>(oi, oo, items, &c->n_items, tasks, cap, P.codes, P.icum, P.splits, d_status);
-      break;
-    case 4:
-      k_top_scatter<4><<<blocks, kLevelThreads, 0, s>>>(oi, oo, items, &c->n_items, tasks, cap, P.codes, P.icum, P.splits, d_status);
-      break;
-    default:
-      k_top_scatter<2><<<blocks, kLevelThreads, 0, s>>>(oi, oo, items, &c->n_items, tasks, cap, P.codes, P.icum, P.splits, d_status);
+    case 8: return go(k_top_scatter<8>);
+    case 4: return go(k_top_scatter<4>);
+    default: return go(k_top_scatter<2>);
   }
+}
+
+// SAH level `base + k`
+static void launch_top_level(BuildPlan& P, cudaStream_t s, uint32_t k, uint32_t* d_status) {
+  const bool odd = k & 1u;
+  const uint32_t *oi = odd ? P.ord_b : P.ord_a;
+  uint32_t* oo = odd ? P.ord_a : P.ord_b;
+  const TopTask* tasks = odd ? P.tasks_b : P.tasks_a;
+  const TopItem* items = odd ? P.items_b : P.items_a;
+  const NextLevel next{odd ? P.tasks_a : P.tasks_b, odd ? P.items_a : P.items_b, odd ? P.bins_a : P.bins_b, P.small,
+                       P.ranges, P.cap_tasks(), P.cap_small(), P.cap_items(), P.nt};
+  uint32_t* bins = odd ? P.bins_b : P.bins_a;
+  launch_top_bin(P, s, oi, oo, items, tasks, bins, next, k, d_status);
+  if (P.chunk() == 8 * kLevelThreads)  // !kSplitWhereBinned
+    k_top_split<<<std::min(kStrideBlocks, P.cap_tasks() / 4u + 1u), 128, 0, s>>>(tasks, P.chunk(), bins, P.splits, P.ctl, k,
+                                                                                 next, P.tree(), d_status);
+  launch_top_scatter(P, s, oi, oo, items, tasks, k, d_status);
 }
 
 // section 5d over every small task and range: persistent blocks, as many as
 // the device holds at the kernel's shared memory
 template <int W>
-static cudaError_t launch_small_tasks_w(BuildPlan& P, cudaStream_t st, uint32_t* d_status) {
-  BuildCtl* c = P.ctl;
+static cudaError_t launch_small_tasks_w(BuildPlan& P, cudaStream_t st, uint32_t k, uint32_t* d_status) {
   const size_t smem = small_smem<W>();
   cudaError_t e = cudaFuncSetAttribute(k_small_tasks<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int dev = 0, sms = 0, per = 0;
@@ -2753,64 +2904,105 @@ static cudaError_t launch_small_tasks_w(BuildPlan& P, cudaStream_t st, uint32_t*
   if (e != cudaSuccess) return e;
   const uint32_t grid = std::min((uint32_t)std::max(1, sms * per), P.cap_small());
   k_small_tasks<W><<<grid, kSmallThreads, smem, st>>>(
-      P.ord_a, P.ord_b, P.tbox, P.small, P.ranges, c->top_ctr, &c->next_job, P.leaf, P.nt, P.cap_small(),
+      P.ord_a, P.ord_b, P.tbox, P.small, P.ranges, P.ctl, k, P.leaf, P.nt, P.cap_small(),
       reinterpret_cast<uint2*>(P.pb), P.tree(), d_status);
   return cudaGetLastError();
 }
 
-static cudaError_t launch_small_tasks(uint32_t W, BuildPlan& P, cudaStream_t st, uint32_t* d_status) {
-  if (W == 2) return launch_small_tasks_w<2>(P, st, d_status);
-  if (W == 8) return launch_small_tasks_w<8>(P, st, d_status);
-  return launch_small_tasks_w<4>(P, st, d_status);
+static cudaError_t launch_small_tasks(uint32_t W, BuildPlan& P, cudaStream_t st, uint32_t k, uint32_t* d_status) {
+  if (W == 2) return launch_small_tasks_w<2>(P, st, k, d_status);
+  if (W == 8) return launch_small_tasks_w<8>(P, st, k, d_status);
+  return launch_small_tasks_w<4>(P, st, k, d_status);
 }
 
-// the default builder's binary tree and its wide nodes (`wide`, in depth-first
-// order): binned-SAH levels down to small tasks, each small task's subtree by
-// one block (and the cost programme up to the root), the placement; the
-// leaf-ordered triangles go to P.tris_out, their positions to P.slot_of
-static cudaError_t enqueue_tree_ploc(BuildPlan& P, float4* wide, cudaStream_t st, cudaStream_t side,
-                                     uint32_t* d_status) {
-  const uint32_t nt = P.nt, W = P.W;
+// The default builder's binary tree and its wide nodes (in depth-first order):
+// binned-SAH levels down to small tasks, each small task's subtree by one
+// block (and the cost programme up to the root), the placement; the
+// leaf-ordered triangles go to P.tris_out, their positions to P.slot_of.
+static void enqueue_top_levels(BuildPlan& P, cudaStream_t st, uint32_t k0, uint32_t k1, uint32_t* d_status) {
+  for (uint32_t k = k0; k < k1; ++k) launch_top_level(P, st, k, d_status);
+}
+static void enqueue_place_levels(BuildPlan& P, cudaStream_t st, uint32_t k0, uint32_t k1, uint32_t* d_status) {
+  for (uint32_t k = k0; k < k1; ++k)
+    launch_collapse_place(P.W, P.box, P.meta, P.tbox, P.soup, k & 1u ? P.pb : P.pa, k & 1u ? P.pa : P.pb, P.ctl, k,
+                          P.nodes ? P.nodes : P.wide, P.tris_out, P.slot_of, P.nt, d_status, st);
+}
+static void enqueue_top_start(BuildPlan& P, cudaStream_t st) {
+  k_top_boxes<<<(P.nt + 255) / 256, 256, 0, st>>>(P.soup, P.nt, P.tbox, P.ord_a);
+  if (P.top_levels())
+    k_top_items<<<std::min(kStrideBlocks, P.cap_items() / 256 + 1), 256, 0, st>>>(P.items_a, P.bins_a, P.nt, P.chunk());
+}
+
+// ... captured: loops after the levels
+static cudaError_t capture_tree_ploc(BuildPlan& P, cudaStream_t st, cudaStream_t side, uint32_t* d_status) {
   BuildCtl* c = P.ctl;
   cudaError_t e = cudaSuccess;
-  const float4* soup = P.soup;
-  k_top_boxes<<<(nt + 255) / 256, 256, 0, st>>>(soup, nt, P.tbox, P.ord_a);
-  J3DG_EQ(cudaSuccess);
-  if (nt > kSmallTask) {
-    const uint32_t chunk = P.chunk();
-    k_top_items<<<std::min(kStrideBlocks, P.cap_items() / 256 + 1), 256, 0, st>>>(P.items_a, P.bins_a, nt, chunk);
-    const uint32_t split_blocks = std::min(kStrideBlocks, P.cap_tasks() / 4u + 1u);
-    // one SAH level: tasks ti, items ii, bins bi, order oi -> the next level's
-    auto level = [&](cudaStream_t s, TopTask* ti, TopTask* to, TopItem* ii, TopItem* io, uint32_t* bi, uint32_t* bo,
-                     uint32_t* oi, uint32_t* oo) {
-      launch_top_bin(P, s, oi, oo, ii, ti, bi, d_status);
-      k_top_split<<<split_blocks, 128, 0, s>>>(ti, &c->n_tasks, chunk, bi, bo, P.splits, c->top_ctr, to, io, P.small,
-                                               P.ranges, P.tree(), P.cap_tasks(), P.cap_small(), P.cap_items(), nt,
-                                               d_status);
-      launch_top_scatter(P, s, oi, oo, ii, ti, d_status);
-    };
-    J3DG_EQ(capture_while(st, side, [&](cudaStream_t s, cudaGraphConditionalHandle h) {
-      level(s, P.tasks_a, P.tasks_b, P.items_a, P.items_b, P.bins_a, P.bins_b, P.ord_a, P.ord_b);
-      k_top_step<<<1, 1, 0, s>>>(c, P.cap_tasks(), P.cap_small(), P.cap_items(), nt, h, 0u);
-      level(s, P.tasks_b, P.tasks_a, P.items_b, P.items_a, P.bins_b, P.bins_a, P.ord_b, P.ord_a);
-      k_top_step<<<1, 1, 0, s>>>(c, P.cap_tasks(), P.cap_small(), P.cap_items(), nt, h, 1u);
-    }));
+  enqueue_top_start(P, st);
+  const uint32_t levels = P.top_levels(), places = P.place_levels();
+  if (levels) {
+    enqueue_top_levels(P, st, 0, levels, d_status);
+    J3DG_EQ(capture_while(
+        st, side, [&](cudaGraphConditionalHandle h) { k_top_more<<<1, 1, 0, st>>>(c, levels, h); },
+        [&](cudaStream_t s, cudaGraphConditionalHandle h) {
+          enqueue_top_levels(P, s, 0, 2, d_status);
+          k_top_more<<<1, 1, 0, s>>>(c, 2u, h);
+        }));
   }
-  J3DG_EQ(launch_small_tasks(W, P, st, d_status));
-  k_tree_done<<<1, 1, 0, st>>>(c, P.meta, nt, P.pa);
-  J3DG_EQ(cudaSuccess);
-  // placement, level by level
-  auto place = [&](cudaStream_t s, const PlaceItem* qi, PlaceItem* qo) {
-    launch_collapse_place(W, P.box, P.meta, P.tbox, soup, qi, &c->n_in, qo, &c->n_out, &c->n_wide, wide, &c->max_depth,
-                          P.tris_out, P.slot_of, nt, d_status, s);
-  };
-  J3DG_EQ(capture_while(st, side, [&](cudaStream_t s, cudaGraphConditionalHandle h) {
-    place(s, P.pa, P.pb);
-    k_place_step<<<1, 1, 0, s>>>(c, nt, h, 0u);
-    place(s, P.pb, P.pa);
-    k_place_step<<<1, 1, 0, s>>>(c, nt, h, 1u);
-  }));
+  J3DG_EQ(launch_small_tasks(P.W, P, st, 0, d_status));
+  k_tree_done<<<1, 1, 0, st>>>(c, 0, P.meta, P.nt, P.pa);
+  enqueue_place_levels(P, st, 0, places, d_status);
+  J3DG_EQ(capture_while(
+      st, side, [&](cudaGraphConditionalHandle h) { k_place_more<<<1, 1, 0, st>>>(c, places, h); },
+      [&](cudaStream_t s, cudaGraphConditionalHandle h) {
+        enqueue_place_levels(P, s, 0, 2, d_status);
+        k_place_more<<<1, 1, 0, s>>>(c, 2u, h);
+      }));
   return e;
+}
+
+// ... on a stream, to its end: h is what the build left
+static cudaError_t run_tree_ploc(BuildPlan& P, cudaStream_t st, uint32_t* d_status, BuildCtl& h) {
+  cudaError_t e = cudaSuccess;
+  enqueue_top_start(P, st);
+  uint32_t levels = 0, places = 0, more_levels = P.top_levels(), more_places = P.place_levels();
+  bool tree = false;
+  for (;;) {
+    if (!tree) {
+      enqueue_top_levels(P, st, levels, levels + more_levels, d_status);
+      levels += more_levels;
+      J3DG_EQ(launch_small_tasks(P.W, P, st, levels, d_status));
+      k_tree_done<<<1, 1, 0, st>>>(P.ctl, levels, P.meta, P.nt, P.pa);
+      if (!P.nodes && !P.wide) {  // the nodes' array first
+        J3DG_EQ(cudaMemcpyAsync(&h, P.ctl, kCtlHead, cudaMemcpyDeviceToHost, st));
+        J3DG_EQ(cudaStreamSynchronize(st));
+        if (e != cudaSuccess || h.error) return e;
+        if (h.top_left == 0) {
+          J3DG_EQ(cudaMallocAsync((void**)&P.nodes, sizeof(float4) * J3DG_NODE_F4(P.W) * (size_t)h.n_wide, st));
+          if (e != cudaSuccess) return e;
+          P.owned.push_back(P.nodes);
+        }
+      }
+    }
+    enqueue_place_levels(P, st, places, places + more_places, d_status);
+    J3DG_EQ(cudaMemcpyAsync(&h, P.ctl, kCtlHead, cudaMemcpyDeviceToHost, st));
+    J3DG_EQ(cudaStreamSynchronize(st));
+    if (e != cudaSuccess || h.error) return e;
+    tree = h.top_left == 0;
+    if (tree) {
+      places += more_places;
+      if (places >= kMaxPlaceLevels || h.place[places] == 0) {
+        if (h.place[std::min(places, kMaxPlaceLevels)]) h.error |= 4u;
+        return e;
+      }
+      more_places = std::min(4u, kMaxPlaceLevels - places);
+    } else {
+      if (levels >= kMaxTopLevels) {
+        h.error |= 1u;
+        return e;
+      }
+      more_levels = std::min(8u, kMaxTopLevels - levels);
+    }
+  }
 }
 
 // the LBVH (J3DG_BUILD_LBVH): Apetrei's one-pass binary tree over the sorted
@@ -2822,7 +3014,7 @@ static cudaError_t enqueue_tree_lbvh(BuildPlan& P, const uint64_t* keys, cudaStr
   BuildCtl* c = P.ctl;
   cudaError_t e = cudaSuccess;
   J3DG_EQ(cudaMemsetAsync(P.other, 0xff, sizeof(uint32_t) * (nt - 1), st));
-  k_lbvh<<<(nt + 255) / 256, 256, 0, st>>>(keys, P.tris_out, nt, P.child, P.box, P.range, P.other, &c->top_ctr[0]);
+  k_lbvh<<<(nt + 255) / 256, 256, 0, st>>>(keys, P.tris_out, nt, P.child, P.box, P.range, P.other, &c->root);
   k_lbvh_root<<<1, 1, 0, st>>>(c, P.qa);
   J3DG_EQ(cudaSuccess);
   J3DG_EQ(capture_while(st, side, [&](cudaStream_t s, cudaGraphConditionalHandle h) {
@@ -2849,9 +3041,9 @@ static cudaError_t enqueue_prefix(BuildPlan& P, const float* dV, const uint32_t*
   cudaError_t e = cudaSuccess;
   J3DG_EQ(cudaMemsetAsync(c, 0, sizeof(BuildCtl), st));
   k_bbox_partial<<<kBBoxBlocks, 256, 0, st>>>(dV, nv, P.part);
-  k_bbox_final<<<1, 1024, 0, st>>>(P.part, kBBoxBlocks, P.bb);
-  k_ctl_init<<<1, 1, 0, st>>>(c, P.tasks_a, P.small, P.ranges, P.bb, nt, P.top ? 1u : 0u, P.chunk());
-  k_tri_prep<<<(nt + 255) / 256, 256, 0, st>>>(dV, nv, dT, nt, P.bb, P.normals, P.k0, P.v0, d_status);
+  k_bbox_final<<<1, 1024, 0, st>>>(P.part, kBBoxBlocks, c->bb);
+  k_ctl_init<<<1, 1, 0, st>>>(c, P.tasks_a, P.small, P.ranges, nt, P.top ? 1u : 0u, P.chunk());
+  k_tri_prep<<<(nt + 255) / 256, 256, 0, st>>>(dV, nv, dT, nt, c->bb, P.normals, P.k0, P.v0, d_status);
   J3DG_EQ(cudaSuccess);
   {
     uint64_t *ka = P.k0, *kb = P.k1;
@@ -2872,15 +3064,14 @@ static cudaError_t enqueue_prefix(BuildPlan& P, const float* dV, const uint32_t*
   return e;
 }
 
-// The rest: the tree, its wide nodes in depth-first order and the triangles'
-// slots; its level loops are conditional while nodes, so `st` must be
-// capturing. The nodes go to P.nodes where it is given, else to P.wide (LBVH:
-// the permutation into depth-first order is then left to the caller).
+// The rest, captured: the tree, its wide nodes in depth-first order and the
+// triangles' slots. The nodes go to P.nodes where it is given, else to P.wide
+// (LBVH: the permutation into depth-first order is then left to the caller).
 static cudaError_t enqueue_tree(BuildPlan& P, cudaStream_t st, cudaStream_t side, uint32_t* d_status) {
   const uint32_t nt = P.nt;
   BuildCtl* c = P.ctl;
   cudaError_t e = cudaSuccess;
-  if (!P.lbvh) return enqueue_tree_ploc(P, P.nodes ? P.nodes : P.wide, st, side, d_status);
+  if (!P.lbvh) return capture_tree_ploc(P, st, side, d_status);
   J3DG_EQ(enqueue_tree_lbvh(P, sorted_keys(P), st, side, d_status));
   // depth-first numbering: subtree sizes bottom-up, positions top-down, permute
   k_dfs_setup<<<1, 1, 0, st>>>(c, P.dfs_pos, 0u);
@@ -2911,14 +3102,12 @@ static cudaError_t enqueue_build(BuildPlan& P, const float* dV, const uint32_t* 
   J3DG_EQ(enqueue_tree(P, st, side, d_status));
   return e;
 }
-#undef J3DG_EQ
 
-// A build through the device-driven graph: allocate, enqueue the prefix
-// (the GPU sorts while the host captures and instantiates the rest), capture
-// the tree's part, launch it, then take the tree's size from the device and
-// keep an exactly sized copy of the nodes.
-static int build_bvh_graph(j3dg_mesh* m, const float* dV, const uint32_t* dT, cudaStream_t st, uint32_t* d_status,
-                           cudaEvent_t done, std::string& err) {
+// One mesh's build: the prefix, then the tree on the same stream (LBVH: the
+// GPU sorts while the host captures and instantiates the tree's part), then
+// the tree's size from the device and an exactly sized copy of the nodes.
+static int build_bvh_tree(j3dg_mesh* m, const float* dV, const uint32_t* dT, cudaStream_t st, uint32_t* d_status,
+                          cudaEvent_t done, std::string& err) {
   BuildPlan P;
   P.nv = m->nv;
   P.nt = m->nt;
@@ -2932,22 +3121,24 @@ static int build_bvh_graph(j3dg_mesh* m, const float* dV, const uint32_t* dT, cu
   cudaGraph_t g = nullptr;
   cudaGraphExec_t ex = nullptr;
   BuildCtl h;
-  float hbb[6];
   int rc = J3DG_OK;
   cudaError_t e = plan_alloc(P, st, true, (m->build_flags & J3DG_BUILD_REBUILDABLE) != 0);
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = enqueue_prefix(P, dV, dT, st, d_status);
-  if (e == cudaSuccess) e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
-  if (e == cudaSuccess) {
-    const cudaError_t eq = enqueue_tree(P, st, side, d_status);
-    e = cudaStreamEndCapture(st, &g);
-    if (eq != cudaSuccess) e = eq;
+  J3DG_EQ(enqueue_prefix(P, dV, dT, st, d_status));
+  if (!P.lbvh) {
+    J3DG_EQ(run_tree_ploc(P, st, d_status, h));
+  } else {
+    J3DG_EQ(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+    if (e == cudaSuccess) e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+      const cudaError_t eq = enqueue_tree(P, st, side, d_status);
+      e = cudaStreamEndCapture(st, &g);
+      if (eq != cudaSuccess) e = eq;
+    }
+    J3DG_EQ(cudaGraphInstantiate(&ex, g, 0));
+    J3DG_EQ(cudaGraphLaunch(ex, st));
+    J3DG_EQ(cudaMemcpyAsync(&h, P.ctl, kCtlHead, cudaMemcpyDeviceToHost, st));
+    J3DG_EQ(cudaStreamSynchronize(st));
   }
-  if (e == cudaSuccess) e = cudaGraphInstantiate(&ex, g, 0);
-  if (e == cudaSuccess) e = cudaGraphLaunch(ex, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&h, P.ctl, sizeof(h), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(hbb, P.bb, sizeof(hbb), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
     err = std::string("build: ") + cudaGetErrorString(e);
     rc = e == cudaErrorMemoryAllocation ? J3DG_ERR_OUT_OF_MEMORY : J3DG_ERR_CUDA;
@@ -2960,42 +3151,34 @@ static int build_bvh_graph(j3dg_mesh* m, const float* dV, const uint32_t* dT, cu
   if (rc == J3DG_OK) {
     m->scale = 0.f;
     for (int k = 0; k < 3; ++k) {
-      m->min_bb[k] = hbb[k];
-      m->max_bb[k] = hbb[3 + k];
+      m->min_bb[k] = h.bb[k];
+      m->max_bb[k] = h.bb[3 + k];
     }
-    for (int k = 0; k < 6; ++k) m->scale = std::max(m->scale, std::fabs(hbb[k]));
+    for (int k = 0; k < 6; ++k) m->scale = std::max(m->scale, std::fabs(h.bb[k]));
     m->n_nodes = h.n_wide;
     m->max_depth = h.max_depth;
     m->root_ref = 0;
-    // the nodes into an array of the tree's size (a rebuildable mesh keeps the
-    // array at the size bound: its nodes are there already)
-    const size_t bytes = sizeof(float4) * J3DG_NODE_F4(P.W) * (size_t)m->n_nodes;
-    if (m->build_flags & J3DG_BUILD_REBUILDABLE) {
-      m->d_nodes = P.nodes;
-      P.nodes = nullptr;
+    // the nodes into an array of the tree's size, unless they are where they
+    // stay (a rebuildable mesh keeps an array at the size bound)
+    if (P.nodes) {
+      m->d_nodes = plan_take(P, P.nodes);
     } else {
-      // the gathered triangles are not needed any more: their memory goes to
-      // the nodes (as an addition to the pool these took 0.85 ms at 778 MB)
-      if (P.soup) cudaFreeAsync(P.soup, st);
-      P.soup = nullptr;
-      e = cudaMallocAsync(&m->d_nodes, bytes ? bytes : sizeof(float4) * J3DG_NODE_F4(P.W), st);
-    }
-    if (e == cudaSuccess && !(m->build_flags & J3DG_BUILD_REBUILDABLE) && m->n_nodes) {
-      if (P.lbvh) {
-        k_dfs_permute<4><<<(m->n_nodes + 255) / 256, 256, 0, st>>>(P.wide, &P.ctl->n_wide, P.dfs_pos, (float4*)m->d_nodes);
-        e = cudaGetLastError();
-      } else {
-        e = cudaMemcpyAsync(m->d_nodes, P.wide, bytes, cudaMemcpyDeviceToDevice, st);
+      const size_t node = sizeof(float4) * J3DG_NODE_F4(P.W);
+      e = cudaMallocAsync(&m->d_nodes, node * std::max(1u, m->n_nodes), st);
+      if (e == cudaSuccess && m->n_nodes) {
+        if (P.lbvh)
+          k_dfs_permute<4><<<(m->n_nodes + 255) / 256, 256, 0, st>>>(P.wide, &P.ctl->n_wide, P.dfs_pos,
+                                                                     (float4*)m->d_nodes);
+        else
+          e = cudaMemcpyAsync(m->d_nodes, P.wide, node * m->n_nodes, cudaMemcpyDeviceToDevice, st);
+        J3DG_EQ(cudaSuccess);
       }
     }
     if (e == cudaSuccess && done) e = cudaEventRecord(done, st);  // the BVH is ready; the rest is clean-up
     if (e == cudaSuccess) {
-      m->d_normals = P.normals;
-      m->d_tris = P.tris_out;
-      m->d_slot_of = P.slot_of;
-      P.normals = nullptr;
-      P.tris_out = nullptr;
-      P.slot_of = nullptr;
+      m->d_normals = plan_take(P, P.normals);
+      m->d_tris = plan_take(P, P.tris_out);
+      m->d_slot_of = plan_take(P, P.slot_of);
     } else {
       err = std::string("build: ") + cudaGetErrorString(e);
       rc = e == cudaErrorMemoryAllocation ? J3DG_ERR_OUT_OF_MEMORY : J3DG_ERR_CUDA;
@@ -3082,10 +3265,10 @@ cudaError_t rebuild_enqueue(RebuildLane* L, const j3dg_mesh* m, cudaStream_t st,
 // mesh fields (bbox, scale, nodes, leaf-ordered triangles, normals); `done`
 // (may be null) is recorded on st once the BVH is ready, before the host's
 // clean-up (the build time is taken up to it). Both builders go through
-// build_bvh_graph; a mesh of at most one leaf is built here.
+// build_bvh_tree; a mesh of at most one leaf is built here.
 int build_bvh(j3dg_mesh* m, const float* dV, const uint32_t* dT, cudaStream_t st, uint32_t* d_status,
               cudaEvent_t done, std::string& err) {
-  if (m->nt > m->leaf_size) return build_bvh_graph(m, dV, dT, st, d_status, done, err);
+  if (m->nt > m->leaf_size) return build_bvh_tree(m, dV, dT, st, d_status, done, err);
   int rc = J3DG_OK;
   const uint32_t nv = m->nv, nt = m->nt;
   float* d_part = nullptr;
@@ -3147,4 +3330,5 @@ cleanup:
   return J3DG_OK;
 }
 
+#undef J3DG_EQ
 }  // namespace j3dg
