@@ -118,7 +118,7 @@ __device__ __forceinline__ uint64_t spread3(uint32_t x) {
 
 __global__ void k_tri_prep(const float* __restrict__ V, uint32_t nv, const uint32_t* __restrict__ T, uint32_t nt,
                            const float* __restrict__ bb, float4* __restrict__ normals, uint64_t* __restrict__ keys,
-                           uint32_t* __restrict__ vals, uint32_t* status) {
+                           uint32_t* status) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nt) return;
   uint32_t a = T[3 * (size_t)i], b = T[3 * (size_t)i + 1], c = T[3 * (size_t)i + 2];
@@ -155,212 +155,204 @@ __global__ void k_tri_prep(const float* __restrict__ V, uint32_t nv, const uint3
     q[k] = (uint32_t)f;
   }
   keys[i] = (spread3(q[0]) << 2) | (spread3(q[1]) << 1) | spread3(q[2]);
-  vals[i] = i;
 }
 
 // ------------------------------------------------------ 3. radix sort ----
 
-static const int kSortThreads = 256;
-static const int kSortItems = 8;  // tiles of 2048 keys: the scatter's shared-memory reorder fits 34 KB
-static const int kSortTile = kSortThreads * kSortItems;
+// Least significant digit first, a kernel a digit: a block takes a tile, ranks
+// its keys within their digits, and learns how many keys of each digit the
+// tiles before it hold by looking back over what they have published
+// (Adinets and Merrill 2022, "Onesweep: A Faster Least Significant Digit Radix
+// Sort for GPUs"), so that a pass reads and writes the keys once; the totals
+// of all digits come from one pass over the keys before.
+//
+// Measured (GB300), all six digits: 82k keys 60 us, 500k 84, 2M 159, 28.09M
+// 1209 (of which the totals 8-75), where counting each tile's digits, scanning
+// the counts of all tiles and then moving the keys, four kernels a digit, took
+// 147 at 82k and 2250 at 28.09M. There a pass moves 674 MB in 189 us. Bound by
+// the ranking (shared memory and votes) and the words looked back at; so a
+// tile is as large as four blocks an SM carry: 16 keys a thread at 64
+// registers (the values fetched once the keys have left theirs), against 1738
+// us with 8 keys and 1740 with 16 and three blocks. match.any in place of the
+// eight votes: 1988. Below 300k keys the tiles are too few for the SMs, and
+// 4 keys a thread are faster (82k: 60 us against 72; 500k: 98 against 84).
 
-__global__ void k_radix_hist(const uint64_t* __restrict__ keys, uint32_t n, int shift, uint32_t num_tiles,
-                             uint32_t* __restrict__ hist) {
-  __shared__ uint32_t h[256];
-  h[threadIdx.x] = 0;
-  __syncthreads();
-  size_t base = (size_t)blockIdx.x * kSortTile;
-#pragma unroll 4
-  for (int j = 0; j < kSortItems; ++j) {
-    size_t idx = base + (size_t)j * kSortThreads + threadIdx.x;
-    if (idx < n) atomicAdd(&h[(keys[idx] >> shift) & 255u], 1u);
-  }
-  __syncthreads();
-  hist[(size_t)threadIdx.x * num_tiles + blockIdx.x] = h[threadIdx.x];
-}
+static const int kSortItems = 16, kSortFew = 4;  // keys per thread
+static const uint32_t kSortLarge = 300000u;      // from this many keys on
+static const uint32_t kSortLook = 8;             // words looked at together
 
-// exclusive scan helpers (over chunks of 1024 elements):
-// k_scan_chunks scans each chunk (256 threads x 4 elements: a sequential
-// scan of the thread's uint4, a shuffle scan of the warp's totals, the
-// eight warp totals through shared memory) and writes the chunk total,
-// k_scan_sums scans the chunk totals, which the readers add. in and out
-// are 16-byte aligned (device allocations); elements past n read as 0 and
-// are not written.
-__global__ void __launch_bounds__(256) k_scan_chunks(const uint32_t* in, uint32_t* out, uint32_t n,
-                                                     uint32_t* __restrict__ sums) {
-  __shared__ uint32_t wsum[8];
-  const uint32_t base = blockIdx.x * 1024u + threadIdx.x * 4u;
-  uint4 v = make_uint4(0u, 0u, 0u, 0u);
-  if (base + 3 < n) {
-    v = *reinterpret_cast<const uint4*>(in + base);
-  } else {
-    if (base < n) v.x = in[base];
-    if (base + 1 < n) v.y = in[base + 1];
-    if (base + 2 < n) v.z = in[base + 2];
-  }
-  const uint32_t tot = v.x + v.y + v.z + v.w;
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  uint32_t inc = tot;  // inclusive scan of the thread totals within the warp
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= (uint32_t)o) inc += y;
-  }
-  if (lane == 31) wsum[warp] = inc;
-  __syncthreads();
-  uint32_t woff = 0, all = 0;
-#pragma unroll
-  for (uint32_t w = 0; w < 8; ++w) {
-    const uint32_t x = wsum[w];
-    woff += w < warp ? x : 0u;
-    all += x;
-  }
-  const uint32_t e = woff + inc - tot;  // exclusive prefix of this thread's first element
-  const uint4 o4 = make_uint4(e, e + v.x, e + v.x + v.y, e + v.x + v.y + v.z);
-  if (base + 3 < n) {
-    *reinterpret_cast<uint4*>(out + base) = o4;
-  } else {
-    if (base < n) out[base] = o4.x;
-    if (base + 1 < n) out[base + 1] = o4.y;
-    if (base + 2 < n) out[base + 2] = o4.z;
-  }
-  if (threadIdx.x == 0) sums[blockIdx.x] = all;
-}
+static const int kSortThreads = 256, kSortWarps = kSortThreads / 32;
 
-__global__ void __launch_bounds__(1024) k_scan_sums(uint32_t* __restrict__ sums, uint32_t n) {
-  // single block of 1024 threads: each thread sums a strip of consecutive
-  // chunk totals, the strip sums are scanned by warp shuffles (within each
-  // warp, then the 32 warp totals by warp 0), and each thread rewrites its
-  // strip as exclusive prefixes
-  __shared__ uint32_t wtot[32];
-  const uint32_t per = (n + 1023) / 1024;
-  const uint32_t b = threadIdx.x * per, e = min(n, b + per);
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  uint32_t acc = 0;
-  for (uint32_t i = b; i < e; ++i) acc += sums[i];
-  uint32_t inc = acc;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= (uint32_t)o) inc += y;
-  }
-  if (lane == 31) wtot[warp] = inc;
+// keys by every digit: totals[pass][256] (zero before)
+__global__ void __launch_bounds__(512) k_radix_totals(const uint64_t* __restrict__ keys, uint32_t n,
+                                                      uint32_t* __restrict__ totals) {
+  __shared__ uint32_t h[kRadixPasses][256];
+  for (uint32_t k = threadIdx.x; k < kRadixPasses * 256u; k += blockDim.x) (&h[0][0])[k] = 0;
   __syncthreads();
-  if (warp == 0) {
-    const uint32_t x = wtot[lane];
-    uint32_t xi = x;
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 4u * stride) {
+    uint64_t k[4];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, xi, o);
-      if (lane >= (uint32_t)o) xi += y;
+    for (uint32_t j = 0; j < 4; ++j) {
+      const uint64_t i = (uint64_t)i0 + (uint64_t)j * stride;
+      k[j] = i < n ? keys[i] : 0ull;
     }
-    wtot[lane] = xi - x;
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j)
+      if ((uint64_t)i0 + (uint64_t)j * stride < n)
+#pragma unroll
+        for (int p = 0; p < kRadixPasses; ++p) atomicAdd(&h[p][(k[j] >> (8 * p)) & 255u], 1u);
   }
   __syncthreads();
-  uint32_t run = wtot[warp] + inc - acc;
-  for (uint32_t i = b; i < e; ++i) {
-    const uint32_t x = sums[i];
-    sums[i] = run;
-    run += x;
+  for (uint32_t k = threadIdx.x; k < kRadixPasses * 256u; k += blockDim.x) {
+    const uint32_t c = (&h[0][0])[k];
+    if (c) atomicAdd(totals + k, c);
   }
 }
 
-// One tile of kSortTile keys per block: each key's rank among the tile's
-// keys of its digit comes from kSortItems rounds of 256 keys (warp
-// match_any ranks, per-warp digit counts scanned across the warps, a
-// running count per digit); the tile is then reordered by digit in shared
-// memory (stable) and written out so that consecutive threads write
-// consecutive positions of one digit's run (coalesced, instead of one
-// scattered 8-byte write per key).
-__global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const uint64_t* __restrict__ kin,
-                                                                const uint32_t* __restrict__ vin,
-                                                                uint64_t* __restrict__ kout, uint32_t* __restrict__ vout,
-                                                                uint32_t n, int shift, uint32_t num_tiles,
-                                                                const uint32_t* __restrict__ offsets,
-                                                                const uint32_t* __restrict__ chunk_offsets,
-                                                                uint32_t* status) {
-  __shared__ uint32_t base[256];     // global position of the tile's first key of each digit
-  __shared__ uint32_t run[256];      // keys of each digit in the tile's earlier rounds, then the digit's local start
-  __shared__ uint32_t wc[kSortThreads / 32][257];
-  __shared__ uint64_t sk[kSortTile];
-  __shared__ uint32_t sv[kSortTile];
-  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  {
-    // offsets: the digit histogram's scan within chunks of 1024 entries;
-    // chunk_offsets: the scanned chunk totals
-    const size_t h = (size_t)tid * num_tiles + blockIdx.x;
-    base[tid] = offsets[h] + chunk_offsets[h >> 10];
-  }
-  run[tid] = 0;
-  const size_t tile = (size_t)blockIdx.x * kSortTile;
-  uint64_t key[kSortItems];
-  uint32_t rnk[kSortItems];  // digit (low 9 bits: 256 = no key) and rank within the tile's digit
+// what a tile publishes per digit: its own count, then the count of all tiles
+// up to it; one word, so no other memory is ordered by it
+static const uint32_t kSortOwn = 1u << 30, kSortUpTo = 2u << 30, kSortCount = kSortOwn - 1u;
+static_assert(J3DG_MAX_TRIANGLES <= kSortOwn, "a count beside the two flag bits");
+static const uint32_t kSortPolls = 1u << 18;  // looks at a tile's word before the sort gives up (> 0.1 s)
+
+template <int ITEMS>
+struct SortMem {
+  union {
+    uint32_t count[kSortWarps][256];  // a warp's keys by digit, then the earlier warps'
+    struct {
+      uint64_t key[ITEMS * kSortThreads];
+      uint32_t val[ITEMS * kSortThreads];
+    };
+  };
+  uint32_t start[256];  // a digit's first key in the tile
+  uint32_t place[256];  // ... its position in the output less that
+  uint64_t wsum[kSortWarps];
+  uint32_t tile;
+};
+
+// One digit (shift): keys and values (vin null: the positions) to kout (null:
+// the keys are not needed any more) and vout. rows: 256 words a tile, zero
+// before; tiles are taken in order (ticket, zero before), so those that a
+// block waits for are running or done.
+template <int ITEMS>
+__global__ void __launch_bounds__(kSortThreads, 4) k_radix_pass(const uint64_t* __restrict__ kin,
+                                                             const uint32_t* __restrict__ vin,
+                                                             uint64_t* __restrict__ kout, uint32_t* __restrict__ vout,
+                                                             uint32_t n, int shift, const uint32_t* __restrict__ totals,
+                                                             uint32_t* rows, uint32_t* ticket, uint32_t* status) {
+  constexpr uint32_t kTile = ITEMS * kSortThreads;
+  extern __shared__ __align__(16) uint8_t sort_raw[];
+  SortMem<ITEMS>& s = *reinterpret_cast<SortMem<ITEMS>*>(sort_raw);
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, below = (1u << lane) - 1u;
+  if (tid == 0) s.tile = atomicAdd(ticket, 1u);
 #pragma unroll
-  for (int j = 0; j < kSortItems; ++j) {
-    for (int w = 0; w < kSortThreads / 32; ++w) wc[w][tid] = 0;
-    if (tid == 0)
-      for (int w = 0; w < kSortThreads / 32; ++w) wc[w][256] = 0;
-    __syncthreads();
-    const size_t idx = tile + (size_t)j * kSortThreads + tid;
-    const bool valid = idx < n;
-    const uint64_t k = valid ? kin[idx] : 0;
-    const uint32_t d = valid ? (uint32_t)((k >> shift) & 255u) : 256u;
-    const uint32_t peers = __match_any_sync(0xffffffffu, d);
-    const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
-    if (rank == 0) wc[warp][d] = __popc(peers);
-    __syncthreads();
-    uint32_t tot = 0;
-    {
-      uint32_t acc = 0;
-      for (int w = 0; w < kSortThreads / 32; ++w) {
-        const uint32_t c = wc[w][tid];
-        wc[w][tid] = acc;
-        acc += c;
+  for (int w = 0; w < kSortWarps; ++w) s.count[w][tid] = 0u;
+  const uint32_t total = totals[tid];
+  __syncthreads();
+  const uint32_t tile = s.tile;
+  const uint64_t first = (uint64_t)tile * kTile;
+  const uint32_t held = (uint32_t)min((uint64_t)kTile, (uint64_t)n - first);  // (the grid has a block per tile)
+  // a warp's keys are consecutive, 32 at a time; past the end: the largest,
+  // which come after the tile's others
+  const uint32_t at = warp * (ITEMS * 32u) + lane;
+  uint64_t key[ITEMS];
+  uint32_t rank[ITEMS];
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) key[j] = at + 32u * j < held ? kin[first + at + 32u * j] : ~0ull;
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const uint32_t d = (uint32_t)(key[j] >> shift) & 255u;
+    uint32_t peers = 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      const bool bit = (d >> b) & 1u;
+      const uint32_t m = __ballot_sync(0xffffffffu, bit);
+      peers &= bit ? m : ~m;
+    }
+    const uint32_t before = s.count[warp][d];
+    __syncwarp();
+    if ((peers & below) == 0u) s.count[warp][d] = before + __popc(peers);
+    __syncwarp();
+    rank[j] = before + __popc(peers & below);
+  }
+  __syncthreads();
+  // thread d: digit d
+  uint32_t own = 0;
+#pragma unroll
+  for (int w = 0; w < kSortWarps; ++w) {
+    const uint32_t c = s.count[w][tid];
+    s.count[w][tid] = own;
+    own += c;
+  }
+  volatile uint32_t* const row = rows + (size_t)tile * 256u + tid;
+  *row = own | (tile == 0u ? kSortUpTo : kSortOwn);
+  // both exclusive scans over the digits in one: of the totals (high) and of
+  // the tile's counts (low 16 bits)
+  const uint64_t x = ((uint64_t)total << 16) | own;
+  uint64_t incl = x;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint64_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= (uint32_t)o) incl += y;
+  }
+  if (lane == 31) s.wsum[warp] = incl;
+  __syncthreads();
+  uint64_t ex = incl - x;
+#pragma unroll
+  for (uint32_t w = 0; w < kSortWarps; ++w)
+    if (w < warp) ex += s.wsum[w];
+  const uint32_t start = (uint32_t)ex & 0xffffu;
+  s.start[tid] = start;
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const uint32_t d = (uint32_t)(key[j] >> shift) & 255u;
+    rank[j] += s.start[d] + s.count[warp][d];
+  }
+  __syncthreads();  // the counts' memory becomes the tile's
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) s.key[rank[j]] = key[j];
+  uint32_t val[ITEMS];  // (fetched here: the keys' registers are free)
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const uint32_t k = at + 32u * j;
+    val[j] = k < held ? (vin ? vin[first + k] : (uint32_t)first + k) : 0u;
+  }
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) s.val[rank[j]] = val[j];
+  // the tiles before, several words at a time
+  uint32_t earlier = 0;
+  if (tile > 0u) {
+    uint32_t t = tile, polls = 0;
+    bool found = false;
+    while (!found) {
+      uint32_t v[kSortLook];
+#pragma unroll
+      for (uint32_t q = 0; q < kSortLook; ++q)
+        v[q] = t > q ? *(volatile uint32_t*)(rows + (size_t)(t - 1u - q) * 256u + tid) : kSortUpTo + 0u;
+#pragma unroll
+      for (uint32_t q = 0; q < kSortLook; ++q) {
+        if (found || v[q] < kSortOwn) break;  // nothing there yet: look again from it
+        earlier += v[q] & kSortCount;
+        --t;
+        found = v[q] >= kSortUpTo;
       }
-      tot = acc;
+      if (!found && ++polls >= kSortPolls) {  // (a stuck tile: the places are wrong, none is out of range)
+        atomicOr(status, J3DG_DEV_VISIT_CAP);
+        break;
+      }
     }
-    __syncthreads();
-    key[j] = k;
-    rnk[j] = d | ((valid ? run[d] + wc[warp][d] + rank : 0u) << 9);
-    __syncthreads();
-    run[tid] += tot;
+    *row = ((earlier + own) & kSortCount) | kSortUpTo;
   }
+  s.place[tid] = (uint32_t)(ex >> 16) + earlier - start;
   __syncthreads();
-  // the digits' starts within the tile: exclusive scan of the counts (run)
-  {
-    const uint32_t c = run[tid];
-    uint32_t incl = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= (uint32_t)o) incl += y;
-    }
-    if (lane == 31) wc[0][warp] = incl;
-    __syncthreads();
-    uint32_t woff = 0;
-    for (uint32_t w = 0; w < warp; ++w) woff += wc[0][w];
-    __syncthreads();
-    run[tid] = woff + incl - c;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < kSortItems; ++j) {
-    const uint32_t d = rnk[j] & 511u;
-    if (d < 256u) {
-      const uint32_t l = run[d] + (rnk[j] >> 9);
-      sk[l] = key[j];
-      sv[l] = vin[tile + (size_t)j * kSortThreads + tid];
-    }
-  }
-  __syncthreads();
-  const uint32_t tile_n = (uint32_t)min((size_t)kSortTile, (size_t)n - tile);
-  for (uint32_t i = tid; i < tile_n; i += kSortThreads) {
-    const uint64_t k = sk[i];
-    const uint32_t d = (uint32_t)((k >> shift) & 255u);
-    const uint32_t pos = base[d] + (i - run[d]);
+  for (uint32_t i = tid; i < held; i += kSortThreads) {
+    const uint64_t k = s.key[i];
+    const uint32_t pos = s.place[(uint32_t)(k >> shift) & 255u] + i;
     if (pos < n) {
-      kout[pos] = k;
-      vout[pos] = sv[i];
+      if (kout) kout[pos] = k;
+      vout[pos] = s.val[i];
     } else {
       atomicOr(status, J3DG_DEV_BAD_INDEX);
     }
@@ -373,7 +365,7 @@ __global__ void k_soup(const float* __restrict__ V, const uint32_t* __restrict__
                        uint32_t nt, uint32_t nv, float4* __restrict__ tris, uint32_t* status) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nt) return;
-  uint32_t id = order[i];
+  uint32_t id = order ? order[i] : i;
   if (id >= nt) {
     atomicOr(status, J3DG_DEV_BAD_INDEX);
     id = 0;
@@ -2672,7 +2664,7 @@ struct BuildPlan {
   // scratch
   float* part = nullptr;
   uint64_t *k0 = nullptr, *k1 = nullptr;
-  uint32_t *v0 = nullptr, *v1 = nullptr, *hist = nullptr, *sums = nullptr;
+  uint32_t *v0 = nullptr, *v1 = nullptr, *sort = nullptr;  // sort: per pass a ticket, the totals, the rows
   uint32_t *ord_a = nullptr, *ord_b = nullptr, *top_up = nullptr, *top_done = nullptr, *bins_a = nullptr, *bins_b = nullptr,
            *icum = nullptr;
   BinNode* tbox = nullptr;
@@ -2699,9 +2691,11 @@ struct BuildPlan {
   // tasks of one level are disjoint, each above kSmallTask; so are the small tasks, each above J3DG_SAH_TOP
   uint32_t cap_tasks() const { return nt / kSmallTask + 1; }
   uint32_t cap_small() const { return nt / J3DG_SAH_TOP + 1; }
-  uint32_t n_tiles() const { return (nt + kSortTile - 1) / kSortTile; }
-  uint32_t hist_n() const { return 256 * n_tiles(); }
-  uint32_t scan_blocks() const { return (hist_n() + 1023) / 1024; }
+  // keys per thread of the sort: the tile is as large as registers and shared
+  // memory carry well where there are tiles for every SM, else smaller
+  uint32_t sort_items() const { return nt >= kSortLarge ? kSortItems : kSortFew; }
+  uint32_t sort_tiles() const { return (nt + sort_items() * kSortThreads - 1) / (sort_items() * kSortThreads); }
+  size_t sort_words() const { return kRadixPasses * (256 * ((size_t)sort_tiles() + 1) + 1); }
   // positions per item of the SAH levels: large ones keep the runs of the
   // binning long and the bins to merge few; below about two items an SM (304
   // on 152 SMs) smaller items fill the device instead
@@ -2761,8 +2755,9 @@ static cudaError_t plan_alloc(BuildPlan& P, cudaStream_t st, bool outputs = true
   A(P.k1, sizeof(uint64_t) * nt);
   A(P.v0, sizeof(uint32_t) * nt);
   A(P.v1, sizeof(uint32_t) * nt);
-  A(P.hist, sizeof(uint32_t) * P.hist_n());
-  A(P.sums, sizeof(uint32_t) * (P.scan_blocks() + 1));
+  // (a lane's smaller meshes may have more tiles)
+  A(P.sort, sizeof(uint32_t) *
+                std::max(P.sort_words(), (size_t)kRadixPasses * (256 * (kSortLarge / (kSortFew * kSortThreads) + 3))));
   if (P.need_ploc) {
     A(P.ord_a, sizeof(uint32_t) * nt);
     A(P.ord_b, sizeof(uint32_t) * nt);
@@ -3031,6 +3026,38 @@ static cudaError_t enqueue_tree_lbvh(BuildPlan& P, const uint64_t* keys, cudaStr
 // the sorted Morton codes after the radix passes (they alternate k0 / k1)
 static const uint64_t* sorted_keys(const BuildPlan& P) { return (kRadixPasses & 1) ? P.k1 : P.k0; }
 
+template <int ITEMS>
+static cudaError_t enqueue_radix_pass(BuildPlan& P, const uint64_t* ka, const uint32_t* va, uint64_t* kb, uint32_t* vb,
+                                      int pass, cudaStream_t st, uint32_t* d_status) {
+  const cudaError_t e =
+      cudaFuncSetAttribute(k_radix_pass<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortMem<ITEMS>));
+  if (e != cudaSuccess) return e;
+  const uint32_t tiles = P.sort_tiles();
+  uint32_t *tickets = P.sort, *totals = tickets + kRadixPasses, *rows = totals + kRadixPasses * 256;
+  k_radix_pass<ITEMS><<<tiles, kSortThreads, sizeof(SortMem<ITEMS>), st>>>(
+      ka, va, kb, vb, P.nt, 8 * pass, totals + 256 * pass, rows + (size_t)pass * tiles * 256, tickets + pass, d_status);
+  return cudaGetLastError();
+}
+
+// keys P.k0 (the passes alternate k0 / k1) to the order of the triangles
+static cudaError_t enqueue_sort(BuildPlan& P, cudaStream_t st, uint32_t* d_status) {
+  cudaError_t e = cudaSuccess;
+  J3DG_EQ(cudaMemsetAsync(P.sort, 0, sizeof(uint32_t) * P.sort_words(), st));
+  k_radix_totals<<<std::min(kStrideBlocks / 4u, (P.nt + 2047u) / 2048u), 512, 0, st>>>(P.k0, P.nt, P.sort + kRadixPasses);
+  J3DG_EQ(cudaSuccess);
+  uint64_t *ka = P.k0, *kb = P.k1;
+  uint32_t *va = P.v0, *vb = P.v1;
+  for (int pass = 0; pass < kRadixPasses; ++pass) {
+    const uint32_t* in = pass ? va : nullptr;
+    uint64_t* out = pass + 1 < kRadixPasses || P.lbvh ? kb : nullptr;  // the LBVH reads the sorted codes
+    J3DG_EQ(P.sort_items() == kSortItems ? enqueue_radix_pass<kSortItems>(P, ka, in, out, vb, pass, st, d_status)
+                                              : enqueue_radix_pass<kSortFew>(P, ka, in, out, vb, pass, st, d_status));
+    std::swap(ka, kb);
+    std::swap(va, vb);
+  }
+  return e;
+}
+
 // A build's first part, whose launches do not depend on the tree: the loop
 // state reset, the bounding box, normals and Morton codes, the radix sort
 // and the gather into Morton order. No host synchronisation.
@@ -3043,23 +3070,11 @@ static cudaError_t enqueue_prefix(BuildPlan& P, const float* dV, const uint32_t*
   k_bbox_partial<<<kBBoxBlocks, 256, 0, st>>>(dV, nv, P.part);
   k_bbox_final<<<1, 1024, 0, st>>>(P.part, kBBoxBlocks, c->bb);
   k_ctl_init<<<1, 1, 0, st>>>(c, P.tasks_a, P.small, P.ranges, nt, P.top ? 1u : 0u, P.chunk());
-  k_tri_prep<<<(nt + 255) / 256, 256, 0, st>>>(dV, nv, dT, nt, c->bb, P.normals, P.k0, P.v0, d_status);
+  k_tri_prep<<<(nt + 255) / 256, 256, 0, st>>>(dV, nv, dT, nt, c->bb, P.normals, P.k0, d_status);
   J3DG_EQ(cudaSuccess);
-  {
-    uint64_t *ka = P.k0, *kb = P.k1;
-    uint32_t *va = P.v0, *vb = P.v1;
-    for (int pass = 0; pass < kRadixPasses; ++pass) {
-      const int shift = 8 * pass;
-      k_radix_hist<<<P.n_tiles(), kSortThreads, 0, st>>>(ka, nt, shift, P.n_tiles(), P.hist);
-      k_scan_chunks<<<P.scan_blocks(), 256, 0, st>>>(P.hist, P.hist, P.hist_n(), P.sums);
-      k_scan_sums<<<1, 1024, 0, st>>>(P.sums, P.scan_blocks());
-      k_radix_scatter<<<P.n_tiles(), kSortThreads, 0, st>>>(ka, va, kb, vb, nt, shift, P.n_tiles(), P.hist, P.sums,
-                                                           d_status);
-      std::swap(ka, kb);
-      std::swap(va, vb);
-    }
-    k_soup<<<(nt + 255) / 256, 256, 0, st>>>(dV, dT, va, nt, nv, P.lbvh ? P.tris_out : P.soup, d_status);
-  }
+  J3DG_EQ(enqueue_sort(P, st, d_status));
+  k_soup<<<(nt + 255) / 256, 256, 0, st>>>(dV, dT, kRadixPasses & 1 ? P.v1 : P.v0, nt, nv, P.lbvh ? P.tris_out : P.soup,
+                                           d_status);
   J3DG_EQ(cudaSuccess);
   return e;
 }
@@ -3274,7 +3289,6 @@ int build_bvh(j3dg_mesh* m, const float* dV, const uint32_t* dT, cudaStream_t st
   float* d_part = nullptr;
   float* d_bb = nullptr;
   uint64_t* k0 = nullptr;
-  uint32_t* v0 = nullptr;
   const int bbox_blocks = 1024;
   float hbb[6];
   const uint32_t W = m->width;
@@ -3299,9 +3313,8 @@ int build_bvh(j3dg_mesh* m, const float* dV, const uint32_t* dT, cudaStream_t st
   J3DG_CK(cudaMallocAsync(&m->d_normals, sizeof(float4) * (size_t)nt, st));
   J3DG_CK(cudaMallocAsync(&m->d_tris, sizeof(float4) * 3 * (size_t)nt, st));
   J3DG_CK(cudaMallocAsync((void**)&k0, sizeof(uint64_t) * nt, st));
-  J3DG_CK(cudaMallocAsync((void**)&v0, sizeof(uint32_t) * nt, st));
-  k_tri_prep<<<1, 256, 0, st>>>(dV, nv, dT, nt, d_bb, (float4*)m->d_normals, k0, v0, d_status);  // v0[i] = i
-  k_soup<<<1, 256, 0, st>>>(dV, dT, v0, nt, nv, (float4*)m->d_tris, d_status);
+  k_tri_prep<<<1, 256, 0, st>>>(dV, nv, dT, nt, d_bb, (float4*)m->d_normals, k0, d_status);
+  k_soup<<<1, 256, 0, st>>>(dV, dT, nullptr, nt, nv, (float4*)m->d_tris, d_status);
   J3DG_CK(cudaGetLastError());
   m->root_ref = J3DG_LEAF_BIT | (nt - 1u);
   m->n_nodes = 0;
@@ -3317,7 +3330,6 @@ cleanup:
   if (d_part) cudaFreeAsync(d_part, st);
   if (d_bb) cudaFreeAsync(d_bb, st);
   if (k0) cudaFreeAsync(k0, st);
-  if (v0) cudaFreeAsync(v0, st);
   {
     cudaError_t e = cudaStreamSynchronize(st);
     if (rc == J3DG_OK && e != cudaSuccess) {
