@@ -625,6 +625,7 @@ struct BuildCtl {
   uint32_t place[kMaxPlaceLevels + 1];  // subtrees to be placed, by level
   uint32_t root;                        // the binary tree's root
   uint32_t top_base, place_base;
+  uint32_t place_jobs;                  // subtrees that a warp places
   uint32_t n_small, n_ranges;           // small tasks and finished ranges
   uint32_t next_job;                    // the next of them to be taken (k_small_tasks)
   struct Level {
@@ -737,146 +738,175 @@ struct PlaceItem {
 // triangles' positions to slot_of). A wide node's place in depth-first order
 // is its parent's, plus one, plus the wide nodes of the slots before it: the
 // wide nodes are written where they stay.
+//
+// A lane makes a slot: it goes down from the wide node's binary node by the
+// decisions, at most W steps of one load's latency each, and holds the slot's
+// box when it arrives. The warp then writes its nodes and copies the
+// triangles of its leaves from shared memory, whole lines at a time. Subtrees
+// above kPlaceJob triangles go level by level; below, a warp places a whole
+// subtree, so that what its nodes share (sectors of the binary tree, lines of
+// the output) is used while it is near, and no queue in global memory is
+// added to. With a lane per wide node (a stack of subtrees, a loop over its
+// leaves' triangles: the latencies of some twenty loads) and levels down to
+// the leaves the placement took 3.35 ms for 28.09M triangles (6.08M nodes),
+// 365 us for 2M, 116 for 82k; a lane per slot, by levels, 3.31, 242 and 67;
+// now 1.78 ms, 203 and 63.
 template <int W>
-__device__ __forceinline__ void collapse_place_one(const BinNode* __restrict__ node, const NodeMeta* __restrict__ meta,
-                                                   const BinNode* __restrict__ tbox, const float4* __restrict__ tris,
-                                                   const PlaceItem* __restrict__ qin, uint32_t t, uint32_t n_in,
-                                                   PlaceItem* __restrict__ qout, uint32_t* __restrict__ n_out,
-                                                   uint32_t n_wide, float4* __restrict__ wide,
-                                                   uint32_t* __restrict__ max_depth, float4* __restrict__ tris_out,
-                                                   uint32_t* __restrict__ slot_of, uint32_t nt, uint32_t* status) {
-  // whole warps come here together (the next level's slots are allocated per
-  // warp); lanes past n_in place nothing
-  const uint32_t lane = threadIdx.x & 31u;
-  const bool valid = t < n_in;
-  const PlaceItem it = valid ? qin[t] : PlaceItem{0u, 0u, 0u, 0u};
-  // the slots the cost decisions give: expand(left, k) then expand(right, W - k)
-  uint32_t ref[W], cnt[W], start[W], sub[W];  // sub: wide nodes in the slot (0: a leaf)
-  float4 lo[W], hi[W];
-  int m = 0;
-  auto count_of = [&](uint32_t r) { return (r & 0x80000000u) ? 1u : meta[r].count; };
+struct PlaceMem {  // a warp's
+  static constexpr int kRow = 8 * W + 4;  // a node's words, and a shift of the banks
+  __align__(16) float node[32 / W * kRow];
+  uint2 tri[32 * J3DG_MAX_LEAF];  // leaf triangles: from, to
+};
+
+// the wide nodes of `it` (lane / W of the warp's; valid: there is one);
+// push(inner, count, item), for whole warps, takes the subtrees to be placed next
+template <int W, class Push>
+__device__ __forceinline__ void place_nodes(PlaceMem<W>& s, const BinNode* __restrict__ node,
+                                            const NodeMeta* __restrict__ meta, const BinNode* __restrict__ tbox,
+                                            const float4* __restrict__ tris, const PlaceItem it, const bool valid,
+                                            uint32_t n_wide, float4* __restrict__ wide, float4* __restrict__ tris_out,
+                                            uint32_t* __restrict__ slot_of, uint32_t nt, uint32_t* status, Push push) {
+  static_assert(J3DG_NODE_F4(W) == 2 * W, "eight rows of W words");
+  const uint32_t lane = threadIdx.x & 31u, slot = lane & (W - 1), group = lane / W;
+  // to the slot-th of the subtrees that the decisions give
+  uint32_t ref = it.bin, start = it.start, cnt = 1u, sub = 0u;  // sub: wide nodes in it (0: a leaf)
+  bool has = valid;
+  float4 lo = make_float4(3.4e38f, 3.4e38f, 3.4e38f, 0.f), hi = make_float4(-3.4e38f, -3.4e38f, -3.4e38f, 0.f);
   if (valid) {
-    struct Slot {
-      uint32_t r, i, start;
-    };
-    Slot stk[2 * W];
-    int sp = 0;
-    const uint32_t k = dec_byte(meta[it.bin], 0) & 0x7fu;
-    const uint32_t cl = left_ref(node[it.bin].lo), cr = right_ref(node[it.bin].hi);
-    stk[sp++] = Slot{cr, (uint32_t)W - k, it.start + count_of(cl)};
-    stk[sp++] = Slot{cl, k, it.start};
-    while (sp > 0 && m < W) {
-      const Slot e = stk[--sp];
-      if (e.r & 0x80000000u) {
-        const BinNode b = tbox[e.r & 0x7fffffffu];
-        ref[m] = e.r, start[m] = e.start, cnt[m] = 1u, sub[m] = 0u, lo[m] = b.lo, hi[m] = b.hi;
-        ++m;
-        continue;
+    uint32_t i = W, at = slot;  // the slots that the subtree takes, ours among them
+    for (int step = 0; step <= W; ++step) {
+      if (ref & 0x80000000u) {  // a triangle takes one
+        has = at == 0u;
+        break;
       }
-      const BinNode b = node[e.r];
-      const NodeMeta M = meta[e.r];
-      uint32_t i = e.i, d = 0u;
-      while (i > 1u && (d = dec_byte(M, i - 1u)) == 0u) --i;  // 0: as with a slot less
-      if (i <= 1u || sp + 2 > 2 * W) {
-        ref[m] = e.r, start[m] = e.start, cnt[m] = M.count, lo[m] = b.lo, hi[m] = b.hi;
-        sub[m] = (M.dec[0] & 0x80u) ? 0u : M.wide;
-        ++m;
-        continue;
+      const BinNode b = node[ref];
+      const NodeMeta M = meta[ref];
+      uint32_t k = 0;
+      if (step == 0) {
+        k = dec_byte(M, 0) & 0x7fu;
+      } else {
+        while (i > 1u && (k = dec_byte(M, i - 1u)) == 0u) --i;  // 0: as with a slot less
+        if (at >= i || i <= 1u) {
+          has = at == 0u;
+          lo = b.lo;
+          hi = b.hi;
+          cnt = M.count;
+          sub = (M.dec[0] & 0x80u) ? 0u : M.wide;
+          break;
+        }
       }
       const uint32_t l = left_ref(b.lo);
-      stk[sp++] = Slot{right_ref(b.hi), i - d, e.start + count_of(l)};
-      stk[sp++] = Slot{l, d, e.start};
+      if (at < k) {
+        ref = l;
+        i = k;
+      } else {
+        start += (l & 0x80000000u) ? 1u : meta[l].count;
+        ref = right_ref(b.hi);
+        at -= k;
+        i -= k;
+      }
+    }
+    if (has && (ref & 0x80000000u)) {
+      const BinNode b = tbox[ref & 0x7fffffffu];
+      lo = b.lo;
+      hi = b.hi;
     }
   }
-  // the next level's queue slots: one atomic per warp (a warp-wide scan of the
-  // lanes' internal slots)
-  uint32_t n_int = 0u;
+  if (!has) {
+    sub = 0u;
+    lo = make_float4(3.4e38f, 3.4e38f, 3.4e38f, 0.f);
+    hi = make_float4(-3.4e38f, -3.4e38f, -3.4e38f, 0.f);
+  }
+  // the wide nodes before it
+  uint32_t next = sub;
 #pragma unroll
-  for (int s = 0; s < W; ++s) n_int += s < m && sub[s] != 0u ? 1u : 0u;
-  uint32_t incl = n_int;
+  for (int o = 1; o < W; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, next, o, W);
+    if (slot >= (uint32_t)o) next += y;
+  }
+  next += it.wide + 1u - sub;
+  const bool inner = sub != 0u;
+  if (inner && next >= n_wide) atomicOr(status, J3DG_DEV_BAD_INDEX);  // (a malformed tree is stopped here)
+  push(inner && next < n_wide, cnt, PlaceItem{ref, next, it.depth + 1, start});
+  const uint32_t out_ref =
+      inner ? next : (has ? J3DG_LEAF_BIT | (start << 3) | (cnt - 1u) : J3DG_EMPTY_REF);
+  // the node: planes [6][W], refs [W], zeros
+  {
+    float* r = s.node + group * PlaceMem<W>::kRow + slot;
+    r[0 * W] = lo.x;
+    r[1 * W] = hi.x;
+    r[2 * W] = lo.y;
+    r[3 * W] = hi.y;
+    r[4 * W] = lo.z;
+    r[5 * W] = hi.z;
+    r[6 * W] = __uint_as_float(out_ref);
+    r[7 * W] = 0.f;
+  }
+  // the leaf's triangles, in depth-first order
+  const uint32_t mine = has && !inner ? min(cnt, J3DG_MAX_LEAF) : 0u;
+  uint32_t off = mine;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= (uint32_t)o) incl += y;
+    const uint32_t y = __shfl_up_sync(0xffffffffu, off, o);
+    if (lane >= (uint32_t)o) off += y;
   }
-  uint32_t q_base = 0u;
-  if (lane == 31u && incl > 0u) q_base = atomicAdd(n_out, incl);
-  uint32_t q = __shfl_sync(0xffffffffu, q_base, 31) + incl - n_int;  // this lane's first queue slot
-  const uint32_t dmax = __reduce_max_sync(0xffffffffu, valid ? it.depth : 0u);
-  if (lane == 0u && dmax > 0u) atomicMax(max_depth, dmax);
-  if (!valid) return;
-  // the node in the width-W layout: planes [6][W], refs [W], zero padding
-  float F[4 * J3DG_NODE_F4(W)];
-#pragma unroll
-  for (int k = 0; k < 4 * J3DG_NODE_F4(W); ++k) F[k] = 0.f;
-  uint32_t next = it.wide + 1u;
-#pragma unroll
-  for (int s = 0; s < W; ++s) {
-    uint32_t out_ref = J3DG_EMPTY_REF;
-    if (s < m) {
-      F[0 * W + s] = lo[s].x;
-      F[1 * W + s] = hi[s].x;
-      F[2 * W + s] = lo[s].y;
-      F[3 * W + s] = hi[s].y;
-      F[4 * W + s] = lo[s].z;
-      F[5 * W + s] = hi[s].z;
-      if (sub[s] == 0u) {
-        out_ref = J3DG_LEAF_BIT | (start[s] << 3) | (cnt[s] - 1u);
-        uint32_t stk[J3DG_MAX_LEAF];
-        int sp = 0;
-        uint32_t k = 0;
-        stk[sp++] = ref[s];
-        while (sp > 0) {
-          const uint32_t r = stk[--sp];
-          if (r & 0x80000000u) {
-            const uint32_t src = r & 0x7fffffffu, dst = start[s] + k++;
-            if (src < nt && dst < nt) {
-              const float4 v0 = tris[3 * (size_t)src], v1 = tris[3 * (size_t)src + 1], v2 = tris[3 * (size_t)src + 2];
-              tris_out[3 * (size_t)dst] = v0;
-              tris_out[3 * (size_t)dst + 1] = v1;
-              tris_out[3 * (size_t)dst + 2] = v2;
-              const uint32_t id = __float_as_uint(v0.w);
-              if (id < nt)
-                slot_of[id] = dst;
-              else
-                atomicOr(status, J3DG_DEV_BAD_INDEX);
-            } else {
-              atomicOr(status, J3DG_DEV_BAD_INDEX);
-            }
-          } else if (sp + 2 <= (int)J3DG_MAX_LEAF) {
-            const BinNode b = node[r];
-            stk[sp++] = right_ref(b.hi);
-            stk[sp++] = left_ref(b.lo);
-          } else {
-            atomicOr(status, J3DG_DEV_STACK_OVERFLOW);
-            break;
-          }
-        }
+  const uint32_t n_tri = __shfl_sync(0xffffffffu, off, 31);
+  off -= mine;
+  if (mine == 1u) {
+    s.tri[off] = make_uint2(ref & 0x7fffffffu, start);
+  } else if (mine) {
+    uint32_t stk[J3DG_MAX_LEAF];
+    int sp = 0;
+    uint32_t k = 0;
+    stk[sp++] = ref;
+    while (sp > 0 && k < mine) {
+      const uint32_t r = stk[--sp];
+      if (r & 0x80000000u) {
+        s.tri[off + k] = make_uint2(r & 0x7fffffffu, start + k);
+        ++k;
+      } else if (sp + 2 <= (int)J3DG_MAX_LEAF) {
+        const BinNode b = node[r];
+        stk[sp++] = right_ref(b.hi);
+        stk[sp++] = left_ref(b.lo);
       } else {
-        // (the queue holds nt entries, the tree n_wide nodes: a malformed
-        // tree is stopped here)
-        if (q < nt && next < n_wide) {
-          qout[q] = PlaceItem{ref[s], next, it.depth + 1, start[s]};
-        } else {
+        break;
+      }
+    }
+    if (k < mine || sp > 0) atomicOr(status, J3DG_DEV_STACK_OVERFLOW);
+    for (; k < mine; ++k) s.tri[off + k] = make_uint2(0xffffffffu, 0xffffffffu);
+  }
+  __syncwarp();
+  // out: two float4 of the nodes a lane
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint32_t y = lane + 32u * h, g = y / (2 * W), x = y % (2 * W);
+    const uint32_t at = __shfl_sync(0xffffffffu, it.wide, (int)(g * W));
+    const bool there = __shfl_sync(0xffffffffu, valid ? 1u : 0u, (int)(g * W));
+    if (there) {
+      if (at < n_wide)
+        wide[2 * W * (size_t)at + x] = *reinterpret_cast<const float4*>(s.node + g * PlaceMem<W>::kRow + 4 * x);
+      else
+        atomicOr(status, J3DG_DEV_BAD_INDEX);
+    }
+  }
+  for (uint32_t k = lane; k < 3u * n_tri; k += 32u) {
+    const uint32_t e = k / 3u, part = k - 3u * e;
+    const uint2 ft = s.tri[e];
+    if (ft.x < nt && ft.y < nt) {
+      const float4 v = tris[3 * (size_t)ft.x + part];
+      tris_out[3 * (size_t)ft.y + part] = v;
+      if (part == 0u) {
+        const uint32_t id = __float_as_uint(v.w);
+        if (id < nt)
+          slot_of[id] = ft.y;
+        else
           atomicOr(status, J3DG_DEV_BAD_INDEX);
-        }
-        out_ref = next;
-        next += sub[s];
-        ++q;
       }
     } else {
-      F[0 * W + s] = F[2 * W + s] = F[4 * W + s] = 3.4e38f;
-      F[1 * W + s] = F[3 * W + s] = F[5 * W + s] = -3.4e38f;
+      atomicOr(status, J3DG_DEV_BAD_INDEX);
     }
-    F[6 * W + s] = __uint_as_float(out_ref);
   }
-  if (it.wide >= n_wide) {
-    atomicOr(status, J3DG_DEV_BAD_INDEX);
-    return;
-  }
-  float4* Wn = wide + J3DG_NODE_F4(W) * (size_t)it.wide;
-#pragma unroll
-  for (int k = 0; k < J3DG_NODE_F4(W); ++k) Wn[k] = make_float4(F[4 * k], F[4 * k + 1], F[4 * k + 2], F[4 * k + 3]);
+  __syncwarp();  // the warp's memory is free for its next nodes
 }
 
 // ------------------------------------------------ 7. depth-first order ----
@@ -969,37 +999,90 @@ static uint32_t wave_blocks128() {
   return blocks;
 }
 
-// level `base + k` of the placement; warp-uniform strides
+static const int kPlaceThreads = 128, kPlaceWarps = kPlaceThreads / 32;
+// a subtree that one warp places: what waits of it are disjoint subtrees of
+// two triangles and more, half as many at most
+// (28.09M triangles, one wave of blocks: 32: 2.96 ms, 64: 2.22, 128: 1.89; the whole
+// build with 256 0.46 ms longer than with 128)
+static const uint32_t kPlaceJob = 128;
+
+// level `base + k` of the placement: subtrees above kPlaceJob triangles to the
+// next level, the others to the jobs; warp-uniform strides
 template <int W>
-__global__ void k_collapse_place(const BinNode* __restrict__ node, const NodeMeta* __restrict__ meta,
-                                 const BinNode* __restrict__ tbox, const float4* __restrict__ tris,
-                                 const PlaceItem* __restrict__ qin, PlaceItem* __restrict__ qout,
-                                 BuildCtl* __restrict__ c, uint32_t k, float4* __restrict__ wide,
-                                 float4* __restrict__ tris_out, uint32_t* __restrict__ slot_of, uint32_t nt,
-                                 uint32_t* status) {
+__global__ void __launch_bounds__(kPlaceThreads) k_collapse_place(
+    const BinNode* __restrict__ node, const NodeMeta* __restrict__ meta, const BinNode* __restrict__ tbox,
+    const float4* __restrict__ tris, const PlaceItem* __restrict__ qin, PlaceItem* __restrict__ qout,
+    PlaceItem* __restrict__ jobs, BuildCtl* __restrict__ c, uint32_t k, float4* __restrict__ wide,
+    float4* __restrict__ tris_out, uint32_t* __restrict__ slot_of, uint32_t nt, uint32_t* status) {
   const uint32_t L = c->place_base + k;
   if (L >= kMaxPlaceLevels) return;
-  const uint32_t n_in = min(c->place[L], nt), n_wide = c->n_wide;
-  const uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t t0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); t0 < n_in; t0 += stride)
-    collapse_place_one<W>(node, meta, tbox, tris, qin, t0 + (threadIdx.x & 31u), n_in, qout, &c->place[L + 1], n_wide,
-                          wide, &c->max_depth, tris_out, slot_of, nt, status);
+  __shared__ PlaceMem<W> mem[kPlaceWarps];
+  const uint32_t n_in = min(c->place[L], nt), n_wide = c->n_wide, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t stride = gridDim.x * (kPlaceThreads / W), below = (1u << lane) - 1u;
+  uint32_t depth = 0;
+  for (uint32_t t0 = blockIdx.x * (kPlaceThreads / W) + warp * (32u / W); t0 < n_in; t0 += stride) {
+    const uint32_t t = t0 + lane / W;
+    const PlaceItem it = t < n_in ? qin[t] : PlaceItem{0u, 0u, 0u, 0u};
+    depth = max(depth, it.depth);
+    place_nodes<W>(mem[warp], node, meta, tbox, tris, it, t < n_in, n_wide, wide, tris_out, slot_of, nt, status,
+                   [&](bool inner, uint32_t count, const PlaceItem& next) {
+                     for (int job = 0; job < 2; ++job) {
+                       const bool mine = inner && (count <= kPlaceJob) == (job == 1);
+                       const uint32_t bal = __ballot_sync(0xffffffffu, mine);
+                       if (!bal) continue;
+                       uint32_t q = 0;
+                       if (lane == 0u) q = atomicAdd(job ? &c->place_jobs : &c->place[L + 1], (uint32_t)__popc(bal));
+                       q = __shfl_sync(0xffffffffu, q, 0) + __popc(bal & below);
+                       if (!mine) continue;
+                       if (q < (job ? nt / 2u : nt))  // (the arrays' ends: a malformed tree is stopped here)
+                         (job ? jobs : qout)[q] = next;
+                       else
+                         atomicOr(status, J3DG_DEV_BAD_INDEX);
+                     }
+                   });
+  }
+  depth = __reduce_max_sync(0xffffffffu, depth);
+  if (lane == 0u && depth > 0u) atomicMax(&c->max_depth, depth);
 }
 
-static void launch_collapse_place(uint32_t W, const BinNode* node, const NodeMeta* meta, const BinNode* tbox,
-                                  const float4* tris, const PlaceItem* qin, PlaceItem* qout, BuildCtl* c, uint32_t k,
-                                  float4* wide, float4* tris_out, uint32_t* slot_of, uint32_t nt, uint32_t* status,
-                                  cudaStream_t st) {
-  auto go = [&](auto kernel) {
-    kernel<<<wave_blocks128(), 128, 0, st>>>(node, meta, tbox, tris, qin, qout, c, k, wide, tris_out, slot_of, nt,
-                                             status);
-  };
-  if (W == 2)
-    go(k_collapse_place<2>);
-  else if (W == 8)
-    go(k_collapse_place<8>);
-  else
-    go(k_collapse_place<4>);
+// the jobs, once the levels up to `base + k` have left nothing
+template <int W>
+__global__ void __launch_bounds__(kPlaceThreads) k_place_jobs(
+    const BinNode* __restrict__ node, const NodeMeta* __restrict__ meta, const BinNode* __restrict__ tbox,
+    const float4* __restrict__ tris, const PlaceItem* __restrict__ jobs, BuildCtl* __restrict__ c, uint32_t k,
+    float4* __restrict__ wide, float4* __restrict__ tris_out, uint32_t* __restrict__ slot_of, uint32_t nt,
+    uint32_t* status) {
+  if (c->place[min(c->place_base + k, kMaxPlaceLevels)]) return;
+  __shared__ PlaceMem<W> mem[kPlaceWarps];
+  __shared__ PlaceItem wait[kPlaceWarps][kPlaceJob / 2];
+  const uint32_t n_jobs = min(c->place_jobs, nt / 2u), n_wide = c->n_wide, lane = threadIdx.x & 31u,
+                 warp = threadIdx.x >> 5, below = (1u << lane) - 1u;
+  uint32_t depth = 0;
+  for (uint32_t j = blockIdx.x * kPlaceWarps + warp; j < n_jobs; j += gridDim.x * kPlaceWarps) {
+    uint32_t n = 1;  // waiting, the last ones first
+    if (lane == 0u) wait[warp][0] = jobs[j];
+    __syncwarp();
+    while (n > 0u) {
+      const uint32_t take = min(n, 32u / W), t = lane / W;
+      const PlaceItem it = t < take ? wait[warp][n - 1u - t] : PlaceItem{0u, 0u, 0u, 0u};
+      n -= take;
+      depth = max(depth, it.depth);
+      __syncwarp();
+      place_nodes<W>(mem[warp], node, meta, tbox, tris, it, t < take, n_wide, wide, tris_out, slot_of, nt, status,
+                     [&](bool inner, uint32_t, const PlaceItem& next) {
+                       const uint32_t bal = __ballot_sync(0xffffffffu, inner), q = n + __popc(bal & below);
+                       if (inner) {
+                         if (q < kPlaceJob / 2u)
+                           wait[warp][q] = next;
+                         else
+                           atomicOr(status, J3DG_DEV_BAD_INDEX);
+                       }
+                       n = min(n + __popc(bal), kPlaceJob / 2u);
+                     });
+    }
+  }
+  depth = __reduce_max_sync(0xffffffffu, depth);
+  if (lane == 0u && depth > 0u) atomicMax(&c->max_depth, depth);
 }
 
 // -------------------------------------------------- 5c. SAH top levels ----
@@ -2730,9 +2813,11 @@ struct BuildPlan {
   }
   uint32_t place_levels() const {
     uint32_t l = 1;
-    for (uint64_t n = W * (uint64_t)leaf; n < nt; n *= W) ++l;
-    return std::min((l + 5u) & ~1u, kMaxPlaceLevels);
+    for (uint64_t n = W * (uint64_t)kPlaceJob; n < nt; n *= W) ++l;
+    return std::min((l + 4u) & ~1u, kMaxPlaceLevels);
   }
+  // the placement's jobs have two triangles and more each; the coverings are done with by then
+  PlaceItem* jobs() const { return reinterpret_cast<PlaceItem*>(dp_cost); }
   Tree tree() const { return Tree{box, meta, top_up, top_done, dp_cost, dp_wide, &ctl->root, &ctl->error}; }
 };
 
@@ -2935,10 +3020,33 @@ static cudaError_t launch_small_tasks(uint32_t W, BuildPlan& P, cudaStream_t st,
 static void enqueue_top_levels(BuildPlan& P, cudaStream_t st, uint32_t k0, uint32_t k1, uint32_t* d_status) {
   for (uint32_t k = k0; k < k1; ++k) launch_top_level(P, st, k, d_status);
 }
-static void enqueue_place_levels(BuildPlan& P, cudaStream_t st, uint32_t k0, uint32_t k1, uint32_t* d_status) {
+template <int W>
+static void enqueue_place_levels_w(BuildPlan& P, cudaStream_t st, uint32_t k0, uint32_t k1, uint32_t* d_status) {
   for (uint32_t k = k0; k < k1; ++k)
-    launch_collapse_place(P.W, P.box, P.meta, P.tbox, P.soup, k & 1u ? P.pb : P.pa, k & 1u ? P.pa : P.pb, P.ctl, k,
-                          P.nodes ? P.nodes : P.wide, P.tris_out, P.slot_of, P.nt, d_status, st);
+    k_collapse_place<W><<<wave_blocks128(), kPlaceThreads, 0, st>>>(
+        P.box, P.meta, P.tbox, P.soup, k & 1u ? P.pb : P.pa, k & 1u ? P.pa : P.pb, P.jobs(), P.ctl, k,
+        P.nodes ? P.nodes : P.wide, P.tris_out, P.slot_of, P.nt, d_status);
+}
+static void enqueue_place_levels(BuildPlan& P, cudaStream_t st, uint32_t k0, uint32_t k1, uint32_t* d_status) {
+  if (P.W == 2)
+    enqueue_place_levels_w<2>(P, st, k0, k1, d_status);
+  else if (P.W == 8)
+    enqueue_place_levels_w<8>(P, st, k0, k1, d_status);
+  else
+    enqueue_place_levels_w<4>(P, st, k0, k1, d_status);
+}
+static void enqueue_place_jobs(BuildPlan& P, cudaStream_t st, uint32_t k, uint32_t* d_status) {
+  auto go = [&](auto kernel) {
+    // more blocks than are resident: the jobs' sizes differ (28.09M triangles: 1.62 ms, in one wave 1.89)
+    kernel<<<std::min(8u * wave_blocks128(), P.nt / 64u + 1u), kPlaceThreads, 0, st>>>(
+        P.box, P.meta, P.tbox, P.soup, P.jobs(), P.ctl, k, P.nodes ? P.nodes : P.wide, P.tris_out, P.slot_of, P.nt, d_status);
+  };
+  if (P.W == 2)
+    go(k_place_jobs<2>);
+  else if (P.W == 8)
+    go(k_place_jobs<8>);
+  else
+    go(k_place_jobs<4>);
 }
 static void enqueue_top_start(BuildPlan& P, cudaStream_t st) {
   k_top_boxes<<<(P.nt + 255) / 256, 256, 0, st>>>(P.soup, P.nt, P.tbox, P.ord_a);
@@ -2970,6 +3078,8 @@ static cudaError_t capture_tree_ploc(BuildPlan& P, cudaStream_t st, cudaStream_t
         enqueue_place_levels(P, s, 0, 2, d_status);
         k_place_more<<<1, 1, 0, s>>>(c, 2u, h);
       }));
+  enqueue_place_jobs(P, st, 0, d_status);
+  J3DG_EQ(cudaSuccess);
   return e;
 }
 
@@ -2997,6 +3107,7 @@ static cudaError_t run_tree_ploc(BuildPlan& P, cudaStream_t st, uint32_t* d_stat
       }
     }
     enqueue_place_levels(P, st, places, places + more_places, d_status);
+    enqueue_place_jobs(P, st, places + more_places, d_status);
     J3DG_EQ(cudaMemcpyAsync(&h, P.ctl, kCtlHead, cudaMemcpyDeviceToHost, st));
     J3DG_EQ(cudaStreamSynchronize(st));
     if (e != cudaSuccess || h.error) return e;
