@@ -349,6 +349,9 @@ __device__ __forceinline__ void sort_children(float (&tc)[W], uint32_t (&rc)[W])
 #undef J3DG_CX
 }
 
+static const int kLeafAt = 8;  // rays at a leaf that a warp stops for (TracerT::warp_step)
+
+
 // ONE: the scene is one object, whose record comes by value with the kernel's
 // parameters (insts points there): its arrays are then read from the constant
 // bank in every step instead of being kept in registers, and the frame needs
@@ -447,60 +450,66 @@ struct TracerT {
   // stack: the caller's per-thread traversal stack of (ref, entry t bits)
   // pairs, one 8-byte access per push or pop (kept out of the struct so
   // that its scalar state can stay in registers).
-  // One traversal step: a pop, a leaf (its triangles, or with TOP an
-  // object entered) or a node. Returns true when the ray is finished.
-  __device__ __forceinline__ bool step(const DevInst* __restrict__ insts, uint32_t n_inst, uint32_t* status,
-                                       uint32_t& visits, uint32_t& tests, uint2* __restrict__ stack) {
-    {
-      const uint32_t c_nt = ONE ? insts[0].nt : nt, c_nodes = ONE ? insts[0].n_nodes : n_nodes;
-      if (cur == J3DG_EMPTY_REF) {
-        bool got = false;
-        while (sp > 0) {
-          --sp;
-          const uint2 e = stack[sp];
-          if (TOP && e.x == kPopTop) {  // the object is done: back to the top level
-            start_top(insts, e.y);
-            continue;
-          }
-          if (__uint_as_float(e.y) <= b.t) {
-            cur = e.x;
-            got = true;
-            break;
-          }
-        }
-        if (!got) {
-          if (TOP || ONE) return true;
-          if (++inst >= n_inst) return true;
-          start_object(insts);
-          return false;
-        }
-      }
-      if (cur & J3DG_LEAF_BIT) {
-        const uint32_t first = (cur & 0x7fffffffu) >> 3, cnt = (cur & 7u) + 1u;
-        if (first + cnt > (TOP ? nt : c_nt)) {
-          atomicOr(status, J3DG_DEV_BAD_INDEX);
-          return true;
-        }
-        if (TOP && inst == kTopInst) {
-          // a top-level leaf: walk its object, then come back
-          if (cnt != 1u || sp + 1 > J3DG_STACK) {
-            atomicOr(status, cnt != 1u ? J3DG_DEV_BAD_INDEX : J3DG_DEV_STACK_OVERFLOW);
-            return true;
-          }
-          stack[sp] = make_uint2(kPopTop, budget);
-          ++sp;
-          inst = first;
-          start_object(insts);
-          return false;
-        }
-#pragma unroll 1
-        for (uint32_t k = 0; k < cnt; ++k) {
-          ++tests;
-          if (tri_test(r, ONE ? insts[0].tris : tris, first + k, ONE ? 0u : inst, b, any) && any) return true;
-        }
-        cur = J3DG_EMPTY_REF;
+  // What the ray does next, in cur: what it has there, or the nearest of the
+  // stack that it still can hit. Returns true when the ray is finished.
+  __device__ __forceinline__ bool fetch(const DevInst* __restrict__ insts, uint32_t n_inst,
+                                        uint2* __restrict__ stack) {
+    while (cur == J3DG_EMPTY_REF) {
+      if (sp == 0) {
+        if (TOP || ONE) return true;
+        if (++inst >= n_inst) return true;
+        start_object(insts);
         return false;
       }
+      --sp;
+      const uint2 e = stack[sp];
+      if (TOP && e.x == kPopTop)  // the object is done: back to the top level
+        start_top(insts, e.y);
+      else if (__uint_as_float(e.y) <= b.t)
+        cur = e.x;
+    }
+    return false;
+  }
+
+  // A leaf (its triangles, or with TOP an object entered). Returns true when
+  // the ray is finished.
+  __device__ __forceinline__ bool leaf(const DevInst* __restrict__ insts, uint32_t* status, uint32_t& tests,
+                                       uint2* __restrict__ stack) {
+    const uint32_t c_nt = ONE ? insts[0].nt : nt;
+    {
+      const uint32_t first = (cur & 0x7fffffffu) >> 3, cnt = (cur & 7u) + 1u;
+      if (first + cnt > (TOP ? nt : c_nt)) {
+        atomicOr(status, J3DG_DEV_BAD_INDEX);
+        return true;
+      }
+      if (TOP && inst == kTopInst) {
+        // a top-level leaf: walk its object, then come back
+        if (cnt != 1u || sp + 1 > J3DG_STACK) {
+          atomicOr(status, cnt != 1u ? J3DG_DEV_BAD_INDEX : J3DG_DEV_STACK_OVERFLOW);
+          return true;
+        }
+        stack[sp] = make_uint2(kPopTop, budget);
+        ++sp;
+        inst = first;
+        start_object(insts);
+        return false;
+      }
+#pragma unroll 1
+      for (uint32_t k = 0; k < cnt; ++k) {
+        ++tests;
+        if (tri_test(r, ONE ? insts[0].tris : tris, first + k, ONE ? 0u : inst, b, any) && any) return true;
+      }
+      cur = J3DG_EMPTY_REF;
+      return false;
+    }
+  }
+
+  // A node: its children that the ray meets, the nearest in cur, the others on
+  // the stack. Returns true on a status.
+  __device__ __forceinline__ bool node(const DevInst* __restrict__ insts, uint32_t* status, uint32_t& visits,
+                                       uint2* __restrict__ stack) {
+    const uint32_t c_nt = ONE ? insts[0].nt : nt, c_nodes = ONE ? insts[0].n_nodes : n_nodes;
+    {
       if (budget-- == 0) {
         atomicOr(status, J3DG_DEV_VISIT_CAP);
         return true;
@@ -558,6 +567,60 @@ struct TracerT {
     }
     return false;
   }
+
+  // One step of a ray: a pop, a leaf or a node. Returns true when the ray is
+  // finished.
+  __device__ __forceinline__ bool step(const DevInst* __restrict__ insts, uint32_t n_inst, uint32_t* status,
+                                       uint32_t& visits, uint32_t& tests, uint2* __restrict__ stack) {
+    if (cur == J3DG_EMPTY_REF) {
+      bool got = false;
+      while (sp > 0) {
+        --sp;
+        const uint2 e = stack[sp];
+        if (TOP && e.x == kPopTop) {  // the object is done: back to the top level
+          start_top(insts, e.y);
+          continue;
+        }
+        if (__uint_as_float(e.y) <= b.t) {
+          cur = e.x;
+          got = true;
+          break;
+        }
+      }
+      if (!got) {
+        if (TOP || ONE) return true;
+        if (++inst >= n_inst) return true;
+        start_object(insts);
+        return false;
+      }
+    }
+    if (cur & J3DG_LEAF_BIT) return leaf(insts, status, tests, stack);
+    return node(insts, status, visits, stack);
+  }
+
+  // One step of a warp's rays (all 32 lanes call it; `active`: this lane has a
+  // ray). Returns true when this lane's ray is finished. Nodes and leaves take
+  // different code, and a warp whose lanes want both runs both, for a few
+  // lanes each. Below a top level, where a leaf may be an object to enter (the
+  // ray brought into its space), the rays at a leaf wait until
+  // kLeafAt of them do or none is at a node: 24 objects, 1279 x 717 with edges,
+  // 449 us -> 350 (kLeafAt 4: 361, 12: 351). With one object the wait costs
+  // more than the lanes it fills: 489 -> 538 us a 1080p frame of 28.09M
+  // triangles, a million incoherent rays 498 -> 515.
+  __device__ __forceinline__ bool warp_step(bool active, const DevInst* __restrict__ insts, uint32_t n_inst,
+                                            uint32_t* status, uint32_t& visits, uint32_t& tests,
+                                            uint2* __restrict__ stack) {
+    if (!TOP) return active && step(insts, n_inst, status, visits, tests, stack);
+    bool done = active && fetch(insts, n_inst, stack);
+    const bool at_leaf = active && !done && (cur & J3DG_LEAF_BIT) != 0, at_node = active && !done && !at_leaf;
+    const uint32_t leaves = __ballot_sync(0xffffffffu, at_leaf);
+    if (__any_sync(0xffffffffu, at_node) && __popc(leaves) < kLeafAt) {
+      if (at_node) done = node(insts, status, visits, stack);
+    } else if (at_leaf) {
+      done = leaf(insts, status, tests, stack);
+    }
+    return done;
+  }
 };
 
 // Persistent warps with per-lane refill (Aila and Laine 2009, "dynamic
@@ -601,7 +664,7 @@ __device__ __forceinline__ void persistent_trace(Src& src, const DevInst* __rest
     if (__all_sync(0xffffffffu, phase == 3)) break;
 #pragma unroll 1
     for (;;) {
-      if (phase == 1 && T.step(insts, n_inst, status, visits, tests, stack)) phase = 2;
+      if (T.warp_step(phase == 1, insts, n_inst, status, visits, tests, stack)) phase = 2;
       if (__all_sync(0xffffffffu, phase != 1)) break;
       if (__popc(__ballot_sync(0xffffffffu, phase == 0 || phase == 2)) >= REFILL) break;
     }

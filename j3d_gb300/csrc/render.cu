@@ -965,7 +965,7 @@ __global__ void __launch_bounds__(kFrameThreads, tier_blocks(kTier))
     // all lanes step together; leave to refill once enough lanes are idle
 #pragma unroll 1
     for (;;) {
-      if ((phase == 1 || phase == 2) && T.step(frame_insts<ONE>(P), P.n_inst, P.status, visits, tests, stack)) {
+      if (T.warp_step(phase == 1 || phase == 2, frame_insts<ONE>(P), P.n_inst, P.status, visits, tests, stack)) {
 #if J3DG_DEFER_FINISH
         phase += 2;
 #else
@@ -1102,9 +1102,9 @@ __global__ void __launch_bounds__(TPB, (MinBlocks<TPB, kThroughput>::value))
     if (__all_sync(0xffffffffu, phase == 0 && exhausted)) break;
 #pragma unroll 1
     for (;;) {
-      if (phase == 1 || phase == 2) {
+      {
         const FrameParams& P = params[frame];
-        if (T.step(P.inst, P.n_inst, P.status, visits, tests, stack)) {
+        if (T.warp_step(phase == 1 || phase == 2, P.inst, P.n_inst, P.status, visits, tests, stack)) {
 #if J3DG_DEFER_FINISH
           phase += 2;
 #else
