@@ -351,7 +351,6 @@ __device__ __forceinline__ void sort_children(float (&tc)[W], uint32_t (&rc)[W])
 
 static const int kLeafAt = 8;  // rays at a leaf that a warp stops for (TracerT::warp_step)
 
-
 // ONE: the scene is one object, whose record comes by value with the kernel's
 // parameters (insts points there): its arrays are then read from the constant
 // bank in every step instead of being kept in registers, and the frame needs
@@ -603,29 +602,29 @@ struct TracerT {
   // different code, and a warp whose lanes want both runs both, for a few
   // lanes each. Below a top level, where a leaf may be an object to enter (the
   // ray brought into its space), the rays at a leaf wait until
-  // kLeafAt of them do or none is at a node: 24 objects, 1279 x 717 with edges,
-  // 449 us -> 350 (kLeafAt 4: 361, 12: 351). With one object the wait costs
+  // kLeafAt of them do or none is at a node (unless `wait` is false): 24
+  // objects, 1279 x 717 with edges, 449 us -> 350 (kLeafAt 4: 361, 12: 351), two
+  // million incoherent rays on 10 objects 1070 -> 815. With one object the wait costs
   // more than the lanes it fills: 489 -> 538 us a 1080p frame of 28.09M
   // triangles, a million incoherent rays 498 -> 515.
   __device__ __forceinline__ bool warp_step(bool active, const DevInst* __restrict__ insts, uint32_t n_inst,
                                             uint32_t* status, uint32_t& visits, uint32_t& tests,
-                                            uint2* __restrict__ stack) {
+                                            uint2* __restrict__ stack, bool wait = true) {
     if (!TOP) return active && step(insts, n_inst, status, visits, tests, stack);
     bool done = active && fetch(insts, n_inst, stack);
     const bool at_leaf = active && !done && (cur & J3DG_LEAF_BIT) != 0, at_node = active && !done && !at_leaf;
     const uint32_t leaves = __ballot_sync(0xffffffffu, at_leaf);
-    if (__any_sync(0xffffffffu, at_node) && __popc(leaves) < kLeafAt) {
-      if (at_node) done = node(insts, status, visits, stack);
-    } else if (at_leaf) {
-      done = leaf(insts, status, tests, stack);
-    }
+    const bool hold = wait && __any_sync(0xffffffffu, at_node) && __popc(leaves) < kLeafAt;
+    if (at_node) done = node(insts, status, visits, stack);
+    if (at_leaf && !hold) done = leaf(insts, status, tests, stack);
     return done;
   }
 };
 
 // Persistent warps with per-lane refill (Aila and Laine 2009, "dynamic
 // fetch"): every lane whose ray finished takes the next work item; the warp
-// fetches for all such lanes with one atomic. Src supplies count(), begin()
+// fetches for all such lanes with one atomic. Src supplies kLaneARay (few
+// items go to a lane each), count(), begin()
 // (returns false when the item needs no tracing and was handled) and
 // finish(). All lanes step together; a lane whose ray finished waits until
 // REFILL lanes are idle, and those finish and refill together.
@@ -641,6 +640,22 @@ __device__ __forceinline__ void persistent_trace(Src& src, const DevInst* __rest
   uint32_t idx = 0;
   int phase = 0;  // 0 idle, 1 tracing, 2 finished, 3 no items left
   uint32_t visits = 0, tests = 0;
+  // Below a top level rays wait for one another (warp_step) while there are
+  // rays to refill with; the last ones don't.
+  bool tail = false;
+  if (TOP && Src::kLaneARay && n <= gridDim.x * N) {
+    // a lane for every ray: the longest rays alone decide, and each goes on by
+    // itself (1000 rays on 5 objects 94 -> 85 us, 100k on 2 objects 120 -> 102;
+    // 200k on 2, two rays a lane, 154 us this way and 143 the other)
+    idx = blockIdx.x * N + threadIdx.x;
+    if (idx < n && src.begin(T, insts, n_inst, idx)) {
+#pragma unroll 1
+      while (!T.step(insts, n_inst, status, visits, tests, stack)) {
+      }
+      src.finish(T, idx);
+    }
+    phase = 3;
+  }
 #pragma unroll 1
   for (;;) {
     if (phase == 2) {
@@ -653,6 +668,7 @@ __device__ __forceinline__ void persistent_trace(Src& src, const DevInst* __rest
       uint32_t base = 0;
       if ((int)lane == leader) base = atomicAdd(counter, (uint32_t)__popc(m));
       base = __shfl_sync(0xffffffffu, base, leader);
+      if (TOP) tail |= base >= n || n - base <= (uint32_t)__popc(m);
       if (phase == 0) {
         idx = base + __popc(m & ((1u << lane) - 1u));
         if (idx >= n)
@@ -664,7 +680,7 @@ __device__ __forceinline__ void persistent_trace(Src& src, const DevInst* __rest
     if (__all_sync(0xffffffffu, phase == 3)) break;
 #pragma unroll 1
     for (;;) {
-      if (T.warp_step(phase == 1, insts, n_inst, status, visits, tests, stack)) phase = 2;
+      if (T.warp_step(phase == 1, insts, n_inst, status, visits, tests, stack, !tail)) phase = 2;
       if (__all_sync(0xffffffffu, phase != 1)) break;
       if (__popc(__ballot_sync(0xffffffffu, phase == 0 || phase == 2)) >= REFILL) break;
     }

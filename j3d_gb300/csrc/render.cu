@@ -866,6 +866,7 @@ __global__ void __launch_bounds__(kResolveThreads) k_resolve(const FrameParams P
 
 // the queued shadow rays, traced by persistent warps
 struct ShadowSrc {
+  static const bool kLaneARay = false;
   const FrameParams* P;
   const ShadowJob* jobs;
   uint32_t n;
@@ -987,6 +988,7 @@ __global__ void __launch_bounds__(kFrameThreads, tier_blocks(kTier))
 template <bool ANY>
 struct BatchSrc {
   static const bool kAny = ANY;
+  static const bool kLaneARay = true;
   const j3dg_ray* rays;
   j3dg_hit* hits;
   uint32_t n;
@@ -1014,8 +1016,10 @@ struct BatchSrc {
   }
 };
 
+// (below a top level the tracer keeps more state: a block an SM fewer, without
+// spills)
 template <bool ANY, bool TOP, bool ONE>
-__global__ void __launch_bounds__(kTraceThreads, J3DG_RAY_BLOCKS)
+__global__ void __launch_bounds__(kTraceThreads, TOP ? J3DG_RAY_BLOCKS - 1 : J3DG_RAY_BLOCKS)
     k_rays(const DevInst* __restrict__ inst, const __grid_constant__ DevInst one, uint32_t n_inst,
            const j3dg_ray* __restrict__ rays, uint32_t n, j3dg_hit* __restrict__ hits, uint32_t* counter,
            uint32_t* status, unsigned long long* counters) {
