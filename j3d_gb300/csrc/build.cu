@@ -1096,10 +1096,10 @@ __global__ void __launch_bounds__(kPlaceThreads) k_place_jobs(
 // partition of the Morton-sorted order keeps every range in Morton order, so
 // each range of at most J3DG_SAH_TOP triangles (a segment) is then clustered
 // by PLOC on its own (neighbours searched within the segment only).
-// Tasks above kSmallTask triangles are split level by level, each cut into
-// items of at most `chunk` positions that a block bins and partitions; a task
-// of at most kSmallTask is taken through the rest of its subtree by one block
-// (section 5d).
+// Tasks above kSmallTask triangles (small builds: kSmallTaskFew) are split
+// level by level, each cut into items of at most `chunk` positions that a
+// block bins and partitions; a smaller task is taken through the rest of its
+// subtree by one block (section 5d).
 //
 // Binary nodes are numbered by position: the node that splits its range at
 // position mid is node mid, and the nodes that PLOC makes in a segment take
@@ -1230,6 +1230,11 @@ struct TopBinner {
 #define J3DG_SMALL_TASK 960
 #endif
 static const uint32_t kSmallTask = J3DG_SMALL_TASK;
+// ... of builds below kSmallFewBelow triangles, whose tasks are fewer than the
+// SMs: two blocks of half the size are done sooner than one, and a level more
+// costs less than that. Build and first frame with 480 / 960: 40k triangles
+// 647 and 674 us, 120k 758 and 771, 250k 918 and 890; with 240 40k 654.
+static const uint32_t kSmallTaskFew = 480, kSmallFewBelow = 130000;
 
 __device__ __forceinline__ float box_half_area(float lx, float ly, float lz, float hx, float hy, float hz) {
   const float dx = hx - lx, dy = hy - ly, dz = hz - lz;
@@ -1559,10 +1564,11 @@ struct NextLevel {
   TopTask* small;
   TopRange* ranges;
   uint32_t cap_tasks, cap_small, cap_items, nt;
+  uint32_t small_max;  // tasks up to this size are one block's
 };
 
 // One warp, after the split S of task T: the children, lanes 0 and 1 one
-// each: a task of the next level above kSmallTask triangles (with its items
+// each: a task of the next level above small_max triangles (with its items
 // and, if they are several, empty bins), a small task above J3DG_SAH_TOP, else
 // a finished range; the task's own node goes under its parent.
 __device__ void warp_children(const TopTask& T, const TopSplit& S, uint32_t chunk, const NextLevel& N,
@@ -1582,7 +1588,7 @@ __device__ void warp_children(const TopTask& T, const TopSplit& S, uint32_t chun
   if (lane < 2) {
     const uint32_t tag = lane | (((T.side >> 1) + 1u) << 1);
     if (len > J3DG_SAH_TOP) {
-      const bool again = len > kSmallTask;
+      const bool again = len > N.small_max;
       if (again) {  // the task and its items in one atomic
         const unsigned long long at = atomicAdd(reinterpret_cast<unsigned long long*>(&c->top[level + 1]),
                                                 1ull | ((unsigned long long)m << 32));
@@ -2604,7 +2610,8 @@ __global__ void k_slot_of(const float4* __restrict__ tris, uint32_t nt, uint32_t
 
 // the root task, by its size: split level by level, by one block, or a segment
 __global__ void k_ctl_init(BuildCtl* __restrict__ c, TopTask* __restrict__ tasks, TopTask* __restrict__ small,
-                           TopRange* __restrict__ ranges, uint32_t nt, uint32_t top, uint32_t chunk) {
+                           TopRange* __restrict__ ranges, uint32_t nt, uint32_t top, uint32_t chunk,
+                           uint32_t small_max) {
   if (top) {
     const float* bb = c->bb;
     TopTask r0;
@@ -2614,7 +2621,7 @@ __global__ void k_ctl_init(BuildCtl* __restrict__ c, TopTask* __restrict__ tasks
     r0.side = 0;
     r0.clo = make_float4(bb[0], bb[1], bb[2], 0.f);  // the vertex bbox holds every centroid
     r0.chi = make_float4(bb[3], bb[4], bb[5], 0.f);
-    if (nt > kSmallTask) {
+    if (nt > small_max) {
       tasks[0] = r0;
       c->top[0].tasks = 1;
       c->top[0].items = (nt + chunk - 1) / chunk;
@@ -2789,8 +2796,9 @@ struct BuildPlan {
   // outputs (the mesh keeps them once `owned` does not)
   float4 *normals = nullptr, *soup = nullptr, *tris_out = nullptr, *nodes = nullptr;
   uint32_t* slot_of = nullptr;
-  // tasks of one level are disjoint, each above kSmallTask; so are the small tasks, each above J3DG_SAH_TOP
-  uint32_t cap_tasks() const { return nt / kSmallTask + 1; }
+  // tasks of one level are disjoint, each above small_task(); so are the small tasks, each above J3DG_SAH_TOP
+  uint32_t small_task() const { return nt >= kSmallFewBelow ? kSmallTask : kSmallTaskFew; }
+  uint32_t cap_tasks() const { return nt / small_task() + 1; }
   uint32_t cap_small() const { return nt / J3DG_SAH_TOP + 1; }
   // keys per thread of the sort: the tile is as large as registers and shared
   // memory carry well where there are tiles for every SM, else smaller
@@ -2808,7 +2816,7 @@ struct BuildPlan {
   // 7, 12, 15 at best), even numbers for the loops behind them
   uint32_t top_levels() const {
     uint32_t l = 0;
-    while ((uint64_t)kSmallTask << l < nt) ++l;
+    while ((uint64_t)small_task() << l < nt) ++l;
     return l ? (l + 4u) & ~1u : 0u;
   }
   uint32_t place_levels() const {
@@ -2866,19 +2874,20 @@ static cudaError_t plan_alloc(BuildPlan& P, cudaStream_t st, bool outputs = true
     A(P.ord_b, sizeof(uint32_t) * nt);
     A(P.tbox, sizeof(BinNode) * nt);
     // (a lane's smaller meshes may have more items, of smaller chunks)
-    const uint32_t items = std::max(P.cap_items(), std::min(P.nt, 600000u) / 512u + P.cap_tasks() + 1);
+    const uint32_t tasks = std::max(P.cap_tasks(), std::min(P.nt, kSmallFewBelow) / kSmallTaskFew + 1);
+    const uint32_t items = std::max(P.cap_items(), std::min(P.nt, 600000u) / 512u + tasks + 1);
     A(P.codes, sizeof(uint16_t) * std::max((size_t)P.cap_items() * P.chunk(), (size_t)items * 512));
     A(P.top_up, sizeof(uint32_t) * nt);
     A(P.top_done, sizeof(uint32_t) * nt);
-    A(P.bins_a, sizeof(uint32_t) * (size_t)P.cap_tasks() * kTopBinRow);
-    A(P.bins_b, sizeof(uint32_t) * (size_t)P.cap_tasks() * kTopBinRow);
+    A(P.bins_a, sizeof(uint32_t) * (size_t)tasks * kTopBinRow);
+    A(P.bins_b, sizeof(uint32_t) * (size_t)tasks * kTopBinRow);
     A(P.icum, sizeof(uint32_t) * (size_t)items * 3 * kTopBins);
     A(P.items_a, sizeof(TopItem) * items);
     A(P.items_b, sizeof(TopItem) * items);
-    A(P.tasks_a, sizeof(TopTask) * P.cap_tasks());
-    A(P.tasks_b, sizeof(TopTask) * P.cap_tasks());
+    A(P.tasks_a, sizeof(TopTask) * tasks);
+    A(P.tasks_b, sizeof(TopTask) * tasks);
     A(P.small, sizeof(TopTask) * P.cap_small());
-    A(P.splits, sizeof(TopSplit) * P.cap_tasks());
+    A(P.splits, sizeof(TopSplit) * tasks);
     A(P.ranges, sizeof(TopRange) * nt);  // at most one range per triangle
   }
   A(P.box, sizeof(BinNode) * nt);
@@ -2980,7 +2989,7 @@ static void launch_top_level(BuildPlan& P, cudaStream_t s, uint32_t k, uint32_t*
   const TopTask* tasks = odd ? P.tasks_b : P.tasks_a;
   const TopItem* items = odd ? P.items_b : P.items_a;
   const NextLevel next{odd ? P.tasks_a : P.tasks_b, odd ? P.items_a : P.items_b, odd ? P.bins_a : P.bins_b, P.small,
-                       P.ranges, P.cap_tasks(), P.cap_small(), P.cap_items(), P.nt};
+                       P.ranges, P.cap_tasks(), P.cap_small(), P.cap_items(), P.nt, P.small_task()};
   uint32_t* bins = odd ? P.bins_b : P.bins_a;
   launch_top_bin(P, s, oi, oo, items, tasks, bins, next, k, d_status);
   if (P.chunk() == 8 * kLevelThreads)  // !kSplitWhereBinned
@@ -3198,7 +3207,7 @@ static cudaError_t enqueue_prefix(BuildPlan& P, const float* dV, const uint32_t*
   J3DG_EQ(cudaMemsetAsync(c, 0, sizeof(BuildCtl), st));
   k_bbox_partial<<<kBBoxBlocks, 256, 0, st>>>(dV, nv, P.part);
   k_bbox_final<<<1, 1024, 0, st>>>(P.part, kBBoxBlocks, c->bb);
-  k_ctl_init<<<1, 1, 0, st>>>(c, P.tasks_a, P.small, P.ranges, nt, P.top ? 1u : 0u, P.chunk());
+  k_ctl_init<<<1, 1, 0, st>>>(c, P.tasks_a, P.small, P.ranges, nt, P.top ? 1u : 0u, P.chunk(), P.small_task());
   k_tri_prep<<<(nt + 255) / 256, 256, 0, st>>>(dV, nv, dT, nt, c->bb, P.normals, P.k0, d_status);
   J3DG_EQ(cudaSuccess);
   J3DG_EQ(enqueue_sort(P, st, d_status));

@@ -8,7 +8,7 @@ LEAF, EMPTY = 0x80000000, 0xffffffff
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("width,leaf", [(4, 2), (2, 1), (8, 8)])
-@pytest.mark.parametrize("nt", [9, 64, 65, 959, 960, 961, 1921, 20011])
+@pytest.mark.parametrize("nt", [9, 64, 65, 479, 480, 481, 959, 960, 961, 1921, 20011, 129_999, 130_000])
 def test_depth_first(gpu_ctx, nt, width, leaf):
     from j3d_gb300 import Mesh
     rng = np.random.default_rng(nt)
