@@ -778,8 +778,7 @@ def primary_rays(pose, pinv, w, h, near, t_near):
 
 def run_build(args):
     """The config-1 mesh's BVH builds alone: warm builds of the 28.09M-triangle
-    torus with the default builder (one CUDA graph with device-driven level
-    loops) and with the LBVH builder, CUDA-event times from the library."""
+    torus with the default builder and with the LBVH builder, CUDA-event times from the library."""
     from j3d_gb300 import Context, Mesh, build as B, workloads as Wk
     B.build()
     wl = Wk.config1(N_CAMERAS, W_, H_)

@@ -134,10 +134,9 @@ typedef struct j3dg_build_opts {
    triangles and parallel locally-ordered clustering (Meister and Bittner
    2018) within them, collapsed by a cost-optimal programme: the fewest node
    visits per ray. J3DG_BUILD_LBVH splits at Morton prefixes instead (4-wide
-   only): about 40 % of the build time (12.0 vs 30.6 ms for 28M triangles),
-   about 19 % more node visits per ray. Either build is one CUDA
-   graph with device-driven level loops. The traversal results are the same
-   for either tree. */
+   only): about half of the build time (9.8 vs 19.5 ms for 28M triangles),
+   about 19 % more node visits per ray. Both are driven by the device, sizes
+   read from its memory. The traversal results are the same for either tree. */
 #define J3DG_BUILD_LBVH 0x1u
 /* BVH width (children per node) of the default builder: 4 unless one of
    these is set. The cost-optimal collapse of the binary tree is run for the

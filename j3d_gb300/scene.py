@@ -127,7 +127,7 @@ class Mesh:
                  rebuildable: bool = False):
         """build: "ploc" (binned-SAH top levels over surface-area
         clustering, the default: fewer node visits per ray) or "lbvh" (Morton
-        splits, 4-wide only, about a third of the build time);
+        splits, 4-wide only, about half the build time);
         width: children per BVH node, 2, 4 (default) or 8; rebuildable: keep
         what a Batch(rebuild=True) rebuilds the BVH from, inside its graph."""
         self.ctx = ctx
