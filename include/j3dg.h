@@ -134,7 +134,7 @@ typedef struct j3dg_build_opts {
    triangles and parallel locally-ordered clustering (Meister and Bittner
    2018) within them, collapsed by a cost-optimal programme: the fewest node
    visits per ray. J3DG_BUILD_LBVH splits at Morton prefixes instead (4-wide
-   only): about half of the build time (9.8 vs 19.5 ms for 28M triangles),
+   only): about half of the build time (9.8 vs 18.5 ms for 28M triangles),
    about 19 % more node visits per ray. Both are driven by the device, sizes
    read from its memory. The traversal results are the same for either tree. */
 #define J3DG_BUILD_LBVH 0x1u

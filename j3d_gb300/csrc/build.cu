@@ -1518,22 +1518,18 @@ __device__ __forceinline__ bool top_goes_left(uint32_t k, uint32_t code, const T
 
 // Stable partition of an item's n positions (from position p0 of its task,
 // which begins at `begin`): left0 of the task's earlier positions go left.
-// Whole block; code_of(k), ord_of(k): the k-th position's.
-template <int K, class Code, class Ord>
+// Whole block; code and o: of the thread's positions, the j-th the item's
+// (j kLevelThreads + tid)-th.
+template <int K>
 __device__ __forceinline__ void partition_item(const TopSplit& S, uint32_t begin, uint32_t p0, uint32_t n, uint32_t end,
-                                               uint32_t left0, uint32_t* s_cnt, Code code_of, Ord ord_of,
-                                               uint32_t* __restrict__ ord2, uint32_t* status) {
+                                               uint32_t left0, uint32_t* s_cnt, const uint32_t (&code)[K],
+                                               const uint32_t (&o)[K], uint32_t* __restrict__ ord2, uint32_t* status) {
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  uint32_t f = 0, o[K];  // the order is fetched with the codes: one wait for both
+  uint32_t f = 0;
 #pragma unroll
   for (int j = 0; j < K; ++j) {
     const uint32_t k = (uint32_t)j * kLevelThreads + tid;
-    o[j] = k < n ? ord_of(k) : 0u;
-  }
-#pragma unroll
-  for (int j = 0; j < K; ++j) {
-    const uint32_t k = (uint32_t)j * kLevelThreads + tid;
-    const bool left = k < n && top_goes_left(p0 + k, code_of(k), S);
+    const bool left = k < n && top_goes_left(p0 + k, code[j], S);
     f |= (left ? 1u : 0u) << j;
     const uint32_t c = __popc(__ballot_sync(0xffffffffu, left));
     if (lane == 0) s_cnt[j * (kLevelThreads / 32) + warp] = c;
@@ -1654,8 +1650,9 @@ __device__ void warp_children(const TopTask& T, const TopSplit& S, uint32_t chun
 // across the banks 19.6. The pass that binned whole chunks of positions, with
 // one warp reduction per 32 triangles and global atomics where a chunk held
 // two tasks, took 0.43 ms a level at 28.09M triangles and, with the passes for
-// flags, scan and scatter, 0.66; this kernel, the split and the scatter take
-// 0.52. Builds of 82k / 2M / 28.09M triangles with their first frame: 1449 ->
+// flags, scan and scatter, 0.66; this kernel, the split and the scatter took
+// 0.52, and 0.42 with the looks at the bins and the scatter's earlier fetches.
+// Builds of 82k / 2M / 28.09M triangles with their first frame: 1449 ->
 // 1230, 4201 -> 3729, 28412 -> 26443 us.
 // the place of an item's k-th box in shared memory: threads read runs of 2, 4
 // or 8 positions, and the low bits are mixed so that the threads of a half
@@ -1763,8 +1760,14 @@ __global__ void __launch_bounds__(kLevelThreads, J3DG_LEVEL_BLOCKS) k_top_bin(
         warp_top_split(sb, T, &s.split, tr);
       }
       __syncthreads();
-      partition_item<K>(s.split, T.begin, 0u, I.n, T.end, 0u, s.cnt, [&](uint32_t k) { return (uint32_t)s.code[k]; },
-                        [&](uint32_t k) { return ord[I.begin + k]; }, ord2, status);
+      uint32_t cd[K], o[K];
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        const uint32_t k = (uint32_t)j * kLevelThreads + tid;
+        o[j] = k < I.n ? ord[I.begin + k] : 0u;
+        cd[j] = k < I.n ? s.code[k] : 0u;
+      }
+      partition_item<K>(s.split, T.begin, 0u, I.n, T.end, 0u, s.cnt, cd, o, ord2, status);
       if (warp == 0) {
         if constexpr (kSplitWhereBinned<K>)
           warp_children(T, s.split, chunk, next, c, level, tr, status);
@@ -1865,6 +1868,17 @@ __global__ void __launch_bounds__(kLevelThreads) k_top_scatter(
     const TopItem I = items[it];
     const TopTask T = tasks[I.task];
     if (T.end - T.begin <= chunk) continue;  // partitioned where it was binned
+    // the positions' codes and order, whatever the split is: their fetch goes
+    // on beside that of the split and of the sums that hang on it (28.09M
+    // triangles, 18 levels: 2.30 -> 1.32 ms; a level of one task moves 281 MB
+    // in 90 us)
+    uint32_t cd[K], o[K];
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const uint32_t k = (uint32_t)j * kLevelThreads + tid;
+      o[j] = k < I.n ? ord[I.begin + k] : 0u;
+      cd[j] = k < I.n ? code[(size_t)it * chunk + k] : 0u;
+    }
     const TopSplit S = splits[I.task];
     uint32_t before = 0;  // lefts of the task's earlier items
     if (S.axis < 3) {
@@ -1882,9 +1896,7 @@ __global__ void __launch_bounds__(kLevelThreads) k_top_scatter(
     } else {
       left0 = min(S.nleft, I.begin - T.begin);
     }
-    partition_item<K>(S, T.begin, I.begin - T.begin, I.n, T.end, left0, s_cnt,
-                   [&](uint32_t k) { return (uint32_t)code[(size_t)it * chunk + k]; },
-                   [&](uint32_t k) { return ord[I.begin + k]; }, ord2, status);
+    partition_item<K>(S, T.begin, I.begin - T.begin, I.n, T.end, left0, s_cnt, cd, o, ord2, status);
     __syncthreads();  // the counts are read before the next item resets them
   }
 }
