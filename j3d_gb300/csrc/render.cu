@@ -242,7 +242,7 @@ __device__ __forceinline__ void frame_exit(const FrameParams& P, bool handed_ove
 #endif
 // A batch of fewer primary items than J3DG_THROUGHPUT_ITEMS runs the latency
 // build instead: 5 blocks per SM with the pixel state in registers (single
-// frames: kTierItems below). Measured on single frames: below about one 1920x1080 frame the
+// frames: tier_items below). Measured on single frames: below about one 1920x1080 frame the
 // extra warps of the throughput build lengthen the frame (a 512x512 frame
 // of the 28M-triangle torus 0.80 -> 0.89 ms); from there on they shorten it.
 #ifndef J3DG_LATENCY_MINBLOCKS
@@ -287,19 +287,33 @@ static const int kFrameThreads = J3DG_FRAME_THREADS;
 // more of the fetches' latency once a frame has the pixels to feed them, fewer
 // let a small frame's last rays run faster.
 //   0 (below 400k items): 20 warps an SM, pixel state in registers
-//   1 (below 2M): 24 warps (a 1280x720 frame of a 1M-triangle torus with
-//     shadows 229 -> 210 us, 800x600 of 24 objects 538 -> 508; a 512x512 frame
-//     of the 28.09M-triangle torus would take 228 instead of 218)
+//   1 (below 2M): 24 warps (20 or 24, views in turn with shadows: 2M triangles
+//     1280x720 209 and 201 us, 850x650 185 and 181; 24 objects 760x600 257 and
+//     241; a 512x512 frame of the 28.09M-triangle torus 218 and 228). A single
+//     object at width 8, where 80 registers are short, from 700k items on
+//     (700x580 169 and 176, one view again and again 268 and 276; 1100x700 207
+//     and 203, 294 and 299).
 //   2: pixel state in shared memory, 28 warps at width 4, whose 72 registers
-//     hold the step without spills now that a single object's arrays come from
-//     the constant bank (1920x1080 of the 28.09M-triangle torus with shadows
-//     525 -> 489 us; 32 warps spill: 497)
-static const int kTiers = 3;
-static const uint32_t kTierItems[kTiers - 1] = {400000u, J3DG_THROUGHPUT_ITEMS};
+//     hold the step of a single object without spills (28.09M triangles at
+//     1920x1080 with shadows, views in turn: 24 or 28 warps 455 and 424 us, a
+//     frame alone 863 both, one view again and again 714 and 721, the slowest
+//     pixels one after the other; 32 warps spill: 497 where 28 took 489)
+__host__ __device__ constexpr uint32_t tier_items(int tier, bool one) {  // the build's frames are below
+  return tier == 0 ? (one && J3DG_W == 8 ? 700000u : 400000u) : J3DG_THROUGHPUT_ITEMS;
+}
 __host__ __device__ constexpr int tier_blocks(int tier) {  // blocks of kFrameThreads an SM
   return (tier == 0 ? J3DG_LATENCY_MINBLOCKS
                     : (tier == 1 || J3DG_W != 4 ? J3DG_TRACE_MINBLOCKS : J3DG_TRACE_MINBLOCKS + 1)) *
          128 / kFrameThreads;
+}
+// Whether a single object's arrays are read from the constant bank in every
+// step: where they would spill as registers. Where they fit, registers are
+// faster (from the constant bank and from registers, alone / in turn / one view
+// again and again: 28.09M triangles 512x512 648 / 272 / 449 and 632 / 268 / 436
+// us, 2M triangles 1280x720 437 / 206 / 308 and 425 / 201 / 296; width 2
+// 1920x1080 alone 711 and 695).
+__host__ __device__ constexpr bool one_by_constant(int tier) {
+  return J3DG_W == 4 ? tier == 2 : (J3DG_W == 8 && tier >= 1);
 }
 
 // Pixel and colour state of a lane: read only at a pixel's start and
@@ -905,7 +919,7 @@ __global__ void __launch_bounds__(kTraceThreads, J3DG_TRACE_MINBLOCKS) k_shadow(
 template <int kTier, bool TOP, bool ONE>
 __global__ void __launch_bounds__(kFrameThreads, tier_blocks(kTier))
     k_frame(const __grid_constant__ FrameParams P) {
-  TracerT<kFrameThreads, TOP, kWidth, ONE> T;
+  TracerT<kFrameThreads, TOP, kWidth, ONE && one_by_constant(kTier)> T;
   uint2 stack[J3DG_STACK];
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t n = primary_count(P);
@@ -1365,8 +1379,8 @@ static cudaError_t launch_frame_tier(const FrameParams& P, bool overlap, cudaStr
 template <bool TOP, bool ONE>
 static cudaError_t launch_frame(const FrameParams& P, bool overlap, cudaStream_t st) {
   const uint32_t items = primary_items(P);
-  if (items < kTierItems[0]) return launch_frame_tier<0, TOP, ONE>(P, overlap, st);
-  if (items < kTierItems[1]) return launch_frame_tier<1, TOP, ONE>(P, overlap, st);
+  if (items < tier_items(0, ONE)) return launch_frame_tier<0, TOP, ONE>(P, overlap, st);
+  if (items < tier_items(1, ONE)) return launch_frame_tier<1, TOP, ONE>(P, overlap, st);
   return launch_frame_tier<2, TOP, ONE>(P, overlap, st);
 }
 
