@@ -141,8 +141,11 @@ __global__ void __launch_bounds__(128, 2) k_umma_gemm(const UmmaArgs g, uint32_t
   const int m0 = blockIdx.y * 128, n0 = blockIdx.x * BN;
   using L = GemmSmem<BN>;
 
-  // a CTA that timed out raised the status word: the rest of the grid stops
-  if (*reinterpret_cast<volatile uint32_t*>(status) & J3DG_DEV_VISIT_CAP) return;
+  // A CTA that timed out raised the status word: the rest of the grid stops.
+  // One thread looks: another CTA may raise it meanwhile, and warps of two
+  // minds would leave the others without the TMEM address and the barriers.
+  if (__syncthreads_or(threadIdx.x == 0 && (*reinterpret_cast<volatile uint32_t*>(status) & J3DG_DEV_VISIT_CAP)))
+    return;
   if (warp == 0) {
     umma::tmem_alloc(umma::smem_u32(&taddr_s), BN);
     umma::tmem_relinquish();
