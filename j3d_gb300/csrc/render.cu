@@ -1077,7 +1077,7 @@ __global__ void __launch_bounds__(kTraceThreads, TOP ? J3DG_RAY_BLOCKS - 1 : J3D
 // single tail. Per-frame parameters live in device memory.
 // blocks per SM that keep registers at or under ~96 for a block of TPB threads
 template <int TPB, bool kThroughput>
-struct MinBlocks {  // the same warps per SM as k_frame
+struct MinBlocks {  // 24 warps an SM, 20 in the latency build
   static const int per128 = kThroughput ? J3DG_TRACE_MINBLOCKS : J3DG_LATENCY_MINBLOCKS;
   static const int value = TPB >= 256 ? per128 / 2 : (TPB >= 128 ? per128 : 2 * per128);
 };
@@ -1149,20 +1149,18 @@ __global__ void __launch_bounds__(TPB, (MinBlocks<TPB, kThroughput>::value))
     if (__all_sync(0xffffffffu, phase == 0 && exhausted)) break;
 #pragma unroll 1
     for (;;) {
-      {
-        const FrameParams& P = params[frame];
-        if (T.warp_step(phase == 1 || phase == 2, P.inst, P.n_inst, P.status, visits, tests, stack)) {
+      const FrameParams& P = params[frame];
+      if (T.warp_step(phase == 1 || phase == 2, P.inst, P.n_inst, P.status, visits, tests, stack)) {
 #if J3DG_DEFER_FINISH
-          phase += 2;
+        phase += 2;
 #else
-          if (phase == 1) {
-            phase = primary_finish(P, T, pix, w0, su, sv) ? 2 : 0;
-          } else {
-            shadow_finish(P, T, pix, w0, su, sv);
-            phase = 0;
-          }
-#endif
+        if (phase == 1) {
+          phase = primary_finish(P, T, pix, w0, su, sv) ? 2 : 0;
+        } else {
+          shadow_finish(P, T, pix, w0, su, sv);
+          phase = 0;
         }
+#endif
       }
       if (__all_sync(0xffffffffu, phase != 1 && phase != 2)) break;
       if (__popc(__ballot_sync(0xffffffffu, (phase == 0 && !exhausted) || phase >= 3)) >= J3DG_REFILL_AT) break;
