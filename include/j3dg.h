@@ -135,8 +135,10 @@ typedef struct j3dg_build_opts {
    2018) within them, collapsed by a cost-optimal programme: the fewest node
    visits per ray. J3DG_BUILD_LBVH splits at Morton prefixes instead (4-wide
    only): about half of the build time (9.8 vs 18.5 ms for 28M triangles),
-   about 19 % more node visits per ray. Both are driven by the device, sizes
-   read from its memory. The traversal results are the same for either tree. */
+   about 19 % more node visits per ray. Both read their sizes on the device;
+   the host looks at the tree at the end, and once before its nodes are made
+   where they may take more than 256 MB. The traversal results are the same
+   for either tree. */
 #define J3DG_BUILD_LBVH 0x1u
 /* BVH width (children per node) of the default builder: 4 unless one of
    these is set. The cost-optimal collapse of the binary tree is run for the

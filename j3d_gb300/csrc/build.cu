@@ -476,7 +476,6 @@ __device__ __forceinline__ float half_area(float4 lo, float4 hi) {
   float dx = hi.x - lo.x, dy = hi.y - lo.y, dz = hi.z - lo.z;
   return dx * dy + dy * dz + dz * dx;
 }
-__device__ __forceinline__ float half_area4(float4 lo, float4 hi) { return half_area(lo, hi); }
 
 // One binary node of the LBVH's 4-wide collapse: it becomes wide node
 // it.wide, whose slots are its children, the largest-area child opened until
@@ -656,9 +655,6 @@ static const size_t kCtlHead = offsetof(BuildCtl, root);
 // dec.x = the k of the node case (bit 7 set: the leaf case is cheaper);
 // dec.y, .z, .w for i = 2, 3, 4: 0 = as i - 1, else the k of the best split.
 
-#ifndef J3DG_SAH_COLLAPSE
-#define J3DG_SAH_COLLAPSE 1
-#endif
 #ifndef J3DG_SAH_CTRI
 #define J3DG_SAH_CTRI 0.5f  // cost of a triangle test relative to a node visit
 #endif
@@ -1106,14 +1102,14 @@ __global__ void __launch_bounds__(kPlaceThreads) k_place_jobs(
 // the segment's positions but the first: every position but position 0
 // numbers one node, without a counter.
 
-// segment size below which PLOC takes over (0: PLOC over the whole mesh).
-// Measured on the 28M-triangle torus frames (node visits per ray, ms per
-// 1080p frame, build ms): PLOC only 6.955 / 0.881 / 39; 4096: 6.402 / 0.862
-// / 67; 256: 6.256 / 0.855 / 76; 64: 6.200 / 0.851 / 87; 16: 6.193 / 0.852
-// / 112.
+// Segment size below which PLOC takes over. Measured on the 28M-triangle torus
+// frames (node visits per ray, ms per 1080p frame, ms of the build of that
+// time): PLOC only 6.955 / 0.881 / 39; 4096: 6.402 / 0.862 / 67; 256: 6.256 /
+// 0.855 / 76; 64: 6.200 / 0.851 / 87; 16: 6.193 / 0.852 / 112.
 #ifndef J3DG_SAH_TOP
 #define J3DG_SAH_TOP 64u
 #endif
+static_assert(J3DG_SAH_TOP > 0, "a segment has a triangle");
 static const int kTopBins = 16;
 static_assert(kTopBins <= 16, "bin codes keep 4 bits per axis");
 // per bin: count, box lo / hi xyz (ordered-float encoded). The children's
@@ -1950,7 +1946,6 @@ static const int kSmallWarps = kSmallThreads / 32;
 static const int kSmallPer = (J3DG_SMALL_TASK + kSmallThreads - 1) / kSmallThreads;  // positions per thread
 static const uint32_t kSmallBins = J3DG_SMALL_BINS;  // local tasks binned at once
 static const uint32_t kSmallTasks = kSmallTask / (J3DG_SAH_TOP + 1u) + 1u;  // tasks of one local level
-static const uint32_t kBinWords = 3 * kTopBins * kTopVals;
 static_assert(kSmallPer <= 32 && kSmallPer * kSmallWarps <= 64, "flag bits and list counts per thread");
 static_assert(kSmallTask <= 4096u && kSmallTasks < 255u && kSmallTasks <= kSmallThreads,
               "12-bit positions, 8-bit local tasks, one thread per task");
@@ -1960,7 +1955,7 @@ struct SmallTaskMem {   // while the levels run
   uint16_t ord[2][kSmallTask];
   uint16_t code[kSmallTask];
   uint8_t tk[2][kSmallTask];
-  uint32_t bins[kSmallBins * kBinWords];
+  uint32_t bins[kSmallBins * kTopBinWords];
 };
 template <int W>
 struct SmallClusterMem {  // while the segments are clustered
@@ -2023,7 +2018,7 @@ __device__ int small_levels(SmallMem<W>& s, uint32_t b0, uint32_t n, uint2* __re
     if (tid == 0) s.n_task[cur ^ 1] = 0;
     for (uint32_t base = 0; base < nlt; base += kSmallBins) {
       const uint32_t m = min(kSmallBins, nlt - base);
-      for (uint32_t k = tid; k < m * kBinWords; k += kSmallThreads) {
+      for (uint32_t k = tid; k < m * kTopBinWords; k += kSmallThreads) {
         const uint32_t v = k % kTopVals;
         s.t.bins[k] = v == 0 ? 0u : (v < 4 ? 0xffffffffu : 0u);
       }
@@ -2046,12 +2041,12 @@ __device__ int small_levels(SmallMem<W>& s, uint32_t b0, uint32_t n, uint2* __re
           const uint32_t cd = B.code(0.5f * (fx.x + fx.y), 0.5f * (fy.x + fy.y), 0.5f * (fz.x + fz.y),
                                      s.task[cur][base + t]);
           s.t.code[p] = (uint16_t)cd;
-          bin_update3(s.t.bins + t * kBinWords, cd, 1u, v);
+          bin_update3(s.t.bins + t * kTopBinWords, cd, 1u, v);
         }
       }
       __syncthreads();
       for (uint32_t t = warp; t < m; t += kSmallWarps)
-        warp_top_split(s.t.bins + t * kBinWords, s.task[cur][base + t], &s.split[base + t], tr);
+        warp_top_split(s.t.bins + t * kTopBinWords, s.task[cur][base + t], &s.split[base + t], tr);
       __syncthreads();
     }
     // the children's tasks
@@ -2139,7 +2134,7 @@ __device__ __forceinline__ float merged_area2(const float2 (&a)[3], const float2
                      make_float4(b[0].x, b[1].x, b[2].x, 0.f), make_float4(b[0].y, b[1].y, b[2].y, 0.f));
 }
 __device__ __forceinline__ float half_area2(const float2 (&a)[3]) {
-  return half_area4(make_float4(a[0].x, a[1].x, a[2].x, 0.f), make_float4(a[0].y, a[1].y, a[2].y, 0.f));
+  return half_area(make_float4(a[0].x, a[1].x, a[2].x, 0.f), make_float4(a[0].y, a[1].y, a[2].y, 0.f));
 }
 
 // PLOC over the block's m clusters (one list, neighbours within a segment
@@ -2365,7 +2360,7 @@ __device__ void climb(const Tree& tr, const BinNode* __restrict__ tbox, uint32_t
   auto covering = [&](uint32_t r, Covering<W>& c) {
     if (r & 0x80000000u) {
       const BinNode b = tbox[r & 0x7fffffffu];
-      c.triangle(half_area4(b.lo, b.hi));
+      c.triangle(half_area(b.lo, b.hi));
     } else {
 #pragma unroll
       for (int i = 1; i <= W; ++i) {
@@ -2383,7 +2378,7 @@ __device__ void climb(const Tree& tr, const BinNode* __restrict__ tbox, uint32_t
     NodeMeta M;
     covering(left_ref(lo), l);
     covering(right_ref(hi), r);
-    collapse_step<W>(l, r, half_area4(lo, hi), tr.meta[n].count, leaf_size, c, M);
+    collapse_step<W>(l, r, half_area(lo, hi), tr.meta[n].count, leaf_size, c, M);
 #pragma unroll
     for (int i = 1; i <= W; ++i) {
       tr.cost[(size_t)n * W + i - 1] = c.cost[i];
@@ -2542,7 +2537,7 @@ __global__ void __launch_bounds__(kSmallThreads, W == 8 ? J3DG_SMALL_BLOCKS - 1 
             l.wide[k] = s.wide16[k - 1][cb];
             r.wide[k] = s.wide16[k - 1][cm];
           }
-          collapse_step<W>(l, r, half_area4(tr.node[node].lo, tr.node[node].hi), (x.y & 0xffffu) - (x.x & 0xffffu), leaf_size,
+          collapse_step<W>(l, r, half_area(tr.node[node].lo, tr.node[node].hi), (x.y & 0xffffu) - (x.x & 0xffffu), leaf_size,
                            c, M);
 #pragma unroll
           for (int k = 1; k <= W; ++k) {
@@ -2595,23 +2590,18 @@ __global__ void k_slot_of(const float4* __restrict__ tris, uint32_t nt, uint32_t
   slot_of[id] = i;
 }
 
-// stream-ordered free of a scratch buffer as soon as it is dead (keeps the
-// build's peak device memory down); the pointer is cleared for the cleanup
-#define J3DG_DROP(p)             \
-  do {                           \
-    if (p) cudaFreeAsync(p, st); \
-    p = nullptr;                 \
-  } while (0)
-
 // ------------------------------------------------ device-driven build ----
 //
-// A build runs with no host round trip but at its end: kernels read their
-// sizes from BuildCtl and stride over them with fixed grids, so the launches
-// do not depend on the tree. The default builder's levels (SAH, placement) are
-// launched a few more of than a balanced tree has; the tree that needs more
-// gets them after the host has looked (j3dg_mesh_build), or from a conditional
-// while node in a captured build (a batch rebuilds its meshes ahead of its
-// frames; a body ends in a one-thread kernel that sets the loop's condition).
+// Kernels read their sizes from BuildCtl and stride over them with fixed grids,
+// so the launches do not depend on the tree, and the host looks at it once, at
+// the build's end (J3DG_BUILD_LBVH too); once before the placement as well where
+// the nodes are made in an array of their number (kStagedNodes), and once more
+// for every set of levels that a deep tree needs. The default builder's levels
+// (SAH, placement) are launched a few more of than a balanced tree has; the
+// tree that needs more gets them after the host has looked (j3dg_mesh_build),
+// or from a conditional while node in a captured build (a batch rebuilds its
+// meshes ahead of its frames; a body ends in a one-thread kernel that sets the
+// loop's condition).
 // A level past the last finds nothing and costs a launch (about 2 us), a round
 // of a loop 13-26 us between its levels, and making the graph of a single
 // build took longer than the radix sort that it ran beside. The LBVH's loops
@@ -3270,7 +3260,8 @@ static cudaError_t enqueue_build(BuildPlan& P, const float* dV, const uint32_t* 
 
 // One mesh's build: the prefix, then the tree on the same stream (LBVH: the
 // GPU sorts while the host captures and instantiates the tree's part), then
-// the tree's size from the device and an exactly sized copy of the nodes.
+// the tree's size from the device and a copy of the nodes of that size, unless
+// they were made where they stay.
 static int build_bvh_tree(j3dg_mesh* m, const float* dV, const uint32_t* dT, cudaStream_t st, uint32_t* d_status,
                           cudaEvent_t done, std::string& err) {
   BuildPlan P;
