@@ -295,11 +295,17 @@ static const int kFrameThreads = J3DG_FRAME_THREADS;
 //     and 203, 294 and 299).
 //   2: pixel state in shared memory, 28 warps at width 4, whose 72 registers
 //     hold the step of a single object without spills (28.09M triangles at
-//     1920x1080 with shadows, views in turn: 24 or 28 warps 455 and 424 us, a
-//     frame alone 863 both, one view again and again 714 and 721, the slowest
-//     pixels one after the other; 32 warps spill: 497 where 28 took 489)
-__host__ __device__ constexpr uint32_t tier_items(int tier, bool one) {  // the build's frames are below
-  return tier == 0 ? (one && J3DG_W == 8 ? 700000u : 400000u) : J3DG_THROUGHPUT_ITEMS;
+//     1920x1080 with shadows, views in turn: build 1 441 us, this one 428; one
+//     view again and again, the slowest pixels one after the other, 698 and
+//     732; 3840x2160 1323 and 1242; 32 warps spill: 497 where 28 took 489).
+//     For a frame that follows none on its canvas the other frame's tail is
+//     not there to be filled, and build 1 is faster up to some 3M items (alone,
+//     28.09M triangles 1920x1080 834 and 861, 2M 541 and 551, 24 objects 815 and
+//     827; 2560x1440 1019 and 1033, 703 and 705; 3000x1700 1229 and 1218, 862
+//     and 852).
+// the build's frames are below
+__host__ __device__ constexpr uint32_t tier_items(int tier, bool one, bool follows) {
+  return tier == 0 ? (one && J3DG_W == 8 ? 700000u : 400000u) : (follows ? J3DG_THROUGHPUT_ITEMS : 3000000u);
 }
 __host__ __device__ constexpr int tier_blocks(int tier) {  // blocks of kFrameThreads an SM
   return (tier == 0 ? J3DG_LATENCY_MINBLOCKS
@@ -1377,8 +1383,9 @@ static cudaError_t launch_frame_tier(const FrameParams& P, bool overlap, cudaStr
 template <bool TOP, bool ONE>
 static cudaError_t launch_frame(const FrameParams& P, bool overlap, cudaStream_t st) {
   const uint32_t items = primary_items(P);
-  if (items < tier_items(0, ONE)) return launch_frame_tier<0, TOP, ONE>(P, overlap, st);
-  if (items < tier_items(1, ONE)) return launch_frame_tier<1, TOP, ONE>(P, overlap, st);
+  const bool follows = P.wait_seq != 0u;
+  if (items < tier_items(0, ONE, follows)) return launch_frame_tier<0, TOP, ONE>(P, overlap, st);
+  if (items < tier_items(1, ONE, follows)) return launch_frame_tier<1, TOP, ONE>(P, overlap, st);
   return launch_frame_tier<2, TOP, ONE>(P, overlap, st);
 }
 
