@@ -302,7 +302,8 @@ static const int kFrameThreads = J3DG_FRAME_THREADS;
 //     not there to be filled, and build 1 is faster up to some 3M items (alone,
 //     28.09M triangles 1920x1080 834 and 861, 2M 541 and 551, 24 objects 815 and
 //     827; 2560x1440 1019 and 1033, 703 and 705; 3000x1700 1229 and 1218, 862
-//     and 852).
+//     and 852). A single object of some 100k triangles gains nothing (244 both,
+//     and 329 against 326 with points splatted after it).
 // the build's frames are below
 __host__ __device__ constexpr uint32_t tier_items(int tier, bool one, bool follows) {
   return tier == 0 ? (one && J3DG_W == 8 ? 700000u : 400000u) : (follows ? J3DG_THROUGHPUT_ITEMS : 3000000u);
@@ -1383,7 +1384,7 @@ static cudaError_t launch_frame_tier(const FrameParams& P, bool overlap, cudaStr
 template <bool TOP, bool ONE>
 static cudaError_t launch_frame(const FrameParams& P, bool overlap, cudaStream_t st) {
   const uint32_t items = primary_items(P);
-  const bool follows = P.wait_seq != 0u;
+  const bool follows = P.wait_seq != 0u || (ONE && P.one.nt < 400000u);
   if (items < tier_items(0, ONE, follows)) return launch_frame_tier<0, TOP, ONE>(P, overlap, st);
   if (items < tier_items(1, ONE, follows)) return launch_frame_tier<1, TOP, ONE>(P, overlap, st);
   return launch_frame_tier<2, TOP, ONE>(P, overlap, st);

@@ -1,6 +1,7 @@
 """Frames of one object on both sides of the sizes where the frame kernel's
 build changes (400,000 pixels, 700,000 at width 8, two million, or three for
-one that follows none on its canvas): its record comes by value there, the batch kernel reads the same scene from a table, and
+one of 400,000 triangles and more that follows none on its canvas): its record
+comes by value there, the batch kernel reads the same scene from a table, and
 the frames are equal byte for byte."""
 import numpy as np
 import pytest
@@ -13,9 +14,20 @@ from test_frame_overlap import _canvas, _same
 @pytest.mark.parametrize("w,h", [(3, 2), (632, 624), (640, 632), (832, 836), (840, 840), (1504, 1328), (1504, 1336), (2000, 1496),
                                  (2000, 1504)])
 def test_frames_equal_a_batch_of_one(gpu_ctx, width, w, h):
+    _compare(gpu_ctx, (300, 150), width, w, h)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width", [2, 4, 8])
+@pytest.mark.parametrize("w,h", [(640, 632), (1504, 1336), (2000, 1496), (2000, 1504)])
+def test_frames_of_a_larger_mesh(gpu_ctx, width, w, h):
+    _compare(gpu_ctx, (640, 320), width, w, h)
+
+
+def _compare(gpu_ctx, grid, width, w, h):
     from j3d_gb300 import Matcap, Mesh, Scene, render_batch, workloads as W
     sc = Scene()
-    sc.add_object(Mesh(gpu_ctx, *W.torus(300, 150), width=width), db_id=1)
+    sc.add_object(Mesh(gpu_ctx, *W.torus(*grid), width=width), db_id=1)
     sc.prepare_scene()
     sc.unzoom()
     mc = Matcap.make(gpu_ctx, 0)
