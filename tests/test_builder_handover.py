@@ -74,3 +74,23 @@ def test_rebuilds_of_all_sizes_in_one_graph(gpu_ctx, width, mixed):
     g.close()
     for cv, _, _ in frames:
         cv.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nt", [3, 40, 65, 481, 2500, 20000])
+@pytest.mark.parametrize("kind", ["infinite", "huge"])
+def test_boxes_without_an_area_are_refused(gpu_ctx, nt, kind):
+    """No pair of clusters has a smallest area: the build says so, places
+    nothing, and the next one is as ever."""
+    from j3d_gb300 import J3dgError, Mesh
+    V, T = _soup(nt, 0.02)
+    good = Mesh(gpu_ctx, V, T, 1, width=2).nodes()
+    W = V.copy()
+    if kind == "infinite":
+        W[1::3, 0] = np.inf
+    else:
+        W *= np.float32(3e38)
+    with pytest.raises(J3dgError, match="malformed tree"):
+        Mesh(gpu_ctx, W, T, 1, width=2)
+    assert np.array_equal(Mesh(gpu_ctx, V, T, 1, width=2).nodes().view(np.uint32), good.view(np.uint32))
+    assert gpu_ctx.device_status() == 0
